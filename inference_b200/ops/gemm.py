@@ -26,10 +26,15 @@ def gemm_workspace(device: torch.device, slot: int = 0) -> torch.Tensor:
 def gemm_bf16(a: torch.Tensor, w: torch.Tensor, *, bias: torch.Tensor | None = None,
               residual: torch.Tensor | None = None, act: str | None = None, out: torch.Tensor | None = None,
               out_dtype: torch.dtype = torch.bfloat16, mode: int = -1, block_n: int = 0, ctas: int = 0,
-              workspace: torch.Tensor | None = None, act_params: tuple[float, float] = (0.0, 0.0)) -> torch.Tensor:
+              workspace: torch.Tensor | None = None, act_params: tuple[float, float] = (0.0, 0.0),
+              static_weight: bool = True) -> torch.Tensor:
     """out[T, N] = act(a[T, K] @ w[N, K]^T + bias) + residual. a and w are bf16 with contiguous rows. act_params: "xielu" (a, b): a z^2 +
-    z / 2 above zero, b (e^z - 1 - z) + z / 2 below; "clamped_pairs" (limit, -)."""
+    z / 2 above zero, b (e^z - 1 - z) + z / 2 below; "clamped_pairs" (limit, -). static_weight=False: w was written by a kernel
+    of this stream that may still be running. The kernels for few tokens start to load a weight before they wait for the
+    kernels in front of them, so such a product takes the tokens-as-M kernel, which waits first."""
     require_cuda(a, w)
+    if not static_weight and mode < 0:
+        mode = 0
     assert a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
     assert a.dim() == 2 and w.dim() == 2 and a.shape[1] == w.shape[1]
     assert a.stride(1) == 1 and w.stride(1) == 1

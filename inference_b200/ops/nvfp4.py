@@ -403,7 +403,8 @@ class Nvfp4Linear:
                                            ptr(self.bias), ws.data_ptr(), ws.numel(), 0, stream_ptr()),
                   "swb_gemm_nvfp4")
         else:
-            out = gemm_bf16(x2, self.dense_bf16(), bias=self.bias)
+            static = self._dense is not None       # expanded by an earlier call
+            out = gemm_bf16(x2, self.dense_bf16(), bias=self.bias, static_weight=static)
         return out.reshape(*lead, t.rows)
 
     __call__ = forward

@@ -94,7 +94,7 @@ def linear_quant(a: torch.Tensor, qw: QuantWeight, bias: torch.Tensor | None = N
     T = a.shape[0]
     assert a.dtype == torch.bfloat16 and a.stride(1) == 1 and a.shape[1] == qw.k
     if T > MAX_FUSED_TOKENS:
-        return gemm_bf16(a, dequantize(qw), bias=bias, out=out)
+        return gemm_bf16(a, dequantize(qw), bias=bias, out=out, static_weight=False)
     if out is None:
         out = torch.empty((T, qw.n), dtype=torch.bfloat16, device=a.device)
     ws = gemm_workspace(a.device)

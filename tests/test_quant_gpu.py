@@ -57,6 +57,23 @@ def test_q4k_matvec_kernel_matches_reference_and_the_tensor_core_path(T, N, K):
     assert (out2.float().cpu() - ref2).abs().max().item() < 2e-2 * max(1.0, ref2.abs().max().item())
 
 
+@pytest.mark.parametrize("T", [65, 130, 256])
+def test_expanded_weights_are_complete_before_they_are_multiplied(T):
+    """Token counts above the fused kernel's expand the weight and multiply it right behind: the product must not start from
+    what the buffer held before. Two weights take turns in the same reused buffer."""
+    from inference_b200.ops import quant
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    N, K = 14336, 4096
+    qws = [quant.quantize_on_device(torch.randn(N, K, generator=g, device="cuda") * s, "Q4_K") for s in (0.05, 5.0)]
+    a = (torch.randn(T, K, generator=g, device="cuda") * 0.5).bfloat16()
+    wants = [a.float() @ quant.dequantize(q).float().t() for q in qws]
+    for _ in range(6):
+        outs = [quant.linear_quant(a, q) for q in qws]
+        for out, want in zip(outs, wants):         # one rounding to bf16 of fp32 sums
+            assert (out.float() - want).abs().max().item() < 2 ** -8 * want.abs().max().item()
+
+
 def test_large_token_count_uses_dense_path():
     from inference_b200.ops import quant
 
