@@ -83,6 +83,8 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
                           c_int, c_int, c_int, c_void_p, c_size_t, c_int, c_int, c_int, c_void_p])
     sig("swb_gemm_bf16_act", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                               c_int, c_int, c_float, c_float, c_int, c_void_p, c_size_t, c_int, c_int, c_int, c_void_p])
+    sig("swb_gemm_bf16_gated", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                                c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p])
     sig("swb_rmsnorm_prefetch", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float,
                                  c_float, c_void_p, c_ll, c_void_p])
     sig("swb_rmsnorm", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_float,

@@ -53,6 +53,35 @@ int swb_gemm_bf16(const void* A, int lda, const void* W, int ldw, void* D, int l
                            workspace_bytes, force_mode, force_block_n, force_ctas, stream);
 }
 
+// D = act(A W^T + bias) * gate + residual on the two-SM kernel; row r takes the gate row r / rows_per_gate (N factors, row stride
+// ld_gate). bf16 output; 16-byte aligned rows. A residual may be D itself.
+int swb_gemm_bf16_gated(const void* A, int lda, const void* W, int ldw, void* D, int ldd, int T, int N, int K, const void* bias,
+                        const void* residual, int ld_res, const void* gate, int ld_gate, int rows_per_gate, int act, void* workspace,
+                        size_t workspace_bytes, void* stream) {
+  if (!gate) return -3;
+  swb::GemmArgs a{};
+  a.A = A;
+  a.lda = lda;
+  a.W = W;
+  a.ldw = ldw;
+  a.D = D;
+  a.ldd = ldd;
+  a.T = T;
+  a.N = N;
+  a.K = K;
+  a.bias = bias;
+  a.residual = residual;
+  a.ld_res = ld_res;
+  a.gate = gate;
+  a.ld_gate = ld_gate;
+  a.rows_per_gate = rows_per_gate;
+  a.act = act;
+  a.workspace = workspace;
+  a.workspace_bytes = workspace_bytes;
+  a.force_mode = -1;
+  return swb::gemm_bf16_launch(a, reinterpret_cast<cudaStream_t>(stream));
+}
+
 // 3x3 convolution, stride 1, zero padding 1, over an NHWC bf16 activation x [n, h, w, c] as an implicit GEMM on the
 // tcgen05 kernel: no patch matrix is written; each reduction block is one window tap over one 64-channel slab, fetched
 // by a 4-D TMA box at the tile's pixel origin shifted by the tap (zero fill outside the image is the padding).

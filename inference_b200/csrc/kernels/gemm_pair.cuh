@@ -1,0 +1,35 @@
+// Parameter block of the two-SM GEMM (kernel in gemm_pair_tcgen05.cu).
+#pragma once
+#include "gemm_tcgen05.cuh"
+
+namespace swb {
+
+struct PairParams {
+  int M, N;
+  int tiles_m, tiles_n;               // tiles of 256 rows x BN columns (grouped: tiles_m bounds the list)
+  int kblocks, kblocks_per_split, splits;
+  void* out;
+  int ldd, out_fp32;
+  const __nv_bfloat16* bias;
+  const __nv_bfloat16* residual;      // D = act(acc + bias) * gate + residual
+  int ld_res;
+  const __nv_bfloat16* gate;          // one row of N factors for each rows_per_gate rows
+  int ld_gate, rows_per_gate;
+  int act;
+  float act_a, act_b;
+  float* workspace;                   // [tile][CTA of the pair][split][BN][128] fp32
+  int* counters;                      // [tile][CTA of the pair][epilogue warp], zero between launches
+  const int4* group_tiles;            // grouped rows: (first row, rows of the group from there on, group, -)
+  const int* group_count;             // entries of the list, on the device
+  // 3x3 convolution (conv_c > 0): a CTA's 128 rows are a box of 2^box_w_log x 2^box_h_log pixels, boxes run row by row
+  int conv_n, conv_h, conv_w, conv_c;
+  int box_w_log, box_h_log, boxes_x, boxes_y;
+};
+
+bool gemm_pair_accepts(const GemmArgs& a);
+// Tile width and number of k-splits for a plain product.
+void gemm_pair_plan(int T, int N, int K, size_t workspace_bytes, int* block_n, int* splits);
+// block_n, splits: 0 = by the plan.
+int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t stream);
+
+}  // namespace swb

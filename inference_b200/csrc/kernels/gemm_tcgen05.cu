@@ -12,6 +12,7 @@
 //     the last-arriving CTA of a tile reduces the fp32 partials in a fixed order (deterministic).
 // Warp roles: warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2..5 = epilogue.
 #include "common.cuh"
+#include "gemm_pair.cuh"
 #include "gemm_tcgen05.cuh"
 
 #include <cudaTypedefs.h>
@@ -778,6 +779,15 @@ int gemm_bf16_launch(const GemmArgs& a, cudaStream_t stream) {
   if ((a.K % 8) != 0 || (a.lda % 8) != 0 || (a.ldw % 8) != 0) return -3;
   if ((reinterpret_cast<uintptr_t>(a.A) & 15) || (reinterpret_cast<uintptr_t>(a.W) & 15)) return -3;
   const int sms = device_sm_count();
+  if (a.gate || a.group_tiles || a.force_mode == 3)
+    return gemm_pair_launch(a, a.force_block_n, a.force_mode == 3 ? a.force_ctas : 0, stream);
+  if (a.force_mode < 0 && a.force_ctas >= 0 && a.force_block_n == 0 && a.T > 64 && a.N >= 128 && gemm_pair_accepts(a))
+    return gemm_pair_launch(a, 0, 0, stream);
+  if (a.force_mode == -2) {
+    GemmArgs b = a;
+    b.force_mode = 0;
+    return gemm_bf16_launch(b, stream);
+  }
 
   int swapped = a.force_mode;
   if (a.scatter) {

@@ -125,7 +125,8 @@ struct GemmArgs {
   int out_fp32;
   void* workspace;
   size_t workspace_bytes;
-  int force_mode;     // -1 auto, 0 tokens-as-M, 1 swapped (weights-as-M), 2 cluster split-K (T <= 64; force_ctas = cluster size)
+  int force_mode;     // -1 auto, 0 tokens-as-M, 1 swapped (weights-as-M), 2 cluster split-K (T <= 64; force_ctas = cluster size),
+                      // 3 pairs of SMs (force_ctas = k-splits), -2 auto without the kernels that load W before the launch dependency
   int force_block_n;  // 0 auto
   int force_ctas;     // 0 auto; > 0 stream-K over that many CTAs; < 0 whole tiles only
   const GemmScatter* scatter = nullptr;
@@ -139,6 +140,12 @@ struct GemmArgs {
   const GemmPeerReduce* peer = nullptr;  // see GemmPeerReduce (decode cluster kernel only)
   int conv_n = 0, conv_h = 0, conv_w = 0, conv_c = 0;   // see GemmParams: A = NHWC activation, T = n h w, K = 9 c
   float act_a = 0.f, act_b = 0.f;
+  // two-SM kernel only (gemm_pair.cuh)
+  const void* gate = nullptr;            // D = act(acc + bias) * gate[row / rows_per_gate] + residual
+  int ld_gate = 0, rows_per_gate = 0;
+  const void* group_tiles = nullptr;     // device int4 list of row tiles, its length in group_count, at most group_max_tiles
+  const int* group_count = nullptr;
+  int group_max_tiles = 0;
 };
 
 int gemm_bf16_launch(const GemmArgs& a, cudaStream_t stream);

@@ -391,15 +391,14 @@ class FluxDiTGpu:
             new = {}
             for s, x, lo, n in (("txt", x_txt, 0, St), ("img", x_img, St, Si)):
                 a = attn[:, lo:lo + n]
-                proj = torch.empty((B, n, H), dtype=torch.bfloat16, device=dev)
+                y = torch.empty((B, n, H), dtype=torch.bfloat16, device=dev)
                 for b in range(B):
-                    self._lin(a[b], f"double_blocks.{i}.{s}_attn.proj", out=proj[b])
-                x = ops.gated_residual(x, proj, mods[s][2], rows_per_batch=n)
-                hm = ops.layernorm_mod(x, scale=mods[s][4], shift=mods[s][3], rows_per_batch=n)
+                    self._lin(a[b], f"double_blocks.{i}.{s}_attn.proj", residual=x[b], gate=mods[s][2][b:b + 1], out=y[b])
+                hm = ops.layernorm_mod(y, scale=mods[s][4], shift=mods[s][3], rows_per_batch=n)
                 h1 = self._lin(hm.view(B * n, H), f"double_blocks.{i}.{s}_mlp.0", act="gelu_tanh")
-                h2 = self._lin(h1, f"double_blocks.{i}.{s}_mlp.2").view(B, n, H)
-                new[s] = ops.gated_residual(x, h2, mods[s][5], rows_per_batch=n)
-                self.launches += 3
+                new[s] = self._lin(h1, f"double_blocks.{i}.{s}_mlp.2", residual=y.view(B * n, H), gate=mods[s][5],
+                                   rows_per_gate=n).view(B, n, H)
+                self.launches += 1
             x_img, x_txt = new["img"], new["txt"]
             r = inj.after_double(i, x_img) if inj is not None else None
             if r is not None:
@@ -416,9 +415,8 @@ class FluxDiTGpu:
             self._lin(xm, p + ".linear1_mlp", act="gelu_tanh", out=buf2.view(B * S, H + M)[:, H:])
             self._cur_norm = (self.w[p + ".norm.query_norm.scale"], self.w[p + ".norm.key_norm.scale"])
             attention(qkv, buf2[:, :, :H])
-            out = self._lin(buf2.view(B * S, H + M), p + ".linear2").view(B, S, H)
-            x = ops.gated_residual(x, out, g, rows_per_batch=S)
-            self.launches += 2
+            x = self._lin(buf2.view(B * S, H + M), p + ".linear2", residual=x.view(B * S, H), gate=g, rows_per_gate=S).view(B, S, H)
+            self.launches += 1
             r = inj.after_single(i, x[:, St:]) if inj is not None else None
             if r is not None:
                 x[:, St:] += r.to(x.dtype)

@@ -399,8 +399,8 @@ class LlamaGpu:
             rope_cos, rope_sin = inp.rope_table
             rope_pos = torch.arange(T, dtype=torch.int32, device=self.device)
         taps = inp.deepstack[1] if inp.deepstack is not None else []
-        # decode-sized steps of a dense model: the norms are folded into a chain of GEMM epilogues
-        chain = (self._chain_ok and inp.decode and T <= 64 and self.quant_format is None and
+        # decode-sized steps of a dense model (short prompts too): the norms are folded into a chain of GEMM epilogues
+        chain = (self._chain_ok and (inp.decode or not self.comm.is_parallel) and T <= 64 and self.quant_format is None and
                  os.environ.get("SWB_NORM_CHAIN", "1") != "0")
         chain = chain and not taps
         fc = self.comm.fused if self.comm.is_parallel else None
@@ -475,8 +475,13 @@ class LlamaGpu:
                 continue
             fused = self.comm.fused if (self.comm.fused is not None and T <= self.comm.fused.max_tokens and
                                         L.post_attn_ln is None and li >= len(taps)) else None
+            # above the decode kernels' sizes the products join the residual stream in their epilogue; a norm then reads it once
+            join = T > 64 and not self.comm.is_parallel
             if fused is not None:
                 h = fused.gemm_allreduce_rmsnorm(attn, L.o, res, L.ln2, eps, woff)
+            elif join and L.post_attn_ln is None:
+                ops.linear_any(attn.reshape(T, -1), L.o, residual=res, out=res)
+                h = ops.rmsnorm(res, L.ln2, eps, w_offset=woff)
             else:
                 branch = ops.linear_any(attn, L.o)
                 branch = self.comm.all_reduce(branch)
@@ -498,6 +503,9 @@ class LlamaGpu:
                 nxt = self.layers[li + 1].ln1 if li + 1 < len(self.layers) else self.norm
                 pending_h = fused.gemm_allreduce_rmsnorm(act, L.down, res, nxt, eps, woff)
                 branch = None
+            elif join and L.post_mlp_ln is None and li >= len(taps):
+                pending_h = branch = None
+                ops.linear_any(act, L.down, residual=res, out=res)
             else:
                 pending_h = None
                 branch = ops.linear_any(act, L.down)
@@ -528,7 +536,7 @@ class LlamaGpu:
         decode-sized step applies the gated activation in the projection's epilogue."""
         if isinstance(gate_up, torch.Tensor) and h.device.type == "cuda":
             y = ops.linear_gated(h, gate_up, self.cfg.mlp_activation)
-            self._mlp_in_launches = 1 if y.shape[0] <= 64 and ops.gated_fused(h.shape[0], *gate_up.shape) else 2
+            self._mlp_in_launches = 1 if ops.gated_epilogue(h, gate_up) else 2
             return y
         self._mlp_in_launches = 2
         return ops.gated_act_mul(ops.linear_any(h, gate_up), self.cfg.mlp_activation, paired=True)

@@ -27,14 +27,15 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, *, bias: torch.Tensor | None = N
               residual: torch.Tensor | None = None, act: str | None = None, out: torch.Tensor | None = None,
               out_dtype: torch.dtype = torch.bfloat16, mode: int = -1, block_n: int = 0, ctas: int = 0,
               workspace: torch.Tensor | None = None, act_params: tuple[float, float] = (0.0, 0.0),
-              static_weight: bool = True) -> torch.Tensor:
+              static_weight: bool = True, gate: torch.Tensor | None = None, rows_per_gate: int = 0) -> torch.Tensor:
     """out[T, N] = act(a[T, K] @ w[N, K]^T + bias) + residual. a and w are bf16 with contiguous rows. act_params: "xielu" (a, b): a z^2 +
     z / 2 above zero, b (e^z - 1 - z) + z / 2 below; "clamped_pairs" (limit, -). static_weight=False: w was written by a kernel
     of this stream that may still be running. The kernels for few tokens start to load a weight before they wait for the
-    kernels in front of them, so such a product takes the tokens-as-M kernel, which waits first."""
+    kernels in front of them, so such a product takes one that waits first.
+    gate bf16 [G, N] (rows may be strided): the product is scaled by gate[row // rows_per_gate] before the residual is added."""
     require_cuda(a, w)
     if not static_weight and mode < 0:
-        mode = 0
+        mode = -2
     assert a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
     assert a.dim() == 2 and w.dim() == 2 and a.shape[1] == w.shape[1]
     assert a.stride(1) == 1 and w.stride(1) == 1
@@ -50,6 +51,16 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, *, bias: torch.Tensor | None = N
         assert bias.dtype == torch.bfloat16 and bias.numel() == N and bias.is_contiguous()
     if workspace is None:
         workspace = gemm_workspace(a.device)
+    if gate is not None:
+        rows = rows_per_gate or T
+        assert gate.dtype == torch.bfloat16 and gate.dim() == 2 and gate.shape[1] == N and gate.stride(1) == 1
+        assert rows * gate.shape[0] >= T and mode < 0 and block_n == 0 and ctas == 0
+        rc = kernels().swb_gemm_bf16_gated(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), T, N, K,
+                                           ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0,
+                                           gate.data_ptr(), gate.stride(0), rows, ACT[act], workspace.data_ptr(), workspace.numel(),
+                                           stream_ptr())
+        check(rc, "swb_gemm_bf16_gated")
+        return out
     rc = kernels().swb_gemm_bf16_act(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0),
                                      T, N, K, ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0,
                                      ACT[act], *act_params, 1 if out.dtype == torch.float32 else 0, workspace.data_ptr(),
@@ -125,19 +136,30 @@ def gated_fused(T: int, N: int, K: int) -> bool:
     return bool(kernels().swb_gemm_gated_supported(T, N, K))
 
 
+def gated_epilogue(x: torch.Tensor, w_pairs: torch.Tensor, out: torch.Tensor | None = None) -> bool:
+    """True when linear_gated of x [T, K] is one launch. Above the decode kernel's 64 tokens the two-SM kernel writes whole
+    16-byte pieces of the half-wide output (8000 tokens of an 8B decoder's layer: 138 us less than the separate pass)."""
+    T, K = x.shape
+    N = w_pairs.shape[0]
+    if gated_fused(T, N, K):
+        return True
+    rows_ok = out is None or (out.stride(-2) % 8 == 0 and out.data_ptr() % 16 == 0)
+    return T > 64 and N >= 128 and N % 16 == 0 and rows_ok
+
+
 def linear_gated(x: torch.Tensor, w_pairs: torch.Tensor, act: str = "silu", out: torch.Tensor | None = None) -> torch.Tensor:
     """act(x W_gate^T) * (x W_up^T) for a gate-up weight whose rows are interleaved (gate_0, up_0, gate_1, ...).
 
-    Decode-sized token counts apply the gated activation in the GEMM's epilogue (the reference runs the projection,
-    a split and two elementwise kernels: candle-llm models/llama.rs:1386-1391); larger ones run the GEMM and the
-    paired activation kernel."""
+    The gated activation is applied in the GEMM's epilogue (the reference runs the projection, a split and two elementwise
+    kernels: candle-llm models/llama.rs:1386-1391); shapes that neither the decode kernel nor the two-SM kernel takes run the
+    GEMM and the paired activation kernel."""
     from .llm import gated_act_mul
 
     x2 = x.reshape(-1, x.shape[-1])
     T, K = x2.shape
     N = w_pairs.shape[0]
     gelu = act in ("gelu", "gelu_tanh")
-    if kernels().swb_gemm_gated_supported(T, N, K):
+    if gated_epilogue(x2, w_pairs, out):
         y = gemm_bf16(x2, w_pairs, act="geglu_pairs" if gelu else "swiglu_pairs", out=out)
     else:
         y = gated_act_mul(gemm_bf16(x2, w_pairs), act, paired=True, out=out)

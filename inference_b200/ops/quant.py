@@ -88,13 +88,14 @@ def dequantize(qw: QuantWeight) -> torch.Tensor:
 
 
 def linear_quant(a: torch.Tensor, qw: QuantWeight, bias: torch.Tensor | None = None, out: torch.Tensor | None = None,
-                 splits: int = 0) -> torch.Tensor:
-    """a [T, K] bf16 -> [T, N] bf16."""
+                 splits: int = 0, residual: torch.Tensor | None = None) -> torch.Tensor:
+    """a [T, K] bf16 -> [T, N] bf16. residual [T, N]: added to the product (more than MAX_FUSED_TOKENS tokens only)."""
     require_cuda(a, qw.packed)
     T = a.shape[0]
     assert a.dtype == torch.bfloat16 and a.stride(1) == 1 and a.shape[1] == qw.k
     if T > MAX_FUSED_TOKENS:
-        return gemm_bf16(a, dequantize(qw), bias=bias, out=out, static_weight=False)
+        return gemm_bf16(a, dequantize(qw), bias=bias, out=out, residual=residual, static_weight=False)
+    assert residual is None
     if out is None:
         out = torch.empty((T, qw.n), dtype=torch.bfloat16, device=a.device)
     ws = gemm_workspace(a.device)
@@ -109,8 +110,8 @@ def linear_any(a: torch.Tensor, w, bias: torch.Tensor | None = None, out: torch.
                ) -> torch.Tensor:
     """a @ w^T for a dense bf16 weight or a QuantWeight (the projections of a model may be either)."""
     if isinstance(w, QuantWeight):
-        assert not kw or set(kw) <= {"out_dtype"} and kw.get("out_dtype") in (None, torch.bfloat16)
-        return linear_quant(a, w, bias=bias, out=out)
+        assert not kw or set(kw) <= {"out_dtype", "residual"} and kw.get("out_dtype") in (None, torch.bfloat16)
+        return linear_quant(a, w, bias=bias, out=out, residual=kw.get("residual"))
     return gemm_bf16(a, w, bias=bias, out=out, **kw)
 
 

@@ -137,3 +137,39 @@ def test_gated_projection_pairs(T, F, K, act):
     fn = torch.nn.functional.silu if act == "silu" else (lambda t: torch.nn.functional.gelu(t, approximate="tanh"))
     torch.testing.assert_close(y.float(), fn(gate) * up, rtol=3e-2, atol=3e-2)
     assert ops.gated_fused(T, 2 * F, K) == (T <= 64)
+
+
+@pytest.mark.parametrize("block_n,splits", [(0, 0), (256, 1), (192, 2), (128, 1), (128, 3), (64, 2)])
+@pytest.mark.parametrize("T,N,K", [(65, 128, 64), (255, 136, 584), (257, 520, 1096), (1000, 776, 2048)])
+def test_pairs_of_sms(T, N, K, block_n, splits):
+    """The two-SM kernel at the edges of its 256-row tiles, with columns and reduction blocks left over, every tile width and
+    k-splits: bias, activation and residual, gates per group of rows, and gated pairs. One rounding to bf16 of an fp32 sum: at most half of the
+    last of 8 bits, 2^-8 of the value; the sum itself is off by less than 1e-4 (terms of size 1, fast exponentials)."""
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    a = torch.randn(T, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    b = torch.randn(N, device="cuda", generator=g).bfloat16()
+    r = torch.randn(T, N, device="cuda", generator=g).bfloat16()
+
+    def close(y, want):
+        ops.check_status()
+        assert ((y.float() - want).abs() <= 2 ** -8 * want.abs() + 1e-4).all()
+
+    kw = dict(mode=3, block_n=block_n, ctas=splits) if block_n else {}
+    z = a.float() @ w.float().t()
+    y = ops.gemm_bf16(a, w, bias=b, residual=r, act="silu", **kw)
+    close(y, torch.nn.functional.silu(z + b.float()) + r.float())
+    assert torch.equal(y, ops.gemm_bf16(a, w, bias=b, residual=r, act="silu", **kw))       # split order, not arrival order
+    out = r.clone()
+    ops.gemm_bf16(a, w, residual=out, out=out, **kw)
+    close(out, z + r.float())
+    torch.testing.assert_close(ops.gemm_bf16(a, w, out_dtype=torch.float32, **kw), z, rtol=1e-5, atol=1e-5)
+    if N % 16 == 0:
+        close(ops.gemm_bf16(a, w, act="swiglu_pairs", **kw), torch.nn.functional.silu(z[:, 0::2]) * z[:, 1::2])
+    if not block_n:
+        gate = torch.randn(2, 2 * N, device="cuda", generator=g).bfloat16()[:, N:]
+        rows = (T + 1) // 2
+        y = ops.gemm_bf16(a, w, bias=b, residual=r, gate=gate, rows_per_gate=rows)
+        close(y, (z + b.float()) * gate.float()[torch.arange(T, device="cuda") // rows] + r.float())
