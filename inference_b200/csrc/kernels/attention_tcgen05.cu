@@ -3,12 +3,13 @@
 // One CTA owns 256 query rows of one head (two 128-row tiles, "q0" and "q1") and walks the keys in tiles of 128.
 //   warp 8 (one lane)   TMA producer: Q once, then K and V tiles through two 2-stage rings (4-D tensor maps over
 //                       [d, head, token, batch], 64-column boxes, 128-byte swizzle).
-//   warp 9 (one lane)   tcgen05.mma issuer. S_q = Q_q K^T accumulates into TMEM; O_q += P_q V reads P from TMEM
+//   warp 9              tcgen05.mma issuer. S_q = Q_q K^T accumulates into TMEM; O_q += P_q V reads P from TMEM
 //                       (P overwrites the first half of S in place as packed bf16) and V from shared memory as an
 //                       MN-major operand, so V needs no transpose. Issue order
 //                           S0(0) S1(0) | PV0(j) S0(j+1) PV1(j) S1(j+1) ...
 //                       keeps the tensor pipe busy with one tile's MMAs while the other tile is in softmax.
-//   warps 0-3 / 4-7     softmax warpgroups for q0 / q1: thread = row. tcgen05.ld the S row, running max with lazy
+//   warps 0-3 / 4-7     softmax warpgroups for q0 / q1: thread = row (plain problems: 16 warps, two threads per row, and the other
+//                       roles are warps 16 and 17). tcgen05.ld the S row, running max with lazy
 //                       rescale (O is only rescaled when the max grew by more than 2^8), exp2, tcgen05.st of P.
 // TMEM map (512 columns): [0,128) S0/P0, [128,256) O0, [256,384) S1/P1, [384,512) O1.
 // It replaces the mma.sync kernel for the FLUX joint attention (reference: candle-gen-flux/src/ip_dit.rs:64-85 runs
@@ -32,7 +33,6 @@ namespace {
 constexpr int BM = 128;          // query rows per tile (two tiles per CTA)
 constexpr int BN = 128;          // keys per tile
 constexpr int MAX_STAGES = 2;
-constexpr int THREADS = 320;
 constexpr uint32_t ATOM_BYTES = BM * 64 * 2;       // 16 KB: 128 rows of one 64-column swizzle atom
 // Tile widths of q / k (QK) and of v (VD). 128 is two swizzle atoms per tile, 64 one atom (half the shared memory and half the
 // MMA work of the padded path); q and k of latent attention take up to three, which leaves room for one V stage.
@@ -47,6 +47,7 @@ struct FaCfg {
   static constexpr uint32_t SMEM_V = SMEM_K + K_STAGES * TILE_BYTES;
   static constexpr uint32_t SMEM_BAR = SMEM_V + V_STAGES * V_TILE_BYTES;
   static constexpr size_t SMEM_BYTES = SMEM_BAR + 256 + 1024 /*alignment slack*/;
+  static constexpr size_t EXCHANGE_BYTES = 2 * 2 * 2 * BM * 4;            // softmax_halves: [tile parity][query tile][half][row] behind the barriers
   static constexpr int ROW_BYTES = VD * 2;                                // one output row of one head
   static constexpr int CHUNKS = ROW_BYTES / 16;                           // 16-byte chunks per row
 };
@@ -153,6 +154,13 @@ __device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t* r) {
       "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
+__device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const float* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "f"(v[0]), "f"(v[1]),
+      "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]),
+      "f"(v[14]), "f"(v[15])
+      : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ float ex2(float x) {
   float y;
@@ -179,11 +187,208 @@ struct Barriers {
   uint64_t k_full[MAX_STAGES], k_empty[MAX_STAGES];
   uint64_t v_full[MAX_STAGES], v_empty[MAX_STAGES];
   uint64_t s_full[2];   // MMA -> softmax q: S_q of the current key tile is complete
-  uint64_t p_full[2];   // softmax q -> MMA: P_q is in TMEM (128 arrivals)
+  uint64_t p_full[2];   // softmax q -> MMA: P_q is in TMEM
   uint64_t o_final;     // every MMA of the CTA has completed
   uint32_t tmem_base;
   int abort;
 };
+
+// Softmax with two threads per query row (plain problems: full or causal masks, packed or paged). Warp = (query tile q, half of the
+// keys, 32 rows): a thread holds 64 scores, so 16 warps fit and each scheduler has four of them whose loads, maxima,
+// exponentials and stores overlap; with 128 scores a thread eight warps left the special-function unit idle half of the time. The halves of
+// a row exchange their maximum through shared memory once per tile; that barrier also orders the stores of P over S behind both
+// halves' loads. Multiply-adds and sums run on two lanes at a time.
+// 4608 tokens x 24 heads: 274 us with a thread per row, 244 with two, 235 (1.11 PFLOP/s) with an eighth of the exponentials' pairs on the
+// multiply-add pipes (259 with a quarter, 235 with a sixteenth); eight causal prompts of 1100 x 32 heads 205 -> 165 us.
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// 2^x of two numbers at once on the multiply-add pipes: x = n + f, |f| <= 1/2, a polynomial in f fitted to 2^f with equal relative
+// ripples (8e-8, evaluated in fp32 within 2.2e-7: as exact as the special-function unit's) times 2^n. x is kept above -126, so what
+// should be zero comes out as 2^-126; what is not a number stays so.
+constexpr float EXP_0 = 1.00000012f, EXP_1 = 0.693146944f, EXP_2 = 0.240221202f, EXP_3 = 0.0555071309f, EXP_4 = 0.00967554096f, EXP_5 = 0.00132764713f;
+__device__ __forceinline__ unsigned long long ex2_fma2(unsigned long long x) {
+  float a, b;
+  unpack2(x, a, b);
+  asm("max.NaN.f32 %0, %0, 0fC2FC0000;" : "+f"(a));
+  asm("max.NaN.f32 %0, %0, 0fC2FC0000;" : "+f"(b));
+  x = pack2(a, b);
+  const unsigned long long magic = pack2(12582912.f, 12582912.f), minus = pack2(-12582912.f, -12582912.f), neg = pack2(-1.f, -1.f);
+  const unsigned long long t = add2(x, magic), f = fma2(add2(t, minus), neg, x);
+  unsigned long long r = fma2(pack2(EXP_5, EXP_5), f, pack2(EXP_4, EXP_4));
+  r = fma2(r, f, pack2(EXP_3, EXP_3));
+  r = fma2(r, f, pack2(EXP_2, EXP_2));
+  r = fma2(r, f, pack2(EXP_1, EXP_1));
+  r = fma2(r, f, pack2(EXP_0, EXP_0));
+  float t0, t1;
+  unpack2(t, t0, t1);
+  const unsigned long long power = pack2(__int_as_float((__float_as_int(t0) << 23) + 0x3f800000), __int_as_float((__float_as_int(t1) << 23) + 0x3f800000));
+  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(r) : "l"(power));
+  return r;
+}
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
+constexpr int FMA_EVERY = 8;   // one pair of exponentials of every FMA_EVERY keys leaves the special-function unit
+
+template <typename C>
+__device__ __forceinline__ void softmax_halves(const FaParams& p, Barriers* bars, uint8_t* smem, uint32_t tmem, int q_base, int q_len, int kv_len,
+                                               int coff, int n_tiles, int tok0, int batch, int head) {
+  constexpr int VD = C::ROW_BYTES / 2, KEYS = BN / 2, OUT = VD / 2;         // scores and output columns of a thread
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int q = warp >> 3, half = (warp >> 2) & 1, w4 = warp & 3;
+  const int my_tiles = (q < p.tiles) ? n_tiles : 0;
+  const uint32_t lane_base = (uint32_t)(w4 * 32) << 16;
+  const uint32_t t_s = tmem + lane_base + (q ? COL_S1 : COL_S0);
+  const uint32_t t_o = tmem + lane_base + (q ? COL_O1 : COL_O0) + half * OUT;
+  float* exchange = reinterpret_cast<float*>(smem + C::SMEM_BAR + 256) + (q * 2) * BM + w4 * 32 + lane;
+  const int pair = 1 + q * 4 + w4;
+  const int row = q_base + q * BM + w4 * 32 + lane;
+  const float scale_log2 = p.scale_log2;
+  const int last_key = p.causal ? min(kv_len - 1, row + coff) : kv_len - 1;
+  const float STOP = __int_as_float(0x7fffffff);                            // handed over instead of a maximum when a wait ran out
+  float m_used = -INFINITY, l = 0.f;
+  bool ok = true;
+  for (int j = 0; j < my_tiles; ++j) {
+    ok = mbar_wait(&bars->s_full[q], j & 1, &bars->abort, 30 + q);
+    ok = __all_sync(0xffffffffu, ok);
+    uint32_t s[KEYS];
+    float mx = STOP;
+    if (ok) {
+      tc_fence_after_sync();
+      tmem_ld_x32(t_s + half * KEYS, s);
+      tmem_ld_x32(t_s + half * KEYS + 32, s + 32);
+      tmem_ld_wait();
+      const int key0 = j * BN + half * KEYS;
+      if (key0 + KEYS > kv_len || (p.causal && key0 + KEYS > q_base + q * BM + coff)) {
+#pragma unroll
+        for (int i = 0; i < KEYS; ++i)
+          if (key0 + i > last_key) s[i] = __float_as_uint(-INFINITY);
+      }
+      float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
+#pragma unroll
+      for (int i = 0; i < KEYS; i += 4) {
+        m0 = fmaxf(m0, __uint_as_float(s[i]));
+        m1 = fmaxf(m1, __uint_as_float(s[i + 1]));
+        m2 = fmaxf(m2, __uint_as_float(s[i + 2]));
+        m3 = fmaxf(m3, __uint_as_float(s[i + 3]));
+      }
+      mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+    }
+    float* slot = exchange + (j & 1) * (4 * BM);
+    slot[half * BM] = mx;
+    pair_sync(pair);
+    const float other = slot[(half ^ 1) * BM];
+    ok = ok && __all_sync(0xffffffffu, __float_as_int(other) != 0x7fffffff);
+    if (!ok) break;                                                         // both halves leave at the same tile
+    const float m_new = fmaxf(fmaxf(mx, other), m_used);
+    const bool grow = (m_new - m_used) * scale_log2 > RESCALE_THRESHOLD;    // true on the first tile (m_used = -inf)
+    if (__any_sync(0xffffffffu, grow)) {
+      const float f = grow ? ex2((m_used - m_new) * scale_log2) : 1.f;      // -inf -> 0 on the first tile
+      if (grow) {
+        l *= f;
+        m_used = m_new;
+      }
+      if (j > 0) {   // O holds nothing before the first PV
+#pragma unroll
+        for (int c = 0; c < OUT / 16; ++c) {        // narrow pieces: the scores stay in registers meanwhile
+          float o[16];
+          tmem_ld_32x32b_x16(t_o + c * 16, o);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) o[i] *= f;
+          tmem_st_x16(t_o + c * 16, o);
+        }
+      }
+    }
+    const float neg_m = -m_used * scale_log2;
+    const unsigned long long sc2 = pack2(scale_log2, scale_log2), nm2 = pack2(neg_m, neg_m);
+    unsigned long long l0 = 0ull, l1 = 0ull;                                // two sums of +0 each
+#pragma unroll
+    for (int i = 0; i < KEYS; i += 4) {   // packed P overwrites the row in place (index i / 2 <= i)
+      float a, b, c, d;
+      unpack2(fma2(pack2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), sc2, nm2), a, b);
+      a = ex2(a), b = ex2(b);
+      const unsigned long long x = fma2(pack2(__uint_as_float(s[i + 2]), __uint_as_float(s[i + 3])), sc2, nm2);
+      if (i % FMA_EVERY == FMA_EVERY - 4) {
+        unpack2(ex2_fma2(x), c, d);
+      } else {
+        unpack2(x, c, d);
+        c = ex2(c), d = ex2(d);
+      }
+      l0 = add2(l0, pack2(a, b));
+      l1 = add2(l1, pack2(c, d));
+      s[i >> 1] = pack_bf16x2(a, b);
+      s[(i >> 1) + 1] = pack_bf16x2(c, d);
+    }
+    float x0, x1;
+    unpack2(add2(l0, l1), x0, x1);
+    l += x0 + x1;
+    tmem_st_x32(t_s + half * (KEYS / 2), s);
+    tmem_st_wait();
+    tc_fence_before_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bars->p_full[q]);
+  }
+  if (my_tiles == 0 || !ok) return;
+  ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_final, 0, &bars->abort, 32 + q));
+  float* slot = exchange + (my_tiles & 1) * (4 * BM);
+  slot[half * BM] = ok ? l : STOP;
+  pair_sync(pair);
+  const float other = slot[(half ^ 1) * BM];
+  if (!ok) return;
+  tc_fence_after_sync();
+  const float sum = half ? other + l : l + other, inv = sum > 0.f ? 1.f / sum : 0.f;
+  // Stage this warp's 32 rows x OUT columns in the (now idle) Q region, then write every row with OUT / 8 lanes x 16 bytes. 16-byte chunk
+  // c of row r sits at c ^ (r & (chunks - 1)).
+  constexpr int BYTES = OUT * 2, CHUNKS = BYTES / 16;
+  uint8_t* slab = smem + C::SMEM_Q + warp * (32 * BYTES);
+#pragma unroll
+  for (int c = 0; c < OUT / 32; ++c) {
+    uint32_t o[32];
+    tmem_ld_x32(t_o + c * 32, o);
+    tmem_ld_wait();
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      uint4 u;
+      u.x = pack_bf16x2(__uint_as_float(o[v * 8 + 0]) * inv, __uint_as_float(o[v * 8 + 1]) * inv);
+      u.y = pack_bf16x2(__uint_as_float(o[v * 8 + 2]) * inv, __uint_as_float(o[v * 8 + 3]) * inv);
+      u.z = pack_bf16x2(__uint_as_float(o[v * 8 + 4]) * inv, __uint_as_float(o[v * 8 + 5]) * inv);
+      u.w = pack_bf16x2(__uint_as_float(o[v * 8 + 6]) * inv, __uint_as_float(o[v * 8 + 7]) * inv);
+      *reinterpret_cast<uint4*>(slab + lane * BYTES + (((c * 4 + v) ^ (lane & (CHUNKS - 1))) << 4)) = u;
+    }
+  }
+  __syncwarp();
+  const int row0 = q_base + q * BM + w4 * 32;
+#pragma unroll
+  for (int it = 0; it < CHUNKS; ++it) {                                     // CHUNKS lanes write one row: 32 / CHUNKS rows per pass
+    const int r = (32 / CHUNKS) * it + lane / CHUNKS, ch = lane % CHUNKS;
+    const int grow = row0 + r;
+    if (grow >= q_len) continue;
+    const uint4 val = *reinterpret_cast<const uint4*>(slab + r * BYTES + ((ch ^ (r & (CHUNKS - 1))) << 4));
+    const int col = head * VD + half * OUT + ch * 8;
+    bf16* dst = p.out + ((long long)batch * p.q_len + tok0 + grow) * p.out_stride_tok + col;
+    if (p.scatter.enabled) {
+      const OutScatter& sc = p.scatter;
+      const int g2 = grow - sc.split;
+      const int rk = grow < sc.split ? grow / sc.n0 : g2 / sc.n1;
+      const int local = grow < sc.split ? grow % sc.n0 : sc.n0 + g2 % sc.n1;
+      dst = sc.peer[rk] + (long long)local * p.out_stride_tok + sc.col_offset + col;
+    }
+    *reinterpret_cast<uint4*>(dst) = val;
+  }
+}
 
 // 168 registers per thread is the cap for ten warps: two of the four scheduler partitions hold three warps, and a
 // partition's file is 16 K registers (a build with 200 registers per thread does not launch).
@@ -193,8 +398,12 @@ struct Barriers {
 // one 64-column atom of the K tile (columns of the other map that fall into it meet zero columns of q), the V tile serves both, and
 // the second map's result is handed to the first one's threads through shared memory for the difference and its norm. DIFF 2 is for
 // caps up to MAX_FIXED_CAP: the scores are bounded, so the exponentials are taken as they are, without a running maximum.
-template <int QK, int VD, bool EXT, bool LAT, int DIFF>
-__global__ void __launch_bounds__(THREADS, 1)
+// HALVES 2 (the plain problems): two threads per query row, each with 64 of a tile's 128 keys. See softmax_halves.
+template <int HALVES>
+constexpr int fa_threads() { return HALVES * 256 + 64; }
+
+template <int QK, int VD, bool EXT, bool LAT, int DIFF, int HALVES>
+__global__ void __launch_bounds__(fa_threads<HALVES>(), 1)
 attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                           const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_q2,
                           const __grid_constant__ CUtensorMap tmap_k2, const FaParams p) {
@@ -206,9 +415,12 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   Barriers* bars = reinterpret_cast<Barriers*>(smem + SMEM_BAR);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  static_assert(HALVES == 1 || !(EXT || LAT || DIFF), "halves: plain problems only");
+  constexpr int TMA_WARP = 8 * HALVES, MMA_WARP = TMA_WARP + 1;
   constexpr int TILE_STEP = DIFF ? 0 : BM;                  // query rows between the two tiles of a CTA
   const int cta_rows = DIFF ? BM : p.tiles * BM;
-  const int q_base = blockIdx.x * cta_rows;
+  // causal blocks: the last queries see the most keys and start first
+  const int q_base = (p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x) * cta_rows;
   constexpr bool WIDE = EXT && !LAT && DIFF == 0;             // v_heads and out_gate are looked at
   const int head = WIDE && p.v_heads > 0 ? blockIdx.y / p.v_heads : blockIdx.y;
   // packed variable-length batch: this CTA's sequence covers tokens [tok0, tok0 + q_len) of one flat token axis
@@ -243,13 +455,13 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
     }
     for (int q = 0; q < 2; ++q) {
       mbar_init(&bars->s_full[q], 1);
-      mbar_init(&bars->p_full[q], BM);
+      mbar_init(&bars->p_full[q], HALVES == 2 ? 8 : BM);      // warps / threads
     }
     mbar_init(&bars->o_final, 1);
     bars->abort = 0;
     mbar_fence_init();
   }
-  if (warp == 8 && lane == 0) {
+  if (warp == TMA_WARP && lane == 0) {
     tma_prefetch_desc(&tmap_q);
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
@@ -258,7 +470,7 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
       tma_prefetch_desc(&tmap_k2);
     }
   }
-  if (warp == 9) {
+  if (warp == MMA_WARP) {
     tmem_alloc(&bars->tmem_base, TMEM_COLS);
     tmem_relinquish();
   }
@@ -269,7 +481,7 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   pdl_launch_dependents();
   pdl_wait();
 
-  if (warp == 8) {
+  if (warp == TMA_WARP) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       mbar_arrive_expect_tx(&bars->q_full, DIFF ? 2 * ATOM_BYTES : p.tiles * TILE_BYTES);
@@ -331,65 +543,77 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
           mbar_wait(&bars->v_full[j % V_STAGES], (j / V_STAGES) & 1, &never, 14);
       }
     }
-  } else if (warp == 9) {
+  } else if (warp == MMA_WARP) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t IDESC_QK = umma_idesc_bf16_f32(BM, BN);
-      constexpr uint32_t IDESC_PV = umma_idesc_bf16_f32(BM, VD) | (1u << 16);   // B is MN-major
-      const uint32_t col_s[2] = {COL_S0, COL_S1}, col_o[2] = {COL_O0, COL_O1};
-      const uint32_t q_addr = smem_u32(smem + SMEM_Q), k_addr = smem_u32(smem + SMEM_K),
-                     v_addr = smem_u32(smem + SMEM_V);
-      auto issue_qk = [&](int q, int s) {
-        if constexpr (DIFF != 0) {
-          for (int k = 0; k < (p.diff.dim + 15) / 16; ++k)
-            umma_f16_ss(tmem + col_s[q], umma_desc_kmajor_sw128(q_addr + q * TILE_BYTES + k * 32),
-                        umma_desc_kmajor_sw128(k_addr + s * TILE_BYTES + q * ATOM_BYTES + k * 32), IDESC_QK, k > 0);
-          umma_commit(&bars->s_full[q]);
-          return;
-        }
+    // The whole warp runs, with one elected lane for the MMAs: their descriptors stay in uniform registers. Issued from one lane of a
+    // divergent warp the 32 MMAs of a key tile took longer than the tensor cores did.
+    constexpr uint32_t IDESC_QK = umma_idesc_bf16_f32(BM, BN);
+    constexpr uint32_t IDESC_PV = umma_idesc_bf16_f32(BM, VD) | (1u << 16);   // B is MN-major
+    const uint32_t col_s[2] = {COL_S0, COL_S1}, col_o[2] = {COL_O0, COL_O1};
+    const uint64_t q_desc = umma_desc_kmajor_sw128(smem_u32(smem + SMEM_Q)), k_desc = umma_desc_kmajor_sw128(smem_u32(smem + SMEM_K)),
+                   v_desc = umma_desc_mnmajor_sw128(smem_u32(smem + SMEM_V));
+    auto wait_all = [&](uint64_t* bar, uint32_t parity, int where) {
+      return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, where)) != 0;
+    };
+    auto issue_qk = [&](int q, int s) {       // one lane; descriptor addresses count 16-byte units
+      const uint64_t qd = q_desc + (uint64_t)(q * (TILE_BYTES >> 4)), kd = k_desc + (uint64_t)(s * (TILE_BYTES >> 4));
+      if constexpr (DIFF != 0) {
+        for (int k = 0; k < (p.diff.dim + 15) / 16; ++k)
+          umma_f16_ss(tmem + col_s[q], qd + k * 2, kd + q * (ATOM_BYTES >> 4) + k * 2, IDESC_QK, k > 0);
+      } else {
 #pragma unroll
         for (int k = 0; k < QK / 16; ++k) {
-          const uint32_t off = (k >> 2) * ATOM_BYTES + (k & 3) * 32;
-          umma_f16_ss(tmem + col_s[q], umma_desc_kmajor_sw128(q_addr + q * TILE_BYTES + off),
-                      umma_desc_kmajor_sw128(k_addr + s * TILE_BYTES + off), IDESC_QK, k > 0);
+          const uint32_t off = ((k >> 2) * ATOM_BYTES + (k & 3) * 32) >> 4;
+          umma_f16_ss(tmem + col_s[q], qd + off, kd + off, IDESC_QK, k > 0);
         }
-        umma_commit(&bars->s_full[q]);
-      };
-      bool ok = mbar_wait(&bars->q_full, 0, abort_flag, 20);
-      if (ok) ok = mbar_wait(&bars->k_full[0], 0, abort_flag, 21);
-      if (ok) {
-        tc_fence_after_sync();
+      }
+      umma_commit(&bars->s_full[q]);
+    };
+    bool ok = wait_all(&bars->q_full, 0, 20);
+    if (ok) ok = wait_all(&bars->k_full[0], 0, 21);
+    if (ok) {
+      tc_fence_after_sync();
+      if (elect_one()) {
         issue_qk(0, 0);
         if (p.tiles == 2) issue_qk(1, 0);
         umma_commit(&bars->k_empty[0]);
       }
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int s = j % V_STAGES, sn = (j + 1) % K_STAGES;
-        const uint32_t ph = (j / V_STAGES) & 1, phn = ((j + 1) / K_STAGES) & 1;
-        ok = mbar_wait(&bars->v_full[s], ph, abort_flag, 22);
-        if (ok && j + 1 < n_tiles) ok = mbar_wait(&bars->k_full[sn], phn, abort_flag, 23);
-        for (int q = 0; q < p.tiles && ok; ++q) {
-          ok = mbar_wait(&bars->p_full[q], j & 1, abort_flag, 24 + q);
-          if (!ok) break;
-          tc_fence_after_sync();
+      __syncwarp();
+    }
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      const int s = j % V_STAGES, sn = (j + 1) % K_STAGES;
+      const uint32_t ph = (j / V_STAGES) & 1, phn = ((j + 1) / K_STAGES) & 1;
+      ok = wait_all(&bars->v_full[s], ph, 22);
+      if (ok && j + 1 < n_tiles) ok = wait_all(&bars->k_full[sn], phn, 23);
+      const uint64_t vd = v_desc + (uint64_t)(s * (V_TILE_BYTES >> 4));
+      for (int q = 0; q < p.tiles && ok; ++q) {
+        ok = wait_all(&bars->p_full[q], j & 1, 24 + q);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const bool last_q = (q == p.tiles - 1);
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < BN / 16; ++k)
-            umma_f16_ts(tmem + col_o[q], tmem + col_s[q] + k * 8,
-                        umma_desc_mnmajor_sw128(v_addr + s * V_TILE_BYTES + k * 2048), IDESC_PV, (j > 0) || (k > 0));
-          const bool last_q = (q == p.tiles - 1);
+            umma_f16_ts(tmem + col_o[q], tmem + col_s[q] + k * 8, vd + k * (2048 >> 4), IDESC_PV, (j > 0) || (k > 0));
           if (last_q) umma_commit(&bars->v_empty[s]);
           if (j + 1 < n_tiles) {
             issue_qk(q, sn);
             if (last_q) umma_commit(&bars->k_empty[sn]);
           }
         }
-      }
-      umma_commit(&bars->o_final);   // also on the abort path: it only tracks MMAs already issued
-      if (!ok) {                     // TMEM must not be freed under MMAs that are still running
-        volatile int never = 0;
-        mbar_wait(&bars->o_final, 0, &never, 27);
+        __syncwarp();
       }
     }
+    __syncwarp();
+    if (elect_one()) umma_commit(&bars->o_final);   // also on the abort path: it only tracks MMAs already issued
+    __syncwarp();
+    if (!ok) {                                      // TMEM must not be freed under MMAs that are still running
+      volatile int never = 0;
+      mbar_wait(&bars->o_final, 0, &never, 27);
+      __syncwarp();
+    }
+  } else if constexpr (HALVES == 2) {
+    softmax_halves<C>(p, bars, smem, tmem, q_base, q_len, kv_len, coff, n_tiles, tok0, batch, head);
   } else {
     // ------------------------------------------------------------------ softmax warpgroups (thread = query row)
     const int q = warp >> 2;
@@ -519,9 +743,9 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
       // a row whose chunk starts beyond this tile has seen no key yet: its exponentials are all zero
       const float neg_m = (EXT && m_used == -INFINITY) ? 0.f : -m_used * scale_log2;
       float l0 = 0.f, l1 = 0.f;
-      // (Measured alternatives for this loop, all slower on B200: every 4th / 2nd exponential as a cubic on the FMA pipe
-      // -8 % / -17 %; pairs of exponentials as one bf16x2 special-function operation -6 %; three-input max with
-      // two-lane fp32 multiply-add and add -30 %, from register-pair moves and spills. The loop is issue-bound.)
+      // (Measured alternatives for this loop with a thread per row, all slower on B200: every 4th / 2nd exponential as a cubic on the FMA
+      // pipe -8 % / -17 %; pairs of exponentials as one bf16x2 special-function operation -6 %; three-input max with two-lane fp32
+      // multiply-add and add -30 %, from register-pair moves and spills.)
 #pragma unroll
       for (int i = 0; i < BN; i += 2) {   // packed P overwrites the row in place (index i/2 <= i)
         const float e0 = ex2(fmaf(__uint_as_float(s[i]), scale_log2, neg_m));
@@ -660,7 +884,7 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == MMA_WARP) {
     tc_fence_after_sync();
     tmem_dealloc(tmem, TMEM_COLS);
   }
@@ -753,8 +977,9 @@ struct FaMaps {
 template <int QK, int VD, bool EXT, bool LAT, int DIFF = 0>
 int launch_fa(dim3 grid, cudaStream_t stream, const FaMaps& m, const FaParams& p) {
   static bool configured[64] = {false};
-  auto kernel = attn_dense_tcgen05_kernel<QK, VD, EXT, LAT, DIFF>;
-  constexpr size_t SMEM = FaCfg<QK, VD>::SMEM_BYTES;
+  constexpr int HALVES = EXT || LAT || DIFF ? 1 : 2;
+  auto kernel = attn_dense_tcgen05_kernel<QK, VD, EXT, LAT, DIFF, HALVES>;
+  constexpr size_t SMEM = FaCfg<QK, VD>::SMEM_BYTES + (HALVES == 2 ? FaCfg<QK, VD>::EXCHANGE_BYTES : 0);
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
@@ -762,7 +987,7 @@ int launch_fa(dim3 grid, cudaStream_t stream, const FaMaps& m, const FaParams& p
     if (e != cudaSuccess) return -(int)e;
     configured[dev] = true;
   }
-  return launch_kernel(kernel, grid, dim3(THREADS), SMEM, stream, m.q, m.k, m.v, m.q2, m.k2, p);
+  return launch_kernel(kernel, grid, dim3(fa_threads<HALVES>()), SMEM, stream, m.q, m.k, m.v, m.q2, m.k2, p);
 }
 
 enum class FaKind { DENSE, EXT, LATENT, DIFF };
