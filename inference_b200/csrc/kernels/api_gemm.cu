@@ -83,10 +83,11 @@ int swb_gemm_bf16_gated(const void* A, int lda, const void* W, int ldw, void* D,
 }
 
 // 3x3 convolution, stride 1, zero padding 1, over an NHWC bf16 activation x [n, h, w, c] as an implicit GEMM on the
-// tcgen05 kernel: no patch matrix is written; each reduction block is one window tap over one 64-channel slab, fetched
+// tcgen05 kernels: no patch matrix is written; each reduction block is one window tap over one 64-channel slab, fetched
 // by a 4-D TMA box at the tile's pixel origin shifted by the tap (zero fill outside the image is the padding).
 // W [cout, (ky, kx, cin)] bf16 rows of 9 c; out [n h w, cout] bf16 (= NHWC); optional bias [cout] and residual
-// [n h w, cout]. Needs c % 64 == 0, h w % 128 == 0 and w a multiple or a divisor of 128; returns -3 otherwise.
+// [n h w, cout]. Needs c % 64 == 0, and either 16-byte rows of out, bias and residual (any image size) or h w % 128 == 0 with w
+// a multiple or a divisor of 128; returns -3 otherwise.
 int swb_conv3x3_nhwc(const void* x, int n, int h, int w, int c, const void* W, int ldw, int cout, void* out, int ldd,
                      const void* bias, const void* residual, int ld_res, int act, void* stream) {
   swb::GemmArgs a;

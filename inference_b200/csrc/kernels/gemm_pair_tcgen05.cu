@@ -602,7 +602,7 @@ int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t st
   CUtensorMap ta, tb;
   int r;
   if (a.conv_c > 0) {
-    if (a.conv_c % BK || a.K != 9 * a.conv_c || (long)a.T != (long)a.conv_n * a.conv_h * a.conv_w) return -3;
+    if (a.conv_n <= 0 || a.conv_h <= 0 || a.conv_w <= 0 || a.conv_c % BK || a.K != 9 * a.conv_c || (long)a.T != (long)a.conv_n * a.conv_h * a.conv_w) return -3;
     // the box of 128 pixels that covers an image with the fewest boxes
     long best = -1;
     for (int wl = 7; wl >= 3; --wl) {

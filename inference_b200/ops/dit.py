@@ -63,11 +63,11 @@ def rgb8_nhwc(x: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def conv3x3_supported(x: torch.Tensor) -> bool:
-    """Shapes the implicit-GEMM convolution takes: 64-channel slabs, whole 128-pixel tiles that are a run of one image
-    row or a stack of whole rows."""
+def conv3x3_supported(x: torch.Tensor, cout: int = 8) -> bool:
+    """Shapes the implicit-GEMM convolution takes: 64-channel slabs, and 16-byte rows of the output (any image size) or whole
+    128-pixel tiles that are a run of one image row or a stack of whole rows."""
     N, H, W, C = x.shape
-    return C % 64 == 0 and (H * W) % 128 == 0 and (W % 128 == 0 or 128 % W == 0)
+    return C % 64 == 0 and (cout % 8 == 0 or ((H * W) % 128 == 0 and (W % 128 == 0 or 128 % W == 0)))
 
 
 def conv3x3_nhwc(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, residual: torch.Tensor | None = None,
@@ -83,7 +83,9 @@ def conv3x3_nhwc(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = N
     Cout = w.shape[0]
     assert x.is_contiguous() and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[1] == 9 * C and w.stride(1) == 1
     res2 = residual.reshape(N * H * W, Cout) if residual is not None else None
-    if not conv3x3_supported(x) or os.environ.get("SWB_CONV3X3", "implicit") == "im2col":
+    rows_ok = ((bias is None or bias.data_ptr() % 16 == 0) and
+               (res2 is None or (res2.data_ptr() % 16 == 0 and res2.stride(0) % 8 == 0)))
+    if not conv3x3_supported(x, Cout if rows_ok else 1) or os.environ.get("SWB_CONV3X3", "implicit") == "im2col":
         return gemm_bf16(im2col3x3_nhwc(x), w, bias=bias, residual=res2, act=act).view(N, H, W, Cout)
     out = torch.empty((N * H * W, Cout), dtype=torch.bfloat16, device=x.device)
     if res2 is not None:

@@ -175,6 +175,27 @@ def test_implicit_conv3x3_matches_conv2d(shape, monkeypatch):
     assert (out.float() - refn).abs().max().item() < 0.03 * max(1.0, refn.abs().max().item())
 
 
+@pytest.mark.parametrize("shape", [(1, 5, 7, 64, 8), (2, 19, 13, 64, 72), (1, 38, 26, 128, 128), (3, 9, 130, 64, 136), (1, 152, 104, 64, 256)])
+def test_implicit_conv3x3_of_any_image_size(shape):
+    """Boxes of pixels that stick out of the image, an odd number of boxes, output widths between the tile widths. The tolerance: two
+    roundings to bf16 (2^-9 each) of the largest result, and fp32 sums of 9 C products."""
+    import torch.nn.functional as F
+
+    from inference_b200 import ops
+
+    N, H, W, C, Co = shape
+    g = torch.Generator(device="cuda").manual_seed(H * W + C)
+    x = torch.randn(N, H, W, C, device="cuda", generator=g).bfloat16()
+    w4 = (torch.randn(Co, C, 3, 3, device="cuda", generator=g) / (9 * C) ** 0.5).bfloat16()
+    b, r = torch.randn(Co, device="cuda", generator=g).bfloat16(), torch.randn(N, H, W, Co, device="cuda", generator=g).bfloat16()
+    wk = w4.permute(0, 2, 3, 1).reshape(Co, 9 * C).contiguous()
+    assert ops.conv3x3_supported(x, Co)
+    want = F.silu(F.conv2d(x.double().permute(0, 3, 1, 2), w4.double(), b.double(), padding=1).permute(0, 2, 3, 1)) + r.double()
+    got = ops.conv3x3_nhwc(x, wk, b, residual=r, act="silu")
+    ops.check_status()
+    assert (got.double() - want).abs().max().item() < 2.0 ** -8 * want.abs().max().item()
+
+
 def test_vae_decoder_matches_oracle():
     from inference_b200.models.vae import OracleVaeDecoder, VaeConfig, VaeDecoderGpu, random_vae_weights
 
