@@ -201,6 +201,31 @@ int swb_gemm_bf16_grouped(const void* A, int lda, const void* W, int ldw, int gr
   return swb::gemm_bf16_launch(a, reinterpret_cast<cudaStream_t>(stream));
 }
 
+// The same for dense segments on the two-SM kernel: row_tiles (int4, on the device) lists (first row, rows from there to the end of its
+// segment, weight group, -) for every 256 rows of a segment, row_tile_count how many there are, at most max_tiles. act may be a gated
+// pair (W's rows in (gate, up) pairs, D [T, N / 2]). N % 8 == 0, 16-byte aligned rows.
+int swb_gemm_bf16_routed(const void* A, int lda, const void* W, int ldw, int groups, const void* row_tiles, const int* row_tile_count,
+                         int max_tiles, void* D, int ldd, int T, int N, int K, int act, float act_a, void* stream) {
+  if (groups <= 0 || !row_tiles || !row_tile_count || max_tiles <= 0) return -3;
+  swb::GemmArgs a{};
+  a.A = A;
+  a.lda = lda;
+  a.W = W;
+  a.ldw = ldw;
+  a.D = D;
+  a.ldd = ldd;
+  a.T = T;
+  a.N = N;
+  a.K = K;
+  a.act = act;
+  a.act_a = act_a;
+  a.groups = groups;
+  a.group_tiles = row_tiles;
+  a.group_count = row_tile_count;
+  a.group_max_tiles = max_tiles;
+  return swb::gemm_bf16_launch(a, reinterpret_cast<cudaStream_t>(stream));
+}
+
 // Decode GEMM inside a folded-RMSNorm chain (T <= 64, cluster kernel): ssq_in (nullable) = per-token sums of squares
 // accumulated by the producer of A, the accumulators are scaled by rsqrt(sum / norm_dim + eps) per token; ssq_out
 // (nullable) accumulates this launch's sums of the rows it stores (after the residual add) and must be zero at

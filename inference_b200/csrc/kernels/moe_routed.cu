@@ -133,7 +133,11 @@ struct RouteParams {
   uint4* rows_out;
   long long ld_in, ld_out;
   int pieces;
+  int4* row_tiles;           // optional: (first row, rows from there to the segment's end, expert, -) of every ROUTED_TILE rows of a segment
+  int* row_tile_count;       // entries of the list
 };
+
+constexpr int ROUTED_TILE = 256;      // rows of a tile of the two-SM GEMM
 
 // First row of every expert's (padded) segment from the counts, by the whole block; start [E + 1] in shared memory.
 __device__ __forceinline__ void segment_starts(const RouteParams& p, int* start) {
@@ -179,6 +183,22 @@ __device__ __forceinline__ void describe_segments(const RouteParams& p, const in
       if (__ldcg(p.counters + e) > 0) p.active[atomicAdd(&n_active, 1)] = e;
     __syncthreads();
     for (int i = n_active + threadIdx.x; i < min(p.E, p.T * p.top); i += blockDim.x) p.active[i] = -1;
+  }
+  if (p.row_tiles && threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int carry = 0;
+    for (int e0 = 0; e0 < p.E; e0 += 32) {
+      const int e = e0 + lane, rows = e < p.E ? __ldcg(p.counters + e) : 0, n = (rows + ROUTED_TILE - 1) / ROUTED_TILE;
+      int s = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += y;
+      }
+      for (int i = 0; i < n; ++i) p.row_tiles[carry + s - n + i] = make_int4(start[e] + i * ROUTED_TILE, rows - i * ROUTED_TILE, e, 0);
+      carry += __shfl_sync(0xffffffffu, s, 31);
+    }
+    if (lane == 0) *p.row_tile_count = carry;
   }
 }
 
@@ -274,6 +294,40 @@ __global__ void __launch_bounds__(256) moe_layout_kernel(const RouteParams p) {
   __syncthreads();
   if (!is_last) return;
   for (int e = threadIdx.x; e < p.E + 2; e += blockDim.x) p.counters[e] = 0;
+}
+
+// out[t] = scale * sum_k weights[t, k] y[dest[t, k]] (+ extra[t] * sigmoid(extra_gate[t])): sums in fp32, slot by slot. A thread has eight
+// columns of a token; four slots' rows are on their way at a time. Bound by reading y: 3650 tokens x 8 slots of 2048 columns take 33 us.
+__global__ void __launch_bounds__(128) moe_combine_kernel(const bf16* __restrict__ y, long long ldy, const int* __restrict__ dest,
+                                                          const float* __restrict__ weights, int top, float scale,
+                                                          const bf16* __restrict__ extra, long long ld_extra,
+                                                          const float* __restrict__ extra_gate, long long ld_gate, bf16* out,
+                                                          long long ldo, int H) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x, c = (blockIdx.y * 128 + threadIdx.x) * 8;
+  if (c >= H) return;
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+#pragma unroll 4
+  for (int k = 0; k < top; ++k) {
+    const float w = weights[(size_t)t * top + k];
+    float v[8];
+    load_row8(y + dest[(size_t)t * top + k] * ldy + c, v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = fmaf(w, v[j], acc[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] *= scale;
+  if (extra) {
+    float v[8];
+    load_row8(extra + t * ld_extra + c, v);
+    const float g = extra_gate ? 1.f / (1.f + expf(-extra_gate[t * ld_gate])) : 1.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = fmaf(g, v[j], acc[j]);
+  }
+  store_row8(out + t * ldo + c, acc);
 }
 
 constexpr int GR_WARPS = 8;
@@ -427,17 +481,19 @@ int swb_moe_table_plan(const long long* ids, int T, const int* tables, int layer
 // [T, top] = their scores, as they are or (renorm) divided by their sum + 1e-20. dest, src, offsets, active, tile_group, pad and rows_cap as in swb_moe_table_plan.
 // expert and rank: int32 scratch [T * top]; counters: int32 [E + 2], zero at the first launch, launches that share it ordered on
 // one stream. rows_in (nullable): bf16 / fp32 rows of `pieces` 16-byte pieces, ld_in pieces apart, copied to rows dest[t, k] of rows_out.
-int swb_moe_route(const float* logits, int ld, int T, int E, int top, int renorm, int pad, int* expert, int* rank, float* weights, int* counters,
-                  int* dest, int* src, int* offsets, int* active, int* tile_group, int rows_cap, const void* rows_in, long long ld_in,
-                  void* rows_out, long long ld_out, int pieces, void* stream) {
+// row_tiles (nullable, needs rows_in and pad 1): int4 [rows_cap / 256 + min(E, rows_cap)], the row tiles of swb_gemm_bf16_routed, their
+// number in row_tile_count.
+int swb_moe_route_tiles(const float* logits, int ld, int T, int E, int top, int renorm, int pad, int* expert, int* rank, float* weights, int* counters,
+                        int* dest, int* src, int* offsets, int* active, int* tile_group, int rows_cap, const void* rows_in, long long ld_in,
+                        void* rows_out, long long ld_out, int pieces, void* row_tiles, int* row_tile_count, void* stream) {
   using namespace swb;
   if (T <= 0) return 0;
   if (top <= 0 || E <= 0 || E > 4096 || top > E || ld < E || (pad != 1 && pad != 128) || (tile_group && (pad != 128 || rows_cap % 128)) ||
       (long long)T * top + (long long)E * (pad - 1) > (long long)rows_cap || !expert || !rank || !weights || !counters || !dest || !offsets ||
-      (rows_in && (!rows_out || pieces <= 0)))
+      (rows_in && (!rows_out || pieces <= 0)) || (row_tiles && (!row_tile_count || !rows_in || pad != 1)))
     return -3;
   const RouteParams p{logits, ld, T, E, top, pad, expert, rank, weights, renorm, counters, dest, src, offsets, active, tile_group, rows_cap,
-                      reinterpret_cast<const uint4*>(rows_in), reinterpret_cast<uint4*>(rows_out), ld_in, ld_out, pieces};
+                      reinterpret_cast<const uint4*>(rows_in), reinterpret_cast<uint4*>(rows_out), ld_in, ld_out, pieces, reinterpret_cast<int4*>(row_tiles), row_tile_count};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const dim3 grid((unsigned)((T + 7) / 8));
   const size_t smem = (size_t)(E + 1) * sizeof(int);
@@ -446,6 +502,26 @@ int swb_moe_route(const float* logits, int ld, int T, int E, int top, int renorm
   if (rc) return rc;
   const long long blocks = ((long long)T * top + 7) / 8;
   return launch_kernel(moe_layout_kernel, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), smem, s, p);
+}
+
+int swb_moe_route(const float* logits, int ld, int T, int E, int top, int renorm, int pad, int* expert, int* rank, float* weights, int* counters,
+                  int* dest, int* src, int* offsets, int* active, int* tile_group, int rows_cap, const void* rows_in, long long ld_in,
+                  void* rows_out, long long ld_out, int pieces, void* stream) {
+  return swb_moe_route_tiles(logits, ld, T, E, top, renorm, pad, expert, rank, weights, counters, dest, src, offsets, active, tile_group, rows_cap,
+                             rows_in, ld_in, rows_out, ld_out, pieces, nullptr, nullptr, stream);
+}
+
+// out[t] = bf16(scale * sum over k < top of weights[t, k] y[dest[t, k]] + extra[t] * sigmoid(extra_gate[t])). extra, extra_gate nullable.
+// H % 8 == 0, 16-byte aligned rows.
+int swb_moe_combine(const void* y, long long ldy, const int* dest, const float* weights, int T, int top, float scale, const void* extra,
+                    long long ld_extra, const float* extra_gate, long long ld_gate, void* out, long long ldo, int H, void* stream) {
+  using namespace swb;
+  if (T <= 0 || H <= 0) return 0;
+  auto bad = [](const void* q, long long ld) { return (reinterpret_cast<uintptr_t>(q) & 15) != 0 || ld % 8 != 0; };
+  if (H % 8 || top <= 0 || !y || !dest || !weights || !out || bad(y, ldy) || bad(out, ldo) || (extra && bad(extra, ld_extra))) return -3;
+  return launch_kernel(moe_combine_kernel, dim3(T, (H + 1023) / 1024), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream),
+                       reinterpret_cast<const bf16*>(y), ldy, dest, weights, top, scale, reinterpret_cast<const bf16*>(extra), ld_extra, extra_gate,
+                       ld_gate, reinterpret_cast<bf16*>(out), ldo, H);
 }
 
 // out[r, :] = act(x[src ? src[r] : r, :] W[e]^T) for every row r of expert e's segment [offsets[e], offsets[e + 1]).

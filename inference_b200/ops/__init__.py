@@ -8,7 +8,7 @@ from .delta import DeltaWeights, channel_delta, delta_key_width, head_delta  # n
 from .hyper import HyperBranch, ShortConv, StreamMix, hyper_step, short_conv  # noqa: F401
 from .latent import (LatentWeights, QueryRotation, SplitPartials, head_product, latent_attention_simple, latent_decode, latent_decode_supported,  # noqa: F401
                      latent_gather, latent_prefill, latent_prefill_supported, latent_prep, latent_width, rotate_queries)
-from .moe import RoutingPlan, gemm_grouped_rows, logits_routing, routed_ffn, routed_gated_ffn, table_routing  # noqa: F401
+from .moe import RoutingPlan, combine_routed, gemm_grouped_rows, gemm_routed, logits_routing, routed_ffn, routed_gated_ffn, routing_counters, table_routing  # noqa: F401
 from .stream import Branch, DepthAverage, NormWeights, RoutedRows, stream_embed, stream_embed_pairs, stream_norm  # noqa: F401
 from .runtime import KernelError, check_status, device_status  # noqa: F401
 from .dit import axpy, conv3x3_nhwc, conv3x3_supported, groupnorm_nhwc, im2col3x3_nhwc, rgb8_nhwc, softmax_rows, upsample2x_nhwc  # noqa: E402,F401

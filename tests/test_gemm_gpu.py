@@ -173,3 +173,37 @@ def test_pairs_of_sms(T, N, K, block_n, splits):
         rows = (T + 1) // 2
         y = ops.gemm_bf16(a, w, bias=b, residual=r, gate=gate, rows_per_gate=rows)
         close(y, (z + b.float()) * gate.float()[torch.arange(T, device="cuda") // rows] + r.float())
+
+
+@pytest.mark.parametrize("T,E,top,H,f,renorm", [(1, 4, 2, 64, 24, True), (33, 8, 8, 128, 72, False), (700, 5, 3, 200, 136, True),
+                                                (2100, 64, 8, 256, 128, False)])
+@pytest.mark.parametrize("shared", [False, True])
+def test_routed_segments_in_row_tiles(T, E, top, H, f, renorm, shared):
+    """Dense expert segments in tiles of 256 rows (none, one row, remainders, several tiles an expert), gated pairs in the epilogue, and
+    the weighted sum per token with a gated extra branch. Rounding: inputs are exact, u and y are bf16 (2^-9 each), the result too."""
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+
+    def rnd(*shape, std=1.0):
+        return (torch.randn(*shape, device="cuda", generator=g) * std).bfloat16()
+    h, up, down, z = rnd(T, H), rnd(E, 2 * f, H, std=H ** -0.5), rnd(E, H, f, std=f ** -0.5), torch.randn(T, E, device="cuda", generator=g)
+    z[:, 0] += 3.0          # a popular expert
+    counters = ops.routing_counters(E, h.device)
+    plan, rows = ops.logits_routing(z, E, top, rows=h, renorm=renorm, counters=counters, tiles256=True)
+    y = ops.routed_gated_ffn(rows, up, down, plan, "silu")
+    extra, gate = (rnd(T, H), torch.randn(T, 3, device="cuda", generator=g)[:, 1]) if shared else (None, None)
+    got = ops.combine_routed(y, plan, 1.5, extra, gate)
+    ops.check_status()
+    assert not counters.any()
+    share, which = z.double().softmax(-1).topk(top, -1)
+    if renorm:
+        share = share / share.sum(-1, keepdim=True)
+    want = torch.zeros(T, H, dtype=torch.float64, device="cuda")
+    for e in range(E):
+        u = h.double() @ up[e].double().T
+        o = (torch.nn.functional.silu(u[:, 0::2]) * u[:, 1::2]) @ down[e].double().T
+        want += 1.5 * o * (share * (which == e)).sum(-1, keepdim=True)
+    if shared:
+        want += extra.double() * torch.sigmoid(gate.double())[:, None]
+    assert (got.double() - want).norm() < 2.0 ** -8 * want.norm()
