@@ -5,8 +5,8 @@ ResnetBlock) -> 4 up levels (ch_mult [1, 2, 4, 4] reversed, num_res_blocks + 1 R
 upsample + conv3x3 between levels) -> GroupNorm(32) -> swish -> conv_out. Latents are unscaled first:
 z / scale_factor + shift_factor.
 
-GPU execution keeps activations NHWC bf16: every convolution is a tcgen05 GEMM (3x3 through a patch gather, 1x1
-directly) with bias and the residual add fused in the epilogue; GroupNorm + SiLU is one fused pass after a
+GPU execution keeps activations NHWC bf16: every convolution is a tcgen05 GEMM (3x3 implicitly, the first one's 16 channels
+through a patch gather, 1x1 directly) with bias and the residual add fused in the epilogue; GroupNorm + SiLU is one fused pass after a
 statistics pass; the mid-block attention is GEMM -> row softmax -> GEMM."""
 from __future__ import annotations
 
