@@ -57,6 +57,25 @@ def test_q4k_matvec_kernel_matches_reference_and_the_tensor_core_path(T, N, K):
     assert (out2.float().cpu() - ref2).abs().max().item() < 2e-2 * max(1.0, ref2.abs().max().item())
 
 
+@pytest.mark.parametrize("T,N,K", [(8, 37, 18432), (4, 4801, 2304), (1, 9473, 512), (6, 2369, 256)])
+def test_q4k_matvec_pairs_of_rows(T, N, K):
+    """A last pair of one row, slices that end inside a row, several pairs per warp, the largest activations. Against 64 bits with the
+    activations rounded as the kernel rounds them (int8 per block of 32), so what is left are fp32 sums and the rounding to bf16."""
+    from inference_b200 import ops
+    from inference_b200.ops import quant
+
+    g = torch.Generator(device="cuda").manual_seed(T * 7 + K)
+    qw = quant.quantize_on_device((torch.randn(N, K, device="cuda", generator=g) * 0.05).bfloat16(), "Q4_K")
+    a = (torch.randn(T, K, device="cuda", generator=g) * 0.5).bfloat16()
+    blocks = a.float().reshape(T, K // 32, 32)
+    top = blocks.abs().amax(-1, keepdim=True)
+    seen = (blocks * (127.0 / top)).round().double() * (top * (1.0 / 127.0)).double()
+    ref = seen.reshape(T, K) @ quant.dequantize_reference(qw).double().cuda().T
+    got = quant.linear_quant(a, qw)
+    ops.check_status()
+    assert (got.double() - ref).abs().max().item() < 2.0 ** -8 * ref.abs().max().item()
+
+
 @pytest.mark.parametrize("T", [65, 130, 256])
 def test_expanded_weights_are_complete_before_they_are_multiplied(T):
     """Token counts above the fused kernel's expand the weight and multiply it right behind: the product must not start from
