@@ -49,10 +49,6 @@ __global__ void __launch_bounds__(256) axpy_f32_kernel(const float* __restrict__
   if (i < n) out[i] = a * x[i] + b * y[i];
 }
 
-// 16-byte loads of a GroupNorm thread on their way at a time. Both passes are bound by memory, and with one load at a time by its
-// latency: 128 channels at 1216 x 832 with SiLU took 229 us for both (3.4 TB/s), with four 231 us.
-constexpr int GN_AHEAD = 4;
-
 // GroupNorm statistics over NHWC bf16: one CTA per (sample, group, chunk of pixels); partial sum / sum of squares are
 // accumulated with atomics into stats[n][g][2] (zeroed by the caller).
 __global__ void __launch_bounds__(256) groupnorm_stats_kernel(const bf16* __restrict__ x, float* stats, int HW, int C,
@@ -116,25 +112,15 @@ __global__ void __launch_bounds__(256) groupnorm_stats_narrow_kernel(const bf16*
   float s[8], ss[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) s[j] = ss[j] = 0.f;
-  auto add = [&](const uint4& u) {
+  for (int p = p0 + lane_p; p < p1; p += stride_p) {
     float f[8];
-    unpack8(u, f);
+    unpack8(*reinterpret_cast<const uint4*>(x + ((size_t)n * HW + p) * C + v * 8), f);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       s[j] += f[j];
       ss[j] += f[j] * f[j];
     }
-  };
-  const bf16* col = x + (size_t)n * HW * C + v * 8;
-  int p = p0 + lane_p;
-  for (; p + (GN_AHEAD - 1) * stride_p < p1; p += GN_AHEAD * stride_p) {
-    uint4 u[GN_AHEAD];
-#pragma unroll
-    for (int i = 0; i < GN_AHEAD; ++i) u[i] = *reinterpret_cast<const uint4*>(col + (size_t)(p + i * stride_p) * C);
-#pragma unroll
-    for (int i = 0; i < GN_AHEAD; ++i) add(u[i]);
   }
-  for (; p < p1; p += stride_p) add(*reinterpret_cast<const uint4*>(col + (size_t)p * C));
   if (cpg >= 8) {
     float st = 0.f, sst = 0.f;
 #pragma unroll
@@ -188,25 +174,16 @@ __global__ void __launch_bounds__(256) groupnorm_apply_kernel(const bf16* __rest
     }
     const uint4* xin = reinterpret_cast<const uint4*>(x) + (size_t)n * HW * c8 + v;
     uint4* yout = reinterpret_cast<uint4*>(out) + (size_t)n * HW * c8 + v;
-    auto one = [&](const uint4& u) {
+    for (unsigned p = tid / c8; p < (unsigned)HW; p += pix_step) {
       float f[8], o[8];
-      unpack8(u, f);
+      unpack8(xin[(size_t)p * c8], f);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float t = fmaf(f[j], sc[j], sh[j]);
         o[j] = silu ? silu_f(t) : t;
       }
-      return pack8(o);
-    };
-    size_t p = tid / c8;
-    for (; p + (size_t)(GN_AHEAD - 1) * pix_step < (size_t)HW; p += (size_t)GN_AHEAD * pix_step) {
-      uint4 u[GN_AHEAD];
-#pragma unroll
-      for (int i = 0; i < GN_AHEAD; ++i) u[i] = xin[(p + (size_t)i * pix_step) * c8];
-#pragma unroll
-      for (int i = 0; i < GN_AHEAD; ++i) yout[(p + (size_t)i * pix_step) * c8] = one(u[i]);
+      yout[(size_t)p * c8] = pack8(o);
     }
-    for (; p < (size_t)HW; p += pix_step) yout[p * c8] = one(xin[p * c8]);
   }
 }
 
