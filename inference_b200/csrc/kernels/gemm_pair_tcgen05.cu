@@ -447,7 +447,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     ItemIter iter(p);
     Item c;
     while (ok && iter.next(c)) {
-      ok = mbar_wait(&bar_tfull[acc], acc_phase, s_abort, 400 + acc);
+      // one answer for the warp: what follows (tcgen05.ld, __syncwarp, the split counter) takes all of its lanes
+      ok = __all_sync(0xffffffffu, mbar_wait(&bar_tfull[acc], acc_phase, s_abort, 400 + acc));
       if (!ok) break;
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * COLS);

@@ -207,3 +207,26 @@ def test_routed_segments_in_row_tiles(T, E, top, H, f, renorm, shared):
     if shared:
         want += extra.double() * torch.sigmoid(gate.double())[:, None]
     assert (got.double() - want).norm() < 2.0 ** -8 * want.norm()
+
+
+def test_pairs_of_sms_give_up_a_wait_together():
+    """The epilogue's wait for one very long reduction (milliseconds) with a limit of a nanosecond: the launch ends by itself, its warps
+    leave together, the status says where, and the next product is right."""
+    from inference_b200 import ops
+    from inference_b200._native import kernels
+
+    L = kernels()
+    K = 1 << 20
+    a, w = (torch.full((n, K), 0.5, dtype=torch.bfloat16, device="cuda") for n in (300, 256))
+    ops.check_status()
+    L.swb_set_wait_limit_ns(1)
+    try:
+        ops.gemm_bf16(a, w, mode=3, block_n=256, ctas=1)
+        st = ops.device_status()
+    finally:
+        L.swb_set_wait_limit_ns(2_000_000_000)
+        L.swb_status_clear()
+    assert st[0] == 1, st      # whichever role noticed first
+    y = ops.gemm_bf16(a[:, :512], w[:, :512], mode=3, block_n=256, ctas=1)
+    ops.check_status()
+    assert (y == 128.0).all()
