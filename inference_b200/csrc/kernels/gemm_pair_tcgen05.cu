@@ -634,7 +634,7 @@ int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t st
   }
   const int pairs = device_sm_count() / 2;
   if (block_n <= 0) {
-    if (a.N <= 32) {
+    if (a.N <= 32 && !gemm_act_pairs(a.act)) {      // a gated pair's epilogue takes 64 accumulator columns or more
       block_n = 32;
       splits = 1;
     } else {

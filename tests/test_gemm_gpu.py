@@ -176,7 +176,7 @@ def test_pairs_of_sms(T, N, K, block_n, splits):
 
 
 @pytest.mark.parametrize("T,E,top,H,f,renorm", [(1, 4, 2, 64, 24, True), (33, 8, 8, 128, 72, False), (700, 5, 3, 200, 136, True),
-                                                (2100, 64, 8, 256, 128, False)])
+                                                (2100, 64, 8, 256, 128, False), (300, 4, 2, 24, 8, True), (150, 3, 2, 72, 16, False)])
 @pytest.mark.parametrize("shared", [False, True])
 def test_routed_segments_in_row_tiles(T, E, top, H, f, renorm, shared):
     """Dense expert segments in tiles of 256 rows (none, one row, remainders, several tiles an expert), gated pairs in the epilogue, and
