@@ -781,8 +781,7 @@ int gemm_bf16_launch(const GemmArgs& a, cudaStream_t stream) {
   const int sms = device_sm_count();
   if (a.gate || a.group_tiles || a.force_mode == 3)
     return gemm_pair_launch(a, a.force_block_n, a.force_mode == 3 ? a.force_ctas : 0, stream);
-  // convolutions have a rule of their own below
-  if (a.conv_c == 0 && a.force_mode < 0 && a.force_ctas >= 0 && a.force_block_n == 0 && a.T > 64 && a.N >= 128 && gemm_pair_accepts(a))
+  if (a.force_mode < 0 && a.force_ctas >= 0 && a.force_block_n == 0 && a.T > 64 && a.N >= 128 && gemm_pair_accepts(a))
     return gemm_pair_launch(a, 0, 0, stream);
   if (a.force_mode == -2) {
     GemmArgs b = a;

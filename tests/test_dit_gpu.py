@@ -196,16 +196,6 @@ def test_implicit_conv3x3_of_any_image_size(shape):
     assert (got.double() - want).abs().max().item() < 2.0 ** -8 * want.abs().max().item()
 
 
-@pytest.mark.parametrize("Co", [64, 256])
-def test_implicit_conv3x3_refuses_gated_pairs(Co):
-    """A convolution's output is as wide as its weight: a gated pair has no meaning for it, whatever the width."""
-    from inference_b200 import ops
-
-    x, w = torch.zeros(1, 16, 16, 64, device="cuda").bfloat16(), torch.zeros(Co, 9 * 64, device="cuda").bfloat16()
-    with pytest.raises(ops.KernelError):
-        ops.conv3x3_nhwc(x, w, act="swiglu_pairs")
-
-
 def test_vae_decoder_matches_oracle():
     from inference_b200.models.vae import OracleVaeDecoder, VaeConfig, VaeDecoderGpu, random_vae_weights
 
