@@ -201,6 +201,7 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
     sig("swb_gemm_bf16_normed", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                  c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p])
     sig("swb_gemm_gated_supported", [c_int, c_int, c_int])
+    sig("swb_gemm_takes_pairs", [c_int] * 8)
     sig("swb_gemm_bf16_peer_reduce", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
                                       c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                       c_int, c_int, c_int, c_void_p])

@@ -302,6 +302,22 @@ int swb_gemm_peer_max_ctas(void) { return swb::SWB_PEER_MAX_CTAS; }
 
 int swb_gemm_gated_supported(int T, int N, int K) { return swb::gemm_bf16_gated_supported(T, N, K); }
 
+// 1 when a product of these sizes with contiguous, aligned rows goes to the two-SM kernel (host only; ldd as the activation has it).
+int swb_gemm_takes_pairs(int T, int N, int K, int act, int out_fp32, int force_mode, int force_block_n, int force_ctas) {
+  swb::GemmArgs a{};
+  a.lda = a.ldw = K;
+  a.ldd = swb::gemm_act_pairs(act) ? N / 2 : N;
+  a.T = T;
+  a.N = N;
+  a.K = K;
+  a.act = act;
+  a.out_fp32 = out_fp32;
+  a.force_mode = force_mode;
+  a.force_block_n = force_block_n;
+  a.force_ctas = force_ctas;
+  return swb::gemm_bf16_takes_pairs(a) ? 1 : 0;
+}
+
 size_t swb_gemm_workspace_min(void) { return swb::SWB_GEMM_COUNTER_BYTES + (size_t)(8u << 20); }
 
 int swb_sm_count(void) { return swb::device_sm_count(); }

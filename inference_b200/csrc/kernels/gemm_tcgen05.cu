@@ -774,15 +774,18 @@ int gemm_bf16_gated_supported(int T, int N, int K) {
          (N % 2) == 0;
 }
 
+// True for products that go to the two-SM kernel. A caller's own tile width or number of CTAs means the one-SM kernels.
+bool gemm_bf16_takes_pairs(const GemmArgs& a) {
+  if (a.gate || a.group_tiles || a.force_mode == 3) return true;
+  return a.force_mode < 0 && a.force_ctas == 0 && a.force_block_n == 0 && a.T > 64 && a.N >= 128 && gemm_pair_accepts(a);
+}
+
 int gemm_bf16_launch(const GemmArgs& a, cudaStream_t stream) {
   if (a.T <= 0 || a.N <= 0 || a.K <= 0) return 0;
   if ((a.K % 8) != 0 || (a.lda % 8) != 0 || (a.ldw % 8) != 0) return -3;
   if ((reinterpret_cast<uintptr_t>(a.A) & 15) || (reinterpret_cast<uintptr_t>(a.W) & 15)) return -3;
   const int sms = device_sm_count();
-  if (a.gate || a.group_tiles || a.force_mode == 3)
-    return gemm_pair_launch(a, a.force_block_n, a.force_mode == 3 ? a.force_ctas : 0, stream);
-  if (a.force_mode < 0 && a.force_ctas >= 0 && a.force_block_n == 0 && a.T > 64 && a.N >= 128 && gemm_pair_accepts(a))
-    return gemm_pair_launch(a, 0, 0, stream);
+  if (gemm_bf16_takes_pairs(a)) return gemm_pair_launch(a, a.force_block_n, a.force_mode == 3 ? a.force_ctas : 0, stream);
   if (a.force_mode == -2) {
     GemmArgs b = a;
     b.force_mode = 0;

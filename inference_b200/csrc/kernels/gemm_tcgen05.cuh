@@ -148,6 +148,7 @@ struct GemmArgs {
   int group_max_tiles = 0;
 };
 
+bool gemm_bf16_takes_pairs(const GemmArgs& a);
 int gemm_bf16_launch(const GemmArgs& a, cudaStream_t stream);
 int gemm_bf16_gated_supported(int T, int N, int K);
 int gemm_decode_cluster_supported(int T);

@@ -43,6 +43,18 @@ def test_swapped_small_tokens(T):
     _check(T, 384, 1024, bias=True, residual=True)
 
 
+@pytest.mark.parametrize("T", [65, 128, 129, 200, 256])
+def test_swapped_kernel_of_many_tokens(T):
+    """The 128- and 256-wide tiles of the weights-as-M kernel and their stream-K sums: asked for, with a number of CTAs, and
+    taken for an odd or a small number of outputs."""
+    _check(T, 512, 256, mode=1)
+    _check(T, 384, 1024, mode=1, bias=True, residual=True)
+    _check(T, 1024, 2048, mode=1, ctas=20, act="silu")
+    _check(T, 384, 1024, ctas=7, bias=True)
+    _check(T, 777, 1032, bias=True, residual=True, act="gelu_tanh")
+    _check(T, 96, 4096, out_dtype=torch.float32)
+
+
 @pytest.mark.parametrize("ctas", [-1, 3, 7, 20, 148])
 def test_stream_k_deterministic(ctas):
     y0 = _check(8, 1024, 2048, mode=1, ctas=ctas, bias=True, act="silu")
