@@ -82,9 +82,9 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
     sig("swb_gemm_bf16", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                           c_int, c_int, c_int, c_void_p, c_size_t, c_int, c_int, c_int, c_void_p])
     sig("swb_gemm_bf16_act", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                              c_int, c_int, c_float, c_float, c_int, c_void_p, c_size_t, c_int, c_int, c_int, c_void_p])
+                              c_int, c_int, c_float, c_float, c_int, c_void_p, c_size_t, c_void_p, c_void_p, c_size_t, c_int, c_int, c_int, c_void_p])
     sig("swb_gemm_bf16_gated", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p])
+                                c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_size_t, c_void_p])
     sig("swb_rmsnorm_prefetch", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float,
                                  c_float, c_void_p, c_ll, c_void_p])
     sig("swb_rmsnorm", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_float,
@@ -202,6 +202,9 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
                                  c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p])
     sig("swb_gemm_gated_supported", [c_int, c_int, c_int])
     sig("swb_gemm_takes_pairs", [c_int] * 8)
+    sig("swb_gemm_split_bytes", [c_int] * 5, c_size_t)
+    sig("swb_gemm_counter_bytes", [], c_size_t)
+    sig("swb_stream_capture_id", [c_void_p], ctypes.c_ulonglong)
     sig("swb_gemm_bf16_peer_reduce", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
                                       c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                       c_int, c_int, c_int, c_void_p])

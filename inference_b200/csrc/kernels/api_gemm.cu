@@ -1,4 +1,5 @@
 // extern "C" entry points for the dense GEMM.
+#include "gemm_pair.cuh"
 #include "gemm_tcgen05.cuh"
 
 namespace swb {
@@ -17,11 +18,16 @@ extern "C" {
 // [13] partials delivered, [14] first group's sum of squares sent). Pass null to switch it off.
 void swb_gemm_set_trace(void* device_buffer) { swb::g_trace = reinterpret_cast<unsigned long long*>(device_buffer); }
 
-// act_a, act_b: parameters of activations that have any (see GemmAct).
+// act_a, act_b: parameters of activations that have any (see GemmAct). split_counters, split_sums (nullable): see GemmArgs; split_bytes as
+// swb_gemm_split_bytes gives them.
 int swb_gemm_bf16_act(const void* A, int lda, const void* W, int ldw, void* D, int ldd, int T, int N, int K,
                       const void* bias, const void* residual, int ld_res, int act, float act_a, float act_b, int out_fp32,
-                      void* workspace, size_t workspace_bytes, int force_mode, int force_block_n, int force_ctas, void* stream) {
+                      void* workspace, size_t workspace_bytes, void* split_counters, void* split_sums, size_t split_bytes, int force_mode,
+                      int force_block_n, int force_ctas, void* stream) {
   swb::GemmArgs a;
+  a.split_counters = split_counters;
+  a.split_sums = split_sums;
+  a.split_bytes = split_bytes;
   a.act_a = act_a;
   a.act_b = act_b;
   a.A = A;
@@ -50,14 +56,14 @@ int swb_gemm_bf16(const void* A, int lda, const void* W, int ldw, void* D, int l
                   const void* bias, const void* residual, int ld_res, int act, int out_fp32, void* workspace,
                   size_t workspace_bytes, int force_mode, int force_block_n, int force_ctas, void* stream) {
   return swb_gemm_bf16_act(A, lda, W, ldw, D, ldd, T, N, K, bias, residual, ld_res, act, 0.f, 0.f, out_fp32, workspace,
-                           workspace_bytes, force_mode, force_block_n, force_ctas, stream);
+                           workspace_bytes, nullptr, nullptr, 0, force_mode, force_block_n, force_ctas, stream);
 }
 
 // D = act(A W^T + bias) * gate + residual on the two-SM kernel; row r takes the gate row r / rows_per_gate (N factors, row stride
 // ld_gate). bf16 output; 16-byte aligned rows. A residual may be D itself.
 int swb_gemm_bf16_gated(const void* A, int lda, const void* W, int ldw, void* D, int ldd, int T, int N, int K, const void* bias,
-                        const void* residual, int ld_res, const void* gate, int ld_gate, int rows_per_gate, int act, void* workspace,
-                        size_t workspace_bytes, void* stream) {
+                        const void* residual, int ld_res, const void* gate, int ld_gate, int rows_per_gate, int act,
+                        void* split_counters, void* split_sums, size_t split_bytes, void* stream) {
   if (!gate) return -3;
   swb::GemmArgs a{};
   a.A = A;
@@ -76,8 +82,9 @@ int swb_gemm_bf16_gated(const void* A, int lda, const void* W, int ldw, void* D,
   a.ld_gate = ld_gate;
   a.rows_per_gate = rows_per_gate;
   a.act = act;
-  a.workspace = workspace;
-  a.workspace_bytes = workspace_bytes;
+  a.split_counters = split_counters;
+  a.split_sums = split_sums;
+  a.split_bytes = split_bytes;
   a.force_mode = -1;
   return swb::gemm_bf16_launch(a, reinterpret_cast<cudaStream_t>(stream));
 }
@@ -316,6 +323,19 @@ int swb_gemm_takes_pairs(int T, int N, int K, int act, int out_fp32, int force_m
   a.force_block_n = force_block_n;
   a.force_ctas = force_ctas;
   return swb::gemm_bf16_takes_pairs(a) ? 1 : 0;
+}
+
+// Bytes of partial sums that a product above 64 rows takes on the two-SM kernel, 0 without k-splits. block_n, splits: 0 = by its plan.
+size_t swb_gemm_split_bytes(int T, int N, int K, int block_n, int splits) { return swb::gemm_pair_split_bytes(T, N, K, block_n, splits); }
+// SWB_GEMM_COUNTER_BYTES: counters of k-splits.
+size_t swb_gemm_counter_bytes(void) { return swb::SWB_GEMM_COUNTER_BYTES; }
+
+// Id of the capture that `stream` takes part in, 0 = none.
+unsigned long long swb_stream_capture_id(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(reinterpret_cast<cudaStream_t>(stream), &status, &id) != cudaSuccess) return 0;
+  return status == cudaStreamCaptureStatusActive ? id : 0;
 }
 
 size_t swb_gemm_workspace_min(void) { return swb::SWB_GEMM_COUNTER_BYTES + (size_t)(8u << 20); }

@@ -549,7 +549,19 @@ double plan_cost(int bn, int splits, long tiles, int kblocks, int pairs) {
 
 }  // namespace
 
-void gemm_pair_plan(int T, int N, int K, size_t workspace_bytes, int* block_n, int* splits) {
+namespace {
+
+constexpr size_t SPLIT_BYTES_MAX = (size_t)96 << 20;
+
+size_t split_bytes(int T, int N, int bn, int splits) {
+  const size_t tiles = (size_t)((T + 2 * BM - 1) / (2 * BM)) * ((N + bn - 1) / bn);
+  return tiles * 2 * splits * BM * bn * sizeof(float);
+}
+bool counters_suffice(long tiles) { return tiles * 2 * EPI_WARPS * (long)sizeof(int) <= (long)SWB_GEMM_COUNTER_BYTES; }
+
+}  // namespace
+
+void gemm_pair_plan(int T, int N, int K, size_t sum_bytes, int* block_n, int* splits) {
   const int pairs = device_sm_count() / 2;
   const int kblocks = (K + BK - 1) / BK;
   const long tm = (T + 2 * BM - 1) / (2 * BM);
@@ -558,14 +570,20 @@ void gemm_pair_plan(int T, int N, int K, size_t workspace_bytes, int* block_n, i
     if (bn > 64 && bn >= 2 * N) continue;
     const long tiles = tm * ((N + bn - 1) / bn);
     for (int s = 1; s <= 8; ++s) {
-      if (s > 1) {
-        const size_t need = SWB_GEMM_COUNTER_BYTES + (size_t)tiles * 2 * s * BM * bn * sizeof(float);
-        if (kblocks / s < 8 || workspace_bytes < need || tiles * 2 * EPI_WARPS * sizeof(int) > SWB_GEMM_COUNTER_BYTES || tiles > pairs) break;
-      }
+      if (s > 1 && (kblocks / s < 8 || sum_bytes < split_bytes(T, N, bn, s) || !counters_suffice(tiles) || tiles > pairs)) break;
       const double c = plan_cost(bn, s, tiles, kblocks, pairs);
       if (c < best) best = c, *block_n = bn, *splits = s;
     }
   }
+}
+
+size_t gemm_pair_split_bytes(int T, int N, int K, int block_n, int splits) {
+  if (block_n <= 0 && N > 32) {
+    int s = 1;
+    gemm_pair_plan(T, N, K, SPLIT_BYTES_MAX, &block_n, &s);
+    if (splits <= 0) splits = s;
+  }
+  return splits > 1 ? split_bytes(T, N, block_n, splits) : 0;
 }
 
 bool gemm_pair_accepts(const GemmArgs& a) {
@@ -633,6 +651,14 @@ int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t st
     p.tiles_m = a.group_max_tiles;
   }
   const int pairs = device_sm_count() / 2;
+  void *counters = a.split_counters, *sums = a.split_sums;
+  size_t sum_bytes = a.split_counters ? a.split_bytes : 0;
+  if (!counters && a.workspace && a.workspace_bytes > SWB_GEMM_COUNTER_BYTES && !a.gate && (a.T <= 256 || a.force_mode == 3)) {
+    counters = a.workspace;
+    sums = reinterpret_cast<uint8_t*>(a.workspace) + SWB_GEMM_COUNTER_BYTES;
+    sum_bytes = std::min(a.workspace_bytes - SWB_GEMM_COUNTER_BYTES, SPLIT_BYTES_MAX);
+  }
+  if (a.conv_c || a.group_tiles) sum_bytes = 0;
   if (block_n <= 0) {
     if (a.N <= 32 && !gemm_act_pairs(a.act)) {      // a gated pair's epilogue takes 64 accumulator columns or more
       block_n = 32;
@@ -640,7 +666,7 @@ int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t st
     } else {
       int s = 1;
       // a convolution's and a group list's rows are not T: plan with the row tiles they have
-      gemm_pair_plan(a.conv_c || a.group_tiles ? p.tiles_m * 2 * BM : a.T, a.N, a.K, a.conv_c || a.group_tiles ? 0 : a.workspace_bytes, &block_n, &s);
+      gemm_pair_plan(a.conv_c || a.group_tiles ? p.tiles_m * 2 * BM : a.T, a.N, a.K, sum_bytes, &block_n, &s);
       splits = splits > 0 ? splits : s;
     }
   }
@@ -656,10 +682,9 @@ int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t st
   p.kblocks_per_split = per;
   const long tiles = (long)p.tiles_m * p.tiles_n;
   if (splits > 1) {
-    const size_t need = SWB_GEMM_COUNTER_BYTES + (size_t)tiles * 2 * splits * BM * block_n * sizeof(float);
-    if (!a.workspace || a.workspace_bytes < need || tiles * 2 * EPI_WARPS * sizeof(int) > SWB_GEMM_COUNTER_BYTES || a.group_tiles) return -4;
-    p.counters = reinterpret_cast<int*>(a.workspace);
-    p.workspace = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(a.workspace) + SWB_GEMM_COUNTER_BYTES);
+    if (!counters || !sums || sum_bytes < split_bytes(a.T, a.N, block_n, splits) || !counters_suffice(tiles)) return -4;
+    p.counters = reinterpret_cast<int*>(counters);
+    p.workspace = reinterpret_cast<float*>(sums);
   }
   const int clusters = (int)std::min<long>(tiles * splits, pairs);
   switch (block_n) {

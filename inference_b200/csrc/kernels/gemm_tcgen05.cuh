@@ -146,6 +146,11 @@ struct GemmArgs {
   const void* group_tiles = nullptr;     // device int4 list of row tiles, its length in group_count, at most group_max_tiles
   const int* group_count = nullptr;
   int group_max_tiles = 0;
+  // its k-splits: SWB_GEMM_COUNTER_BYTES of counters, zero between launches that are ordered, and room for the partial sums. Without
+  // them products of up to 256 rows split in `workspace`, larger ones not at all.
+  void* split_counters = nullptr;
+  void* split_sums = nullptr;
+  size_t split_bytes = 0;
 };
 
 bool gemm_bf16_takes_pairs(const GemmArgs& a);

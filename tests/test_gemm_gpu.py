@@ -187,6 +187,47 @@ def test_pairs_of_sms(T, N, K, block_n, splits):
         close(y, (z + b.float()) * gate.float()[torch.arange(T, device="cuda") // rows] + r.float())
 
 
+@pytest.mark.parametrize("T,N,K", [(300, 1024, 8192), (200, 512, 4096)])
+def test_products_split_along_k_run_beside_each_other(T, N, K):
+    """Products with k-splits on several streams at once, launched one by one and replayed from graphs: each gives the bits it gives
+    alone. Streams and captures have counters of their own, which are zero afterwards."""
+    from inference_b200 import ops
+    from inference_b200._native import kernels
+    from inference_b200.ops import gemm
+
+    assert kernels().swb_gemm_split_bytes(T, N, K, 0, 0) > 0
+    g = torch.Generator(device="cuda").manual_seed(T)
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    data = [(torch.randn(T, K, device="cuda", generator=g).bfloat16(), torch.randn(N, K, device="cuda", generator=g).bfloat16()) for _ in streams]
+    want = [ops.gemm_bf16(a, w) for a, w in data]
+    torch.cuda.synchronize()
+    graphs, outs = [], []
+    for a, w in data:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            outs.append(ops.gemm_bf16(a, w))
+        graphs.append(graph)
+    for _ in range(20):
+        got = []
+        for s, (a, w) in zip(streams, data):
+            with torch.cuda.stream(s):
+                got.append([ops.gemm_bf16(a, w) for _ in range(3)])
+        torch.cuda.synchronize()
+        assert all(torch.equal(x, y) for xs, y in zip(got, want) for x in xs)
+        for o in outs:
+            o.zero_()
+        torch.cuda.synchronize()
+        for s, graph in zip(streams, graphs):
+            with torch.cuda.stream(s):
+                graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(x, y) for x, y in zip(outs, want))
+    ops.check_status()
+    used = {k: t for k, t in gemm._SPLIT_COUNTERS.items() if k[1] in {s.cuda_stream for s in streams} and k[2] == 0}
+    assert len({t.data_ptr() for t in used.values()}) == len(streams) and not any(t.any() for t in used.values())
+    assert len({k[2] for k in gemm._SPLIT_COUNTERS}) > len(graphs)
+
+
 @pytest.mark.parametrize("T,E,top,H,f,renorm", [(1, 4, 2, 64, 24, True), (33, 8, 8, 128, 72, False), (700, 5, 3, 200, 136, True),
                                                 (2100, 64, 8, 256, 128, False), (300, 4, 2, 24, 8, True), (150, 3, 2, 72, 16, False)])
 @pytest.mark.parametrize("shared", [False, True])
