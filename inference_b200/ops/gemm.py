@@ -55,6 +55,15 @@ def split_counters(device: torch.device) -> torch.Tensor:
     return t
 
 
+def clear_split_counters() -> None:
+    """All counters of k-splits back to zero (nothing may be running)."""
+    with _SPLIT_LOCK:
+        for t in _SPLIT_COUNTERS.values():
+            t.zero_()
+    for ws in _WORKSPACES.values():
+        ws[:kernels().swb_gemm_counter_bytes()].zero_()
+
+
 def gemm_bf16(a: torch.Tensor, w: torch.Tensor, *, bias: torch.Tensor | None = None,
               residual: torch.Tensor | None = None, act: str | None = None, out: torch.Tensor | None = None,
               out_dtype: torch.dtype = torch.bfloat16, mode: int = -1, block_n: int = 0, ctas: int = 0,

@@ -8,6 +8,9 @@ import torch
 from .._native import kernels
 
 
+WAIT_TIMEOUT = 1        # status code of a bounded wait that ran out
+
+
 class KernelError(RuntimeError):
     """A native launch returned an error code, or a bounded device-side wait ran out."""
 
@@ -32,10 +35,16 @@ def require_cuda(*tensors: torch.Tensor) -> None:
 
 
 def device_status() -> list[int]:
-    """Synchronises and returns the 8-int status word (index 0 is the sticky error code)."""
+    """Synchronises and returns the 8-int status word (index 0 is the sticky error code). A launch that gave up a wait may have counted
+    only some of its k-splits: the counters are cleared then, so that later products are right."""
     out = (ctypes.c_int * 8)()
     torch.cuda.synchronize()
     kernels().swb_status_read(out)
+    if out[0] == WAIT_TIMEOUT:
+        from .gemm import clear_split_counters
+
+        clear_split_counters()
+        torch.cuda.synchronize()
     return list(out)
 
 

@@ -283,3 +283,33 @@ def test_pairs_of_sms_give_up_a_wait_together():
     y = ops.gemm_bf16(a[:, :512], w[:, :512], mode=3, block_n=256, ctas=1)
     ops.check_status()
     assert (y == 128.0).all()
+
+
+def test_counters_are_zero_again_after_a_wait_ran_out():
+    """A launch that gives up may leave its k-splits partly counted (here: counters set by hand beside one such launch). Reading its
+    status clears them, and the next split products are right."""
+    from inference_b200 import ops
+    from inference_b200._native import kernels
+    from inference_b200.ops import gemm
+
+    L = kernels()
+    K = 1 << 20
+    a, w = (torch.full((n, K), 0.5, dtype=torch.bfloat16, device="cuda") for n in (300, 256))
+    dev = a.device
+    ops.gemm_bf16(a[:, :4096], w[:, :4096])
+    ops.check_status()
+    L.swb_set_wait_limit_ns(1)
+    try:
+        ops.gemm_bf16(a, w, mode=3, block_n=256, ctas=2)
+        gemm.split_counters(dev).fill_(1)
+        ops.gemm_workspace(dev)[:L.swb_gemm_counter_bytes()].fill_(1)
+        with pytest.raises(ops.KernelError):
+            ops.check_status()
+    finally:
+        L.swb_set_wait_limit_ns(2_000_000_000)
+        L.swb_status_clear()
+    assert not gemm.split_counters(dev).any() and not ops.gemm_workspace(dev)[:L.swb_gemm_counter_bytes()].any()
+    for T in (300, 200, 64):
+        y = ops.gemm_bf16(a[:T, :8192], w[:, :8192], mode=3 if T > 64 else 1, block_n=128, ctas=2 if T > 64 else 20)
+        ops.check_status()
+        assert (y == 2048.0).all()
