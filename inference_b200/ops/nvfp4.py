@@ -370,7 +370,10 @@ class Nvfp4Linear:
         out = torch.empty((t.rows, t.cols), dtype=torch.bfloat16, device=t.packed.device)
         check(kernels().swb_dequant_nvfp4(t.packed.data_ptr(), t.scales.data_ptr(), t.global_scale, out.data_ptr(),
                                           t.rows, t.cols, stream_ptr()), "swb_dequant_nvfp4")
-        if self.keep_dense:
+        # A kept expansion is waited for, once: the kernels for few rows load a weight before they wait for the kernels in front of them. One
+        # inside a capture is not kept, since it is written by replays only.
+        if self.keep_dense and not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream().synchronize()
             self._dense = out
         return out
 
@@ -403,8 +406,8 @@ class Nvfp4Linear:
                                            ptr(self.bias), ws.data_ptr(), ws.numel(), 0, stream_ptr()),
                   "swb_gemm_nvfp4")
         else:
-            static = self._dense is not None       # expanded by an earlier call
-            out = gemm_bf16(x2, self.dense_bf16(), bias=self.bias, static_weight=static)
+            w = self.dense_bf16()
+            out = gemm_bf16(x2, w, bias=self.bias, static_weight=w is self._dense)
         return out.reshape(*lead, t.rows)
 
     __call__ = forward

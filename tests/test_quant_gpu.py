@@ -93,6 +93,52 @@ def test_expanded_weights_are_complete_before_they_are_multiplied(T):
             assert (out.float() - want).abs().max().item() < 2 ** -8 * want.abs().max().item()
 
 
+@pytest.mark.parametrize("T,N,K", [(65, 3581, 4096), (200, 5117, 4096), (256, 96, 14336), (130, 120, 14336)])
+def test_expanded_weights_are_complete_on_the_one_sm_kernels(T, N, K):
+    """The same for shapes that the two-SM kernel does not take (odd or small output widths). Their kernel for so many tokens loads a
+    weight ahead, so an expanded one goes to the kernel that waits."""
+    from inference_b200._native import kernels
+    from inference_b200.ops import quant
+
+    assert not kernels().swb_gemm_takes_pairs(T, N, K, 0, 0, -2, 0, 0)
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    qws = [quant.quantize_on_device(torch.randn(N, K, generator=g, device="cuda") * s, "Q8_0") for s in (0.05, 5.0)]
+    a = (torch.randn(T, K, generator=g, device="cuda") * 0.5).bfloat16()
+    wants = [a.float() @ quant.dequantize(q).float().t() for q in qws]
+    for _ in range(6):
+        outs = [quant.linear_quant(a, q) for q in qws]
+        for out, want in zip(outs, wants):         # one rounding to bf16 of fp32 sums
+            assert (out.float() - want).abs().max().item() < 2 ** -8 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("first,then", [(100, 5), (100, 60), (200, 100)])
+def test_a_kept_nvfp4_expansion_is_complete_before_it_is_read_ahead(first, then):
+    """Products right behind the one that expanded the weight for good. An expansion inside a capture is not kept: its buffer is written
+    by replays only."""
+    from inference_b200.ops import nvfp4 as nv
+
+    g = torch.Generator(device="cuda").manual_seed(first + then)
+    N, K = 4099, 4096
+    x = torch.randn(first, K, device="cuda", generator=g).bfloat16()
+    for s in (0.02, 2.0, 0.02, 2.0):
+        t = nv.Nvfp4Tensor.pack(torch.randn(N, K, device="cuda", generator=g) * s)
+        want = x.float() @ t.dequantize().float().T
+        torch.cuda.synchronize()
+        lin = nv.Nvfp4Linear(t, keep_dense=True)
+        whole, part = lin(x), lin(x[:then])
+        assert (whole.float() - want).abs().max().item() < 2 ** -7 * want.abs().max().item()      # the weight and the result in bf16
+        assert (part.float() - want[:then]).abs().max().item() < 2 ** -7 * want.abs().max().item()
+        assert torch.equal(lin(x), whole) and lin.dense_bf16() is lin._dense
+    lin = nv.Nvfp4Linear(t, keep_dense=True)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = lin(x)
+    assert lin._dense is None
+    graph.replay()
+    torch.cuda.synchronize()
+    assert (y.float() - want).abs().max().item() < 2 ** -7 * want.abs().max().item()
+
+
 def test_large_token_count_uses_dense_path():
     from inference_b200.ops import quant
 
