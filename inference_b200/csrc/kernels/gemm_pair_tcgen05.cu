@@ -210,33 +210,49 @@ template <int COLS, typename Load>
 __device__ __forceinline__ void store_columns(const PairParams& p, const RowMap& rows, int col0, uint8_t* slab, int lane, Load load) {
   const bool pairs = gemm_act_pairs(p.act);
   const long long my_row = rows(lane);
-  if (p.out_fp32) {      // 128 contiguous bytes per thread and load
+  const int swz = lane & 7;
+  const int sub = lane >> 3, chunk = lane & 7;           // coalesced phases: four rows at a time, eight lanes each
+  if (p.out_fp32) {      // a slab holds 32 rows x 32 fp32 of D, 16-byte chunk c of row r at c ^ (r & 7)
 #pragma unroll 1
     for (int c = 0; c < COLS; c += 32) {
+      const int a0 = col0 + c;
+      if (a0 >= p.N) break;
       float v[32];
       __syncwarp();
       load(c, v);
-      float* out = reinterpret_cast<float*>(p.out) + my_row * p.ldd + col0 + c;
+      if (p.bias) {
 #pragma unroll
-      for (int j = 0; j < 32; j += 4) {
-        if (my_row < 0 || col0 + c + j >= p.N) continue;
+        for (int j = 0; j < 32; j += 8)
+          if (a0 + j < p.N) add_bf16x8(v + j, __ldg(reinterpret_cast<const uint4*>(p.bias + a0 + j)));
+      }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (p.bias) v[j + i] += __bfloat162float(p.bias[col0 + c + j + i]);
-          v[j + i] = pair_act(v[j + i], p);
-          if (p.residual) v[j + i] += __bfloat162float(p.residual[my_row * p.ld_res + col0 + c + j + i]);
+      for (int j = 0; j < 8; ++j) {
+        float4 f = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        if (p.act != SWB_ACT_NONE) f = make_float4(pair_act(f.x, p), pair_act(f.y, p), pair_act(f.z, p), pair_act(f.w, p));
+        *reinterpret_cast<float4*>(slab + lane * 128 + ((j ^ swz) << 4)) = f;
+      }
+      __syncwarp();
+      const int d = a0 + chunk * 4;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = i * 4 + sub;
+        const long long row = rows(r);
+        if (row < 0 || d >= p.N) continue;
+        float4 f = *reinterpret_cast<const float4*>(slab + r * 128 + ((chunk ^ (r & 7)) << 4));
+        if (p.residual) {
+          const uint2 u = *reinterpret_cast<const uint2*>(p.residual + row * p.ld_res + d);
+          f.x += __uint_as_float(u.x << 16), f.y += __uint_as_float(u.x & 0xffff0000u);
+          f.z += __uint_as_float(u.y << 16), f.w += __uint_as_float(u.y & 0xffff0000u);
         }
-        *reinterpret_cast<float4*>(out + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + row * p.ldd + d) = f;
       }
     }
     return;
   }
   // A slab holds 32 rows x 64 bf16 of D; its 16-byte chunk c of row r lies at c ^ (r & 7).
   uint8_t* my_slab = slab + lane * 128;
-  const int swz = lane & 7;
   const int step = pairs ? 128 : 64;
   const int width = pairs ? p.N / 2 : p.N;              // columns of D
-  const int sub = lane >> 3, chunk = lane & 7;           // coalesced phases: four rows at a time, eight lanes each
   const bf16* gate = p.gate ? p.gate + (long long)(my_row < 0 ? 0 : (int)my_row / p.rows_per_gate) * p.ld_gate : nullptr;
 #pragma unroll 1
   for (int s = 0; s < COLS; s += step) {

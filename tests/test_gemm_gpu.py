@@ -178,6 +178,8 @@ def test_pairs_of_sms(T, N, K, block_n, splits):
     ops.gemm_bf16(a, w, residual=out, out=out, **kw)
     close(out, z + r.float())
     torch.testing.assert_close(ops.gemm_bf16(a, w, out_dtype=torch.float32, **kw), z, rtol=1e-5, atol=1e-5)
+    y = ops.gemm_bf16(a, w, bias=b, residual=r, act="silu", out_dtype=torch.float32, **kw)
+    torch.testing.assert_close(y, torch.nn.functional.silu(z + b.float()) + r.float(), rtol=1e-5, atol=1e-4)
     if N % 16 == 0:
         close(ops.gemm_bf16(a, w, act="swiglu_pairs", **kw), torch.nn.functional.silu(z[:, 0::2]) * z[:, 1::2])
     if not block_n:
