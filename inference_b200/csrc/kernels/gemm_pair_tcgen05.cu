@@ -191,6 +191,11 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+__device__ __forceinline__ void copy_async16(void* smem_dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Where the rows of this warp's 32 TMEM lanes lie in D (and in the residual): -1 = no such row.
 struct RowMap {
   const PairParams& p;
@@ -259,15 +264,14 @@ __device__ __forceinline__ void store_columns(const PairParams& p, const RowMap&
     const int d0 = pairs ? (col0 + s) >> 1 : col0 + s;   // first column of D in this slab
     if (d0 >= width) break;
     const bool in = d0 + chunk * 8 < width && chunk * 8 < (pairs ? (COLS - s) / 2 : COLS - s);
-    if (p.residual) {
+    if (p.residual) {      // copies straight to the slab: all on their way at a time, without registers
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int r = i * 4 + sub;
         const long long row = rows(r);
-        if (row >= 0 && in)
-          *reinterpret_cast<uint4*>(slab + r * 128 + ((chunk ^ (r & 7)) << 4)) =
-              *reinterpret_cast<const uint4*>(p.residual + row * p.ld_res + d0 + chunk * 8);
+        if (row >= 0 && in) copy_async16(slab + r * 128 + ((chunk ^ (r & 7)) << 4), p.residual + row * p.ld_res + d0 + chunk * 8);
       }
+      copy_async_wait();
       __syncwarp();
     }
 #pragma unroll 1
@@ -318,9 +322,11 @@ __device__ __forceinline__ void store_columns(const PairParams& p, const RowMap&
     }
     __syncwarp();
     bf16* out = reinterpret_cast<bf16*>(p.out) + d0 + chunk * 8;
+    int first = sub;
+    asm volatile("" : "+r"(first));      // places of rows are computed again: kept from the residual's copies they would spill
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int r = i * 4 + sub;
+      const int r = i * 4 + first;
       const long long row = rows(r);
       if (row >= 0 && in)
         *reinterpret_cast<uint4*>(out + row * p.ldd) = *reinterpret_cast<const uint4*>(slab + r * 128 + ((chunk ^ (r & 7)) << 4));
