@@ -201,7 +201,8 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
     sig("swb_gemm_bf16_normed", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                  c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p])
     sig("swb_gemm_gated_supported", [c_int, c_int, c_int])
-    sig("swb_gemm_takes_pairs", [c_int] * 8)
+    sig("swb_gemm_takes_pairs", [c_int] * 10)
+    sig("swb_gemm_gated_in_pairs", [c_int, c_int, c_int])
     sig("swb_gemm_split_bytes", [c_int] * 5, c_size_t)
     sig("swb_gemm_counter_bytes", [], c_size_t)
     sig("swb_stream_capture_id", [c_void_p], ctypes.c_ulonglong)

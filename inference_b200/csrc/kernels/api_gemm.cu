@@ -309,20 +309,35 @@ int swb_gemm_peer_max_ctas(void) { return swb::SWB_PEER_MAX_CTAS; }
 
 int swb_gemm_gated_supported(int T, int N, int K) { return swb::gemm_bf16_gated_supported(T, N, K); }
 
-// 1 when a product of these sizes with contiguous, aligned rows goes to the two-SM kernel (host only; ldd as the activation has it).
-int swb_gemm_takes_pairs(int T, int N, int K, int act, int out_fp32, int force_mode, int force_block_n, int force_ctas) {
+// 1 when a product of these sizes with contiguous, aligned rows and scratch for k-splits goes to the two-SM kernel (host only).
+int swb_gemm_takes_pairs(int T, int N, int K, int bias, int residual, int act, int out_fp32, int force_mode, int force_block_n, int force_ctas) {
   swb::GemmArgs a{};
   a.lda = a.ldw = K;
   a.ldd = swb::gemm_act_pairs(act) ? N / 2 : N;
   a.T = T;
   a.N = N;
   a.K = K;
+  alignas(16) static const char some[16] = {};
+  a.bias = bias ? some : nullptr;
+  a.residual = residual ? some : nullptr;
+  a.ld_res = N;
   a.act = act;
   a.out_fp32 = out_fp32;
   a.force_mode = force_mode;
   a.force_block_n = force_block_n;
   a.force_ctas = force_ctas;
+  a.split_counters = &a;
+  a.split_bytes = swb::GEMM_SPLIT_BYTES_MAX;
   return swb::gemm_bf16_takes_pairs(a) ? 1 : 0;
+}
+
+// 1 when a gated projection (N accumulator columns in pairs) of more than 64 rows is one launch on the two-SM kernel; else the plain product
+// and a pass over its T x N outputs (read, and half written, at 6 TB/s; its launch costs what the gated epilogue adds) are faster: 257 rows
+// of 5632 x 2048 take 23.7 us so and 25.4 in one launch, 400 rows 37.3 and 25.8.
+int swb_gemm_gated_in_pairs(int T, int N, int K) {
+  if (T <= 64 || N < 128 || N % 16) return 0;
+  const double pass_us = 3e-6 * T * N / 6.0;
+  return swb::gemm_bf16_prefers_one_sm(T, N, K, swb::GEMM_SPLIT_BYTES_MAX, 0.0, pass_us) ? 0 : 1;
 }
 
 // Bytes of partial sums that a product above 64 rows takes on the two-SM kernel, 0 without k-splits. block_n, splits: 0 = by its plan.

@@ -27,10 +27,11 @@ struct PairParams {
 };
 
 bool gemm_pair_accepts(const GemmArgs& a);
-// Tile width and number of k-splits for a plain product whose partial sums may take sum_bytes.
-void gemm_pair_plan(int T, int N, int K, size_t sum_bytes, int* block_n, int* splits);
+// Tile width and number of k-splits for a plain product whose partial sums may take sum_bytes. Returns its estimated microseconds.
+double gemm_pair_plan(int T, int N, int K, size_t sum_bytes, int* block_n, int* splits);
 // Bytes of partial sums of a product (block_n, splits: 0 = by the plan); 0 = no k-splits.
 size_t gemm_pair_split_bytes(int T, int N, int K, int block_n, int splits);
+constexpr size_t GEMM_SPLIT_BYTES_MAX = (size_t)96 << 20;
 // block_n, splits: 0 = by the plan.
 int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t stream);
 

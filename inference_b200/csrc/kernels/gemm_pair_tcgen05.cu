@@ -556,7 +556,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const PairParams& 
   return launch_kernel(kern, dim3(2 * clusters), dim3(THREADS), PairCfg<BN>::SMEM_BYTES, stream, ta, tb, p);
 }
 
-// Estimated microseconds of a plan, without the 8 us that all plans share. Fitted to sweeps of every tile width and up to six splits over
+// Estimated microseconds of a plan, without what gemm_pair_plan adds to the best one. Fitted to sweeps of every tile width and up to six splits over
 // token counts 100..8000 and the projections of an 8B decoder and a 12B image transformer. A k-block costs more the fuller the chip
 // is (operand traffic, power): 0.29 us at BN = 256 on half of the pairs, 0.35 us on all of them. Narrower tiles move the same A for less
 // work but fill a last wave better: 975 x 9216 x 3072 takes 41.8 us at 256, 45.9 at 192, 52.3 at 128; 700 x 4096 x 4096 takes 27.2, 22.5, 32.1.
@@ -573,8 +573,6 @@ double plan_cost(int bn, int splits, long tiles, int kblocks, int pairs) {
 
 namespace {
 
-constexpr size_t SPLIT_BYTES_MAX = (size_t)96 << 20;
-
 size_t split_bytes(int T, int N, int bn, int splits) {
   const size_t tiles = (size_t)((T + 2 * BM - 1) / (2 * BM)) * ((N + bn - 1) / bn);
   return tiles * 2 * splits * BM * bn * sizeof(float);
@@ -583,7 +581,7 @@ bool counters_suffice(long tiles) { return tiles * 2 * EPI_WARPS * (long)sizeof(
 
 }  // namespace
 
-void gemm_pair_plan(int T, int N, int K, size_t sum_bytes, int* block_n, int* splits) {
+double gemm_pair_plan(int T, int N, int K, size_t sum_bytes, int* block_n, int* splits) {
   const int pairs = device_sm_count() / 2;
   const int kblocks = (K + BK - 1) / BK;
   const long tm = (T + 2 * BM - 1) / (2 * BM);
@@ -597,12 +595,13 @@ void gemm_pair_plan(int T, int N, int K, size_t sum_bytes, int* block_n, int* sp
       if (c < best) best = c, *block_n = bn, *splits = s;
     }
   }
+  return best + 3.35 + 2.89 * *block_n / 256.0;      // launch, first loads and the last tile's epilogue
 }
 
 size_t gemm_pair_split_bytes(int T, int N, int K, int block_n, int splits) {
   if (block_n <= 0 && N > 32) {
     int s = 1;
-    gemm_pair_plan(T, N, K, SPLIT_BYTES_MAX, &block_n, &s);
+    gemm_pair_plan(T, N, K, GEMM_SPLIT_BYTES_MAX, &block_n, &s);
     if (splits <= 0) splits = s;
   }
   return splits > 1 ? split_bytes(T, N, block_n, splits) : 0;
@@ -678,7 +677,7 @@ int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t st
   if (!counters && a.workspace && a.workspace_bytes > SWB_GEMM_COUNTER_BYTES && !a.gate && (a.T <= 256 || a.force_mode == 3)) {
     counters = a.workspace;
     sums = reinterpret_cast<uint8_t*>(a.workspace) + SWB_GEMM_COUNTER_BYTES;
-    sum_bytes = std::min(a.workspace_bytes - SWB_GEMM_COUNTER_BYTES, SPLIT_BYTES_MAX);
+    sum_bytes = std::min(a.workspace_bytes - SWB_GEMM_COUNTER_BYTES, GEMM_SPLIT_BYTES_MAX);
   }
   if (a.conv_c || a.group_tiles) sum_bytes = 0;
   if (block_n <= 0) {

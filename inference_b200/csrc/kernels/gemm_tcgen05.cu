@@ -774,10 +774,53 @@ int gemm_bf16_gated_supported(int T, int N, int K) {
          (N % 2) == 0;
 }
 
-// True for products that go to the two-SM kernel. A caller's own tile width or number of CTAs means the one-SM kernels.
+namespace {
+
+// Tile width of the tokens-as-M kernel, and how full its waves of tiles are. With few row tiles a 128-wide tile can fill the SMs better
+// than a 256-wide one does, at roughly 0.85 of its per-SM rate.
+int whole_tile_width(int T, int N, int sms, double* fill, long* waves) {
+  const long tm = (T + BM - 1) / BM;
+  auto fill_of = [&](int bn) {
+    const long tiles = tm * ((N + bn - 1) / bn);
+    *waves = (tiles + sms - 1) / sms;
+    return (double)tiles / (double)(*waves * sms);
+  };
+  int bn = N >= 256 ? 256 : N >= 128 ? 128 : N >= 64 ? 64 : N >= 32 ? 32 : 16;
+  if (bn == 256 && fill_of(128) * 0.85 > fill_of(256) * 1.02) bn = 128;
+  *fill = fill_of(bn);
+  return bn;
+}
+
+// Estimated microseconds of the tokens-as-M kernel. epilogue_us: what each 256-wide tile's epilogue takes longer than on the two-SM
+// kernel, which has twice the warps for it.
+double whole_tile_cost(int T, int N, int K, double epilogue_us, int sms) {
+  double fill;
+  long waves;
+  const int bn = whole_tile_width(T, N, sms, &fill, &waves);
+  const double t = bn == 256 ? 0.32 + 0.106 * fill : 0.242 + 0.035 * fill;
+  return waves * ((K + BK - 1) / BK * t + 0.5 + epilogue_us * bn / 256.0) + 3.89 + 1.92 * bn / 256.0;
+}
+
+}  // namespace
+
+bool gemm_bf16_prefers_one_sm(int T, int N, int K, size_t split_bytes, double epilogue_us, double extra_us) {
+  int bn, splits;
+  return T > 256 && N >= 128 &&
+         whole_tile_cost(T, N, K, epilogue_us, device_sm_count()) + extra_us < gemm_pair_plan(T, N, K, split_bytes, &bn, &splits);
+}
+
+// True for products that go to the two-SM kernel. Up to 256 rows it is the faster one throughout (6144 x 4096 at 65 and 256 rows: 21 us against
+// 30 and 62 on one SM), and for fp32 rows. Above, tiles of 128 rows can fill the chip where those of 256 do not: 257..384 rows x 12288 x
+// 3072 are 144 one-SM tiles in one wave (28 us) but 96 two-SM tiles in two (31 us); 400 rows 48 and 33 us. Bias and activation
+// make up for it (the same product with both: 56 us on one SM, 50 on pairs). Both estimates were fitted to 890 products of 257..4000
+// rows, bare, with residual, bias or SiLU: no choice loses more than 8 % to the other kernel, 0.1 % on average. Gated pairs are for the two-SM kernel alone:
+// callers ask gemm_bf16_prefers_one_sm first. A caller's own tile width or number of CTAs means the one-SM kernels.
 bool gemm_bf16_takes_pairs(const GemmArgs& a) {
   if (a.gate || a.group_tiles || a.force_mode == 3) return true;
-  return a.force_mode < 0 && a.force_ctas == 0 && a.force_block_n == 0 && a.T > 64 && a.N >= 128 && gemm_pair_accepts(a);
+  if (a.force_mode >= 0 || a.force_ctas != 0 || a.force_block_n != 0 || a.T <= 64 || a.N < 128 || !gemm_pair_accepts(a)) return false;
+  if (gemm_act_pairs(a.act) || a.out_fp32) return true;
+  const double epilogue_us = (a.bias ? 7.45 : 0.0) + (a.act != SWB_ACT_NONE ? 8.6 : 0.0);
+  return !gemm_bf16_prefers_one_sm(a.T, a.N, a.K, a.split_counters ? a.split_bytes : 0, epilogue_us, 0.0);
 }
 
 int gemm_bf16_launch(const GemmArgs& a, cudaStream_t stream) {
@@ -879,18 +922,9 @@ int gemm_bf16_launch(const GemmArgs& a, cudaStream_t stream) {
     if (r) return r;
     p.vec_ok = 0;
   } else {
-    block_n = a.N >= 256 ? 256 : a.N >= 128 ? 128 : a.N >= 64 ? 64 : a.N >= 32 ? 32 : 16;
-    if (block_n == 256) {
-      // wave quantisation: with few row tiles a 128-wide tile can fill the SMs better than a 256-wide one does,
-      // at roughly 0.85 of its per-SM rate
-      const long tm = (a.T + BM - 1) / BM;
-      auto fill = [&](int bn) {
-        const long tiles = tm * ((a.N + bn - 1) / bn);
-        const long waves = (tiles + sms - 1) / sms;
-        return (double)tiles / (double)(waves * sms);
-      };
-      if (fill(128) * 0.85 > fill(256) * 1.02) block_n = 128;
-    }
+    double fill;
+    long waves;
+    block_n = whole_tile_width(a.T, a.N, sms, &fill, &waves);
     if (a.force_block_n > 0) block_n = a.force_block_n;
     p.M = a.T;
     p.N = a.N;

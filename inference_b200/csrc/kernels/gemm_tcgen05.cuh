@@ -154,6 +154,9 @@ struct GemmArgs {
 };
 
 bool gemm_bf16_takes_pairs(const GemmArgs& a);
+// True when a product of more than 256 rows is faster on the tokens-as-M kernel, whose epilogue takes epilogue_us longer per 256-wide
+// tile and which leaves extra_us of work to others.
+bool gemm_bf16_prefers_one_sm(int T, int N, int K, size_t split_bytes, double epilogue_us, double extra_us);
 int gemm_bf16_launch(const GemmArgs& a, cudaStream_t stream);
 int gemm_bf16_gated_supported(int T, int N, int K);
 int gemm_decode_cluster_supported(int T);

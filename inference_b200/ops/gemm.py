@@ -185,13 +185,14 @@ def gated_fused(T: int, N: int, K: int) -> bool:
 
 def gated_epilogue(x: torch.Tensor, w_pairs: torch.Tensor, out: torch.Tensor | None = None) -> bool:
     """True when linear_gated of x [T, K] is one launch. Above the decode kernel's 64 tokens the two-SM kernel writes whole
-    16-byte pieces of the half-wide output (8000 tokens of an 8B decoder's layer: 138 us less than the separate pass)."""
+    16-byte pieces of the half-wide output (8000 tokens of an 8B decoder's layer: 138 us less than the separate pass), unless the plain
+    product is so much faster on single SMs that it pays for the pass."""
     T, K = x.shape
     N = w_pairs.shape[0]
     if gated_fused(T, N, K):
         return True
     rows_ok = out is None or (out.stride(-2) % 8 == 0 and out.data_ptr() % 16 == 0)
-    return T > 64 and N >= 128 and N % 16 == 0 and rows_ok
+    return rows_ok and bool(kernels().swb_gemm_gated_in_pairs(T, N, K))
 
 
 def linear_gated(x: torch.Tensor, w_pairs: torch.Tensor, act: str = "silu", out: torch.Tensor | None = None) -> torch.Tensor:

@@ -100,7 +100,7 @@ def test_expanded_weights_are_complete_on_the_one_sm_kernels(T, N, K):
     from inference_b200._native import kernels
     from inference_b200.ops import quant
 
-    assert not kernels().swb_gemm_takes_pairs(T, N, K, 0, 0, -2, 0, 0)
+    assert not kernels().swb_gemm_takes_pairs(T, N, K, 0, 0, 0, 0, -2, 0, 0)
     g = torch.Generator(device="cuda").manual_seed(T + N)
     qws = [quant.quantize_on_device(torch.randn(N, K, generator=g, device="cuda") * s, "Q8_0") for s in (0.05, 5.0)]
     a = (torch.randn(T, K, generator=g, device="cuda") * 0.5).bfloat16()
