@@ -3,7 +3,6 @@ from __future__ import annotations
 
 import functools
 import threading
-from collections import OrderedDict
 
 import torch
 
@@ -17,8 +16,8 @@ WORKSPACE_BYTES = 64 * 1024 + (96 << 20)
 
 
 def gemm_workspace(device: torch.device, slot: int = 0) -> torch.Tensor:
-    """Per-(device, slot) split-K scratch. Launches sharing a slot must be ordered on one stream: products of up to 64 rows whose output
-    is wider than the decode kernel takes, of 65 to 256 rows that the two-SM kernel does not take, and packed weights."""
+    """Per-(device, slot) split-K scratch. Launches sharing a slot must be ordered on one stream: products of up to 256 rows without gate,
+    and packed weights."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
     key = (idx, slot)
     ws = _WORKSPACES.get(key)
@@ -28,8 +27,8 @@ def gemm_workspace(device: torch.device, slot: int = 0) -> torch.Tensor:
     return ws
 
 
-_SPLIT_COUNTERS: OrderedDict[tuple[int, int, int], torch.Tensor] = OrderedDict()
-_SPLIT_COUNTERS_MAX = 32        # streams and captures in use at a time, 64 KB each
+_SPLIT_COUNTERS: dict[tuple[int, int, int], torch.Tensor] = {}
+_SPLIT_COUNTERS_MAX = 32        # streams and captures, 64 KB each; the oldest goes first
 _SPLIT_LOCK = threading.Lock()
 
 
@@ -38,20 +37,20 @@ def _split_bytes(T: int, N: int, K: int, block_n: int, splits: int) -> int:
     return kernels().swb_gemm_split_bytes(T, N, K, block_n, splits)
 
 
-def split_counters(device: torch.device) -> torch.Tensor:
+def split_counters(device: torch.device, stream: int | None = None) -> torch.Tensor:
     """Zeroed counters for the k-splits of the two-SM kernel, which leaves them zero. One buffer for each stream, and for each stream of
     each graph capture: products that run at the same time share none, and a graph's buffer lies in its own memory pool and is
     cleared by every replay."""
-    stream = stream_ptr()
-    key = (device.index if device.index is not None else torch.cuda.current_device(), stream, kernels().swb_stream_capture_id(stream))
-    with _SPLIT_LOCK:
-        t = _SPLIT_COUNTERS.get(key)
-        if t is None:
-            t = _SPLIT_COUNTERS[key] = torch.zeros(kernels().swb_gemm_counter_bytes(), dtype=torch.uint8, device=device)
-            if len(_SPLIT_COUNTERS) > _SPLIT_COUNTERS_MAX:      # its memory goes back to its own stream, behind what still uses it
-                _SPLIT_COUNTERS.popitem(last=False)
-        else:
-            _SPLIT_COUNTERS.move_to_end(key)
+    stream = stream_ptr() if stream is None else stream
+    capture = kernels().swb_stream_capture_id(stream) if torch.cuda.is_current_stream_capturing() else 0
+    key = (device.index if device.index is not None else torch.cuda.current_device(), stream, capture)
+    t = _SPLIT_COUNTERS.get(key)
+    if t is None:
+        t = torch.zeros(kernels().swb_gemm_counter_bytes(), dtype=torch.uint8, device=device)
+        with _SPLIT_LOCK:
+            while len(_SPLIT_COUNTERS) >= _SPLIT_COUNTERS_MAX:      # its memory goes back to its own stream, behind what still uses it
+                del _SPLIT_COUNTERS[next(iter(_SPLIT_COUNTERS))]
+            _SPLIT_COUNTERS[key] = t
     return t
 
 
@@ -92,26 +91,28 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, *, bias: torch.Tensor | None = N
         assert bias.dtype == torch.bfloat16 and bias.numel() == N and bias.is_contiguous()
     if workspace is None:
         workspace = gemm_workspace(a.device)
-    # the two-SM kernel's partial sums are the call's own, so that it may run beside others; ctas is its number of splits in mode 3
+    stream = stream_ptr()
+    # Above 256 rows (and with a gate) the partial sums of k-splits are the call's own, so that it may run beside others. ctas is the
+    # number of splits in mode 3.
     splits = (None, None, 0)
-    if mode == 3 or (mode < 0 and block_n == 0 and ctas == 0 and (T > 64 or gate is not None)):
+    if (T > 256 or gate is not None) and (mode == 3 or (mode < 0 and block_n == 0 and ctas == 0)):
         need = _split_bytes(T, N, K, block_n, ctas)
         if need:
-            sums = torch.empty(need, dtype=torch.uint8, device=a.device)
-            splits = (split_counters(a.device).data_ptr(), sums.data_ptr(), need)
+            sums, counters = torch.empty(need, dtype=torch.uint8, device=a.device), split_counters(a.device, stream)
+            splits = (counters.data_ptr(), sums.data_ptr(), need)
     if gate is not None:
         rows = rows_per_gate or T
         assert gate.dtype == torch.bfloat16 and gate.dim() == 2 and gate.shape[1] == N and gate.stride(1) == 1
         assert rows * gate.shape[0] >= T and mode < 0 and block_n == 0 and ctas == 0
         rc = kernels().swb_gemm_bf16_gated(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), T, N, K,
                                            ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0,
-                                           gate.data_ptr(), gate.stride(0), rows, ACT[act], *splits, stream_ptr())
+                                           gate.data_ptr(), gate.stride(0), rows, ACT[act], *splits, stream)
         check(rc, "swb_gemm_bf16_gated")
         return out
     rc = kernels().swb_gemm_bf16_act(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0),
                                      T, N, K, ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0,
                                      ACT[act], *act_params, 1 if out.dtype == torch.float32 else 0, workspace.data_ptr(),
-                                     workspace.numel(), *splits, mode, block_n, ctas, stream_ptr())
+                                     workspace.numel(), *splits, mode, block_n, ctas, stream)
     check(rc, "swb_gemm_bf16")
     return out
 

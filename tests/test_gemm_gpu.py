@@ -189,7 +189,7 @@ def test_pairs_of_sms(T, N, K, block_n, splits):
         close(y, (z + b.float()) * gate.float()[torch.arange(T, device="cuda") // rows] + r.float())
 
 
-@pytest.mark.parametrize("T,N,K", [(300, 1024, 8192), (200, 512, 4096)])
+@pytest.mark.parametrize("T,N,K", [(300, 1024, 8192), (700, 512, 4096)])
 def test_products_split_along_k_run_beside_each_other(T, N, K):
     """Products with k-splits on several streams at once, launched one by one and replayed from graphs: each gives the bits it gives
     alone. Streams and captures have counters of their own, which are zero afterwards."""
