@@ -209,7 +209,7 @@ class VaeDecoderGpu:
         return self.load_state_dict(random_vae_weights(self.cfg, seed, device=self.device))
 
     def _conv3(self, x, name, residual=None):
-        self.launches += 1 if ops.conv3x3_supported(x, self.w[name + ".weight"].shape[0]) else 2
+        self.launches += 1 if ops.conv3x3_implicit(x, self.w[name + ".weight"].shape[0]) else 2
         return ops.conv3x3_nhwc(x, self.w[name + ".weight"], self.w[name + ".bias"], residual)
 
     def _conv1(self, x, name, residual=None):

@@ -70,12 +70,19 @@ def conv3x3_supported(x: torch.Tensor, cout: int = 8) -> bool:
     return C % 64 == 0 and (cout % 8 == 0 or ((H * W) % 128 == 0 and (W % 128 == 0 or 128 % W == 0)))
 
 
+def conv3x3_implicit(x: torch.Tensor, cout: int = 8) -> bool:
+    """True when conv3x3_nhwc writes no patch matrix. Up to 64 pixels it does: the matrix is small, and its product runs on the decode kernel,
+    which splits the reduction over the chip. 8 x 8 pixels, 512 -> 512 channels take 7.9 us so and 24.9 as one row of implicit
+    tiles; 6 x 12 pixels 45 and 25."""
+    return x.shape[0] * x.shape[1] * x.shape[2] > 64 and conv3x3_supported(x, cout)
+
+
 def conv3x3_nhwc(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, residual: torch.Tensor | None = None,
                  act: str | None = None) -> torch.Tensor:
     """3x3 convolution (stride 1, zero padding 1) of x [N, H, W, C] bf16 with w [Cout, 9 * C] (columns ordered ky, kx,
     c) -> [N, H, W, Cout], bias / activation / residual [N, H, W, Cout] in the epilogue. Implicit GEMM on the tcgen05
     kernel: the nine shifted views of x are fetched by TMA, no patch matrix is materialised. Shapes outside
-    `conv3x3_supported` take the patch-gather + GEMM path."""
+    `conv3x3_implicit` take the patch-gather + GEMM path."""
     from .gemm import ACT, gemm_bf16
 
     require_cuda(x, w)
@@ -85,7 +92,7 @@ def conv3x3_nhwc(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = N
     res2 = residual.reshape(N * H * W, Cout) if residual is not None else None
     rows_ok = ((bias is None or bias.data_ptr() % 16 == 0) and
                (res2 is None or (res2.data_ptr() % 16 == 0 and res2.stride(0) % 8 == 0)))
-    if not conv3x3_supported(x, Cout if rows_ok else 1) or os.environ.get("SWB_CONV3X3", "implicit") == "im2col":
+    if not conv3x3_implicit(x, Cout if rows_ok else 1) or os.environ.get("SWB_CONV3X3", "implicit") == "im2col":
         return gemm_bf16(im2col3x3_nhwc(x), w, bias=bias, residual=res2, act=act).view(N, H, W, Cout)
     out = torch.empty((N * H * W, Cout), dtype=torch.bfloat16, device=x.device)
     if res2 is not None:

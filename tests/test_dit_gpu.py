@@ -175,7 +175,8 @@ def test_implicit_conv3x3_matches_conv2d(shape, monkeypatch):
     assert (out.float() - refn).abs().max().item() < 0.03 * max(1.0, refn.abs().max().item())
 
 
-@pytest.mark.parametrize("shape", [(1, 5, 7, 64, 8), (2, 19, 13, 64, 72), (1, 38, 26, 128, 128), (3, 9, 130, 64, 136), (1, 152, 104, 64, 256)])
+@pytest.mark.parametrize("shape", [(1, 5, 7, 64, 8), (2, 19, 13, 64, 72), (1, 38, 26, 128, 128), (3, 9, 130, 64, 136), (1, 152, 104, 64, 256), (1, 8, 8, 128, 64),
+                                   (1, 5, 13, 128, 64)])
 def test_implicit_conv3x3_of_any_image_size(shape):
     """Boxes of pixels that stick out of the image, an odd number of boxes, output widths between the tile widths. The tolerance: two
     roundings to bf16 (2^-9 each) of the largest result, and fp32 sums of 9 C products."""

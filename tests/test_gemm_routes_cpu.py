@@ -1,5 +1,6 @@
 """Which kernel a product goes to, by the library's own rule (host code; no launch)."""
 import pytest
+import torch
 
 from inference_b200._native import kernels
 
@@ -41,3 +42,12 @@ def test_gated_projections_pay_for_a_pass_only_where_that_is_faster():
     assert not any(fused(T, 2 * F, K) for T, F, K in [(257, 5632, 2048), (384, 5632, 2048), (257, 11008, 4096), (384, 11008, 4096), (64, 1024, 4096)])
     assert all(fused(T, 2 * F, K) for T, F, K in [(65, 14336, 4096), (256, 5632, 2048), (400, 5632, 2048), (900, 11008, 4096), (900, 14336, 4096),
                                                   (300, 8192, 2048), (300, 1024, 2048), (8000, 14336, 4096), (300, 64, 512)])
+
+
+def test_convolutions_of_few_pixels_go_through_a_patch_matrix():
+    from inference_b200 import ops
+
+    def implicit(n, h, w, c, cout):
+        return ops.conv3x3_implicit(torch.empty(n, h, w, c, device="meta"), cout)
+    assert not any(implicit(*s) for s in [(1, 8, 8, 512, 512), (1, 1, 1, 64, 64), (4, 4, 4, 128, 128), (1, 9, 9, 32, 64), (1, 9, 9, 64, 4)])
+    assert all(implicit(*s) for s in [(1, 5, 13, 512, 512), (1, 6, 12, 64, 8), (2, 6, 6, 64, 72), (1, 8, 16, 64, 3), (1, 152, 104, 512, 512)])
