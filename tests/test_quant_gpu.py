@@ -57,9 +57,9 @@ def test_q4k_matvec_kernel_matches_reference_and_the_tensor_core_path(T, N, K):
     assert (out2.float().cpu() - ref2).abs().max().item() < 2e-2 * max(1.0, ref2.abs().max().item())
 
 
-@pytest.mark.parametrize("T,N,K", [(8, 37, 18432), (4, 4801, 2304), (1, 9473, 512), (6, 2369, 256)])
+@pytest.mark.parametrize("T,N,K", [(8, 37, 18432), (4, 4801, 2304), (1, 9473, 512), (6, 2369, 256), (5, 2368, 768), (3, 1, 4352), (8, 130, 256)])
 def test_q4k_matvec_pairs_of_rows(T, N, K):
-    """A last pair of one row, slices that end inside a row, several pairs per warp, the largest activations. Against 64 bits with the
+    """A last pair of one row, slices that end inside a row, several pairs per warp, a row per warp and its limit, the largest activations. Against 64 bits with the
     activations rounded as the kernel rounds them (int8 per block of 32), so what is left are fp32 sums and the rounding to bf16."""
     from inference_b200 import ops
     from inference_b200.ops import quant
