@@ -750,8 +750,9 @@ __global__ void __launch_bounds__(256) embedding_kernel(const long long* __restr
   *reinterpret_cast<uint4*>(out + (size_t)t * H + v * 8) = u;
 }
 
-// out = a + gate * b (gate per batch row-vector), or out = a + b when gate == nullptr.
-__global__ void __launch_bounds__(256) gated_residual_kernel(const bf16* __restrict__ a, const bf16* __restrict__ b,
+// out = a + gate * b (gate per batch row-vector), or out = a + b when gate == nullptr. b is bf16 or fp32.
+template <typename B>
+__global__ void __launch_bounds__(256) gated_residual_kernel(const bf16* __restrict__ a, const B* __restrict__ b,
                                                             const bf16* __restrict__ gate, int ld_gate,
                                                             int rows_per_batch, bf16* out, int T, int H) {
   pdl_launch_dependents();
@@ -763,7 +764,7 @@ __global__ void __launch_bounds__(256) gated_residual_kernel(const bf16* __restr
   const int v = (int)(idx % nvec);
   float fa[8], fb[8], o[8];
   unpack8(*reinterpret_cast<const uint4*>(a + (size_t)t * H + v * 8), fa);
-  unpack8(*reinterpret_cast<const uint4*>(b + (size_t)t * H + v * 8), fb);
+  load_row8(b + (size_t)t * H + v * 8, fb);
   if (gate) {
     float g[8];
     const int bi = rows_per_batch > 0 ? t / rows_per_batch : 0;
@@ -975,14 +976,18 @@ int swb_embedding(const long long* ids, const void* table, void* out, int T, int
   return last_err();
 }
 
-int swb_gated_residual(const void* a, const void* b, const void* gate, int ld_gate, int rows_per_batch, void* out,
+int swb_gated_residual(const void* a, const void* b, int b_fp32, const void* gate, int ld_gate, int rows_per_batch, void* out,
                        int T, int H, void* stream) {
   using namespace swb;
   if (T <= 0) return 0;
   if (H % 8 != 0 || (gate && ld_gate % 8 != 0)) return -3;
-  const long long n = (long long)T * (H / 8);
-  launch_rc = launch_kernel(gated_residual_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const bf16*>(a), reinterpret_cast<const bf16*>(b), reinterpret_cast<const bf16*>(gate), ld_gate,
-      rows_per_batch, reinterpret_cast<bf16*>(out), T, H);
+  const dim3 grid((unsigned)(((long long)T * (H / 8) + 255) / 256));
+  auto launch = [&](auto kernel, auto* rows) {
+    launch_rc = launch_kernel(kernel, grid, dim3(256), 0, reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const bf16*>(a), rows,
+                              reinterpret_cast<const bf16*>(gate), ld_gate, rows_per_batch, reinterpret_cast<bf16*>(out), T, H);
+  };
+  if (b_fp32) launch(gated_residual_kernel<float>, reinterpret_cast<const float*>(b));
+  else launch(gated_residual_kernel<bf16>, reinterpret_cast<const bf16*>(b));
   return last_err();
 }
 

@@ -204,7 +204,7 @@ def embedding(ids: torch.Tensor, table: torch.Tensor, *, scale: float = 1.0, voc
 
 def gated_residual(a: torch.Tensor, b: torch.Tensor, gate: torch.Tensor | None = None, rows_per_batch: int = 0,
                    out: torch.Tensor | None = None) -> torch.Tensor:
-    """out = a + gate[batch] * b (DiT gated residual) or a + b."""
+    """out = a + gate[batch] * b (DiT gated residual) or a + b. a, gate and out bf16, b bf16 or fp32."""
     require_cuda(a, b)
     H = a.shape[-1]
     a2, b2 = a.reshape(-1, H), b.reshape(-1, H)
@@ -214,7 +214,8 @@ def gated_residual(a: torch.Tensor, b: torch.Tensor, gate: torch.Tensor | None =
     ld_gate = 0
     if gate is not None:
         ld_gate = gate.stride(0) if gate.dim() >= 2 and gate.shape[0] > 1 else H
-    rc = kernels().swb_gated_residual(a2.data_ptr(), b2.data_ptr(), ptr(gate), ld_gate, rows_per_batch,
+    assert b2.dtype in (torch.bfloat16, torch.float32)
+    rc = kernels().swb_gated_residual(a2.data_ptr(), b2.data_ptr(), 1 if b2.dtype == torch.float32 else 0, ptr(gate), ld_gate, rows_per_batch,
                                       out.data_ptr(), a2.shape[0], H, stream_ptr())
     check(rc, "swb_gated_residual")
     return out.reshape(a.shape)

@@ -189,6 +189,31 @@ def test_pairs_of_sms(T, N, K, block_n, splits):
         close(y, (z + b.float()) * gate.float()[torch.arange(T, device="cuda") // rows] + r.float())
 
 
+@pytest.mark.parametrize("T,N,K", [(1, 128, 512), (16, 776, 1096), (63, 3072, 4096), (64, 520, 584), (64, 512, 128)])
+def test_gates_of_few_rows(T, N, K):
+    """Gate and residual behind the decode kernel's fp32 sums (and, below its smallest reduction, in the two-SM kernel): one rounding to bf16.
+    Rows that are not aligned are refused by either."""
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    a = torch.randn(T, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    b, r = torch.randn(N, device="cuda", generator=g).bfloat16(), torch.randn(T, N, device="cuda", generator=g).bfloat16()
+    gate = torch.randn(2, 2 * N, device="cuda", generator=g).bfloat16()[:, N:]
+    rows = (T + 1) // 2
+    want = (a.double() @ w.double().t() + b.double()) * gate.double()[torch.arange(T, device="cuda") // rows] + r.double()
+    y, out = ops.gemm_bf16(a, w, bias=b, residual=r, gate=gate, rows_per_gate=rows), r.clone()
+    ops.gemm_bf16(a, w, bias=b, residual=out, gate=gate, rows_per_gate=rows, out=out)
+    ops.check_status()
+    assert ((y.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-4).all() and torch.equal(y, out)
+    odd = torch.empty(T * N + 1, device="cuda", dtype=torch.bfloat16)[1:].view(T, N)
+    for kw in (dict(residual=odd), dict(residual=r, out=odd)):
+        with pytest.raises(ops.KernelError):
+            ops.gemm_bf16(a, w, gate=gate, rows_per_gate=rows, **kw)
+    with pytest.raises(ops.KernelError):
+        ops.gemm_bf16(a, w, residual=r, gate=torch.zeros(2 * N + 1, device="cuda", dtype=torch.bfloat16)[1:].view(2, N), rows_per_gate=rows)
+
+
 @pytest.mark.parametrize("T,N,K", [(300, 1024, 8192), (700, 512, 4096)])
 def test_products_split_along_k_run_beside_each_other(T, N, K):
     """Products with k-splits on several streams at once, launched one by one and replayed from graphs: each gives the bits it gives
