@@ -308,7 +308,7 @@ class FluxDiTGpu:
         return sum(t.numel() * 2 for t in self.w.values())
 
     def _lin(self, x, name, **kw):
-        self.launches += 1
+        self.launches += 2 if "gate" in kw and ops.gated_fused(x.shape[0], *self.w[name + ".weight"].shape) else 1
         return ops.gemm_bf16(x, self.w[name + ".weight"], bias=self.w[name + ".bias"], **kw)
 
     def _embed(self, x, name):

@@ -496,7 +496,7 @@ class LlamaGpu:
             if L.moe is not None:
                 pending_h = None
                 branch = self.comm.all_reduce(self._moe_ffn(h, L.moe, moe_counters))
-                n += 6
+                n += 6 + self._moe_launches
                 if li < len(taps):      # the stream after this layer is res + branch: the tap joins the pending branch
                     branch.index_add_(0, inp.deepstack[0], taps[li].to(branch.dtype))
                 continue
@@ -559,8 +559,10 @@ class LlamaGpu:
         T, E, k = h.shape[0], m.router.shape[0], moe.num_experts_per_tok
         logits = ops.gemm_bf16(h, m.router, out_dtype=torch.float32)
         shared = shared_gate = None
+        shared_launches = 0
         if m.shared_gate_up is not None:
             shared = ops.gemm_bf16(ops.linear_gated(h, m.shared_gate_up, act), m.shared_down)
+            shared_launches = (2 if h.device.type == "cuda" and ops.gated_epilogue(h, m.shared_gate_up) else 3) + (m.shared_gate is not None)
             if m.shared_gate is not None:
                 shared_gate = ops.gemm_bf16(h, m.shared_gate, out_dtype=torch.float32)[:, 0]
         if h.device.type != "cuda" or os.environ.get("SWB_MOE") == "loop":
@@ -568,12 +570,15 @@ class LlamaGpu:
             if moe.norm_topk_prob:
                 topv = topv / topv.sum(-1, keepdim=True)
             out = self._moe_experts_loop(h, m, topv * moe.routed_scaling_factor, topi)
+            self._moe_launches = 1 + shared_launches + 3 * topi.unique().numel()
             if shared is not None:
                 out += shared.float() if shared_gate is None else shared.float() * torch.sigmoid(shared_gate[:, None])
             return out.to(torch.bfloat16)
         if counters is None:
             counters = ops.routing_counters(E, h.device)
         spread = T * k > LlamaGpu.rows_per_expert_small * E
+        # router, one or two for the plan, two expert products, sum
+        self._moe_launches = shared_launches + (5 if T <= 128 and not spread else 6)
         plan, rows = ops.logits_routing(logits, E, k, rows=h if spread else None, renorm=moe.norm_topk_prob, counters=counters, tiles256=spread)
         y = ops.routed_gated_ffn(rows if spread else h, m.gate_up, m.down, plan, act)
         return ops.combine_routed(y, plan, moe.routed_scaling_factor, shared, shared_gate)

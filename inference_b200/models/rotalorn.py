@@ -238,7 +238,7 @@ class RotalornGpu(LatentDecoder):
         T, f, fast = h.shape[0], ff.spec, self.dtype == torch.bfloat16
         if isinstance(f, DenseSpec):
             if fast:
-                self.launches += 1 if ops.gated_fused(T, *ff.gate_up.shape) else 2
+                self.launches += 1 if ops.gated_epilogue(h, ff.gate_up, out) else 2
                 ops.linear_gated(h, ff.gate_up, "gelu", out=out)
             else:
                 self.launches += 1

@@ -197,6 +197,27 @@ def test_implicit_conv3x3_of_any_image_size(shape):
     assert (got.double() - want).abs().max().item() < 2.0 ** -8 * want.abs().max().item()
 
 
+@pytest.mark.parametrize("side,text", [(4, 8), (8, 16), (16, 40), (16, 128)])
+def test_launches_of_an_image_step_are_the_ones_counted(side, text):
+    """Gated products of up to 64 rows are two launches, larger ones one."""
+    from torch.profiler import ProfilerActivity, profile
+
+    from inference_b200.models.dit_flux import FluxConfig, FluxDiTGpu, make_ids, rope_table
+
+    cfg = FluxConfig(depth=1, depth_single=1, guidance_embed=False)
+    dit = FluxDiTGpu(cfg, device=torch.device("cuda", torch.cuda.current_device())).init_random(0)
+    txt_ids, img_ids = make_ids(side, side, text, device="cuda")
+    rnd = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    x = dict(img=rnd(1, side * side, cfg.in_channels), img_ids=img_ids, txt=rnd(1, text, cfg.context_in_dim), txt_ids=txt_ids,
+             timesteps=torch.rand(1, device="cuda"), y=rnd(1, cfg.vec_in_dim), rope=rope_table(torch.cat([txt_ids, img_ids]), cfg.axes_dim, cfg.theta))
+    dit.forward(**x)
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        dit.forward(**x)
+        torch.cuda.synchronize()
+    assert sum(e.count for e in prof.key_averages() if "swb::" in e.key) == dit.launches
+
+
 def test_vae_decoder_matches_oracle():
     from inference_b200.models.vae import OracleVaeDecoder, VaeConfig, VaeDecoderGpu, random_vae_weights
 

@@ -476,3 +476,35 @@ def test_split_decode_steps_match_whole_steps():
         for a, b in zip(steps, ref):
             assert a.shape == b.shape
             assert (a - b).abs().max().item() < 0.03 * max(1.0, b.abs().max().item())
+
+
+def _kernels_of(run) -> int:
+    """Launches of this library's kernels while run() runs, as the device's trace has them."""
+    from torch.profiler import ProfilerActivity, profile
+
+    run()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        run()
+        torch.cuda.synchronize()
+    return sum(e.count for e in prof.key_averages() if "swb::" in e.key)
+
+
+@pytest.mark.parametrize("T", [20, 64, 65, 100, 300])
+@pytest.mark.parametrize("shared", [0, 128])
+def test_launches_of_a_sparse_prompt_are_the_ones_counted(T, shared):
+    from inference_b200.engine.llm_engine import EngineConfig, LlmEngine
+    from inference_b200.models import ModelConfig
+    from inference_b200.models.llama import LlamaGpu
+
+    cfg = ModelConfig.from_json({"model_type": "qwen2_moe", "hidden_size": 512, "intermediate_size": 512, "num_hidden_layers": 3, "vocab_size": 1024,
+                                 "num_attention_heads": 4, "num_key_value_heads": 2, "head_dim": 128, "num_experts": 8, "num_experts_per_tok": 2,
+                                 "moe_intermediate_size": 256, "shared_expert_intermediate_size": shared, "rope_theta": 1e4, "rms_norm_eps": 1e-5})
+    model = LlamaGpu(cfg, device=torch.device("cuda")).init_random(seed=0)
+    eng = LlmEngine(model, EngineConfig(max_batch=1, max_seq_len=512))
+    s = eng.new_sequence()
+
+    def run():
+        s.truncate(0)
+        eng.runner.prefill([s], [list(range(1, T + 1))], want_logits=True)
+    assert _kernels_of(run) == model.launches
