@@ -107,9 +107,7 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
                              c_float, c_int, c_int, c_void_p])
     sig("swb_moe_table_plan", [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                c_void_p, c_void_p, c_int, c_void_p])
-    sig("swb_moe_route", [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                          c_void_p, c_void_p, c_int, c_void_p, c_ll, c_void_p, c_ll, c_int, c_void_p])
-    sig("swb_moe_route_tiles", [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+    sig("swb_moe_route", [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_ll, c_void_p, c_ll, c_int, c_void_p, c_void_p, c_void_p])
     sig("swb_moe_combine", [c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_int,
                             c_void_p])

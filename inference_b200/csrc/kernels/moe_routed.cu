@@ -483,7 +483,7 @@ int swb_moe_table_plan(const long long* ids, int T, const int* tables, int layer
 // one stream. rows_in (nullable): bf16 / fp32 rows of `pieces` 16-byte pieces, ld_in pieces apart, copied to rows dest[t, k] of rows_out.
 // row_tiles (nullable, needs rows_in and pad 1): int4 [rows_cap / 256 + min(E, rows_cap)], the row tiles of swb_gemm_bf16_routed, their
 // number in row_tile_count.
-int swb_moe_route_tiles(const float* logits, int ld, int T, int E, int top, int renorm, int pad, int* expert, int* rank, float* weights, int* counters,
+int swb_moe_route(const float* logits, int ld, int T, int E, int top, int renorm, int pad, int* expert, int* rank, float* weights, int* counters,
                         int* dest, int* src, int* offsets, int* active, int* tile_group, int rows_cap, const void* rows_in, long long ld_in,
                         void* rows_out, long long ld_out, int pieces, void* row_tiles, int* row_tile_count, void* stream) {
   using namespace swb;
@@ -502,13 +502,6 @@ int swb_moe_route_tiles(const float* logits, int ld, int T, int E, int top, int 
   if (rc) return rc;
   const long long blocks = ((long long)T * top + 7) / 8;
   return launch_kernel(moe_layout_kernel, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), smem, s, p);
-}
-
-int swb_moe_route(const float* logits, int ld, int T, int E, int top, int renorm, int pad, int* expert, int* rank, float* weights, int* counters,
-                  int* dest, int* src, int* offsets, int* active, int* tile_group, int rows_cap, const void* rows_in, long long ld_in,
-                  void* rows_out, long long ld_out, int pieces, void* stream) {
-  return swb_moe_route_tiles(logits, ld, T, E, top, renorm, pad, expert, rank, weights, counters, dest, src, offsets, active, tile_group, rows_cap,
-                             rows_in, ld_in, rows_out, ld_out, pieces, nullptr, nullptr, stream);
 }
 
 // out[t] = bf16(scale * sum over k < top of weights[t, k] y[dest[t, k]] + extra[t] * sigmoid(extra_gate[t])). extra, extra_gate nullable.
