@@ -198,8 +198,9 @@ struct Barriers {
 // exponentials and stores overlap; with 128 scores a thread eight warps left the special-function unit idle half of the time. The halves of
 // a row exchange their maximum through shared memory once per tile; that barrier also orders the stores of P over S behind both
 // halves' loads. Multiply-adds and sums run on two lanes at a time.
-// 4608 tokens x 24 heads: 274 us with a thread per row, 244 with two, 235 (1.11 PFLOP/s) with an eighth of the exponentials' pairs on the
-// multiply-add pipes (259 with a quarter, 235 with a sixteenth); eight causal prompts of 1100 x 32 heads 205 -> 165 us.
+// 4608 tokens x 24 heads of 128: 274 us with a thread per row, 244 with two, 235 (1.11 PFLOP/s) with a quarter of the exponentials' pairs on
+// the multiply-add pipes (259 with half of them, 235 with an eighth), 229 with whole-warp MMA issue on another box; eight causal prompts of 1100 x 32 heads
+// 209 -> 164 us. Heads of 64: 4608 tokens x 24 heads 251 -> 198 us, 2 x 4250 x 38 718 -> 569 us, 8 x 197 x 12 10.4 -> 8.9 us.
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -241,7 +242,7 @@ __device__ __forceinline__ unsigned long long ex2_fma2(unsigned long long x) {
 }
 __device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 
-constexpr int FMA_EVERY = 8;   // one pair of exponentials of every FMA_EVERY keys leaves the special-function unit
+constexpr int FMA_EVERY = 8;   // one of the four pairs of exponentials of every FMA_EVERY keys leaves the special-function unit
 
 template <typename C>
 __device__ __forceinline__ void softmax_halves(const FaParams& p, Barriers* bars, uint8_t* smem, uint32_t tmem, int q_base, int q_len, int kv_len,

@@ -329,3 +329,63 @@ def test_varlen_causal_attention_tcgen05(lens, Hq, Hkv):
         err = (out[lo:lo + n].float() - ref).abs().max().item()
         assert err < 3e-2, (n, err)
         lo += n
+
+
+def _one_by_one(a, b, D, causal=False):
+    """softmax of the scores a_i b_j (exact products of bf16 numbers), probability by probability: the values are rows of the unit
+    matrix for D keys at a time. a [queries], b [keys] -> [queries, keys], bf16 as the kernel stores it."""
+    from inference_b200 import ops
+
+    n, m = a.numel(), b.numel()
+    q, k = torch.zeros(1, n, 1, D, device="cuda", dtype=torch.bfloat16), torch.zeros(1, m, 1, D, device="cuda", dtype=torch.bfloat16)
+    q[0, :, 0, 0], k[0, :, 0, 0] = a, b
+    got = torch.empty(n, m, device="cuda", dtype=torch.bfloat16)
+    for j in range(0, m, D):
+        v = torch.zeros_like(k)
+        w = min(D, m - j)
+        v[0, j:j + w, 0, :w] = torch.eye(w, device="cuda")
+        if causal:
+            cu = torch.tensor([0, n], dtype=torch.int32, device="cuda")
+            out = ops.varlen_causal_attention(q[0], k[0], v[0], cu, n, scale=1.0)
+        else:
+            out = ops.dense_attention(q, k, v, scale=1.0)[0]
+        got[:, j:j + w] = out[:, :w]
+    ops.check_status()
+    return got
+
+
+@pytest.mark.parametrize("D,keys,causal", [(128, 300, False), (64, 300, False), (128, 300, True), (64, 129, False), (128, 1100, True)])
+def test_dense_attention_probabilities_one_by_one(D, keys, causal):
+    """Scores from 0 down to -140, in an order whose maximum grows by little and by much from tile to tile. Two roundings to bf16 (the weight
+    and the result, 2^-8 each: half of the last of 8 bits) and 1e-4 for the exponent in fp32. What is masked or far below stays under 2^-120."""
+    g = torch.Generator(device="cuda").manual_seed(keys + D)
+    b = (-140 * torch.rand(keys, device="cuda", generator=g) ** 2).bfloat16()
+    b[:128] -= 60
+    b[keys // 2] = 0
+    a = torch.tensor([1.0, 0.5, 0.75, 0.0078125, 1.25, 0.0], device="cuda").bfloat16().repeat(keys // 6 + 1)[:keys]
+    got = _one_by_one(a, b, D, causal).double()
+    scores = a.double()[:, None] * b.double()[None, :]
+    if causal:
+        scores = scores.masked_fill(torch.arange(keys, device="cuda")[None, :] > torch.arange(keys, device="cuda")[:, None], -torch.inf)
+    want = scores.softmax(-1)
+    assert ((got - want).abs() <= (2.0 ** -7 + 1e-4) * want + 2.0 ** -120).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_dense_attention_numbers_that_are_none(D):
+    """A query that is not a number and one whose score overflows give rows that are none; a key at minus infinity has no weight; the
+    other rows are as they are without them."""
+    a = torch.linspace(0.5, 1.0, 200, device="cuda").bfloat16()
+    b = torch.linspace(-20.0, -1.0, 333, device="cuda").bfloat16()
+    clean = _one_by_one(a, b, D)
+    a2 = a.clone()
+    a2[7], a2[150] = torch.nan, -3e38
+    got = _one_by_one(a2, b, D)
+    rows = torch.ones(200, dtype=torch.bool, device="cuda")
+    rows[7] = rows[150] = False
+    assert got[~rows].isnan().all() and torch.equal(got[rows], clean[rows])
+    b2 = b.clone()
+    b2[40], b2[332] = -torch.inf, -torch.inf
+    got = _one_by_one(a, b2, D).double()
+    want = (a.double()[:, None] * b2.double()[None, :]).softmax(-1)
+    assert ((got - want).abs() <= (2.0 ** -7 + 1e-4) * want + 2.0 ** -120).all()
