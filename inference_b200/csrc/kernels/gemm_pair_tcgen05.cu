@@ -3,7 +3,8 @@
 // A cluster of two CTAs computes a 256 x BN tile (BN = 32 .. 256) with tcgen05.mma.cta_group::2: each CTA brings its own 128 rows
 // of A and half of the tile's weight rows, so a k-block of 64 costs an SM 32 KB of operands (BN = 256) instead of the 48 KB
 // of a 128 x 256 tile on one SM. That traffic out of L2 is what bounded the one-SM kernel at prompt sizes
-// (gemm_tcgen05.cu, which keeps the peer-scatter epilogues and the shapes without 16-byte rows).
+// (gemm_tcgen05.cu, which keeps the peer-scatter epilogues, the shapes without 16-byte rows and those where 128-row tiles fill the
+// chip better: gemm_bf16_takes_pairs).
 //   warp 0      TMA producer of this CTA; all copies of a stage complete on the even CTA's barrier
 //   warp 1      TMEM owner; in the even CTA it issues the MMAs of the pair
 //   warps 2..9  epilogue: warp = (32 TMEM lanes, half of the columns); two accumulators, so it overlaps the next tile's
