@@ -479,7 +479,7 @@ int swb_moe_table_plan(const long long* ids, int T, const int* tables, int layer
 
 // Routing plan of one layer from router logits [T, ld] (fp32): the `top` experts of the largest softmax scores over all E, weights
 // [T, top] = their scores, as they are or (renorm) divided by their sum + 1e-20. dest, src, offsets, active, tile_group, pad and rows_cap as in swb_moe_table_plan.
-// expert and rank: int32 scratch [T * top]; counters: int32 [E + 2], zero at the first launch, launches that share it ordered on
+// E <= 12000 (segment starts in shared memory). expert and rank: int32 scratch [T * top]; counters: int32 [E + 2], zero at the first launch, launches that share it ordered on
 // one stream. rows_in (nullable): bf16 / fp32 rows of `pieces` 16-byte pieces, ld_in pieces apart, copied to rows dest[t, k] of rows_out.
 // row_tiles (nullable, needs rows_in and pad 1): int4 [rows_cap / 256 + min(E, rows_cap)], the row tiles of swb_gemm_bf16_routed, their
 // number in row_tile_count.
@@ -488,7 +488,7 @@ int swb_moe_route(const float* logits, int ld, int T, int E, int top, int renorm
                         void* rows_out, long long ld_out, int pieces, void* row_tiles, int* row_tile_count, void* stream) {
   using namespace swb;
   if (T <= 0) return 0;
-  if (top <= 0 || E <= 0 || E > 4096 || top > E || ld < E || (pad != 1 && pad != 128) || (tile_group && (pad != 128 || rows_cap % 128)) ||
+  if (top <= 0 || E <= 0 || E > 12000 || top > E || ld < E || (pad != 1 && pad != 128) || (tile_group && (pad != 128 || rows_cap % 128)) ||
       (long long)T * top + (long long)E * (pad - 1) > (long long)rows_cap || !expert || !rank || !weights || !counters || !dest || !offsets ||
       (rows_in && (!rows_out || pieces <= 0)) || (row_tiles && (!row_tile_count || !rows_in || pad != 1)))
     return -3;

@@ -98,7 +98,8 @@ def logits_routing(logits: torch.Tensor, num_experts: int, top: int, *, rows: to
     per = 16 // rows.element_size() if spread else 1
     assert not spread or (rows.stride(1) == 1 and rows.stride(0) % per == 0 and rows.shape[1] % per == 0)
     assert counters is None or (counters.dtype == torch.int32 and counters.numel() >= E + 2)
-    counters = _counters(dev) if counters is None else counters
+    if counters is None:
+        counters = _counters(dev) if E <= 4096 else routing_counters(E, dev)
     rc = kernels().swb_moe_route(logits.data_ptr(), logits.stride(0), T, E, top, 1 if renorm else 0, TILE if padded else 1, scratch[0].data_ptr(),
                                  scratch[1].data_ptr(), weights.data_ptr(), counters.data_ptr(), dest.data_ptr(), ptr(src),
                                  offsets.data_ptr(), ptr(active), ptr(tiles), cap, ptr(rows), rows.stride(0) // per if spread else 0, ptr(buf),

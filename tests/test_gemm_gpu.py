@@ -189,6 +189,24 @@ def test_pairs_of_sms(T, N, K, block_n, splits):
         close(y, (z + b.float()) * gate.float()[torch.arange(T, device="cuda") // rows] + r.float())
 
 
+@pytest.mark.parametrize("T,N,K", [(1100, 2048, 512), (300, 12288, 3072)])
+def test_residual_in_place_above_256_rows(T, N, K):
+    """The same product in place on the kernel of its choice (one SM a tile here) and on pairs of SMs: one rounding of fp32 sums each."""
+    from inference_b200 import ops
+    from inference_b200._native import kernels
+
+    assert not kernels().swb_gemm_takes_pairs(T, N, K, 0, 1, 0, 0, -1, 0, 0)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    a, r = torch.randn(T, K, device="cuda", generator=g).bfloat16(), torch.randn(T, N, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    want = a.float() @ w.float().t() + r.float()
+    for kw in ({}, dict(mode=3)):
+        out = r.clone()
+        ops.gemm_bf16(a, w, residual=out, out=out, **kw)
+        ops.check_status()
+        assert ((out.float() - want).abs() <= 2 ** -8 * want.abs() + 1e-4).all(), kw
+
+
 @pytest.mark.parametrize("T,N,K", [(1, 128, 512), (16, 776, 1096), (63, 3072, 4096), (64, 520, 584), (64, 512, 128)])
 def test_gates_of_few_rows(T, N, K):
     """Gate and residual behind the decode kernel's fp32 sums (and, below its smallest reduction, in the two-SM kernel): one rounding to bf16.
@@ -256,7 +274,8 @@ def test_products_split_along_k_run_beside_each_other(T, N, K):
 
 
 @pytest.mark.parametrize("T,E,top,H,f,renorm", [(1, 4, 2, 64, 24, True), (33, 8, 8, 128, 72, False), (700, 5, 3, 200, 136, True),
-                                                (2100, 64, 8, 256, 128, False), (300, 4, 2, 24, 8, True), (150, 3, 2, 72, 16, False)])
+                                                (2100, 64, 8, 256, 128, False), (300, 4, 2, 24, 8, True), (150, 3, 2, 72, 16, False),
+                                                (40, 5003, 2, 64, 8, True), (20100, 5003, 2, 64, 8, False)])
 @pytest.mark.parametrize("shared", [False, True])
 def test_routed_segments_in_row_tiles(T, E, top, H, f, renorm, shared):
     """Dense expert segments in tiles of 256 rows (none, one row, remainders, several tiles an expert), gated pairs in the epilogue, and
