@@ -200,9 +200,8 @@ def test_implicit_conv3x3_of_any_image_size(shape):
 @pytest.mark.parametrize("side,text", [(4, 8), (8, 16), (16, 40), (16, 128)])
 def test_launches_of_an_image_step_are_the_ones_counted(side, text):
     """Gated products of up to 64 rows are two launches, larger ones one."""
-    from torch.profiler import ProfilerActivity, profile
-
     from inference_b200.models.dit_flux import FluxConfig, FluxDiTGpu, make_ids, rope_table
+    from inference_b200.utils.tracing import LaunchTimeline
 
     cfg = FluxConfig(depth=1, depth_single=1, guidance_embed=False)
     dit = FluxDiTGpu(cfg, device=torch.device("cuda", torch.cuda.current_device())).init_random(0)
@@ -212,10 +211,10 @@ def test_launches_of_an_image_step_are_the_ones_counted(side, text):
              timesteps=torch.rand(1, device="cuda"), y=rnd(1, cfg.vec_in_dim), rope=rope_table(torch.cat([txt_ids, img_ids]), cfg.axes_dim, cfg.theta))
     dit.forward(**x)
     torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+    with LaunchTimeline() as timeline:
         dit.forward(**x)
         torch.cuda.synchronize()
-    assert sum(e.count for e in prof.key_averages() if "swb::" in e.key) == dit.launches
+    assert len(timeline.records()) == dit.launches
 
 
 def test_vae_decoder_matches_oracle():
