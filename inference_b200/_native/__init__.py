@@ -196,6 +196,9 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
     sig("swb_sample_device", [c_void_p, c_int, c_ll, c_int, c_int, c_float, c_int, c_float, c_void_p, c_void_p, c_void_p,
                               c_void_p, c_void_p])
     sig("swb_argmax_peer_merge", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    sig("swb_gemv_q4k_supported", [c_int, c_int])
+    sig("swb_gemv_q4k_normed", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
+                                c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p])
     sig("swb_gemm_bf16_normed", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                  c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p])
     sig("swb_gemm_gated_supported", [c_int, c_int, c_int])

@@ -368,6 +368,12 @@ class LlamaGpu:
         self.quant_format = fmt
         return self
 
+    def _packed_chain(self, T: int) -> bool:
+        """Whether packed projections run as a chain of products that join the stream and scale by its norm (6 kernels per layer and not 9), on an
+        fp32 stream."""
+        return (self.norm_folded and not self.comm.is_parallel and self.device.type == "cuda" and
+                all(ops.normed_supported(T, w) for L in self.layers for w in (L.qkv, L.o, L.gate_up, L.down)))
+
     # bytes of the next projection's weights each decode-step norm prefetches into L2 (0 = all of them, < 0 = off).
     # Off by default: measured on B200 the prefetches lengthen the norm kernel that the GEMM's dependency waits on
     # (Llama-3-8B step 5.27 ms without, 5.50 ms with 24-48 MB, 6.06 ms with 96 MB).
@@ -402,8 +408,8 @@ class LlamaGpu:
             rope_pos = torch.arange(T, dtype=torch.int32, device=self.device)
         taps = inp.deepstack[1] if inp.deepstack is not None else []
         # decode-sized steps of a dense model (short prompts too): the norms are folded into a chain of GEMM epilogues
-        chain = (self._chain_ok and (inp.decode or not self.comm.is_parallel) and T <= 64 and self.quant_format is None and
-                 os.environ.get("SWB_NORM_CHAIN", "1") != "0")
+        chain = (T <= 64 and (inp.decode or not self.comm.is_parallel) and os.environ.get("SWB_NORM_CHAIN", "1") != "0" and
+                 (self._chain_ok if self.quant_format is None else self._packed_chain(T)))
         chain = chain and not taps
         fc = self.comm.fused if self.comm.is_parallel else None
         if chain and self.comm.is_parallel:
@@ -422,6 +428,8 @@ class LlamaGpu:
         # optional: each norm asks L2 for (the first megabytes of) its consumer's weights (see l2_prefetch_bytes)
         pf_bytes = self.l2_prefetch_bytes if inp.decode else -1
         pf = (lambda t: t if (pf_bytes >= 0 and isinstance(t, torch.Tensor)) else None)
+        ssq = (self._ssq if self.quant_format is None else torch.empty((2, ops.SSQ_WORDS), dtype=torch.int64, device=self.device).unbind(0)) if chain else None
+        packed = chain and self.quant_format is not None
         ssq_prev = None                 # partial sums of squares of `res` (valid while branch is None)
         H = cfg.hidden_size
         moe_counters = ops.routing_counters(cfg.moe.num_experts, self.device) if self.has_moe else None
@@ -436,7 +444,9 @@ class LlamaGpu:
                 h = ops.rmsnorm(branch, L.ln1, eps, residual=res, w_offset=woff, prefetch=pf(L.qkv),
                                 prefetch_bytes=pf_bytes)
             if h is None:
-                qkv = ops.gemm_bf16_normed(res, L.qkv, bias=L.qkv_bias, ssq_in=ssq_prev, norm_dim=H, eps=eps)
+                qkv = ops.linear_normed(res, L.qkv, bias=L.qkv_bias, ssq_in=ssq_prev, norm_dim=H, eps=eps)
+            elif packed:       # the step's own accumulators: the first product clears what the next one adds to
+                qkv = ops.linear_normed(h, L.qkv, bias=L.qkv_bias, ssq_zero=ssq[0])
             else:
                 qkv = ops.linear_any(h, L.qkv, bias=L.qkv_bias)
             ops.rope_kv_write(qkv, rope_pos, inp.slot_mapping, rope_cos, rope_sin, kv_pool[li, 0], kv_pool[li, 1],
@@ -460,20 +470,23 @@ class LlamaGpu:
                     res.add_(branch)
                     branch = None
                     n += 1
+                if packed and h is not None:    # the stream of packed products is kept in 32 bits until the last layer
+                    res = res.float()
+                    n += 1
                 gelu = cfg.mlp_activation in ("gelu", "gelu_tanh")
                 if fc is not None:
-                    fc.gemm_peer_reduce(attn.reshape(T, -1), L.o, res, 0, ssq_out=self._ssq[0], ssq_zero=self._ssq[1])
+                    fc.gemm_peer_reduce(attn.reshape(T, -1), L.o, res, 0, ssq_out=ssq[0], ssq_zero=ssq[1])
                 else:
-                    ops.gemm_bf16_normed(attn.reshape(T, -1), L.o, out=res, residual=res, ssq_out=self._ssq[0],
-                                         ssq_zero=self._ssq[1])
-                act = ops.gemm_bf16_normed(res, L.gate_up, act="geglu_pairs" if gelu else "swiglu_pairs",
-                                           ssq_in=self._ssq[0], norm_dim=H, eps=eps)
+                    ops.linear_normed(attn.reshape(T, -1), L.o, out=res, residual=res, ssq_out=ssq[0],
+                                         ssq_zero=ssq[1])
+                act = ops.linear_normed(res, L.gate_up, act="geglu_pairs" if gelu else "swiglu_pairs",
+                                           ssq_in=ssq[0], norm_dim=H, eps=eps)
                 if fc is not None:
-                    fc.gemm_peer_reduce(act, L.down, res, 1, ssq_out=self._ssq[1], ssq_zero=self._ssq[0])
+                    fc.gemm_peer_reduce(act, L.down, res, 1, ssq_out=ssq[1], ssq_zero=ssq[0])
                 else:
-                    ops.gemm_bf16_normed(act, L.down, out=res, residual=res, ssq_out=self._ssq[1],
-                                         ssq_zero=self._ssq[0])
-                ssq_prev, pending_h = self._ssq[1], None
+                    ops.linear_normed(act, L.down, out=res, residual=res, ssq_out=ssq[1],
+                                         ssq_zero=ssq[0])
+                ssq_prev, pending_h = ssq[1], None
                 n += 6 + (1 if h is not None else 0)
                 continue
             fused = self.comm.fused if (self.comm.fused is not None and T <= self.comm.fused.max_tokens and
@@ -519,6 +532,9 @@ class LlamaGpu:
             if li < len(taps):
                 branch.index_add_(0, inp.deepstack[0], taps[li].to(branch.dtype))
             n += 7 + self._mlp_in_launches
+        if packed:
+            res = res.to(torch.bfloat16)
+            n += 1
         self.launches = n
         if not last_stage:
             assert pending_h is None

@@ -9,7 +9,7 @@ import numpy as np
 import torch
 
 from .._native import kernels
-from .gemm import gemm_bf16, gemm_workspace
+from .gemm import ACT, SSQ_WORDS, _PAIRS, gemm_bf16, gemm_bf16_normed, gemm_workspace
 from .runtime import check, ptr, require_cuda, stream_ptr
 
 FORMATS = {"Q4_K": 0, "Q8_0": 1, "AFFINE4": 2, "AFFINE8": 3}
@@ -103,6 +103,37 @@ def linear_quant(a: torch.Tensor, qw: QuantWeight, bias: torch.Tensor | None = N
                                   ptr(qw.biases), out.data_ptr(), out.stride(0), T, qw.n, qw.k, ptr(bias),
                                   ws.data_ptr(), ws.numel(), splits, stream_ptr())
     check(rc, "swb_gemm_quant")
+    return out
+
+
+def normed_supported(T: int, w) -> bool:
+    """True when linear_normed takes T tokens of this packed weight."""
+    return isinstance(w, QuantWeight) and w.fmt == "Q4_K" and bool(kernels().swb_gemv_q4k_supported(T, w.k))
+
+
+def linear_normed(a: torch.Tensor, w, *, out: torch.Tensor | None = None, bias: torch.Tensor | None = None,
+                  residual: torch.Tensor | None = None, act: str | None = None, ssq_in: torch.Tensor | None = None,
+                  ssq_out: torch.Tensor | None = None, ssq_zero: torch.Tensor | None = None, norm_dim: int = 0, eps: float = 0.0) -> torch.Tensor:
+    """`gemm_bf16_normed` for a dense weight or one that `normed_supported` answers for (whose norm weight was folded in before it was packed).
+    With a packed weight the stream may be fp32: a, or out and residual."""
+    if not isinstance(w, QuantWeight):
+        return gemm_bf16_normed(a, w, out=out, bias=bias, residual=residual, act=act, ssq_in=ssq_in, ssq_out=ssq_out, ssq_zero=ssq_zero,
+                                norm_dim=norm_dim, eps=eps)
+    require_cuda(a, w.packed)
+    T, K = a.shape
+    n_out = w.n // 2 if ACT[act] in _PAIRS else w.n
+    if out is None:
+        out = torch.empty((T, n_out), dtype=torch.bfloat16, device=a.device)
+    f32, either = torch.float32, (torch.bfloat16, torch.float32)
+    assert out.shape == (T, n_out) and out.dtype in either and out.stride(1) == 1 and a.dtype in either and a.stride(1) == 1
+    assert w.fmt == "Q4_K" and K == w.k and (bias is None or (bias.dtype == torch.bfloat16 and bias.numel() == w.n and bias.is_contiguous()))
+    assert residual is None or (residual.dtype == out.dtype and residual.shape == out.shape and residual.stride(1) == 1)
+    for b in (ssq_in, ssq_out, ssq_zero):
+        assert b is None or (b.dtype == torch.int64 and b.numel() >= SSQ_WORDS and b.is_contiguous())
+    rc = kernels().swb_gemv_q4k_normed(a.data_ptr(), a.stride(0), int(a.dtype == f32), w.packed.data_ptr(), out.data_ptr(), out.stride(0),
+                                       int(out.dtype == f32), T, w.n, K, ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0,
+                                       ACT[act], ptr(ssq_in), ptr(ssq_out), ptr(ssq_zero), norm_dim, eps, stream_ptr())
+    check(rc, "swb_gemv_q4k_normed")
     return out
 
 

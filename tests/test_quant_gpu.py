@@ -76,6 +76,115 @@ def test_q4k_matvec_pairs_of_rows(T, N, K):
     assert (got.double() - ref).abs().max().item() < 2.0 ** -8 * ref.abs().max().item()
 
 
+# a tile of one row; more than 16 tiles of a CTA; one, two and four passes over the reduction index; activations far apart in size
+@pytest.mark.parametrize("T,N,K", [(1, 1, 256), (4, 16 * 148 * 16 + 18, 256), (7, 2390, 4096), (8, 98, 14336), (8, 34, 28416), (5, 64, 1536), (3, 4096, 512)])
+def test_q4k_matvec_chain_links(T, N, K):
+    """Both links of a folded-norm chain and gated pairs, against 64 bits. Operands are exact, so what is left are fp32 sums (K of them at 2^-24) and
+    the rounding to bf16; activations that are 10^5 times smaller than others of their super-block count as much as the rest."""
+    from inference_b200 import ops
+    from inference_b200.ops import quant
+
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    qw = quant.quantize_on_device((torch.randn(N, K, device="cuda", generator=g) * 0.05).bfloat16(), "Q4_K")
+    w = quant.dequantize_reference(qw).double().cuda()
+    assert ops.normed_supported(T, qw)
+    a = torch.randn(T, K, device="cuda", generator=g)
+    a[:, : K // 2] *= 1e-5
+    a[:, 32:64] = 0
+    a[T - 1] *= 1e2
+    a = a.bfloat16()
+    bias = (torch.randn(N, generator=g, device="cuda") * 0.1).bfloat16()
+    res = torch.randn(T, N, device="cuda", generator=g).bfloat16()
+
+    def product(x):
+        return x.double() @ w.T, x.double().abs() @ w.abs().T * (2.0 ** -22 + K * 2.0 ** -26)
+
+    out, zero = ops.ssq_buffer(a.device), torch.ones(64, dtype=torch.int64, device="cuda")
+    y = res.clone()
+    ops.linear_normed(a, qw, out=y, bias=bias, residual=y, ssq_out=out, ssq_zero=zero)
+    ops.check_status()
+    exact, near = product(a)
+    exact += bias.double()
+    want = exact + res.double()
+    assert ((y.double() - want).abs() - near - 2.0 ** -8 * (exact.abs() + want.abs())).max().item() <= 0
+    assert not zero.any() and not out[T:].any()
+    torch.testing.assert_close(ops.ssq_values(out)[:T], y.float().pow(2).sum(1), rtol=1e-5, atol=1e-5)
+
+    y32 = ops.linear_normed(a.float(), qw, out=res.float(), bias=bias, residual=res.float())      # bf16 values in fp32: the same operands
+    assert ((y32.double() - want).abs() - near - 2.0 ** -22 * want.abs()).max().item() <= 0
+
+    ssq = ops.ssq_buffer(a.device)
+    ssq[:T] = (a.double().pow(2).sum(1) * 2.0 ** 24).round().long()
+    rms = (a.double().pow(2).mean(1, keepdim=True) + 1e-5).rsqrt()
+    exact, near = (t * rms for t in product(a))
+    z = ops.linear_normed(a, qw, ssq_in=ssq, norm_dim=K, eps=1e-5)
+    assert ((z.double() - exact).abs() - near - 2.0 ** -8 * exact.abs()).max().item() <= 0
+    if N % 2 == 0:
+        for act, f in (("swiglu_pairs", torch.nn.functional.silu), ("geglu_pairs", lambda t: torch.nn.functional.gelu(t, approximate="tanh"))):
+            u = ops.linear_normed(a, qw, act=act, ssq_in=ssq, norm_dim=K, eps=1e-5)
+            gate, up = exact[:, 0::2], exact[:, 1::2]
+            e_gate, e_up = (near + 2.0 ** -8 * exact.abs())[:, 0::2], (near + 2.0 ** -8 * exact.abs())[:, 1::2]
+            bound = 1.2 * e_gate * (up.abs() + e_up) + f(gate).abs() * e_up      # slopes of both functions stay below 1.2
+            assert ((u.double() - f(gate) * up).abs() - bound - 2.0 ** -8 * (f(gate) * up).abs()).max().item() <= 1e-6
+
+
+def test_q4k_matvec_chain_sees_small_activations():
+    """Tokens and super-blocks of any size: what one holds is not measured by another's largest."""
+    from inference_b200 import ops
+    from inference_b200.ops import quant
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    qw = quant.quantize_on_device((torch.randn(64, 768, device="cuda", generator=g) * 0.05).bfloat16(), "Q4_K")
+    w = quant.dequantize_reference(qw).double().cuda()
+    a = torch.randn(6, 768, device="cuda", generator=g)
+    a *= torch.tensor([1e-30, 1e-12, 0.0, 1.0, 1e9, 1e30], device="cuda")[:, None]
+    a = a.bfloat16()
+    got, want = ops.linear_normed(a, qw).double(), a.double() @ w.T
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -20 * (a.double().abs() @ w.abs().T)).all()
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_q4k_matvec_chain_keeps_what_is_no_number_in_its_token(value):
+    from inference_b200 import ops
+    from inference_b200.ops import quant
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    qw = quant.quantize_on_device((torch.randn(48, 512, device="cuda", generator=g) * 0.05).bfloat16(), "Q4_K")
+    a = torch.randn(3, 512, device="cuda", generator=g).bfloat16()
+    want = ops.linear_normed(a, qw)
+    a[1, 300] = value
+    got = ops.linear_normed(a, qw)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[2], want[2]) and not got[1].isfinite().any()
+
+
+def test_a_q4k_decoder_chains_its_products_in_decode():
+    """Steps of up to eight rows join the stream and apply its norm inside the products: six launches a layer. The same logits as with the
+    kernels in between, within the rounding of what those store in bf16."""
+    import os
+
+    from inference_b200.engine.llm_engine import EngineConfig, LlmEngine
+    from inference_b200.models import ModelConfig
+    from inference_b200.models.llama import LlamaGpu
+
+    cfg = ModelConfig.from_json({"hidden_size": 512, "intermediate_size": 1024, "num_hidden_layers": 3, "num_attention_heads": 4,
+                                 "num_key_value_heads": 2, "head_dim": 128, "vocab_size": 1024, "rope_theta": 10000.0})
+    model = LlamaGpu(cfg).init_random(seed=1).quantize_("Q4_K")
+    logits, launches = {}, {}
+    for chain in ("1", "0"):
+        os.environ["SWB_NORM_CHAIN"] = chain
+        try:
+            eng = LlmEngine(model, EngineConfig(max_batch=8, max_seq_len=64))
+            seqs = [eng.new_sequence() for _ in range(3)]
+            eng.runner.prefill(seqs, [[1, 2, 3], [4, 5], [6, 7, 8, 9]])
+            for _ in range(2):
+                logits[chain] = eng.runner.decode(seqs, [3, 4, 5], want_logits=True).clone()
+            launches[chain] = eng.runner.launches_last
+        finally:
+            del os.environ["SWB_NORM_CHAIN"]
+    assert launches["1"] == launches["0"] - 3 * 3 + 3        # the first norm stays, the stream is converted to 32 bits and back
+    assert (logits["1"] - logits["0"]).norm() < 0.03 * logits["0"].norm()
+
+
 @pytest.mark.parametrize("T", [65, 130, 256])
 def test_expanded_weights_are_complete_before_they_are_multiplied(T):
     """Token counts above the fused kernel's expand the weight and multiply it right behind: the product must not start from
