@@ -58,6 +58,23 @@ def test_media_kernels():
     assert torch.equal(u8, ref)
 
 
+@pytest.mark.parametrize("pad", [0, 3, 4])
+@pytest.mark.parametrize("cols", [1, 4, 252, 255, 4096, 4100, 8192, 8196, 15808, 16384, 16388])
+def test_softmax_rows_of_any_width(cols, pad):
+    """Rows that stay in 4, 8 or 16 vectors of a thread, wider ones and ones that do not start on 16 bytes."""
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    s = (torch.randn(5, cols + pad, device="cuda", generator=g) * 8)[:, :cols]
+    if cols > 1:
+        s[1, cols // 2] = -float("inf")
+    s[2] += 1e4
+    p = ops.softmax_rows(s, 0.5)
+    want = torch.softmax(s.double() * 0.5, -1)
+    # the scaled score rounded to 32 bits, the exponential's 2^-21 and the rounding to bf16
+    assert ((p.double() - want).abs() <= want * (2.0 ** -8 + s.abs().amax(1, keepdim=True).clamp_max(1e6).nan_to_num(0) * 2.0 ** -23)).all()
+
+
 def test_rope_in_place_updates_k_without_cache():
     from inference_b200 import ops
 
