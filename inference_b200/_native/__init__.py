@@ -171,6 +171,8 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
     sig("swb_axpy", [c_void_p, c_void_p, c_void_p, c_ll, c_float, c_float, c_int, c_void_p])
     sig("swb_groupnorm", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int,
                           c_void_p])
+    sig("swb_groupnorm_apply", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int,
+                          c_void_p])
     sig("swb_upsample2x", [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
     sig("swb_attn_dense_set_impl", [c_int], None)
     sig("swb_attn_dense_set_tiles", [c_int], None)
@@ -229,6 +231,8 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
     sig("swb_rgb8", [c_void_p, c_void_p, c_ll, c_int, c_void_p])
     sig("swb_comm_max_ctas", [])
     sig("swb_comm_flag_words", [])
+    sig("swb_conv3x3_nhwc_stats", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p,
+                             c_int, c_int, c_void_p, c_int, c_void_p])
     sig("swb_allreduce_rmsnorm", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int,
                                   c_void_p, c_float, c_float, c_void_p, c_int, c_void_p])
     sig("swb_flag_wait", [c_void_p, ctypes.c_uint, c_void_p, c_void_p])

@@ -95,8 +95,10 @@ int swb_gemm_bf16_gated(const void* A, int lda, const void* W, int ldw, void* D,
 // W [cout, (ky, kx, cin)] bf16 rows of 9 c; out [n h w, cout] bf16 (= NHWC); optional bias [cout] and residual
 // [n h w, cout]. Needs c % 64 == 0, and either 16-byte rows of out, bias and residual (any image size) or h w % 128 == 0 with w
 // a multiple or a divisor of 128; returns -3 otherwise.
-int swb_conv3x3_nhwc(const void* x, int n, int h, int w, int c, const void* W, int ldw, int cout, void* out, int ldd,
-                     const void* bias, const void* residual, int ld_res, int act, void* stream) {
+// stats (nullable): fp32 [n, groups, 2]; the sum and the sum of squares of every group of neighbouring output channels, as stored, are added to it.
+// Needs groups of 4, 8, 16 or 32 channels and 16-byte rows of everything.
+int swb_conv3x3_nhwc_stats(const void* x, int n, int h, int w, int c, const void* W, int ldw, int cout, void* out, int ldd,
+                           const void* bias, const void* residual, int ld_res, int act, void* stats, int groups, void* stream) {
   swb::GemmArgs a;
   a.A = x;
   a.lda = c;
@@ -121,7 +123,13 @@ int swb_conv3x3_nhwc(const void* x, int n, int h, int w, int c, const void* W, i
   a.conv_h = h;
   a.conv_w = w;
   a.conv_c = c;
+  a.conv_stats = reinterpret_cast<float*>(stats);
+  a.stats_groups = groups;
   return swb::gemm_bf16_launch(a, reinterpret_cast<cudaStream_t>(stream));
+}
+int swb_conv3x3_nhwc(const void* x, int n, int h, int w, int c, const void* W, int ldw, int cout, void* out, int ldd,
+                     const void* bias, const void* residual, int ld_res, int act, void* stream) {
+  return swb_conv3x3_nhwc_stats(x, n, h, w, c, W, ldw, cout, out, ldd, bias, residual, ld_res, act, nullptr, 0, stream);
 }
 
 // GEMM whose epilogue dispatches the output head-sharded to peers (see GemmScatter): D is not written locally.

@@ -174,7 +174,9 @@ __global__ void __launch_bounds__(256) groupnorm_apply_kernel(const bf16* __rest
     }
     const uint4* xin = reinterpret_cast<const uint4*>(x) + (size_t)n * HW * c8 + v;
     uint4* yout = reinterpret_cast<uint4*>(out) + (size_t)n * HW * c8 + v;
-    for (unsigned p = tid / c8; p < (unsigned)HW; p += pix_step) {
+    // last pixels first: of what the kernel in front of this one wrote they are the part that L2 still holds
+    for (unsigned i = tid / c8; i < (unsigned)HW; i += pix_step) {
+      const unsigned p = (unsigned)HW - 1 - i;
       float f[8], o[8];
       unpack8(xin[(size_t)p * c8], f);
 #pragma unroll
@@ -246,6 +248,9 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(const float* __restri
   pdl_wait();
   __shared__ float red[8];
   const float* row = s + (size_t)blockIdx.x * ld_in;
+  bf16* o = out + (size_t)blockIdx.x * ld_out;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float4 v[VECS > 0 ? VECS : 1];
   float mx = -INFINITY;
   if constexpr (VECS > 0) {
 #pragma unroll
@@ -261,9 +266,6 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(const float* __restri
   } else {
     for (int i = threadIdx.x; i < cols; i += blockDim.x) mx = fmaxf(mx, row[i] * scale);
   }
-  bf16* o = out + (size_t)blockIdx.x * ld_out;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float4 v[VECS > 0 ? VECS : 1];
   mx = warp_max(mx);
   if (lane == 0) red[warp] = mx;
   __syncthreads();
@@ -358,6 +360,27 @@ int swb_axpy(const void* x, const void* y, void* out, long long n, float a, floa
                        reinterpret_cast<const bf16*>(y), reinterpret_cast<bf16*>(out), n / 8, a, b);
 }
 
+// x, out: NHWC bf16 [N, H*W, C]; stats: fp32 [N, G, 2], sums and sums of squares of every group (of G groups of C / G neighbouring channels).
+int swb_groupnorm_apply(const void* x, const void* stats, const void* gamma, const void* beta, void* out, int N, int HW, int C,
+                        int G, float eps, int silu, void* stream) {
+  using namespace swb;
+  if (N <= 0 || HW <= 0) return 0;
+  if (C % G != 0 || C % 8 != 0) return -3;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const long long n8 = (long long)N * HW * C / 8;
+  if (256 % (C / 8) == 0) {
+    // about four vectors per thread, at most eight CTAs per SM's worth of blocks
+    const long long per_sample = (long long)HW * (C / 8);
+    const int blocks = (int)std::max<long long>(1, std::min<long long>((per_sample + 1023) / 1024, 148 * 8));
+    return launch_kernel(groupnorm_apply_kernel, dim3(blocks), dim3(256), 0, s, reinterpret_cast<const bf16*>(x),
+                         reinterpret_cast<const float*>(stats), reinterpret_cast<const bf16*>(gamma),
+                         reinterpret_cast<const bf16*>(beta), reinterpret_cast<bf16*>(out), N, HW, C, G, eps, silu);
+  }
+  return launch_kernel(groupnorm_apply_any_kernel, dim3(blocks_for(n8)), dim3(256), 0, s, reinterpret_cast<const bf16*>(x),
+                       reinterpret_cast<const float*>(stats), reinterpret_cast<const bf16*>(gamma),
+                       reinterpret_cast<const bf16*>(beta), reinterpret_cast<bf16*>(out), n8, HW, C, G, eps, silu);
+}
+
 // stats: fp32 [N, G, 2] scratch. x, out: NHWC bf16 [N, H*W, C]; C / G a multiple of 8, or one of 1, 2, 4 (then
 // C/8 must divide 256 and G <= 512).
 int swb_groupnorm(const void* x, void* stats, const void* gamma, const void* beta, void* out, int N, int HW, int C,
@@ -380,18 +403,7 @@ int swb_groupnorm(const void* x, void* stats, const void* gamma, const void* bet
                   : launch_kernel(groupnorm_stats_kernel, grid, dim3(256), 0, s, reinterpret_cast<const bf16*>(x),
                                   reinterpret_cast<float*>(stats), HW, C, G, chunk);
   if (rc) return rc;
-  const long long n8 = (long long)N * HW * C / 8;
-  if (256 % (C / 8) == 0) {
-    // about four vectors per thread, at most eight CTAs per SM's worth of blocks
-    const long long per_sample = (long long)HW * (C / 8);
-    const int blocks = (int)std::max<long long>(1, std::min<long long>((per_sample + 1023) / 1024, 148 * 8));
-    return launch_kernel(groupnorm_apply_kernel, dim3(blocks), dim3(256), 0, s, reinterpret_cast<const bf16*>(x),
-                         reinterpret_cast<const float*>(stats), reinterpret_cast<const bf16*>(gamma),
-                         reinterpret_cast<const bf16*>(beta), reinterpret_cast<bf16*>(out), N, HW, C, G, eps, silu);
-  }
-  return launch_kernel(groupnorm_apply_any_kernel, dim3(blocks_for(n8)), dim3(256), 0, s, reinterpret_cast<const bf16*>(x),
-                       reinterpret_cast<const float*>(stats), reinterpret_cast<const bf16*>(gamma),
-                       reinterpret_cast<const bf16*>(beta), reinterpret_cast<bf16*>(out), n8, HW, C, G, eps, silu);
+  return swb_groupnorm_apply(x, stats, gamma, beta, out, N, HW, C, G, eps, silu, stream);
 }
 
 int swb_upsample2x(const void* x, void* out, int N, int H, int W, int C, void* stream) {

@@ -24,6 +24,8 @@ struct PairParams {
   // 3x3 convolution (conv_c > 0): a CTA's 128 rows are a box of 2^box_w_log x 2^box_h_log pixels, boxes run row by row
   int conv_n, conv_h, conv_w, conv_c;
   int box_w_log, box_h_log, boxes_x, boxes_y;
+  float* stats;                       // optional [conv_n][N / group_channels][2]: sums and sums of squares of what is stored are added
+  int group_channels;                 // 4, 8, 16 or 32
 };
 
 bool gemm_pair_accepts(const GemmArgs& a);

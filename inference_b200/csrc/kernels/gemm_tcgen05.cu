@@ -849,6 +849,7 @@ int gemm_bf16_launch(const GemmArgs& a, cudaStream_t stream) {
   // Convolutions whose output has 16-byte rows go to the two-SM kernel, whose tiles are boxes of pixels of any image size. 512 -> 512
   // channels at 304 x 208 take 188 us there (1.58 PFLOP/s) and 427 us through a patch matrix, 128 -> 128 at 1216 x 832 354 us and 1320 us.
   if (a.conv_c > 0 && !gemm_act_pairs(a.act) && gemm_pair_accepts(a)) return gemm_pair_launch(a, 0, 0, stream);
+  if (a.conv_stats) return -3;
   if (a.conv_c > 0) {
     // implicit 3x3 convolution: tokens-as-M only; a 128-pixel tile is a run of one image row or whole rows
     const long hw = (long)a.conv_h * a.conv_w;

@@ -139,6 +139,8 @@ struct GemmArgs {
   float norm_eps = 0.f;
   const GemmPeerReduce* peer = nullptr;  // see GemmPeerReduce (decode cluster kernel only)
   int conv_n = 0, conv_h = 0, conv_w = 0, conv_c = 0;   // see GemmParams: A = NHWC activation, T = n h w, K = 9 c
+  float* conv_stats = nullptr;           // two-SM kernel only: see PairParams
+  int stats_groups = 0;
   float act_a = 0.f, act_b = 0.f;
   // two-SM kernel only (gemm_pair.cuh)
   const void* gate = nullptr;            // D = act(acc + bias) * gate[row / rows_per_gate] + residual

@@ -180,6 +180,9 @@ class OracleVaeEncoder(OracleVaeDecoder):
         return (moments[:, : cfg.z_channels] - cfg.shift_factor) * cfg.scale_factor
 
 
+GROUPS = 32      # of every norm of the decoder
+
+
 class VaeDecoderGpu:
     def __init__(self, cfg: VaeConfig, device: torch.device | None = None):
         self.cfg = cfg
@@ -208,9 +211,12 @@ class VaeDecoderGpu:
     def init_random(self, seed: int = 0) -> "VaeDecoderGpu":
         return self.load_state_dict(random_vae_weights(self.cfg, seed, device=self.device))
 
-    def _conv3(self, x, name, residual=None):
-        self.launches += 1 if ops.conv3x3_implicit(x, self.w[name + ".weight"].shape[0]) else 2
-        return ops.conv3x3_nhwc(x, self.w[name + ".weight"], self.w[name + ".bias"], residual)
+    def _conv3(self, x, name, residual=None, sums=None):
+        """The convolution and, where it adds them up for the norm behind it, its output's group sums. sums: room for those of a whole pass, taken in turn."""
+        w, bias = self.w[name + ".weight"], self.w[name + ".bias"]
+        mine = next(sums) if sums is not None and ops.conv3x3_sums(x, w, bias, residual, GROUPS) else None
+        self.launches += 1 if ops.conv3x3_implicit(x, w.shape[0]) else 2
+        return ops.conv3x3_nhwc(x, w, bias, residual, sums=mine), mine
 
     def _conv1(self, x, name, residual=None):
         N, H, W, C = x.shape
@@ -219,18 +225,18 @@ class VaeDecoderGpu:
         self.launches += 1
         return y.view(N, H, W, -1)
 
-    def _gn(self, x, name, silu):
-        self.launches += 2
-        return ops.groupnorm_nhwc(x, self.w[name + ".weight"], self.w[name + ".bias"], 32, 1e-6, silu)
+    def _gn(self, x, name, silu, sums=None):
+        self.launches += 2 if sums is None else 1
+        return ops.groupnorm_nhwc(x, self.w[name + ".weight"], self.w[name + ".bias"], GROUPS, 1e-6, silu, sums=sums)
 
-    def _res(self, x, name):
-        h = self._conv3(self._gn(x, name + ".norm1", True), name + ".conv1")
+    def _res(self, x, x_sums, name, sums):
+        h, h_sums = self._conv3(self._gn(x, name + ".norm1", True, x_sums), name + ".conv1", sums=sums)
         skip = self._conv1(x, name + ".nin_shortcut") if (name + ".nin_shortcut.weight") in self.w else x
-        return self._conv3(self._gn(h, name + ".norm2", True), name + ".conv2", residual=skip)
+        return self._conv3(self._gn(h, name + ".norm2", True, h_sums), name + ".conv2", residual=skip, sums=sums)
 
-    def _attn(self, x, name):
+    def _attn(self, x, x_sums, name):
         N, H, W, C = x.shape
-        h = self._gn(x, name + ".norm", False)
+        h = self._gn(x, name + ".norm", False, x_sums)
         q, k, v = (self._conv1(h, f"{name}.{n}").view(N, H * W, C) for n in "qkv")
         outs = []
         for b in range(N):
@@ -254,17 +260,19 @@ class VaeDecoderGpu:
         cfg = self.cfg
         self.launches = 0
         x = (z.float() / cfg.scale_factor + cfg.shift_factor).permute(0, 2, 3, 1).contiguous().bfloat16()
-        h = self._conv3(x, "decoder.conv_in")
-        h = self._res(h, "decoder.mid.block_1")
-        h = self._attn(h, "decoder.mid.attn_1")
-        h = self._res(h, "decoder.mid.block_2")
+        convs = sum(k.endswith(".weight") and ".conv" in k for k in self.w)
+        sums = iter(torch.zeros((convs, z.shape[0], GROUPS, 2), dtype=torch.float32, device=x.device))
+        h, s = self._conv3(x, "decoder.conv_in", sums=sums)
+        h, s = self._res(h, s, "decoder.mid.block_1", sums)
+        h, s = self._attn(h, s, "decoder.mid.attn_1"), None
+        h, s = self._res(h, s, "decoder.mid.block_2", sums)
         for lvl in reversed(range(len(cfg.ch_mult))):
             for i in range(cfg.num_res_blocks + 1):
-                h = self._res(h, f"decoder.up.{lvl}.block.{i}")
+                h, s = self._res(h, s, f"decoder.up.{lvl}.block.{i}", sums)
             if lvl != 0:
-                h = self._conv3(ops.upsample2x_nhwc(h), f"decoder.up.{lvl}.upsample.conv")
+                h, s = self._conv3(ops.upsample2x_nhwc(h), f"decoder.up.{lvl}.upsample.conv", sums=sums)
                 self.launches += 1
-        return self._conv3(self._gn(h, "decoder.norm_out", True), "decoder.conv_out")
+        return self._conv3(self._gn(h, "decoder.norm_out", True, s), "decoder.conv_out")[0]
 
     def decode_rgb8(self, z: torch.Tensor) -> torch.Tensor:
         return ops.rgb8_nhwc(self.decode(z))

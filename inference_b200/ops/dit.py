@@ -22,13 +22,20 @@ def axpy(a: float, x: torch.Tensor, b: float, y: torch.Tensor, out: torch.Tensor
 
 
 def groupnorm_nhwc(x: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, groups: int = 32, eps: float = 1e-6,
-                   silu: bool = False, out: torch.Tensor | None = None) -> torch.Tensor:
-    """x: [N, H, W, C] bf16 channels-last. GroupNorm with optional fused SiLU."""
+                   silu: bool = False, out: torch.Tensor | None = None, sums: torch.Tensor | None = None) -> torch.Tensor:
+    """x: [N, H, W, C] bf16 channels-last. GroupNorm with optional fused SiLU. sums fp32 [N, groups, 2]: each group's sum and sum of squares, where
+    the kernel that made x has them (see conv3x3_sums); x is then read once."""
     require_cuda(x)
     N, H, W, C = x.shape
     assert x.is_contiguous() and x.dtype == torch.bfloat16
     if out is None:
         out = torch.empty_like(x)
+    if sums is not None:
+        assert sums.shape == (N, groups, 2) and sums.dtype == torch.float32 and sums.is_contiguous()
+        rc = kernels().swb_groupnorm_apply(x.data_ptr(), sums.data_ptr(), gamma.data_ptr(), beta.data_ptr(), out.data_ptr(), N, H * W, C, groups,
+                                           eps, 1 if silu else 0, stream_ptr())
+        check(rc, "swb_groupnorm_apply")
+        return out
     stats = torch.empty((N, groups, 2), dtype=torch.float32, device=x.device)
     rc = kernels().swb_groupnorm(x.data_ptr(), stats.data_ptr(), gamma.data_ptr(), beta.data_ptr(), out.data_ptr(), N,
                                  H * W, C, groups, eps, 1 if silu else 0, stream_ptr())
@@ -77,12 +84,25 @@ def conv3x3_implicit(x: torch.Tensor, cout: int = 8) -> bool:
     return x.shape[0] * x.shape[1] * x.shape[2] > 64 and conv3x3_supported(x, cout)
 
 
+def _rows_of_16_bytes(bias: torch.Tensor | None, res2: torch.Tensor | None) -> bool:
+    return (bias is None or bias.data_ptr() % 16 == 0) and (res2 is None or (res2.data_ptr() % 16 == 0 and res2.stride(0) % 8 == 0))
+
+
+def conv3x3_sums(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, residual: torch.Tensor | None, groups: int) -> bool:
+    """Whether conv3x3_nhwc of these operands can add up the sums of its output for a norm over `groups` groups of channels."""
+    cout = w.shape[0]
+    res2 = residual.reshape(-1, cout) if residual is not None else None
+    return (cout % 8 == 0 and cout % groups == 0 and cout // groups in (4, 8, 16, 32) and _rows_of_16_bytes(bias, res2) and
+            conv3x3_implicit(x, cout) and os.environ.get("SWB_CONV3X3", "implicit") != "im2col")
+
+
 def conv3x3_nhwc(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, residual: torch.Tensor | None = None,
-                 act: str | None = None) -> torch.Tensor:
+                 act: str | None = None, sums: torch.Tensor | None = None) -> torch.Tensor:
     """3x3 convolution (stride 1, zero padding 1) of x [N, H, W, C] bf16 with w [Cout, 9 * C] (columns ordered ky, kx,
     c) -> [N, H, W, Cout], bias / activation / residual [N, H, W, Cout] in the epilogue. Implicit GEMM on the tcgen05
     kernel: the nine shifted views of x are fetched by TMA, no patch matrix is materialised. Shapes outside
-    `conv3x3_implicit` take the patch-gather + GEMM path."""
+    `conv3x3_implicit` take the patch-gather + GEMM path. sums fp32 [N, groups, 2] (where conv3x3_sums says so): the sum and the sum of squares of
+    each group of neighbouring output channels are added to it."""
     from .gemm import ACT, gemm_bf16
 
     require_cuda(x, w)
@@ -90,15 +110,16 @@ def conv3x3_nhwc(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = N
     Cout = w.shape[0]
     assert x.is_contiguous() and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[1] == 9 * C and w.stride(1) == 1
     res2 = residual.reshape(N * H * W, Cout) if residual is not None else None
-    rows_ok = ((bias is None or bias.data_ptr() % 16 == 0) and
-               (res2 is None or (res2.data_ptr() % 16 == 0 and res2.stride(0) % 8 == 0)))
+    rows_ok = _rows_of_16_bytes(bias, res2)
+    assert sums is None or (sums.dtype == torch.float32 and sums.is_contiguous() and sums.shape[::2] == (N, 2) and conv3x3_sums(x, w, bias, residual, sums.shape[1]))
     if not conv3x3_implicit(x, Cout if rows_ok else 1) or os.environ.get("SWB_CONV3X3", "implicit") == "im2col":
         return gemm_bf16(im2col3x3_nhwc(x), w, bias=bias, residual=res2, act=act).view(N, H, W, Cout)
     out = torch.empty((N * H * W, Cout), dtype=torch.bfloat16, device=x.device)
     if res2 is not None:
         assert res2.dtype == torch.bfloat16 and res2.stride(1) == 1
-    rc = kernels().swb_conv3x3_nhwc(x.data_ptr(), N, H, W, C, w.data_ptr(), w.stride(0), Cout, out.data_ptr(), out.stride(0),
-                                    ptr(bias), ptr(res2), res2.stride(0) if res2 is not None else 0, ACT[act], stream_ptr())
+    rc = kernels().swb_conv3x3_nhwc_stats(x.data_ptr(), N, H, W, C, w.data_ptr(), w.stride(0), Cout, out.data_ptr(), out.stride(0),
+                                          ptr(bias), ptr(res2), res2.stride(0) if res2 is not None else 0, ACT[act], ptr(sums),
+                                          sums.shape[1] if sums is not None else 0, stream_ptr())
     check(rc, "swb_conv3x3_nhwc")
     return out.view(N, H, W, Cout)
 

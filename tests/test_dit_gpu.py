@@ -75,6 +75,31 @@ def test_softmax_rows_of_any_width(cols, pad):
     assert ((p.double() - want).abs() <= want * (2.0 ** -8 + s.abs().amax(1, keepdim=True).clamp_max(1e6).nan_to_num(0) * 2.0 ** -23)).all()
 
 
+# groups of 4 to 32 channels; images that end inside a box of pixels and inside a pair of boxes; several column blocks and images of a CTA
+@pytest.mark.parametrize("N,H,W,C,cout,G", [(1, 9, 13, 64, 128, 32), (2, 40, 24, 128, 256, 32), (3, 17, 33, 64, 512, 32), (1, 64, 96, 64, 1024, 32),
+                                            (1, 31, 40, 64, 64, 16), (5, 9, 9, 64, 192, 12), (1, 200, 150, 64, 128, 32)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_convolution_adds_up_the_sums_of_its_output(N, H, W, C, cout, G, residual):
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(H + cout)
+    x = torch.randn(N, H, W, C, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(cout, 9 * C, device="cuda", generator=g) / (3 * C ** 0.5)).bfloat16()
+    bias = torch.randn(cout, device="cuda", generator=g).bfloat16()
+    res = torch.randn(N, H, W, cout, device="cuda", generator=g).bfloat16() if residual else None
+    assert ops.conv3x3_sums(x, w, bias, res, G) and not ops.conv3x3_sums(x, w, bias, res, cout // 2)
+    sums = torch.zeros(N, G, 2, device="cuda")
+    y = ops.conv3x3_nhwc(x, w, bias, res, sums=sums)
+    assert torch.equal(y, ops.conv3x3_nhwc(x, w, bias, res))
+    t = y.double().reshape(N, H * W, G, cout // G)
+    n = H * W * cout // G
+    assert ((sums[..., 0].double() - t.sum((1, 3))).abs() <= n * 2.0 ** -20 * t.abs().mean((1, 3))).all()      # fp32 sums, in parts of some thousand
+    assert ((sums[..., 1].double() - t.pow(2).sum((1, 3))).abs() <= n * 2.0 ** -20 * t.pow(2).mean((1, 3))).all()
+    gamma, beta = (torch.randn(cout, device="cuda", generator=g).bfloat16() for _ in range(2))
+    a, b = ops.groupnorm_nhwc(y, gamma, beta, G, silu=True, sums=sums), ops.groupnorm_nhwc(y, gamma, beta, G, silu=True)
+    assert (a.float() - b.float()).abs().max() <= 2.0 ** -7 * b.float().abs().max()
+
+
 def test_rope_in_place_updates_k_without_cache():
     from inference_b200 import ops
 
