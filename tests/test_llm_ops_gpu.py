@@ -105,6 +105,43 @@ def test_qk_norm_rope():
     assert torch.allclose(got, q, atol=4e-2, rtol=2e-2)
 
 
+# a CTA per 32 (16) heads of a token below 296 tokens, all of a token's heads from there on; heads that fill the last round in part; rows 16 bytes apart
+# from a whole vector go to the general kernel
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("T,Hq,Hkv,ld_extra", [(1, 1, 1, 0), (3, 40, 7, 8), (295, 5, 3, 0), (296, 33, 2, 0), (300, 7, 7, 0), (9, 3, 1, 2)])
+def test_rope_of_whole_heads(interleaved, T, Hq, Hkv, ld_extra):
+    from inference_b200 import ops
+
+    D, bs = 128, 16
+    g = torch.Generator(device="cuda").manual_seed(T + Hq)
+    width = (Hq + 2 * Hkv) * D
+    qkv = torch.randn(T, width + ld_extra, device="cuda", generator=g).bfloat16()[:, :width]
+    pos = torch.randint(0, 500, (T,), device="cuda", dtype=torch.int32, generator=g)
+    nblk = (T + bs - 1) // bs + 1
+    slots = torch.randperm(nblk * bs, device="cuda", generator=g)[:T].to(torch.int64)
+    slots[T // 2] = -1                      # this token's keys and values go to no cache
+    cos, sin = _rope_tables(512, D)
+    qw, kw = ((torch.rand(D, device="cuda", generator=g) + 0.5).bfloat16() for _ in range(2))
+    kc, vc = (torch.full((nblk, Hkv, bs, D), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    x = qkv.double().reshape(T, Hq + 2 * Hkv, D)
+    w = torch.cat([qw.double().expand(Hq, D), kw.double().expand(Hkv, D)])
+    n = (x[:, :Hq + Hkv] * (x[:, :Hq + Hkv].pow(2).mean(-1, keepdim=True) + 1e-6).rsqrt() * w).bfloat16().double()
+    c, s = cos[pos.long()].double()[:, None], sin[pos.long()].double()[:, None]
+    a, b = (n[..., 0::2], n[..., 1::2]) if interleaved else (n[..., :64], n[..., 64:])
+    ref = torch.stack([a * c - b * s, b * c + a * s], -1).flatten(-2) if interleaved else torch.cat([a * c - b * s, b * c + a * s], -1)
+    values = qkv.reshape(T, -1, D)[:, Hq + Hkv:].clone()
+    ops.rope_kv_write(qkv, pos, slots, cos, sin, kc, vc, Hq, Hkv, D, q_norm=qw, k_norm=kw, norm_eps=1e-6, interleaved=interleaved, block_size=bs)
+    got = qkv.reshape(T, -1, D)
+    bound = 2.0 ** -8 * 2 * n.abs().amax(-1, keepdim=True)      # a norm that falls to the other side of a rounding, and the rounding of the result
+    assert ((got[:, :Hq + Hkv].double() - ref).abs() <= bound).all()
+    blk, off = slots // bs, slots % bs
+    kept = slots >= 0
+    assert torch.equal(kc[blk, :, off][kept], got[:, Hq:Hq + Hkv][kept]) and torch.equal(vc[blk, :, off][kept], values[kept])
+    rest = torch.ones(nblk * bs, dtype=torch.bool, device="cuda")
+    rest[slots[kept]] = False
+    assert (kc.transpose(1, 2).reshape(nblk * bs, -1)[rest] == 7.0).all() and (vc.transpose(1, 2).reshape(nblk * bs, -1)[rest] == 7.0).all()
+
+
 def test_gated_act_embedding_argmax():
     from inference_b200 import ops
 
