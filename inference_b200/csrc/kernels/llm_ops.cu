@@ -102,7 +102,9 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_kernel(const bf16* __restrict
 }
 
 // LayerNorm without affine followed by adaLN modulation: out = LN(x) * (1 + scale) + shift, where
-// scale/shift are per-batch vectors (row / rows_per_batch selects the batch).
+// scale/shift are per-batch vectors (row / rows_per_batch selects the batch). Bound by the latency of a row's loads and sums: 1231 rows of 3072 columns take 6.6 us
+// (7.1 with 256 threads to a row, the second half of them without a second vector, and scale and shift requested behind the sums). A warp per row
+// took 8.6: its written-out code is longer than it runs.
 template <int THREADS, int VPT>
 __global__ void __launch_bounds__(THREADS) layernorm_mod_kernel(const bf16* __restrict__ x, int ldx,
                                                                const bf16* __restrict__ scale,
@@ -115,13 +117,26 @@ __global__ void __launch_bounds__(THREADS) layernorm_mod_kernel(const bf16* __re
   __shared__ float red[32];
   const int row = blockIdx.x;
   const int nvec = H / 8;
+  const int b = rows_per_batch > 0 ? row / rows_per_batch : 0;
   float vals[VPT][8];
+  uint4 raw[VPT], sc8[VPT], sh8[VPT];      // all that the row meets is requested before its first sum
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int v = threadIdx.x + i * THREADS;
+    if (v < nvec) raw[i] = *reinterpret_cast<const uint4*>(x + (size_t)row * ldx + v * 8);
+  }
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int v = threadIdx.x + i * THREADS;
+    if (v < nvec && scale) sc8[i] = *reinterpret_cast<const uint4*>(scale + (size_t)b * ld_mod + v * 8);
+    if (v < nvec && shift) sh8[i] = *reinterpret_cast<const uint4*>(shift + (size_t)b * ld_mod + v * 8);
+  }
   float s = 0.f;
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int v = threadIdx.x + i * THREADS;
     if (v < nvec) {
-      unpack8(*reinterpret_cast<const uint4*>(x + (size_t)row * ldx + v * 8), vals[i]);
+      unpack8(raw[i], vals[i]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) s += vals[i][j];
     }
@@ -140,7 +155,6 @@ __global__ void __launch_bounds__(THREADS) layernorm_mod_kernel(const bf16* __re
     }
   }
   const float inv = rsqrtf(block_sum<THREADS>(ss, red) / (float)H + eps);
-  const int b = rows_per_batch > 0 ? row / rows_per_batch : 0;
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int v = threadIdx.x + i * THREADS;
@@ -162,13 +176,13 @@ __global__ void __launch_bounds__(THREADS) layernorm_mod_kernel(const bf16* __re
       }
       if (scale) {
         float sc[8];
-        unpack8(*reinterpret_cast<const uint4*>(scale + (size_t)b * ld_mod + v * 8), sc);
+        unpack8(sc8[i], sc);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] *= (1.f + sc[j]);
       }
       if (shift) {
         float sh[8];
-        unpack8(*reinterpret_cast<const uint4*>(shift + (size_t)b * ld_mod + v * 8), sh);
+        unpack8(sh8[i], sh);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] += sh[j];
       }
@@ -851,13 +865,18 @@ int swb_layernorm_mod(const void* x, int ldx, const void* scale, const void* shi
   if (T <= 0) return 0;
   if (H % 8 != 0 || ldx % 8 != 0 || ldo % 8 != 0 || ld_mod % 8 != 0) return -3;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  return launch_norm(H, [&](auto TH, auto VP) {
+  const bf16 *px = reinterpret_cast<const bf16*>(x), *psc = reinterpret_cast<const bf16*>(scale), *psh = reinterpret_cast<const bf16*>(shift),
+             *pg = reinterpret_cast<const bf16*>(gamma), *pb = reinterpret_cast<const bf16*>(beta);
+  bf16* po = reinterpret_cast<bf16*>(out);
+  auto launch = [&](auto TH, auto VP) {
     constexpr int THREADS = decltype(TH)::value, VPT = decltype(VP)::value;
-    launch_rc = launch_kernel(layernorm_mod_kernel<THREADS, VPT>, dim3(T), dim3(THREADS), 0, s, reinterpret_cast<const bf16*>(x), ldx, reinterpret_cast<const bf16*>(scale),
-        reinterpret_cast<const bf16*>(shift), ld_mod, rows_per_batch, reinterpret_cast<const bf16*>(gamma),
-        reinterpret_cast<const bf16*>(beta), reinterpret_cast<bf16*>(out), ldo, H, eps);
+    launch_rc = launch_kernel(layernorm_mod_kernel<THREADS, VPT>, dim3(T), dim3(THREADS), 0, s, px, ldx, psc, psh, ld_mod, rows_per_batch, pg, pb, po, ldo, H,
+                              eps);
     return last_err();
-  });
+  };
+  // three whole vectors of 128 threads instead of one and a half of 256
+  if (H / 8 > 256 && H / 8 <= 384) return launch(std::integral_constant<int, 128>{}, std::integral_constant<int, 3>{});
+  return launch_norm(H, launch);
 }
 
 // fp32 = 1: qkv and both caches hold floats (q_norm_w / k_norm_w stay bf16). Dv: width of the v heads and of the v cache.

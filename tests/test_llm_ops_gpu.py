@@ -49,6 +49,21 @@ def test_layernorm_mod_and_gated_residual():
     assert torch.allclose(z.float(), refz, atol=3e-2, rtol=2e-2)
 
 
+# one, two and three vectors of a thread, the last of them in part; rows further apart than they are long
+@pytest.mark.parametrize("T,H,per,ld", [(1, 1024, 0, 1024), (5, 1032, 3, 1040), (7, 2048, 2, 2048), (9, 2056, 4, 2056), (6, 3072, 5, 3080), (3, 3080, 1, 3080)])
+def test_layernorm_of_any_width(T, H, per, ld):
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(H)
+    x = (torch.randn(T, ld, device="cuda", generator=g) * 3 + 20).bfloat16()[:, :H]
+    B = (T + per - 1) // per if per else 1
+    mods = [(torch.randn(B, H, device="cuda", generator=g) * 0.3).bfloat16() for _ in range(2)]
+    y = ops.layernorm_mod(x, scale=mods[0], shift=mods[1], rows_per_batch=per or T)
+    rows = torch.arange(T, device="cuda") // (per or T)
+    want = torch.nn.functional.layer_norm(x.double(), (H,), eps=1e-6) * (1 + mods[0].double()[rows]) + mods[1].double()[rows]
+    assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()      # fp32 sums of values that are 7 times their spread
+
+
 @pytest.mark.parametrize("interleaved", [False, True])
 @pytest.mark.parametrize("D,rot", [(128, 128), (64, 64), (128, 64), (96, 32)])
 def test_rope_kv_write(interleaved, D, rot):
