@@ -180,6 +180,10 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
                                    c_int, c_int, c_int, c_int, c_float, c_void_p])
     sig("swb_attn_paged_prefill_tc", [c_void_p, c_ll, c_int, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p])
+    sig("swb_attn_paged_prefill_split", [c_void_p, c_ll, c_int, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                      c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_size_t, c_void_p])
+    sig("swb_attn_prefill_splits", [c_int, c_int, c_int, c_int, c_ll])
+    sig("swb_attn_prefill_part_bytes", [c_int, c_int, c_int], c_size_t)
     sig("swb_attn_dense_scatter", [c_void_p, c_ll, c_int, c_void_p, c_void_p, c_ll, c_int, c_void_p, c_int,
                                    c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                                    c_void_p])
@@ -227,12 +231,12 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
     sig("swb_im2col3x3", [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
     sig("swb_conv3x3_nhwc", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p,
                              c_int, c_int, c_void_p])
+    sig("swb_conv3x3_nhwc_stats", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p,
+                             c_int, c_int, c_void_p, c_int, c_void_p])
     sig("swb_softmax_rows", [c_void_p, c_void_p, c_int, c_int, c_ll, c_ll, c_float, c_void_p])
     sig("swb_rgb8", [c_void_p, c_void_p, c_ll, c_int, c_void_p])
     sig("swb_comm_max_ctas", [])
     sig("swb_comm_flag_words", [])
-    sig("swb_conv3x3_nhwc_stats", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p,
-                             c_int, c_int, c_void_p, c_int, c_void_p])
     sig("swb_allreduce_rmsnorm", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int,
                                   c_void_p, c_float, c_float, c_void_p, c_int, c_void_p])
     sig("swb_flag_wait", [c_void_p, ctypes.c_uint, c_void_p, c_void_p])

@@ -586,10 +586,11 @@ int swb_attn_varlen_causal(const void* q, long long q_stride_tok, int q_stride_h
 // pages block_table[s, :]; its queries sit at the last positions (bottom-right aligned causal mask). Caches:
 // [num_blocks, Hkv, block_size, 128] contiguous, block_size a multiple of 8 dividing 128. Returns -3 when the problem
 // is outside the kernel's reach (the caller then takes swb_attn_paged).
-int swb_attn_paged_prefill_tc(const void* q, long long q_stride_tok, int q_stride_head, void* out, long long out_stride_tok,
+int swb_attn_paged_prefill_split(const void* q, long long q_stride_tok, int q_stride_head, void* out, long long out_stride_tok,
                               const void* kcache, const void* vcache, const int* block_table, int max_blocks,
                               int block_size, int num_blocks, const int* cu_q, const int* kv_lens, int num_seqs,
-                              int max_q_len, int total_tokens, int Hq, int Hkv, float scale, int causal, void* stream) {
+                              int max_q_len, int total_tokens, int Hq, int Hkv, float scale, int causal, int splits, void* parts,
+                                 size_t part_bytes, void* stream) {
   using namespace swb;
   if (num_seqs <= 0 || total_tokens <= 0) return 0;
   if (g_dense_impl != 0 || !cu_q || !kv_lens || !block_table || max_q_len <= 0 || Hq % Hkv != 0) return -3;
@@ -598,8 +599,20 @@ int swb_attn_paged_prefill_tc(const void* q, long long q_stride_tok, int q_strid
   return attn_dense_tcgen05_launch(q, q_stride_tok, q_stride_head, kcache, vcache, 128, 128, out, out_stride_tok,
                                    num_seqs, max_q_len, max_q_len, Hq, Hkv, scale, reinterpret_cast<cudaStream_t>(stream),
                                    nullptr, 0, 0, 0, 0, 0, causal, cu_q, total_tokens, 128, kv_lens, block_table,
-                                   max_blocks, block_size, num_blocks);
+                                   max_blocks, block_size, num_blocks, splits, parts, part_bytes);
 }
+int swb_attn_paged_prefill_tc(const void* q, long long q_stride_tok, int q_stride_head, void* out, long long out_stride_tok,
+                              const void* kcache, const void* vcache, const int* block_table, int max_blocks,
+                              int block_size, int num_blocks, const int* cu_q, const int* kv_lens, int num_seqs,
+                              int max_q_len, int total_tokens, int Hq, int Hkv, float scale, int causal, void* stream) {
+  return swb_attn_paged_prefill_split(q, q_stride_tok, q_stride_head, out, out_stride_tok, kcache, vcache, block_table, max_blocks, block_size, num_blocks,
+                                      cu_q, kv_lens, num_seqs, max_q_len, total_tokens, Hq, Hkv, scale, causal, 1, nullptr, 0, stream);
+}
+// How many splits of the keys a step should take (contexts of up to max_kv tokens), and the bytes of their parts (16-byte aligned; the call's own).
+int swb_attn_prefill_splits(int max_q_len, int total_tokens, int Hq, int num_seqs, long long max_kv) {
+  return swb::attn_prefill_splits(max_q_len, total_tokens, Hq, num_seqs, max_kv);
+}
+size_t swb_attn_prefill_part_bytes(int total_tokens, int Hq, int splits) { return swb::attn_prefill_part_bytes(total_tokens, Hq, splits); }
 
 // Attention with per-tensor head widths, chunked masking and sinks over the paged cache (kcache [num_blocks, Hkv,
 // block_size, D], vcache [num_blocks, Hkv, block_size, Dv], contiguous) or, with block_table == nullptr, over fresh keys

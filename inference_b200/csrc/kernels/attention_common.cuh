@@ -103,7 +103,10 @@ int attn_dense_tcgen05_launch(const void* q, long long q_stride_tok, int q_strid
                               void* const* peers = nullptr, int world = 0, int split = 0, int n0 = 0, int n1 = 0,
                               int col_offset = 0, int causal = 0, const int* cu_q = nullptr, int total_tokens = 0,
                               int head_dim = 128, const int* kv_lens = nullptr, const int* block_table = nullptr,
-                              int max_blocks = 0, int block_size = 0, int num_blocks = 0);
+                              int max_blocks = 0, int block_size = 0, int num_blocks = 0, int splits = 1, void* parts = nullptr,
+                              size_t part_bytes = 0);
+int attn_prefill_splits(int max_q_len, int total_tokens, int Hq, int num_seqs, long long max_kv);
+size_t attn_prefill_part_bytes(int total_tokens, int Hq, int splits);
 int attn_ext_tcgen05_launch(const void* q, long long q_stride_tok, const void* k, long long k_stride_tok, const void* v,
                             long long v_stride_tok, void* out, long long out_stride_tok, int num_seqs, int max_q_len,
                             int total_tokens, int Hq, int Hkv, int D, int Dv, float scale, int chunk, const float* sink,

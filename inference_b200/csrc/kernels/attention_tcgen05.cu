@@ -78,6 +78,12 @@ struct FaParams {
   const int* kv_lens;
   const int* block_table;
   int max_blocks, block_size;
+  // Paged problems may split the keys (plain instantiation): CTAs of split z take the z-th part of the key tiles that their rows see and leave
+  // un-normalised rows in part_o [split][head][rows][VD] with their maximum (log2 units) and sum in part_ml, for attn_split_merge_kernel.
+  int splits;
+  long long part_rows;
+  float* part_o;
+  float2* part_ml;
   // Extended problems (the EXT instantiations only):
   int chunk;           // > 0: query i sees key j <= i only if floor(i / chunk) == floor(j / chunk), positions of the sequence
   const float* sink;   // optional [Hq]: exp(sink[h]) joins the softmax denominator (no key, no value, not scaled)
@@ -246,7 +252,7 @@ constexpr int FMA_EVERY = 8;   // one of the four pairs of exponentials of every
 
 template <typename C>
 __device__ __forceinline__ void softmax_halves(const FaParams& p, Barriers* bars, uint8_t* smem, uint32_t tmem, int q_base, int q_len, int kv_len,
-                                               int coff, int n_tiles, int tok0, int batch, int head) {
+                                               int coff, int n_tiles, int tok0, int batch, int head, int j0, int split) {
   constexpr int VD = C::ROW_BYTES / 2, KEYS = BN / 2, OUT = VD / 2;         // scores and output columns of a thread
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = warp >> 3, half = (warp >> 2) & 1, w4 = warp & 3;
@@ -272,7 +278,7 @@ __device__ __forceinline__ void softmax_halves(const FaParams& p, Barriers* bars
       tmem_ld_x32(t_s + half * KEYS, s);
       tmem_ld_x32(t_s + half * KEYS + 32, s + 32);
       tmem_ld_wait();
-      const int key0 = j * BN + half * KEYS;
+      const int key0 = (j + j0) * BN + half * KEYS;
       if (key0 + KEYS > kv_len || (p.causal && key0 + KEYS > q_base + q * BM + coff)) {
 #pragma unroll
         for (int i = 0; i < KEYS; ++i)
@@ -313,7 +319,7 @@ __device__ __forceinline__ void softmax_halves(const FaParams& p, Barriers* bars
         }
       }
     }
-    const float neg_m = -m_used * scale_log2;
+    const float neg_m = m_used == -INFINITY ? 0.f : -m_used * scale_log2;     // no key of a split so far is visible to this row
     const unsigned long long sc2 = pack2(scale_log2, scale_log2), nm2 = pack2(neg_m, neg_m);
     unsigned long long l0 = 0ull, l1 = 0ull;                                // two sums of +0 each
 #pragma unroll
@@ -351,6 +357,23 @@ __device__ __forceinline__ void softmax_halves(const FaParams& p, Barriers* bars
   if (!ok) return;
   tc_fence_after_sync();
   const float sum = half ? other + l : l + other, inv = sum > 0.f ? 1.f / sum : 0.f;
+  if (p.splits > 1) {
+    const long long at = ((long long)split * p.Hq + head) * p.part_rows + tok0 + row;
+#pragma unroll
+    for (int c = 0; c < OUT / 32; ++c) {
+      uint32_t o[32];
+      tmem_ld_x32(t_o + c * 32, o);
+      tmem_ld_wait();
+      if (row < q_len) {
+        float4* to = reinterpret_cast<float4*>(p.part_o + at * VD + half * OUT + c * 32);
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+          to[v] = make_float4(__uint_as_float(o[v * 4]), __uint_as_float(o[v * 4 + 1]), __uint_as_float(o[v * 4 + 2]), __uint_as_float(o[v * 4 + 3]));
+      }
+    }
+    if (half == 0 && row < q_len) p.part_ml[at] = make_float2(m_used * scale_log2, sum);
+    return;
+  }
   // Stage this warp's 32 rows x OUT columns in the (now idle) Q region, then write every row with OUT / 8 lanes x 16 bytes. 16-byte chunk
   // c of row r sits at c ^ (r & (chunks - 1)).
   constexpr int BYTES = OUT * 2, CHUNKS = BYTES / 16;
@@ -421,7 +444,10 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   constexpr int TILE_STEP = DIFF ? 0 : BM;                  // query rows between the two tiles of a CTA
   const int cta_rows = DIFF ? BM : p.tiles * BM;
   // causal blocks: the last queries see the most keys and start first
-  const int q_base = (p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x) * cta_rows;
+  constexpr bool PLAIN = HALVES == 2;                         // p.splits is looked at
+  const int row_tiles = PLAIN && p.splits > 1 ? (int)gridDim.x / p.splits : (int)gridDim.x;
+  const int split = PLAIN && p.splits > 1 ? (int)blockIdx.x / row_tiles : 0, row_tile = (int)blockIdx.x - split * row_tiles;
+  const int q_base = (p.causal ? row_tiles - 1 - row_tile : row_tile) * cta_rows;
   constexpr bool WIDE = EXT && !LAT && DIFF == 0;             // v_heads and out_gate are looked at
   const int head = WIDE && p.v_heads > 0 ? blockIdx.y / p.v_heads : blockIdx.y;
   // packed variable-length batch: this CTA's sequence covers tokens [tok0, tok0 + q_len) of one flat token axis
@@ -442,8 +468,15 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
     if (p.window > 0) first = max(first, pos - p.window + 1);
     return first;
   };
-  const int j0 = EXT ? first_key_of(q_base + coff) / BN : 0;
-  const int n_tiles = (kv_end + BN - 1) / BN - j0;
+  const int all_tiles = (kv_end + BN - 1) / BN, per_split = PLAIN && p.splits > 1 ? (all_tiles + p.splits - 1) / p.splits : all_tiles;
+  const int j0 = EXT ? first_key_of(q_base + coff) / BN : split * per_split;
+  const int n_tiles = EXT ? all_tiles - j0 : min(all_tiles, j0 + per_split) - j0;
+  if (PLAIN && n_tiles <= 0) {      // fewer key tiles than splits; uniform for the whole CTA
+    pdl_wait();
+    for (int r = threadIdx.x; r < cta_rows && q_base + r < q_len; r += blockDim.x)
+      p.part_ml[((long long)split * p.Hq + head) * p.part_rows + tok0 + q_base + r] = make_float2(-INFINITY, 0.f);
+    return;
+  }
   volatile int* abort_flag = &bars->abort;
 
   if (threadIdx.x == 0) {
@@ -614,7 +647,7 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
       __syncwarp();
     }
   } else if constexpr (HALVES == 2) {
-    softmax_halves<C>(p, bars, smem, tmem, q_base, q_len, kv_len, coff, n_tiles, tok0, batch, head);
+    softmax_halves<C>(p, bars, smem, tmem, q_base, q_len, kv_len, coff, n_tiles, tok0, batch, head, j0, split);
   } else {
     // ------------------------------------------------------------------ softmax warpgroups (thread = query row)
     const int q = warp >> 2;
@@ -966,6 +999,36 @@ int make_tmap_heads(CUtensorMap* out, const void* ptr, int hd, int heads, int to
 
 }  // namespace
 
+namespace {
+
+// Sum of the splits of a row and head: a warp each, a lane has four columns.
+__global__ void __launch_bounds__(256) attn_split_merge_kernel(const float* __restrict__ part_o, const float2* __restrict__ part_ml, int splits,
+                                                              long long rows, int Hq, bf16* out, long long out_stride) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);      // heads run fastest: a row of the output is written together
+  const int lane = threadIdx.x & 31;
+  if (i >= rows * Hq) return;
+  const long long row = i / Hq, head = i - row * Hq;
+  float top = -INFINITY;
+  for (int s = 0; s < splits; ++s) top = fmaxf(top, part_ml[(s * Hq + head) * rows + row].x);
+  float sum = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s = 0; s < splits; ++s) {
+    const long long at = (s * Hq + head) * rows + row;
+    const float2 ml = part_ml[at];
+    if (ml.y <= 0.f) continue;                                             // no key of this split was visible (its rows may not have been written)
+    const float w = ex2(ml.x - top);
+    const float4 o = *reinterpret_cast<const float4*>(part_o + at * 128 + lane * 4);
+    sum = fmaf(w, ml.y, sum);
+    acc.x = fmaf(w, o.x, acc.x), acc.y = fmaf(w, o.y, acc.y), acc.z = fmaf(w, o.z, acc.z), acc.w = fmaf(w, o.w, acc.w);
+  }
+  const float inv = sum > 0.f ? 1.f / sum : 0.f;
+  store_row4(out + row * out_stride + head * 128 + lane * 4, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
+}
+
+}  // namespace
+
 int g_force_tiles = 0;   // 0: choose per problem; 1 / 2: fixed query tiles per CTA (comparison runs)
 void attn_dense_tcgen05_set_tiles(int tiles) { g_force_tiles = tiles; }
 
@@ -1005,8 +1068,8 @@ int launch_tiles(int qk, FaKind kind, int q_len, int Hq, int batch, cudaStream_t
   const int sms = 148;
   const long c2 = (long)((q_len + 2 * BM - 1) / (2 * BM)) * Hq * batch, c1 = (long)((q_len + BM - 1) / BM) * Hq * batch;
   const double t2 = (double)((c2 + sms - 1) / sms), t1 = 0.85 * (double)((c1 + sms - 1) / sms);
-  p.tiles = (g_force_tiles == 1 || g_force_tiles == 2) ? g_force_tiles : (t1 < t2 ? 1 : 2);
-  const dim3 grid((q_len + p.tiles * BM - 1) / (p.tiles * BM), Hq, batch);
+  p.tiles = (g_force_tiles == 1 || g_force_tiles == 2) ? g_force_tiles : (t1 < t2 && p.splits <= 1 ? 1 : 2);
+  const dim3 grid((q_len + p.tiles * BM - 1) / (p.tiles * BM) * (p.splits > 1 ? p.splits : 1), Hq, batch);
   if (kind == FaKind::LATENT)
     return qk == 192 ? launch_fa<192, 128, true, true>(grid, stream, m, p) : launch_fa<128, 128, true, true>(grid, stream, m, p);
   if (kind == FaKind::EXT) {
@@ -1034,7 +1097,7 @@ int attn_dense_tcgen05_launch(const void* q, long long q_stride_tok, int q_strid
                               int batch, int q_len, int kv_len, int Hq, int Hkv, float scale, cudaStream_t stream,
                               void* const* peers, int world, int split, int n0, int n1, int col_offset, int causal,
                               const int* cu_q, int total_tokens, int head_dim, const int* kv_lens,
-                              const int* block_table, int max_blocks, int block_size, int num_blocks) {
+                              const int* block_table, int max_blocks, int block_size, int num_blocks, int splits, void* parts, size_t part_bytes) {
   if (head_dim != 64 && head_dim != 128) return -3;
   const bool paged = block_table != nullptr;
   if (paged && (head_dim != 128 || !cu_q || !kv_lens || block_size < 8 || block_size % 8 || BN % block_size ||
@@ -1076,7 +1139,38 @@ int attn_dense_tcgen05_launch(const void* q, long long q_stride_tok, int q_strid
     p.scatter.n1 = n1;
     p.scatter.col_offset = col_offset;
   }
-  return launch_tiles(head_dim, FaKind::DENSE, q_len, Hq, batch, stream, m, p);
+  if (splits > 1) {
+    if (!paged || !parts || part_bytes < attn_prefill_part_bytes(total_tokens, Hq, splits) || (reinterpret_cast<uintptr_t>(parts) & 15)) return -5;
+    p.splits = splits;
+    p.part_rows = total_tokens;
+    p.part_o = reinterpret_cast<float*>(parts);
+    p.part_ml = reinterpret_cast<float2*>(p.part_o + (size_t)splits * Hq * total_tokens * 128);
+  }
+  rc = launch_tiles(head_dim, FaKind::DENSE, q_len, Hq, batch, stream, m, p);
+  if (rc || splits <= 1) return rc;
+  const long long warps = (long long)total_tokens * Hq;
+  return launch_kernel(attn_split_merge_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, stream, (const float*)p.part_o, (const float2*)p.part_ml,
+                       splits, (long long)total_tokens, Hq, reinterpret_cast<bf16*>(out), out_stride_tok);
+}
+
+size_t attn_prefill_part_bytes(int total_tokens, int Hq, int splits) { return splits > 1 ? (size_t)splits * Hq * total_tokens * (128 * 4 + 8) : 0; }
+
+// Splits of the keys of a paged prompt step: its CTAs have 256 rows of a head each, one to an SM, so that few rows on a long context leave SMs idle or
+// a last wave nearly empty. Microseconds: 2.5 per 128 keys of a CTA, 4 for its start and end; parts are written and read back at about 4 TB/s. 700 rows x
+// 32 heads on 5900 cached tokens are 96 CTAs of 52 key tiles: 124 us whole, 146, 115 and 136 in 2, 3 and 4 parts. 512 rows on 6000: 110, 79, 109, 93; 45 on
+// 6000: 103, 62, 46, 40; 1500 on 4000: 191, 188, 196, 232.
+int attn_prefill_splits(int max_q_len, int total_tokens, int Hq, int num_seqs, long long max_kv) {
+  const long ctas = (long)((max_q_len + 2 * BM - 1) / (2 * BM)) * Hq * num_seqs;
+  const int sms = 148;
+  const long tiles = (long)((max_kv + BN - 1) / BN);
+  double best = 1e30;
+  int best_s = 1;
+  for (int s = 1; s <= 8 && (s == 1 || tiles / s >= 4); ++s) {
+    const double t = (double)((ctas * s + sms - 1) / sms) * (2.5 * (double)((tiles + s - 1) / s) + 4.0) +
+                     (s > 1 ? 5.0 + (double)total_tokens * Hq * 1024.0 * s / 4e6 : 0.0);
+    if (t < 0.95 * best) best = t, best_s = s;
+  }
+  return best_s;
 }
 
 // Attention over queries and keys of any head widths up to 128 (multiples of 8), with chunked masking and sinks: the

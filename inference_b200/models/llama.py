@@ -430,6 +430,8 @@ class LlamaGpu:
         pf = (lambda t: t if (pf_bytes >= 0 and isinstance(t, torch.Tensor)) else None)
         ssq = (self._ssq if self.quant_format is None else torch.empty((2, ops.SSQ_WORDS), dtype=torch.int64, device=self.device).unbind(0)) if chain else None
         packed = chain and self.quant_format is not None
+        normed = ops.linear_normed if packed else ops.gemm_bf16_normed
+        prefill_splits = None
         ssq_prev = None                 # partial sums of squares of `res` (valid while branch is None)
         H = cfg.hidden_size
         moe_counters = ops.routing_counters(cfg.moe.num_experts, self.device) if self.has_moe else None
@@ -444,9 +446,9 @@ class LlamaGpu:
                 h = ops.rmsnorm(branch, L.ln1, eps, residual=res, w_offset=woff, prefetch=pf(L.qkv),
                                 prefetch_bytes=pf_bytes)
             if h is None:
-                qkv = ops.linear_normed(res, L.qkv, bias=L.qkv_bias, ssq_in=ssq_prev, norm_dim=H, eps=eps)
+                qkv = normed(res, L.qkv, bias=L.qkv_bias, ssq_in=ssq_prev, norm_dim=H, eps=eps)
             elif packed:       # the step's own accumulators: the first product clears what the next one adds to
-                qkv = ops.linear_normed(h, L.qkv, bias=L.qkv_bias, ssq_zero=ssq[0])
+                qkv = normed(h, L.qkv, bias=L.qkv_bias, ssq_zero=ssq[0])
             else:
                 qkv = ops.linear_any(h, L.qkv, bias=L.qkv_bias)
             ops.rope_kv_write(qkv, rope_pos, inp.slot_mapping, rope_cos, rope_sin, kv_pool[li, 0], kv_pool[li, 1],
@@ -461,10 +463,14 @@ class LlamaGpu:
                                                    qkv[:, q_cols + kv_cols:].view(T, self.hkv, D), inp.cu_q,
                                                    inp.max_q_len, scale=cfg.attn_scale)
             else:
+                if prefill_splits is None:
+                    on_tc = ops.paged_prefill_on_tensor_memory(q, kv_pool[li, 0], cfg.attn_logit_softcap or 0.0, inp.decode)
+                    prefill_splits = ops.paged_prefill_splits(q, inp.block_table, inp.num_seqs, inp.max_q_len, block_size) if on_tc else 1
                 attn = ops.paged_attention(q, kv_pool[li, 0], kv_pool[li, 1], inp.block_table, inp.kv_lens,
                                            cu_q=inp.cu_q, max_q_len=inp.max_q_len, scale=cfg.attn_scale, causal=True,
                                            decode=inp.decode, num_splits=inp.attn_splits,
-                                           softcap=cfg.attn_logit_softcap or 0.0)
+                                           softcap=cfg.attn_logit_softcap or 0.0, prefill_splits=prefill_splits)
+                n += prefill_splits > 1         # the sum of the splits
             if chain:
                 if branch is not None:          # first layer of the chain: fold the pending branch into the stream
                     res.add_(branch)
@@ -477,14 +483,14 @@ class LlamaGpu:
                 if fc is not None:
                     fc.gemm_peer_reduce(attn.reshape(T, -1), L.o, res, 0, ssq_out=ssq[0], ssq_zero=ssq[1])
                 else:
-                    ops.linear_normed(attn.reshape(T, -1), L.o, out=res, residual=res, ssq_out=ssq[0],
+                    normed(attn.reshape(T, -1), L.o, out=res, residual=res, ssq_out=ssq[0],
                                          ssq_zero=ssq[1])
-                act = ops.linear_normed(res, L.gate_up, act="geglu_pairs" if gelu else "swiglu_pairs",
+                act = normed(res, L.gate_up, act="geglu_pairs" if gelu else "swiglu_pairs",
                                            ssq_in=ssq[0], norm_dim=H, eps=eps)
                 if fc is not None:
                     fc.gemm_peer_reduce(act, L.down, res, 1, ssq_out=ssq[1], ssq_zero=ssq[0])
                 else:
-                    ops.linear_normed(act, L.down, out=res, residual=res, ssq_out=ssq[1],
+                    normed(act, L.down, out=res, residual=res, ssq_out=ssq[1],
                                          ssq_zero=ssq[0])
                 ssq_prev, pending_h = ssq[1], None
                 n += 6 + (1 if h is not None else 0)

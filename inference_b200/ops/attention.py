@@ -22,17 +22,29 @@ def decode_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     return ws
 
 
+def paged_prefill_on_tensor_memory(q: torch.Tensor, kcache: torch.Tensor, softcap: float, decode: bool) -> bool:
+    bs = kcache.shape[2]
+    return (not decode and q.shape[2] == 128 and softcap == 0.0 and bs % 8 == 0 and 128 % bs == 0
+            and os.environ.get("SWB_PAGED_PREFILL", "tcgen05") != "legacy")
+
+
+def paged_prefill_splits(q: torch.Tensor, block_table: torch.Tensor, num_seqs: int, max_q_len: int, block_size: int) -> int:
+    """Parts into which a prompt step on cached context splits its keys: more than one costs a second launch, which sums them."""
+    return kernels().swb_attn_prefill_splits(max_q_len, q.shape[0], q.shape[1], num_seqs, block_table.shape[1] * block_size)
+
+
 def paged_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, block_table: torch.Tensor,
                     kv_lens: torch.Tensor, *, cu_q: torch.Tensor | None, max_q_len: int, scale: float,
                     causal: bool = True, decode: bool = False, num_splits: int = 1, softcap: float = 0.0,
                     out: torch.Tensor | None = None, workspace: torch.Tensor | None = None,
-                    use_tma: bool = True) -> torch.Tensor:
+                    use_tma: bool = True, prefill_splits: int | None = None) -> torch.Tensor:
     """q: [T, Hq, 128] (any token/head strides, unit inner stride); caches [blocks, Hkv, block_size, 128];
     block_table int32 [num_seqs, max_blocks]; kv_lens int32 [num_seqs] (context length including the new
     tokens); cu_q int32 [num_seqs + 1] or None when every sequence has exactly max_q_len query tokens.
     Bottom-right aligned causal mask like the reference SDPA (candle-llm/src/primitives/attention.rs:154-186).
     Prefill (decode=False) with page sizes that divide 128 and no soft cap runs on the tcgen05 kernel, which reads the
-    pages through TMA; SWB_PAGED_PREFILL=legacy keeps the mma.sync kernel (comparison runs)."""
+    pages through TMA; SWB_PAGED_PREFILL=legacy keeps the mma.sync kernel (comparison runs). prefill_splits: parts that its keys are
+    split into (default: paged_prefill_splits)."""
     require_cuda(q, kcache, vcache, block_table, kv_lens)
     T, Hq, D = q.shape
     Hkv, bs = kcache.shape[1], kcache.shape[2]
@@ -41,17 +53,19 @@ def paged_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor,
     num_seqs = kv_lens.numel()
     if out is None:
         out = torch.empty((T, Hq * D), dtype=q.dtype, device=q.device)
-    if (not decode and D == 128 and softcap == 0.0 and use_tma and bs % 8 == 0 and 128 % bs == 0
-            and os.environ.get("SWB_PAGED_PREFILL", "tcgen05") != "legacy"):
+    if paged_prefill_on_tensor_memory(q, kcache, softcap, decode) and use_tma:
         if cu_q is None:
             cu_q = torch.arange(num_seqs + 1, dtype=torch.int32, device=q.device) * max_q_len
-        rc = kernels().swb_attn_paged_prefill_tc(q.data_ptr(), q.stride(0), q.stride(1), out.data_ptr(), out.stride(0),
-                                                 kcache.data_ptr(), vcache.data_ptr(), block_table.data_ptr(),
-                                                 block_table.stride(0), bs, kcache.shape[0], cu_q.data_ptr(),
-                                                 kv_lens.data_ptr(), num_seqs, max_q_len, T, Hq, Hkv, scale,
-                                                 1 if causal else 0, stream_ptr())
+        splits = paged_prefill_splits(q, block_table, num_seqs, max_q_len, bs) if prefill_splits is None else prefill_splits
+        nbytes = kernels().swb_attn_prefill_part_bytes(T, Hq, splits)
+        parts = torch.empty(nbytes, dtype=torch.uint8, device=q.device) if nbytes else None
+        rc = kernels().swb_attn_paged_prefill_split(q.data_ptr(), q.stride(0), q.stride(1), out.data_ptr(), out.stride(0),
+                                                    kcache.data_ptr(), vcache.data_ptr(), block_table.data_ptr(),
+                                                    block_table.stride(0), bs, kcache.shape[0], cu_q.data_ptr(),
+                                                    kv_lens.data_ptr(), num_seqs, max_q_len, T, Hq, Hkv, scale,
+                                                    1 if causal else 0, splits, ptr(parts), nbytes, stream_ptr())
         if rc != -3:
-            check(rc, "swb_attn_paged_prefill_tc")
+            check(rc, "swb_attn_paged_prefill_split")
             return out
     ws_ptr, ws_bytes = None, 0
     if decode and num_splits > 1:

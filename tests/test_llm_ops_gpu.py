@@ -157,6 +157,42 @@ def test_rope_of_whole_heads(interleaved, T, Hq, Hkv, ld_extra):
     assert (kc.transpose(1, 2).reshape(nblk * bs, -1)[rest] == 7.0).all() and (vc.transpose(1, 2).reshape(nblk * bs, -1)[rest] == 7.0).all()
 
 
+# sequences with fewer key tiles than parts, rows that see no key of the last part, one row, a last tile that ends inside a page
+@pytest.mark.parametrize("splits", [2, 3, 8])
+@pytest.mark.parametrize("news,olds,Hq,Hkv,bs", [([700], [1900], 4, 2, 16), ([130, 1, 300], [1000, 2500, 0], 2, 1, 32), ([5, 257], [3, 640], 3, 3, 64)])
+def test_paged_prefill_with_split_keys(news, olds, Hq, Hkv, bs, splits):
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(sum(news))
+    T, lens = sum(news), [n + o for n, o in zip(news, olds)]
+    need = [(x + bs - 1) // bs for x in lens]
+    perm = torch.randperm(sum(need), device="cuda", generator=g).int()
+    table = torch.zeros(len(news), max(need), dtype=torch.int32, device="cuda")
+    for i, parts in enumerate(perm.split(need)):
+        table[i, :need[i]] = parts
+    kc, vc = (torch.randn(sum(need), Hkv, bs, 128, device="cuda", generator=g).bfloat16() for _ in range(2))
+    q = torch.randn(T, Hq, 128, device="cuda", generator=g).bfloat16() * 2
+    cu = torch.tensor([0, *torch.tensor(news).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
+    kvl = torch.tensor(lens, dtype=torch.int32, device="cuda")
+
+    def run(n):
+        return ops.paged_attention(q, kc, vc, table, kvl, cu_q=cu, max_q_len=max(news), scale=128 ** -0.5, prefill_splits=n).double()
+
+    whole, split = run(1), run(splits)
+    ops.check_status()
+    want, at = torch.empty_like(whole), 0
+    for i, (n, o) in enumerate(zip(news, olds)):
+        rows = table[i, :need[i]].long()
+        k, v = (c[rows].transpose(1, 2).reshape(-1, Hkv, 128)[:n + o].double().repeat_interleave(Hq // Hkv, 1) for c in (kc, vc))
+        s = torch.einsum("qhd,khd->hqk", q[at:at + n].double(), k) * 128 ** -0.5
+        seen = torch.arange(n + o, device="cuda")[None] <= torch.arange(o, o + n, device="cuda")[:, None]
+        want[at:at + n] = torch.einsum("hqk,khd->qhd", s.masked_fill(~seen, -math.inf).softmax(-1), v).reshape(n, -1)
+        at += n
+    # probabilities in bf16 on both sides, rounded against different maxima
+    assert (split - want).norm() <= 1.2 * (whole - want).norm() + 1e-4 * want.norm()
+    assert (split - want).abs().max() <= 2.0 ** -6 * want.abs().max()
+
+
 def test_gated_act_embedding_argmax():
     from inference_b200 import ops
 
