@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(192, 2) attn_decode_tma_kernel(const __grid_co
   volatile int* s_abort = reinterpret_cast<volatile int*>(bar_empty + STAGES);
   float* sMerge = reinterpret_cast<float*>(ring);        // reused after the loop (33 KB)
   float* sRed = sMerge + STAGES * STAGE_BYTES / 4 - 32;  // DIFF: 32 floats behind it
+  float* sPart = sMerge + 4 * 16 * HD + 128;             // cluster merge: maximum and sum of each of the 16 rows
 
   const int split = blockIdx.x;
   const int v_heads = EXT && p.v_heads > 0 ? p.v_heads : 1;
@@ -111,6 +112,7 @@ __global__ void __launch_bounds__(192, 2) attn_decode_tma_kernel(const __grid_co
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
   }
+  __syncthreads();           // the barriers exist: the producer starts without waiting for the queries
   pdl_wait(TL_ATTN_DECODE);  // everything below reads what the preceding kernels wrote (q, the newest K/V, kv_lens)
 
   const int q_start = p.cu_q ? p.cu_q[seq] : seq * p.uniform_q_len;
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(192, 2) attn_decode_tma_kernel(const __grid_co
   const int k_halves = (k_dim + 63) >> 6, v_halves = (v_dim + 63) >> 6;
 
   // Q rows -> shared (row r = query token r / G, head kvh * G + r % G), zero rows past nrows
-  for (int idx = threadIdx.x; idx < 256; idx += blockDim.x) {
+  for (int idx = threadIdx.x; warp < 4 && idx < 256; idx += 128) {
     const int row = idx >> 4, c = idx & 15;
     uint4 val = make_uint4(0, 0, 0, 0);
     const int qtok = row / p.G, hg = row % p.G;
@@ -142,7 +144,7 @@ __global__ void __launch_bounds__(192, 2) attn_decode_tma_kernel(const __grid_co
     *reinterpret_cast<uint4*>(sQp + q_off(row, c)) = val;
   }
   if (EXT && !DIFF && p.gate) {          // the gates are read by the merge: have them near by then
-    for (int i = threadIdx.x; i < nrows * 2; i += blockDim.x) {
+    for (int i = threadIdx.x; warp < 4 && i < nrows * 2; i += 128) {
       const int row = i >> 1, half = i & 1;
       if (half * 64 < v_dim) {
         const bf16* g = p.gate + (size_t)(q_start + row / p.G) * p.gate_stride + (size_t)(kvh * p.G + row % p.G) * v_dim + half * 64;
@@ -150,7 +152,7 @@ __global__ void __launch_bounds__(192, 2) attn_decode_tma_kernel(const __grid_co
       }
     }
   }
-  __syncthreads();
+  if (warp < 4) asm volatile("bar.sync 2, 128;" ::: "memory");
 
   float o[16][4];
 #pragma unroll
@@ -357,6 +359,9 @@ __global__ void __launch_bounds__(192, 2) attn_decode_tma_kernel(const __grid_co
         if (DIFF) {
           sMerge[row * HD + d] = acc * inv;      // warp 0's partial of this row and column, read by this thread alone
         } else if (d < v_dim) put(row, d, acc * inv);
+      } else if (!DIFF && p.cluster_merge) {
+        sMerge[row * HD + d] = acc;              // as above: the cluster reads it from here
+        if (d == 0) *reinterpret_cast<float2*>(sPart + row * 2) = make_float2(M, L);
       } else {
         const size_t base = part0 + (size_t)split * 16 + row;
         p.part_o[base * HD + d] = acc;
@@ -386,6 +391,47 @@ __global__ void __launch_bounds__(192, 2) attn_decode_tma_kernel(const __grid_co
   };
   if (DIFF && p.num_splits == 1) {
     if (threadIdx.x < 128) store_pairs(sMerge);
+    return;
+  }
+  if (!DIFF && p.num_splits > 1 && p.cluster_merge) {
+    // The splits of a (sequence, kv head) are one thread-block cluster: every CTA merges its share of the rows out of all CTAs' shared memory (through
+    // global memory and one merging CTA the partials take two trips through L2 more).
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int S = p.num_splits, d = threadIdx.x;           // S <= 8
+    if (d < v_dim) {
+      const uint32_t at_o = smem_u32(sMerge) + (uint32_t)d * 4, at_ml = smem_u32(sPart);
+      for (int row = split; row < nrows; row += S) {
+        float m[8], l[8], v[8];
+#pragma unroll
+        for (int sp = 0; sp < 8; ++sp) {
+          m[sp] = -INFINITY, l[sp] = v[sp] = 0.f;
+          if (sp < S) {
+            uint32_t remote_ml, remote_o;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_ml) : "r"(at_ml + (uint32_t)row * 8), "r"(sp));
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_o) : "r"(at_o + (uint32_t)row * (HD * 4)), "r"(sp));
+            asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(m[sp]), "=f"(l[sp]) : "r"(remote_ml) : "memory");
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[sp]) : "r"(remote_o) : "memory");
+          }
+        }
+        float M = -INFINITY;
+#pragma unroll
+        for (int sp = 0; sp < 8; ++sp) M = fmaxf(M, m[sp]);
+        const float Ms = (M == -INFINITY) ? 0.f : M;
+        float L = 0.f, acc = 0.f;
+#pragma unroll
+        for (int sp = 0; sp < 8; ++sp) {
+          const float sc = exp2f(m[sp] - Ms);
+          L += sc * l[sp];
+          acc += sc * v[sp];
+        }
+        put(row, d, acc * softmax_inv<EXT>(p, kvh * p.G + row % p.G, M, L));
+      }
+    }
+    // nobody's shared memory goes away while another CTA reads it
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     return;
   }
   if (p.num_splits > 1 && p.split_counters) {
