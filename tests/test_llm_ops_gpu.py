@@ -193,6 +193,40 @@ def test_paged_prefill_with_split_keys(news, olds, Hq, Hkv, bs, splits):
     assert (split - want).abs().max() <= 2.0 ** -6 * want.abs().max()
 
 
+@pytest.mark.parametrize("T", [5, 150])
+@pytest.mark.parametrize("E,top", [(1, 1), (32, 32), (33, 4), (64, 8), (100, 7), (128, 3), (200, 40), (256, 6), (257, 5)])
+def test_routing_chooses_in_order(E, top, T):
+    """The largest logits, ties (and the two zeros) by number of the expert, at every number of registers per lane."""
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(E)
+    z = (torch.randn(T, E, device="cuda", generator=g) * 4).round() / 2
+    z[0] = 0.0
+    z[0, ::3] = -0.0
+    z[1, : E // 2] = -math.inf
+    z[2] = z[2].abs() * -1e30
+    plan, _ = ops.logits_routing(z, E, top)
+    ops.check_status()
+    order = torch.sort(z, dim=-1, descending=True, stable=True).indices[:, :top]
+    expert = torch.repeat_interleave(torch.arange(E, device="cuda"), plan.offsets.long().diff())[plan.dest.long()]
+    assert torch.equal(expert, order)
+    want = torch.softmax(z.double(), -1).gather(1, order)
+    assert torch.allclose(plan.weights.double(), want, rtol=1e-5, atol=1e-30)
+    assert torch.equal(plan.src.long()[plan.dest.long()], torch.arange(T, device="cuda")[:, None].expand(T, top))
+
+
+@pytest.mark.parametrize("value", [math.nan, math.inf, -math.inf])
+def test_routing_of_what_is_no_number_names_experts(value):
+    from inference_b200 import ops
+
+    z = torch.full((4, 40), value, device="cuda")
+    z[1:, :3] = torch.tensor([1.0, 2.0, 3.0], device="cuda")
+    plan, _ = ops.logits_routing(z, 40, 6)
+    ops.check_status()
+    expert = torch.repeat_interleave(torch.arange(40, device="cuda"), plan.offsets.long().diff())[plan.dest.long()]
+    assert all(len(set(row)) == 6 for row in expert.tolist())
+
+
 def test_gated_act_embedding_argmax():
     from inference_b200 import ops
 
