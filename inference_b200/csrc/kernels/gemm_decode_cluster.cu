@@ -349,7 +349,7 @@ gemm_decode_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __g
   // depend on the cluster, so they are requested between the barrier's arrive and wait.
   constexpr int R8 = R / 8;
   constexpr int ITEMS = (R8 * BLOCK_N + EPI_THREADS - 1) / EPI_THREADS;
-  constexpr bool PREFETCH_RES = ITEMS <= 4;     // (more items would not stay in registers)
+  constexpr bool PREFETCH_RES = PEER ? ITEMS <= 4 : ITEMS == 1;     // (registers are not indexed by a loop)
   uint4 resv[PREFETCH_RES ? ITEMS : 1];
   __syncwarp();
   if (CLUSTER > 1) cluster_arrive();
@@ -528,7 +528,9 @@ gemm_decode_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __g
   } else if (warp >= 2) {
     const int et = (warp - 2) * 32 + lane;  // 0 .. EPI_THREADS - 1
     const bool res_vec = PREFETCH_RES && p.residual && p.vec_ok && (p.ld_res & 7) == 0;
-#pragma unroll(ITEMS < 4 ? ITEMS : 4)
+    // As a loop: written out, four groups are instructions that no cache holds when the accumulator is complete, fetched line after line behind the
+    // weights of the other SMs. At 64 tokens the gate-up product of an 8B decoder spent 13000 clocks here, as a loop 4400.
+#pragma unroll 1
     for (int it = 0; it < ITEMS; ++it) {
       const int idx = et + it * EPI_THREADS;
       const int f8 = idx % R8;         // consecutive threads -> consecutive 16-byte feature groups of one token
