@@ -172,20 +172,23 @@ class PagedSequence:
         slots = []
         if self.state_slot < 0 and self.stateful:
             self.state_slot = self.pool.slots.alloc()
-        for _ in range(n_tokens):
+        left = n_tokens
+        while left > 0:         # a block at a time: what holds for its first new token holds for the others
             bi, off = divmod(self.length, bs)
             if bi == len(self.blocks):
                 self.blocks.append(self.pool.allocator.alloc())
-            elif off == 0 or self.pool.allocator.refcount(self.blocks[bi]) > 1:
+            elif self.pool.allocator.refcount(self.blocks[bi]) > 1:
                 # writing into a shared block: unshare it first (copy-on-write)
-                if self.pool.allocator.refcount(self.blocks[bi]) > 1:
-                    fresh = self.pool.allocator.alloc()
-                    self.pool.copy_block(self.blocks[bi], fresh)
-                    self.pool.allocator.release(self.blocks[bi])
-                    self.blocks[bi] = fresh
-                    self.epoch += 1
-            slots.append(self.blocks[bi] * bs + off)
-            self.length += 1
+                fresh = self.pool.allocator.alloc()
+                self.pool.copy_block(self.blocks[bi], fresh)
+                self.pool.allocator.release(self.blocks[bi])
+                self.blocks[bi] = fresh
+                self.epoch += 1
+            take = min(bs - off, left)
+            first = self.blocks[bi] * bs + off
+            slots.extend(range(first, first + take))
+            self.length += take
+            left -= take
         return slots
 
     @property

@@ -11,6 +11,7 @@ from dataclasses import dataclass
 
 import os
 
+import numpy as np
 import torch
 
 from ..models.llama import LlamaGpu, StepInputs, splits_for as _splits_for
@@ -104,7 +105,7 @@ class ModelRunner:
             sl = s.reserve(len(toks))
             ids += toks
             delta = getattr(s, "rope_delta", 0)
-            pos += list(range(start + delta, start + delta + len(toks)))
+            pos.extend(range(start + delta, start + delta + len(toks)))
             slots += sl
             cu.append(cu[-1] + len(toks))
             kvl.append(s.length)
@@ -112,24 +113,21 @@ class ModelRunner:
         if want is not None:
             rows = [cu[i] + w for i, places in enumerate(want) for w in places]
         maxb = max(len(s.blocks) for s in seqs)
-        table = torch.zeros((len(seqs), maxb), dtype=torch.int32)
-        for i, s in enumerate(seqs):
-            table[i, : len(s.blocks)] = torch.tensor(s.blocks, dtype=torch.int32)
         max_q = max(len(t) for t in new_tokens)
         G = self.model.cfg.groups
         decode = max_q * G <= 16 and all(len(t) == max_q for t in new_tokens)
+        states = [s.state_slot for s in seqs] if self._stateful else []
+        d_ids, d_slots, d_rows, d_pos, d_cu, d_kvl, d_states, d_table = self._upload(
+            (ids, slots, [] if all_positions else rows), (pos, cu, kvl, states), [s.blocks for s in seqs], maxb)
         inp = StepInputs(
-            input_ids=torch.tensor(ids, dtype=torch.int64, device=dev),
-            positions=torch.tensor(pos, dtype=torch.int32, device=dev),
-            slot_mapping=torch.tensor(slots, dtype=torch.int64, device=dev),
-            block_table=table.to(dev), kv_lens=torch.tensor(kvl, dtype=torch.int32, device=dev),
-            cu_q=None if decode else torch.tensor(cu, dtype=torch.int32, device=dev), max_q_len=max_q,
+            input_ids=d_ids, positions=d_pos, slot_mapping=d_slots, block_table=d_table, kv_lens=d_kvl,
+            cu_q=None if decode else d_cu, max_q_len=max_q,
             num_seqs=len(seqs), decode=decode, fresh_prefill=fresh and not decode,
             attn_splits=self._splits(len(seqs), max(kvl)) if decode else 1,
-            logits_rows=None if all_positions else torch.tensor(rows, dtype=torch.int64, device=dev),
+            logits_rows=None if all_positions else d_rows,
             spans=[(len(t), n) for t, n in zip(new_tokens, kvl)])
         if self._stateful:
-            inp.state_slots = torch.tensor([s.state_slot for s in seqs], dtype=torch.int32, device=dev)
+            inp.state_slots = d_states
             for s, toks in zip(seqs, new_tokens):
                 s.fed(toks)
         if embed_overrides is not None:
@@ -149,6 +147,34 @@ class ModelRunner:
             if want_logits or all_positions or want is not None:
                 return self.model.logits(hidden)
             return self.model.greedy_tokens(hidden)
+
+    def _upload(self, wide, narrow, tables, maxb: int):
+        """Lists of int64 and of int32 and a ragged int32 table as device tensors, by one copy from pinned memory of the call's own: the host prepares the
+        next step while this one runs. (Copies from pageable memory, one per list, each wait for the stream.)"""
+        dev = self.model.device
+        n64, n32 = sum(map(len, wide)), sum(map(len, narrow))
+        host = torch.zeros(2 * n64 + n32 + len(tables) * maxb, dtype=torch.int32, pin_memory=dev.type == "cuda")
+        words = host.numpy()
+        longs, at = words[:2 * n64].view(np.int64), 0
+        for values in wide:
+            longs[at:at + len(values)] = values
+            at += len(values)
+        at = 2 * n64
+        for values in narrow:
+            words[at:at + len(values)] = values
+            at += len(values)
+        rows = words[at:].reshape(len(tables), maxb)
+        for row, blocks in zip(rows, tables):
+            row[:len(blocks)] = blocks
+        got = host.to(dev, non_blocking=True)
+        out, at = [], 0
+        for values in wide:
+            out.append(got[at:at + 2 * len(values)].view(torch.int64))
+            at += 2 * len(values)
+        for values in narrow:
+            out.append(got[at:at + len(values)])
+            at += len(values)
+        return (*out, got[at:].view(len(tables), maxb))
 
     def _apply_mrope(self, inp: StepInputs, seqs, overrides, cu: list[int]) -> None:
         """Per-token rotary table for a step in which some sequences carry three-axis positions (the others keep their
