@@ -3,18 +3,18 @@
 // At this size the packed weights are the only stream that matters (4.5 bits per weight), and the arithmetic must not cost more than
 // their arrival. A step of it is 16 weight rows x one super-block of 256 x 8 tokens, in a warp of its own: mma.sync.m16n8k16 in f16
 // on operands that are exact.
-//   weights      q * sc (4-bit code times 6-bit block scale, at most 945) is a whole number that f16 holds exactly. A code becomes f16 by
-//                or-ing it under the exponent of 1024; one packed multiply-add takes the 1024 away again and applies the scale. High nibbles
-//                stay 16 times too large, their activations are 16 times too small.
+//   weights      a 4-bit code as the bits of an f16 is code * 2^-24, a subnormal number that the tensor cores multiply exactly: two masks and a shift per word and
+//                no conversion. High nibbles are 16 times too large, their activations 16 times too small. Block scales (6 bits, the same way) multiply the
+//                fp32 sums of the 32 weights of a block. (Scales multiplied into f16 codes, which is exact too, kept the half-rate FMA pipe busy
+//                with 64 packed multiply-adds per step: 23.1 us where this takes 21.0 for 28672 x 4096 at 4 tokens.)
 //   activations  bf16 times a power of two of the (token, super-block) that takes the largest to 2^9 .. 2^10: f16 holds them exactly down to 2^-19 of
 //                that one, and below it to 2^-35 of it. Those of an fp32 stream are rounded to 11 bits.
 //   minima       sum over blocks of m * (sum of the block's activations): one more MMA per super-block, the sums as two f16 parts.
-// The order of the reduction index is free as long as both operands agree, so a lane multiplies the 16-byte pieces of a row as they lie
-// and has four block scales to decode per row and super-block. d and dmin are applied to the fp32 result of each super-block.
-// The cost per weight does not depend on T. 28672 x 4096 takes 21.1 / 23.3 / 25.2 us at 1 / 4 / 8 tokens, 4096 x 14336 14.7 / 20.0 / 29.0; the kernel of single
+// The order of the reduction index is free as long as both operands agree. d and dmin are applied to the fp32 result of each super-block.
+// The cost per weight does not depend on T. 28672 x 4096 takes 19.6 / 21.0 / 22.6 us at 1 / 4 / 8 tokens, 4096 x 14336 13.6 / 17.8 / 25.9; the kernel of single
 // products (gemv_q4k.cu: dp4a on activations that are rounded to int8) 23.5 / 34.2 / 50.4 and 13.5 / 21.6 / 32.2. What is left above the weights' arrival
-// (10.2 and 5.1 us) is latency: half of the issue slots are idle with four warps to a scheduler, and about 5 us of a launch lie before the
-// first and behind the last weight. A decode step of 4 tokens of an 8B decoder went from 3.26 to 2.55 ms, its error against 64 bits from 0.029 to 0.004.
+// (10.2 and 5.1 us): about 5 us of a launch before the first and behind the last weight, shared memory (activations 4 KB and weights 2.3 KB per step) and
+// latency with four warps to a scheduler. A decode step of 4 tokens of an 8B decoder went from 3.27 to 2.50 ms, its error against 64 bits from 0.029 to 0.004.
 //
 // One CTA of 16 warps per SM. A CTA has every gridDim-th tile of 16 rows; the (tile, super-block) steps of its tiles lie on one line that is cut
 // into 16 equal parts, one per warp, so that few warps meet in a tile and none is idle. Packed bytes come through a ring of
@@ -75,41 +75,38 @@ __device__ __forceinline__ void mma_f16(float* c, uint32_t a0, uint32_t a1, uint
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// the same onto zeros
+__device__ __forceinline__ void mma_f16_first(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
 __device__ __forceinline__ __half2 bits_h2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
-// (v & mask) | 0x6400 in both halves: whole numbers on top of 1024
-__device__ __forceinline__ uint32_t on_1024(uint32_t v, uint32_t mask) {
-  uint32_t r;
-  asm("lop3.b32 %0, %1, %2, 0x64006400, 0xEA;" : "=r"(r) : "r"(v), "r"(mask));
-  return r;
-}
 
-// What a lane needs of one row's super-block header.
+// A row's super-block header: block scales as fp32 and the lane's two minima as f16, both times 2^-24.
 struct RowScales {
-  __half2 sc[4], off[4];       // [set * 2 + (low | high nibbles)]: block scale, -1024 times it
-  uint32_t mins;               // two minima as f16
-  float d, dmin;
+  float sc[8], d, dmin;
+  uint32_t mins;
 };
-// sel0 / sel1: byte 2 (tig / 2) and the next one, each twice under 0x64; msel: bytes 2 (tig mod 2) and the next one.
-__device__ __forceinline__ RowScales decode_header(const uint4 h, uint32_t sel0, uint32_t sel1, uint32_t msel, bool upper) {
+// msel: bytes 2 (tig mod 2) and the next one, each under a zero byte
+__device__ __forceinline__ RowScales decode_header(const uint4 h, uint32_t msel, bool upper) {
   RowScales r;
   const float2 dd = __half22float2(bits_h2(h.x));
-  r.d = dd.x, r.dmin = dd.y;
-  const uint32_t s_lo = h.y & 0x3f3f3f3fu, m_lo = h.z & 0x3f3f3f3fu;
-  const uint32_t s_hi = (h.w & 0x0f0f0f0fu) | ((h.y >> 2) & 0x30303030u), m_hi = ((h.w >> 4) & 0x0f0f0f0fu) | ((h.z >> 2) & 0x30303030u);
-  const __half2 base = bits_h2(0x64006400u), minus = bits_h2(0xE400E400u);      // 1024, -1024
-  const uint32_t w[4] = {__byte_perm(s_lo, 0x64646464u, sel0), __byte_perm(s_lo, 0x64646464u, sel1), __byte_perm(s_hi, 0x64646464u, sel0),
-                         __byte_perm(s_hi, 0x64646464u, sel1)};
+  r.d = dd.x * 281474976710656.f, r.dmin = dd.y * 16777216.f;      // takes the 2^-48 of code and scale, and the 2^-24 of a minimum, away again
+  const uint32_t s_lo = h.y & 0x3f3f3f3fu, s_hi = (h.w & 0x0f0f0f0fu) | ((h.y >> 2) & 0x30303030u);
+  const uint32_t m = upper ? ((h.w >> 4) & 0x0f0f0f0fu) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3f3f3f3fu;
+  const uint32_t two[4] = {__byte_perm(s_lo, 0, 0x4140), __byte_perm(s_lo, 0, 0x4342), __byte_perm(s_hi, 0, 0x4140), __byte_perm(s_hi, 0, 0x4342)};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    r.sc[i] = __hsub2(bits_h2(w[i]), base);
-    r.off[i] = __hmul2(r.sc[i], minus);
+    const float2 f = __half22float2(bits_h2(two[i]));
+    r.sc[2 * i] = f.x, r.sc[2 * i + 1] = f.y;
   }
-  r.mins = h2_bits(__hsub2(bits_h2(__byte_perm(upper ? m_hi : m_lo, 0x64646464u, msel)), base));
+  r.mins = __byte_perm(m, 0, msel);
   return r;
 }
 
-// Shared memory: activations [super-block of the pass][T][8 parts][4 lanes] uint4, parts of odd tokens swapped pairwise (eight lanes read two
+// Shared memory: activations [super-block of the pass][T][8 blocks][4 lanes] uint4, blocks of odd tokens swapped pairwise (eight lanes read two
 // tokens: other banks), their block sums [super-block][T][4] uint2, powers of two
 // [super-block][8] float, parts [GV_ROUND + GV_WARPS][8][GV_TOK_STRIDE] float, stages [warp][stages][GV_STAGE].
 size_t gv_act_bytes(int T, int kb) { return (size_t)kb * (512 * T + 32 * T + 32); }
@@ -156,9 +153,7 @@ __global__ void __launch_bounds__(GV_THREADS, 1) gemv_q4k_chain_kernel(const GvP
 
   // ---- fragment constants of this lane ----
   const int tok = min(g, T - 1);                          // column of B; columns past T repeat the last token
-  const uint32_t b2 = (uint32_t)(tig >> 1) * 2, m2 = (uint32_t)(tig & 1) * 2;
-  const uint32_t sel0 = b2 | (4u << 4) | (b2 << 8) | (4u << 12), sel1 = (b2 + 1) | (4u << 4) | ((b2 + 1) << 8) | (4u << 12);
-  const uint32_t msel = m2 | (4u << 4) | ((m2 + 1) << 8) | (4u << 12);
+  const uint32_t m2 = (uint32_t)(tig & 1) * 2, msel = m2 | (4u << 4) | ((m2 + 1) << 8) | (4u << 12);
   const bool upper = tig >= 2;
   const uint8_t* rows_at = ring + (size_t)warp * p.stages * GV_STAGE + (g >> 1) * 336 + (g & 1) * 192;     // row g; row g + 8 is 4 * 336 further
 
@@ -191,18 +186,40 @@ __global__ void __launch_bounds__(GV_THREADS, 1) gemv_q4k_chain_kernel(const GvP
       }
       // ---- activations of this pass: a warp per (token, super-block), a lane has eight neighbours ----
       if (round == 0 || p.passes > 1) {
-        for (int i = warp; i < T * nk; i += GV_WARPS) {
-          const int t = i % T, sb = i / T;
+        constexpr int AHEAD = 4;                          // units of a warp whose loads are on their way together: one by one each waits for L2
+        for (int i0 = warp; i0 < T * nk; i0 += AHEAD * GV_WARPS) {
+          uint4 raw[AHEAD][2];
+#pragma unroll
+          for (int n = 0; n < AHEAD; ++n) {
+            const int i = min(i0 + n * GV_WARPS, T * nk - 1);
+            const size_t at = (size_t)(i % T) * p.lda + (size_t)(k0 + i / T) * 256 + lane * 8;
+            if (p.a_f32) {
+              raw[n][0] = *reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(p.a) + at);
+              raw[n][1] = *reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(p.a) + at + 4);
+            } else {
+              raw[n][0] = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(p.a) + at);
+            }
+          }
+#pragma unroll
+          for (int n = 0; n < AHEAD; ++n) {
+          const int i = i0 + n * GV_WARPS, t = i % T, sb = i / T;
+          if (i >= T * nk) break;                         // the whole warp
+          const uint4 r0 = raw[n][0], r1 = raw[n][1];
           float v[8];
-          const size_t at = (size_t)t * p.lda + (size_t)(k0 + sb) * 256 + lane * 8;
-          if (p.a_f32) load_row8(reinterpret_cast<const float*>(p.a) + at, v);
-          else load_row8(reinterpret_cast<const bf16*>(p.a) + at, v);
+          if (p.a_f32) {
+            v[0] = __uint_as_float(r0.x), v[1] = __uint_as_float(r0.y), v[2] = __uint_as_float(r0.z), v[3] = __uint_as_float(r0.w);
+            v[4] = __uint_as_float(r1.x), v[5] = __uint_as_float(r1.y), v[6] = __uint_as_float(r1.z), v[7] = __uint_as_float(r1.w);
+          } else {
+            const uint32_t w[4] = {r0.x, r0.y, r0.z, r0.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[2 * e] = __uint_as_float(w[e] << 16), v[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+          }
           float top = 0.f;
 #pragma unroll
           for (int e = 0; e < 8; ++e) top = fmaxf(top, fabsf(v[e]));
           top = warp_max(top);
           const int exp = min(9 - ((int)(__float_as_uint(top) >> 23) - 127), 126);
-          const int block = lane >> 2, piece = (block >> 1) * 2 + ((lane >> 1) & 1), high = block & 1;
+          const int block = lane >> 2, high = block & 1;
           const float put = __uint_as_float((uint32_t)(127 + exp) << 23) * (high ? 0.0625f : 1.f);
           float sum = 0.f;                                // of what the product sees
           uint32_t f[4];
@@ -214,7 +231,7 @@ __global__ void __launch_bounds__(GV_THREADS, 1) gemv_q4k_chain_kernel(const GvP
             sum += seen.x + seen.y;
             f[q] = h2_bits(h);
           }
-          act[((sb * T + t) * 8 + (((piece >> 2) * 4 + high * 2 + (lane & 1)) ^ (t & 1))) * 4 + (piece & 3)] = make_uint4(f[0], f[1], f[2], f[3]);
+          act[(sb * T + t) * 32 + (lane ^ ((t & 1) << 2))] = make_uint4(f[0], f[1], f[2], f[3]);
           sum += __shfl_xor_sync(0xffffffffu, sum, 1);
           sum += __shfl_xor_sync(0xffffffffu, sum, 2);
           if ((lane & 3) == 0) {
@@ -224,6 +241,7 @@ __global__ void __launch_bounds__(GV_THREADS, 1) gemv_q4k_chain_kernel(const GvP
             to[0] = s_hi, to[2] = s_lo;
           }
           if (lane == 0) pow2[sb * 8 + t] = __uint_as_float((uint32_t)(127 - exp) << 23);
+          }
         }
       }
       __syncthreads();
@@ -237,48 +255,44 @@ __global__ void __launch_bounds__(GV_THREADS, 1) gemv_q4k_chain_kernel(const GvP
         else cp_async_wait<1>();
         __syncwarp();
         const uint8_t* at = rows_at + slot * GV_STAGE;
-        uint4 h[2], q[2][2];                              // [row g | row g + 8][pieces tig | tig + 4]
+        uint4 h[2];                                       // [row g | row g + 8]
+        uint2 q[2][4];                                    // eight bytes of each chunk of 32
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const uint4* row = reinterpret_cast<const uint4*>(at + r * 4 * 336);
-          h[r] = row[0];
-          q[r][0] = row[1 + tig];
-          q[r][1] = row[5 + tig];
+          h[r] = *reinterpret_cast<const uint4*>(at + r * 4 * 336);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) q[r][j] = *reinterpret_cast<const uint2*>(at + r * 4 * 336 + 16 + j * 32 + tig * 8);
         }
         __syncwarp();                                     // all lanes have read the stage
         request_next(slot);
         if (++slot == p.stages) slot = 0;
 
-        const RowScales s0 = decode_header(h[0], sel0, sel1, msel, upper), s1 = decode_header(h[1], sel0, sel1, msel, upper);
-        float sum[4] = {0.f, 0.f, 0.f, 0.f}, sum2[4] = {0.f, 0.f, 0.f, 0.f}, low[4] = {0.f, 0.f, 0.f, 0.f};
-        const uint4* bp = act + (ls * T + tok) * 32 + tig;
+        const RowScales s0 = decode_header(h[0], msel, upper), s1 = decode_header(h[1], msel, upper);
+        float sum[4] = {0.f, 0.f, 0.f, 0.f}, low[4];
+        const uint4 *b_low = act + (ls * T + tok) * 32 + tig + ((tok & 1) << 2), *b_high = act + (ls * T + tok) * 32 + tig + ((~tok & 1) << 2);
 #pragma unroll
-        for (int set = 0; set < 2; ++set) {
-          const uint32_t w0[4] = {q[0][set].x, q[0][set].y, q[0][set].z, q[0][set].w};
-          const uint32_t w1[4] = {q[1][set].x, q[1][set].y, q[1][set].z, q[1][set].w};
-          const __half2 scl0 = s0.sc[set * 2], scl1 = s1.sc[set * 2], sch0 = s0.sc[set * 2 + 1], sch1 = s1.sc[set * 2 + 1];
-          const __half2 ofl0 = s0.off[set * 2], ofl1 = s1.off[set * 2], ofh0 = s0.off[set * 2 + 1], ofh1 = s1.off[set * 2 + 1];
-#pragma unroll
-          for (int v = 0; v < 2; ++v) {
-            const uint4 bl = bp[((set * 4 + v) ^ (tok & 1)) * 4], bh = bp[((set * 4 + 2 + v) ^ (tok & 1)) * 4];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const uint32_t x = w0[v * 2 + e], y = w1[v * 2 + e], x8 = x >> 8, y8 = y >> 8;
-              auto scaled = [](uint32_t w, uint32_t mask, __half2 sc, __half2 off) { return h2_bits(__hfma2(bits_h2(on_1024(w, mask)), sc, off)); };
-              mma_f16(sum, scaled(x, 0x000f000fu, scl0, ofl0), scaled(y, 0x000f000fu, scl1, ofl1), scaled(x8, 0x000f000fu, scl0, ofl0),
-                      scaled(y8, 0x000f000fu, scl1, ofl1), e ? bl.z : bl.x, e ? bl.w : bl.y);
-              mma_f16(sum2, scaled(x, 0x00f000f0u, sch0, ofh0), scaled(y, 0x00f000f0u, sch1, ofh1), scaled(x8, 0x00f000f0u, sch0, ofh0),
-                      scaled(y8, 0x00f000f0u, sch1, ofh1), e ? bh.z : bh.x, e ? bh.w : bh.y);
-            }
-          }
+        for (int j = 0; j < 4; ++j) {
+          const uint4 bl = b_low[j * 8], bh = b_high[j * 8];
+          const uint32_t x = q[0][j].x, y = q[1][j].x, u0 = q[0][j].y, u1 = q[1][j].y;
+          const uint32_t x8 = x >> 8, y8 = y >> 8, u08 = u0 >> 8, u18 = u1 >> 8;
+          constexpr uint32_t LO = 0x000f000fu, HI = 0x00f000f0u;
+          float a[4], b[4];
+          mma_f16_first(a, x & LO, y & LO, x8 & LO, y8 & LO, bl.x, bl.y);
+          mma_f16_first(b, x & HI, y & HI, x8 & HI, y8 & HI, bh.x, bh.y);
+          mma_f16(a, u0 & LO, u1 & LO, u08 & LO, u18 & LO, bl.z, bl.w);
+          mma_f16(b, u0 & HI, u1 & HI, u08 & HI, u18 & HI, bh.z, bh.w);
+          sum[0] = fmaf(s0.sc[2 * j], a[0], fmaf(s0.sc[2 * j + 1], b[0], sum[0]));
+          sum[1] = fmaf(s0.sc[2 * j], a[1], fmaf(s0.sc[2 * j + 1], b[1], sum[1]));
+          sum[2] = fmaf(s1.sc[2 * j], a[2], fmaf(s1.sc[2 * j + 1], b[2], sum[2]));
+          sum[3] = fmaf(s1.sc[2 * j], a[3], fmaf(s1.sc[2 * j + 1], b[3], sum[3]));
         }
         const uint2 bs = sums[(size_t)(ls * T + tok) * 4 + tig];
-        mma_f16(low, s0.mins, s1.mins, s0.mins, s1.mins, bs.x, bs.y);
+        mma_f16_first(low, s0.mins, s1.mins, s0.mins, s1.mins, bs.x, bs.y);
         const float2 e2 = *reinterpret_cast<const float2*>(pow2 + ls * 8 + tig * 2);
-        acc[0] += e2.x * (s0.d * (sum[0] + sum2[0]) - s0.dmin * low[0]);
-        acc[1] += e2.y * (s0.d * (sum[1] + sum2[1]) - s0.dmin * low[1]);
-        acc[2] += e2.x * (s1.d * (sum[2] + sum2[2]) - s1.dmin * low[2]);
-        acc[3] += e2.y * (s1.d * (sum[3] + sum2[3]) - s1.dmin * low[3]);
+        acc[0] = fmaf(e2.x, s0.d * sum[0] - s0.dmin * low[0], acc[0]);
+        acc[1] = fmaf(e2.y, s0.d * sum[1] - s0.dmin * low[1], acc[1]);
+        acc[2] = fmaf(e2.x, s1.d * sum[2] - s1.dmin * low[2], acc[2]);
+        acc[3] = fmaf(e2.y, s1.d * sum[3] - s1.dmin * low[3], acc[3]);
         if (++ls == nk || u + 1 == u1) {                  // the end of this warp's part of the tile: part number tile + warp, in order along the line
           float* part = parts + (size_t)(lt + warp) * GV_PART;
           part[tig * 2 * GV_TOK_STRIDE + g] = acc[0];
