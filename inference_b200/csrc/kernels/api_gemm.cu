@@ -89,6 +89,31 @@ int swb_gemm_bf16_gated(const void* A, int lda, const void* W, int ldw, void* D,
   return swb::gemm_bf16_launch(a, reinterpret_cast<cudaStream_t>(stream));
 }
 
+// One product into two outputs: columns [0, first_n) go to D1 with act1, columns [first_n, N) to D2 with act2 (W [N, K], bias [N]). On the two-SM kernel;
+// -3 where it does not take the rows (16-byte pieces, first_n a multiple of 64, no gated pairs).
+int swb_gemm_bf16_two(const void* A, int lda, const void* W, int ldw, void* D1, int ldd1, int act1, void* D2, int ldd2, int act2, int first_n, int T, int N,
+                      int K, const void* bias, void* stream) {
+  swb::GemmArgs a{};
+  a.A = A;
+  a.lda = lda;
+  a.W = W;
+  a.ldw = ldw;
+  a.D = D1;
+  a.ldd = ldd1;
+  a.act = act1;
+  a.D2 = D2;
+  a.ldd2 = ldd2;
+  a.act2 = act2;
+  a.first_n = first_n;
+  a.T = T;
+  a.N = N;
+  a.K = K;
+  a.bias = bias;
+  if (T <= 0) return 0;
+  if (!D2 || N <= 0 || K <= 0 || K % 8 || lda % 8 || ldw % 8 || ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15)) return -3;
+  return swb::gemm_pair_launch(a, 0, 1, reinterpret_cast<cudaStream_t>(stream));
+}
+
 // 3x3 convolution, stride 1, zero padding 1, over an NHWC bf16 activation x [n, h, w, c] as an implicit GEMM on the
 // tcgen05 kernels: no patch matrix is written; each reduction block is one window tap over one 64-channel slab, fetched
 // by a 4-D TMA box at the tile's pixel origin shifted by the tap (zero fill outside the image is the padding).

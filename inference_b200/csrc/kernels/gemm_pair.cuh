@@ -17,6 +17,9 @@ struct PairParams {
   int ld_gate, rows_per_gate;
   int act;
   float act_a, act_b;
+  int first_n;                        // > 0: columns from here on (a multiple of the tile width) go to out2 and take act2
+  void* out2;
+  int ldd2, act2;
   float* workspace;                   // [tile][CTA of the pair][split][BN][128] fp32
   int* counters;                      // [tile][CTA of the pair][epilogue warp], zero between launches
   const int4* group_tiles;            // grouped rows: (first row, rows of the group from there on, group, -)
@@ -30,7 +33,8 @@ struct PairParams {
 
 bool gemm_pair_accepts(const GemmArgs& a);
 // Tile width and number of k-splits for a plain product whose partial sums may take sum_bytes. Returns its estimated microseconds.
-double gemm_pair_plan(int T, int N, int K, size_t sum_bytes, int* block_n, int* splits);
+// multiple > 0: only widths that divide it.
+double gemm_pair_plan(int T, int N, int K, size_t sum_bytes, int* block_n, int* splits, int multiple = 0);
 // Bytes of partial sums of a product (block_n, splits: 0 = by the plan); 0 = no k-splits.
 size_t gemm_pair_split_bytes(int T, int N, int K, int block_n, int splits);
 constexpr size_t GEMM_SPLIT_BYTES_MAX = (size_t)96 << 20;

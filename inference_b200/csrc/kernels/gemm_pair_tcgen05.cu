@@ -168,8 +168,8 @@ __device__ __forceinline__ Box box_of(const PairParams& p, int index) {
   return b;
 }
 
-__device__ __forceinline__ float pair_act(float x, const PairParams& p) {
-  switch (p.act) {
+__device__ __forceinline__ float pair_act(float x, const PairParams& p, int act) {
+  switch (act) {
     case SWB_ACT_SILU: return silu_f(x);
     case SWB_ACT_GELU_TANH: return gelu_tanh_f(x);
     case SWB_ACT_RELU2: return relu2_f(x);
@@ -196,6 +196,16 @@ __device__ __forceinline__ void copy_async16(void* smem_dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Where the columns of a tile go.
+struct OutSel {
+  void* out;
+  int ldd, act, first;       // first accumulator column of this output
+  __device__ __forceinline__ OutSel(const PairParams& p, int col0) {
+    const bool second = p.first_n > 0 && col0 >= p.first_n;
+    out = second ? p.out2 : p.out, ldd = second ? p.ldd2 : p.ldd, act = second ? p.act2 : p.act, first = second ? p.first_n : 0;
+  }
+};
 
 // Where the rows of this warp's 32 TMEM lanes lie in D (and in the residual): -1 = no such row.
 struct RowMap {
@@ -246,6 +256,7 @@ struct GroupSums {
 // COLS accumulator columns of this warp's 32 rows (thread = row) -> D. `load(c, v)` gives columns c .. c + 31.
 template <int COLS, bool STATS, typename Load>
 __device__ __forceinline__ void store_columns(const PairParams& p, const RowMap& rows, int col0, uint8_t* slab, int lane, GroupSums& sums, Load load) {
+  const OutSel to(p, col0);
   const bool pairs = gemm_act_pairs(p.act);
   const long long my_row = rows(lane);
   const int swz = lane & 7;
@@ -266,7 +277,7 @@ __device__ __forceinline__ void store_columns(const PairParams& p, const RowMap&
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         float4 f = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        if (p.act != SWB_ACT_NONE) f = make_float4(pair_act(f.x, p), pair_act(f.y, p), pair_act(f.z, p), pair_act(f.w, p));
+        if (p.act != SWB_ACT_NONE) f = make_float4(pair_act(f.x, p, p.act), pair_act(f.y, p, p.act), pair_act(f.z, p, p.act), pair_act(f.w, p, p.act));
         *reinterpret_cast<float4*>(slab + lane * 128 + ((j ^ swz) << 4)) = f;
       }
       __syncwarp();
@@ -330,9 +341,9 @@ __device__ __forceinline__ void store_columns(const PairParams& p, const RowMap&
         *reinterpret_cast<uint4*>(my_slab + ((k ^ swz) << 4)) = pack8(o);
         *reinterpret_cast<uint4*>(my_slab + (((k + 1) ^ swz) << 4)) = pack8(o + 8);
       } else {
-        if (p.act != SWB_ACT_NONE) {
+        if (to.act != SWB_ACT_NONE) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = pair_act(v[j], p);
+          for (int j = 0; j < 32; ++j) v[j] = pair_act(v[j], p, to.act);
         }
         const int k0 = (c - s) >> 3;
         if (gate) {
@@ -354,7 +365,7 @@ __device__ __forceinline__ void store_columns(const PairParams& p, const RowMap&
       }
     }
     __syncwarp();
-    bf16* out = reinterpret_cast<bf16*>(p.out) + d0 + chunk * 8;
+    bf16* out = reinterpret_cast<bf16*>(to.out) + (d0 - to.first) + chunk * 8;
     int first = sub;
     asm volatile("" : "+r"(first));      // places of rows are computed again: kept from the residual's copies they would spill
     float t[4] = {0.f, 0.f, 0.f, 0.f};
@@ -364,7 +375,7 @@ __device__ __forceinline__ void store_columns(const PairParams& p, const RowMap&
       const long long row = rows(r);
       if (row >= 0 && in) {
         const uint4 u = *reinterpret_cast<const uint4*>(slab + r * 128 + ((chunk ^ (r & 7)) << 4));
-        *reinterpret_cast<uint4*>(out + row * p.ldd) = u;
+        *reinterpret_cast<uint4*>(out + row * to.ldd) = u;
         if constexpr (STATS) {
           const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
@@ -647,13 +658,13 @@ bool counters_suffice(long tiles) { return tiles * 2 * EPI_WARPS * (long)sizeof(
 
 }  // namespace
 
-double gemm_pair_plan(int T, int N, int K, size_t sum_bytes, int* block_n, int* splits) {
+double gemm_pair_plan(int T, int N, int K, size_t sum_bytes, int* block_n, int* splits, int multiple) {
   const int pairs = device_sm_count() / 2;
   const int kblocks = (K + BK - 1) / BK;
   const long tm = (T + 2 * BM - 1) / (2 * BM);
   double best = 1e30;
   for (int bn : {256, 192, 128, 64}) {
-    if (bn > 64 && bn >= 2 * N) continue;
+    if ((bn > 64 && bn >= 2 * N) || multiple % bn) continue;
     const long tiles = tm * ((N + bn - 1) / bn);
     for (int s = 1; s <= 8; ++s) {
       if (s > 1 && (kblocks / s < 8 || sum_bytes < split_bytes(T, N, bn, s) || !counters_suffice(tiles) || tiles > pairs)) break;
@@ -679,6 +690,9 @@ bool gemm_pair_accepts(const GemmArgs& a) {
   const size_t esz = a.out_fp32 ? 4 : 2;
   if (pairs && (a.out_fp32 || a.residual || a.N % 16)) return false;
   if (a.gate && (a.out_fp32 || pairs)) return false;
+  if (a.D2 && (a.first_n <= 0 || a.first_n >= a.N || a.first_n % 64 || a.conv_c || a.group_tiles || a.out_fp32 || pairs || gemm_act_pairs(a.act2) || a.residual || a.gate ||
+               a.ldd2 % 8 || (reinterpret_cast<uintptr_t>(a.D2) & 15)))
+    return false;
   if (a.conv_stats) {
     const int gc = a.stats_groups > 0 && a.N % a.stats_groups == 0 ? a.N / a.stats_groups : 0;
     if (!a.conv_c || a.out_fp32 || pairs || (gc != 4 && gc != 8 && gc != 16 && gc != 32)) return false;
@@ -708,6 +722,7 @@ int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t st
   p.act = a.act;
   p.act_a = a.act_a;
   p.act_b = a.act_b;
+  if (a.D2) p.first_n = a.first_n, p.out2 = a.D2, p.ldd2 = a.ldd2, p.act2 = a.act2;
   p.tiles_m = (a.T + 2 * BM - 1) / (2 * BM);
   CUtensorMap ta, tb;
   int r;
@@ -759,7 +774,7 @@ int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t st
     } else {
       int s = 1;
       // a convolution's and a group list's rows are not T: plan with the row tiles they have
-      gemm_pair_plan(a.conv_c || a.group_tiles ? p.tiles_m * 2 * BM : a.T, a.N, a.K, sum_bytes, &block_n, &s);
+      gemm_pair_plan(a.conv_c || a.group_tiles ? p.tiles_m * 2 * BM : a.T, a.N, a.K, sum_bytes, &block_n, &s, a.D2 ? a.first_n : 0);
       splits = splits > 0 ? splits : s;
     }
   }

@@ -145,6 +145,8 @@ struct GemmArgs {
   // two-SM kernel only (gemm_pair.cuh)
   const void* gate = nullptr;            // D = act(acc + bias) * gate[row / rows_per_gate] + residual
   int ld_gate = 0, rows_per_gate = 0;
+  void* D2 = nullptr;                    // columns first_n .. N of the product, with an activation of their own
+  int ldd2 = 0, act2 = 0, first_n = 0;
   const void* group_tiles = nullptr;     // device int4 list of row tiles, its length in group_count, at most group_max_tiles
   const int* group_count = nullptr;
   int group_max_tiles = 0;

@@ -252,12 +252,14 @@ class FluxDiTGpu:
     def load_state_dict(self, weights: dict[str, torch.Tensor]) -> "FluxDiTGpu":
         self.w = {k: v.to(device=self.device, dtype=torch.bfloat16).contiguous() for k, v in weights.items()}
         H = self.cfg.hidden_size
-        # split single-block linear1 into its qkv and MLP row blocks so the MLP part takes the fused GELU epilogue
+        # single-block linear1 as its qkv and MLP row blocks (views): the MLP part takes the fused GELU epilogue
+        self._linear1: dict[int, tuple[torch.Tensor, torch.Tensor]] = {}
         for i in range(self.cfg.depth_single):
             p = f"single_blocks.{i}.linear1"
             W, b = self.w.pop(p + ".weight"), self.w.pop(p + ".bias")
-            self.w[p + "_qkv.weight"], self.w[p + "_mlp.weight"] = W[: 3 * H].contiguous(), W[3 * H:].contiguous()
-            self.w[p + "_qkv.bias"], self.w[p + "_mlp.bias"] = b[: 3 * H].contiguous(), b[3 * H:].contiguous()
+            self.w[p + "_qkv.weight"], self.w[p + "_mlp.weight"] = W[: 3 * H], W[3 * H:]
+            self.w[p + "_qkv.bias"], self.w[p + "_mlp.bias"] = b[: 3 * H], b[3 * H:]
+            self._linear1[i] = (W, b)
         self._build_modulation_table()
         return self
 
@@ -310,6 +312,20 @@ class FluxDiTGpu:
     def _lin(self, x, name, **kw):
         self.launches += 2 if "gate" in kw and ops.gated_fused(x.shape[0], *self.w[name + ".weight"].shape) else 1
         return ops.gemm_bf16(x, self.w[name + ".weight"], bias=self.w[name + ".bias"], **kw)
+
+    def _linear1_of(self, x, i, qkv, mlp):
+        """Both parts of a single block's linear1, as one product above the sizes at which each has a kernel of its own: 1231 rows are 420 tiles on 74 pairs of
+        SMs, six waves, and 180 + 240 of them seven."""
+        p = f"single_blocks.{i}.linear1"
+        W, b = self._linear1.get(i, (None, None))
+        # (adapters put other tensors in place of the parts)
+        whole = W is not None and all(self.w[f"{p}_{n}.{k}"].data_ptr() == t.data_ptr() + o * t.stride(0) * t.element_size()
+                                      for n, o in (("qkv", 0), ("mlp", qkv.shape[1])) for k, t in (("weight", W), ("bias", b)))
+        if x.shape[0] > 256 and whole and ops.gemm_bf16_two(x, W, qkv, mlp, bias=b, act=(None, "gelu_tanh")):
+            self.launches += 1
+            return
+        self._lin(x, p + "_qkv", out=qkv)
+        self._lin(x, p + "_mlp", act="gelu_tanh", out=mlp)
 
     def _embed(self, x, name):
         return self._lin(self._lin(x, name + ".in_layer", act="silu"), name + ".out_layer")
@@ -411,8 +427,7 @@ class FluxDiTGpu:
             m = mod[p + ".modulation.lin"]
             sh, sc, g = m[:, :H], m[:, H:2 * H], m[:, 2 * H:]
             xm = ops.layernorm_mod(x, scale=sc, shift=sh, rows_per_batch=S).view(B * S, H)
-            self._lin(xm, p + ".linear1_qkv", out=qkv.view(B * S, 3 * H))
-            self._lin(xm, p + ".linear1_mlp", act="gelu_tanh", out=buf2.view(B * S, H + M)[:, H:])
+            self._linear1_of(xm, i, qkv.view(B * S, 3 * H), buf2.view(B * S, H + M)[:, H:])
             self._cur_norm = (self.w[p + ".norm.query_norm.scale"], self.w[p + ".norm.key_norm.scale"])
             attention(qkv, buf2[:, :, :H])
             x = self._lin(buf2.view(B * S, H + M), p + ".linear2", residual=x.view(B * S, H), gate=g, rows_per_gate=S).view(B, S, H)

@@ -1,7 +1,7 @@
 """Python wrappers over the sm_100a kernel library (tensors in, tensors out, current CUDA stream)."""
 from .attention import (Differential, chunk_attention, dense_attention, dense_attention_padded, exchange_attention, exchange_decode_fits,  # noqa: F401
                         narrow_heads_on_kernel, paged_attention, paged_prefill_on_tensor_memory, paged_prefill_splits, varlen_causal_attention)
-from .gemm import SSQ_WORDS, ssq_buffer, ssq_values, gemm_bf16, gemm_bf16_grouped, gemm_bf16_normed, gemm_f32, gated_epilogue, gated_fused, gemm_workspace, linear, linear_gated  # noqa: F401
+from .gemm import SSQ_WORDS, ssq_buffer, ssq_values, gemm_bf16, gemm_bf16_grouped, gemm_bf16_normed, gemm_bf16_two, gemm_f32, gated_epilogue, gated_fused, gemm_workspace, linear, linear_gated  # noqa: F401
 from .llm import (argmax, sample_device, embedding, gated_act_mul, gated_residual, layernorm_mod, poly_norm, rmsnorm, rope_kv_write, row_rope_kv_write, diff_combine, head_mix, head_mix_weights,  # noqa: F401
                   spec_verify_greedy)
 from .delta import DeltaWeights, channel_delta, delta_key_width, head_delta  # noqa: F401

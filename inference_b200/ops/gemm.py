@@ -127,6 +127,23 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, *, bias: torch.Tensor | None = N
     return out
 
 
+def gemm_bf16_two(a: torch.Tensor, w: torch.Tensor, first: torch.Tensor, second: torch.Tensor, *, bias: torch.Tensor | None = None,
+                  act: tuple[str | None, str | None] = (None, None)) -> bool:
+    """One product a @ w^T + bias into two outputs, `first` and `second` [T, N1], [T, N2] of w [N1 + N2, K], each with its activation: two weights that read the
+    same rows fill the waves of tiles of one launch. False (and nothing done) where the two-SM kernel does not take the operands."""
+    require_cuda(a, w, first, second)
+    T, K = a.shape
+    n1, n2 = first.shape[1], second.shape[1]
+    assert w.shape == (n1 + n2, K) and first.shape[0] == second.shape[0] == T and a.stride(1) == w.stride(1) == first.stride(1) == second.stride(1) == 1
+    assert all(t.dtype == torch.bfloat16 for t in (a, w, first, second)) and (bias is None or (bias.dtype == torch.bfloat16 and bias.numel() == n1 + n2))
+    rc = kernels().swb_gemm_bf16_two(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), first.data_ptr(), first.stride(0), ACT[act[0]], second.data_ptr(),
+                                     second.stride(0), ACT[act[1]], n1, T, n1 + n2, K, ptr(bias), stream_ptr())
+    if rc == -3:
+        return False
+    check(rc, "swb_gemm_bf16_two")
+    return True
+
+
 def gemm_bf16_grouped(a: torch.Tensor, w: torch.Tensor, tile_groups: torch.Tensor, *, act: str | None = None,
                       out: torch.Tensor | None = None) -> torch.Tensor:
     """Grouped GEMM (replaces the reference's per-expert serial matmuls, candle-llm/src/models/llama.rs:1415-1488).

@@ -359,3 +359,24 @@ def test_counters_are_zero_again_after_a_wait_ran_out():
         y = ops.gemm_bf16(a[:T, :8192], w[:, :8192], mode=3 if T > 64 else 1, block_n=128, ctas=2 if T > 64 else 20)
         ops.check_status()
         assert (y == 2048.0).all()
+
+
+# widths that 256, 192 and 64 divide; a last tile of rows that is not full; columns that end inside a tile
+@pytest.mark.parametrize("T,n1,n2,K", [(300, 768, 1024, 256), (513, 576, 400, 512), (1000, 64, 72, 128), (257, 9216, 12288, 192)])
+@pytest.mark.parametrize("acts", [(None, "gelu_tanh"), ("silu", None)])
+def test_one_product_into_two_outputs(T, n1, n2, K, acts):
+    """The same bits as two products on the same kernel."""
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    a = torch.randn(T, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(n1 + n2, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    bias = torch.randn(n1 + n2, device="cuda", generator=g).bfloat16()
+    first = torch.full((T, n1 + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    second = torch.full((T, n2 + 24), 7.0, device="cuda", dtype=torch.bfloat16)
+    assert ops.gemm_bf16_two(a, w, first[:, :n1], second[:, 16:16 + n2], bias=bias, act=acts)
+    ops.check_status()
+    for got, rows, act in ((first[:, :n1], slice(0, n1), acts[0]), (second[:, 16:16 + n2], slice(n1, None), acts[1])):
+        assert torch.equal(got, ops.gemm_bf16(a, w[rows], bias=bias[rows].contiguous(), act=act, mode=3, ctas=1))
+    assert (first[:, n1:] == 7.0).all() and (second[:, :16] == 7.0).all() and (second[:, 16 + n2:] == 7.0).all()
+    assert not ops.gemm_bf16_two(a, w, torch.empty(T, n1 + 8, device="cuda", dtype=torch.bfloat16)[:, 4:n1 + 4], second[:, 16:16 + n2], act=acts)
