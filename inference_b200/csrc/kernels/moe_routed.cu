@@ -475,8 +475,9 @@ __device__ __forceinline__ void grouped_pass(const GroupedRowsParams& p, const b
   __syncthreads();
 }
 
-template <int MT>
-__global__ void __launch_bounds__(GR_WARPS * 32) grouped_rows_kernel(const GroupedRowsParams p) {
+// BLOCKS: CTAs to an SM that the registers allow. A CTA is short (32 weight rows), its loads pause while it sums its parts, and other CTAs fill the pause.
+template <int MT, int BLOCKS>
+__global__ void __launch_bounds__(GR_WARPS * 32, BLOCKS) grouped_rows_kernel(const GroupedRowsParams p) {
   pdl_launch_dependents();
   __shared__ float red[GR_WARPS * 32 * (16 * MT + 1)];
   if (!p.plan_ahead) pdl_wait();
@@ -576,10 +577,13 @@ int swb_gemm_grouped_rows(const void* x, int ldx, const int* src, const int* off
   GroupedRowsParams p{reinterpret_cast<const bf16*>(x), ldx, src, offsets, active, reinterpret_cast<const bf16*>(w),
                       reinterpret_cast<bf16*>(out), ldo, N, K, act, act_a, plan_ahead};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  // 32 weight rows per CTA halve the token re-reads; 16 when that is needed to give every SM two CTAs
-  if ((long long)((N + 31) / 32) * n_active >= 2 * 148)
-    return launch_kernel(grouped_rows_kernel<2>, dim3((N + 31) / 32, n_active), dim3(GR_WARPS * 32), 0, s, p);
-  return launch_kernel(grouped_rows_kernel<1>, dim3((N + 15) / 16, n_active), dim3(GR_WARPS * 32), 0, s, p);
+  // 32 weight rows per CTA halve the token re-reads; 16 when that is needed to give every SM two CTAs. Three to an SM once they make two waves: both products
+  // of 64 experts of 2048 x 1024 take 105.2 us with two and 99.0 with three at 8 tokens (40 experts), 169.8 and 162.6 at 64, but 26.1 and 29.5 for one token
+  // (8 experts, 512 CTAs).
+  const long long ctas = (long long)((N + 31) / 32) * n_active;
+  if (ctas >= 2 * 3 * 148) return launch_kernel(grouped_rows_kernel<2, 3>, dim3((N + 31) / 32, n_active), dim3(GR_WARPS * 32), 0, s, p);
+  if (ctas >= 2 * 148) return launch_kernel(grouped_rows_kernel<2, 2>, dim3((N + 31) / 32, n_active), dim3(GR_WARPS * 32), 0, s, p);
+  return launch_kernel(grouped_rows_kernel<1, 3>, dim3((N + 15) / 16, n_active), dim3(GR_WARPS * 32), 0, s, p);
 }
 
 }  // extern "C"
