@@ -9,6 +9,7 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 
+import gc
 import os
 
 import numpy as np
@@ -421,8 +422,15 @@ class ModelRunner:
         fused = self.model.comm.fused
         if fused is not None:
             fused.begin_capture()
-        with torch.cuda.graph(graph):
-            toks, logits = self._decode_body(B, splits, want_logits, feedback)
+        # A graph of an engine that nobody holds any more must not be collected now: destroying one is an error in any capture.
+        collecting = gc.isenabled()
+        gc.disable()
+        try:
+            with torch.cuda.graph(graph):
+                toks, logits = self._decode_body(B, splits, want_logits, feedback)
+        finally:
+            if collecting:
+                gc.enable()
         if fused is not None:
             fused.end_capture()
         return _DecodeGraph(graph, toks, logits, self.model.launches)
