@@ -171,6 +171,7 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
     sig("swb_axpy", [c_void_p, c_void_p, c_void_p, c_ll, c_float, c_float, c_int, c_void_p])
     sig("swb_groupnorm", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int,
                           c_void_p])
+    sig("swb_norm_silu_conv3x3_few", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p])
     sig("swb_groupnorm_apply", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int,
                           c_void_p])
     sig("swb_upsample2x", [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p])

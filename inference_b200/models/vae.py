@@ -272,7 +272,16 @@ class VaeDecoderGpu:
             if lvl != 0:
                 h, s = self._conv3(ops.upsample2x_nhwc(h), f"decoder.up.{lvl}.upsample.conv", sums=sums)
                 self.launches += 1
-        return self._conv3(self._gn(h, "decoder.norm_out", True, s), "decoder.conv_out")[0]
+        return self._out(h, s)
+
+    def _out(self, h, h_sums):
+        if h_sums is not None:
+            norm, conv = (tuple(self.w[f"decoder.{n}.{part}"] for part in ("weight", "bias")) for n in ("norm_out", "conv_out"))
+            y = ops.conv3x3_of_norm(h, h_sums, *norm, 1e-6, *conv)
+            if y is not None:
+                self.launches += 1
+                return y
+        return self._conv3(self._gn(h, "decoder.norm_out", True, h_sums), "decoder.conv_out")[0]
 
     def decode_rgb8(self, z: torch.Tensor) -> torch.Tensor:
         return ops.rgb8_nhwc(self.decode(z))

@@ -11,5 +11,5 @@ from .latent import (LatentWeights, QueryRotation, SplitPartials, head_product, 
 from .moe import RoutingPlan, combine_routed, gemm_grouped_rows, gemm_routed, logits_routing, routed_ffn, routed_gated_ffn, routing_counters, table_routing  # noqa: F401
 from .stream import Branch, DepthAverage, NormWeights, RoutedRows, stream_embed, stream_embed_pairs, stream_norm  # noqa: F401
 from .runtime import KernelError, check_status, device_status  # noqa: F401
-from .dit import axpy, conv3x3_implicit, conv3x3_nhwc, conv3x3_sums, conv3x3_supported, groupnorm_nhwc, im2col3x3_nhwc, rgb8_nhwc, softmax_rows, upsample2x_nhwc  # noqa: E402,F401
+from .dit import axpy, conv3x3_implicit, conv3x3_nhwc, conv3x3_of_norm, conv3x3_sums, conv3x3_supported, groupnorm_nhwc, im2col3x3_nhwc, rgb8_nhwc, softmax_rows, upsample2x_nhwc  # noqa: E402,F401
 from .quant import QuantWeight, dequantize, linear_any, linear_normed, linear_quant, normed_supported, quantize_weight  # noqa: E402,F401

@@ -124,6 +124,24 @@ def conv3x3_nhwc(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = N
     return out.view(N, H, W, Cout)
 
 
+def conv3x3_of_norm(x: torch.Tensor, sums: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, eps: float, w: torch.Tensor,
+                    bias: torch.Tensor) -> torch.Tensor | None:
+    """conv3x3_nhwc(groupnorm_nhwc(x, gamma, beta, groups, eps, silu=True, sums=sums), w, bias) for the eight output channels in which a decoder
+    ends, in one pass over x that stores no normed copy of it. None where the kernel is not made for these operands (64 or 128 channels in, eight out, a bias)."""
+    require_cuda(x)
+    N, H, W, C = x.shape
+    if C not in (64, 128) or w.shape != (8, 9 * C) or os.environ.get("SWB_CONV3X3", "implicit") == "im2col":
+        return None
+    if any(t.dtype != torch.bfloat16 or not t.is_contiguous() or t.data_ptr() % 16 for t in (x, gamma, beta, w, bias)) or sums.data_ptr() % 16:
+        return None
+    assert sums.shape[::2] == (N, 2) and sums.dtype == torch.float32 and sums.is_contiguous() and C % sums.shape[1] == 0
+    assert gamma.numel() == beta.numel() == C and bias.numel() == 8
+    out = torch.empty((N, H, W, 8), dtype=torch.bfloat16, device=x.device)
+    check(kernels().swb_norm_silu_conv3x3_few(x.data_ptr(), N, H, W, C, sums.data_ptr(), sums.shape[1], gamma.data_ptr(), beta.data_ptr(), eps,
+                                              w.data_ptr(), bias.data_ptr(), out.data_ptr(), stream_ptr()), "swb_norm_silu_conv3x3_few")
+    return out
+
+
 def im2col3x3_nhwc(x: torch.Tensor) -> torch.Tensor:
     """[N, H, W, C] bf16 -> [N*H*W, 9*C] patches (stride 1, zero padding 1), column order (kh, kw, c)."""
     require_cuda(x)

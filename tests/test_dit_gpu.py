@@ -100,6 +100,26 @@ def test_convolution_adds_up_the_sums_of_its_output(N, H, W, C, cout, G, residua
     assert (a.float() - b.float()).abs().max() <= 2.0 ** -7 * b.float().abs().max()
 
 
+@pytest.mark.parametrize("N,H,W,C,G", [(1, 1, 1, 64, 32), (1, 8, 32, 128, 32), (2, 9, 33, 128, 32), (3, 17, 31, 64, 16), (1, 7, 200, 128, 4), (5, 130, 75, 128, 32)])
+def test_last_convolution_norms_its_input(N, H, W, C, G):
+    """One kernel against the norm and the convolution apart: the operands of the products are rounded alike (a scale that is contracted otherwise may move one in some
+    thousand by 2^-8 of itself), so what is left is the order of fp32 sums and one rounding to bf16."""
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(H * W + C)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)      # noqa: E731
+    x, w, bias = (rnd(N, H, W, C) * 3 + 1).bfloat16(), (rnd(8, 9 * C) / (3 * C ** 0.5)).bfloat16(), rnd(8).bfloat16()
+    gamma, beta = rnd(C).bfloat16(), rnd(C).bfloat16()
+    t = x.float().view(N, H * W, G, C // G)
+    sums = torch.stack((t.sum((1, 3)), t.pow(2).sum((1, 3))), -1).contiguous()
+    got = ops.conv3x3_of_norm(x, sums, gamma, beta, 1e-6, w, bias)
+    normed = ops.groupnorm_nhwc(x, gamma, beta, G, 1e-6, True, sums=sums)
+    want = torch.nn.functional.conv2d(normed.double().permute(0, 3, 1, 2), w.double().view(8, 3, 3, C).permute(0, 3, 1, 2), bias.double(), padding=1)
+    want = want.permute(0, 2, 3, 1)
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * (want.abs() + 0.25 * want.abs().max())).all()
+    assert ops.conv3x3_of_norm(x, sums, gamma, beta, 1e-6, w[:, 9:].contiguous(), bias) is None
+
+
 def test_rope_in_place_updates_k_without_cache():
     from inference_b200 import ops
 
