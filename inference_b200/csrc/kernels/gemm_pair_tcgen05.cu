@@ -40,7 +40,7 @@ struct PairCfg {
   static constexpr uint32_t A_BYTES = BM * BK * 2;
   static constexpr uint32_t B_BYTES = BN / 2 * BK * 2;
   static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr uint32_t TMEM_COLS = BN == 192 ? 512 : 2 * BN;
+  static constexpr uint32_t TMEM_COLS = BN > 128 ? 512 : 2 * BN;
   static constexpr uint32_t SLAB_BYTES = 32 * 128;
   static constexpr uint32_t SMEM_SLABS = STAGES * STAGE_BYTES;
   static constexpr uint32_t SMEM_BARS = SMEM_SLABS + EPI_WARPS * SLAB_BYTES;
@@ -253,9 +253,9 @@ struct GroupSums {
   }
 };
 
-// COLS accumulator columns of this warp's 32 rows (thread = row) -> D. `load(c, v)` gives columns c .. c + 31.
-template <int COLS, bool STATS, typename Load>
-__device__ __forceinline__ void store_columns(const PairParams& p, const RowMap& rows, int col0, uint8_t* slab, int lane, GroupSums& sums, Load load) {
+// cols accumulator columns of this warp's 32 rows (thread = row) -> D. `load(c, v)` gives columns c .. c + 31.
+template <bool STATS, typename Load>
+__device__ __forceinline__ void store_columns(int cols, const PairParams& p, const RowMap& rows, int col0, uint8_t* slab, int lane, GroupSums& sums, Load load) {
   const OutSel to(p, col0);
   const bool pairs = gemm_act_pairs(p.act);
   const long long my_row = rows(lane);
@@ -263,7 +263,7 @@ __device__ __forceinline__ void store_columns(const PairParams& p, const RowMap&
   const int sub = lane >> 3, chunk = lane & 7;           // coalesced phases: four rows at a time, eight lanes each
   if (p.out_fp32) {      // a slab holds 32 rows x 32 fp32 of D, 16-byte chunk c of row r at c ^ (r & 7)
 #pragma unroll 1
-    for (int c = 0; c < COLS; c += 32) {
+    for (int c = 0; c < cols; c += 32) {
       const int a0 = col0 + c;
       if (a0 >= p.N) break;
       float v[32];
@@ -304,10 +304,10 @@ __device__ __forceinline__ void store_columns(const PairParams& p, const RowMap&
   const int width = pairs ? p.N / 2 : p.N;              // columns of D
   const bf16* gate = p.gate ? p.gate + (long long)(my_row < 0 ? 0 : (int)my_row / p.rows_per_gate) * p.ld_gate : nullptr;
 #pragma unroll 1
-  for (int s = 0; s < COLS; s += step) {
+  for (int s = 0; s < cols; s += step) {
     const int d0 = pairs ? (col0 + s) >> 1 : col0 + s;   // first column of D in this slab
     if (d0 >= width) break;
-    const bool in = d0 + chunk * 8 < width && chunk * 8 < (pairs ? (COLS - s) / 2 : COLS - s);
+    const bool in = d0 + chunk * 8 < width && chunk * 8 < (pairs ? (cols - s) / 2 : cols - s);
     if (p.residual) {      // copies straight to the slab: all on their way at a time, without registers
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -319,7 +319,7 @@ __device__ __forceinline__ void store_columns(const PairParams& p, const RowMap&
       __syncwarp();
     }
 #pragma unroll 1
-    for (int c = s; c < min(s + step, COLS); c += 32) {
+    for (int c = s; c < min(s + step, cols); c += 32) {
       float v[32];
       load(c, v);
       const int a0 = col0 + c;                           // first accumulator column
@@ -522,8 +522,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else {
     // ------------------------------ epilogue ------------------------------
-    constexpr int COLS = BN / 2 < 32 ? 32 : BN / 2;       // columns of one warp; with BN = 32 the second half's warps idle
+    // columns of one warp, in slabs of 64 where there are as many; with BN = 32 the second half's warps idle, with 224 they have one load less
+    constexpr int COLS = BN / 2 < 32 ? 32 : BN == 224 ? 128 : BN / 2;
     const int quarter = warp & 3, half = (warp - 2) >> 2;
+    const int cols = BN == 224 && half ? BN - COLS : COLS;
     const bool idle = BN < 64 && half == 1;
     uint8_t* slab = smem + Cfg::SMEM_SLABS + (warp - 2) * Cfg::SLAB_BYTES;
     int acc = 0;
@@ -549,7 +551,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         sums.img = rows.box.img, sums.col0 = col0;
       }
       if (p.splits == 1) {
-        if (!idle) store_columns<COLS, STATS>(p, rows, col0, slab, lane, sums, [&](int cc, float* v) { tmem_ld_32(taddr + cc, v); });
+        if (!idle) store_columns<STATS>(cols, p, rows, col0, slab, lane, sums, [&](int cc, float* v) { tmem_ld_32(taddr + cc, v); });
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive_even(smem_u32(&bar_tempty[acc]));
@@ -560,7 +562,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         if (!idle) {
           float* ws = p.workspace + (tile_slot + c.split) * SLOT + mine;
 #pragma unroll 1
-          for (int cc = 0; cc < COLS; cc += 32) {
+          for (int cc = 0; cc < cols; cc += 32) {
             float v[32];
             tmem_ld_32(taddr + cc, v);
 #pragma unroll
@@ -583,7 +585,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         if (last && !idle) {
           __threadfence();
           const float* ws = p.workspace + tile_slot * SLOT + mine;
-          store_columns<COLS, false>(p, rows, col0, slab, lane, sums, [&](int cc, float* v) {
+          store_columns<false>(cols, p, rows, col0, slab, lane, sums, [&](int cc, float* v) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __ldcg(ws + (size_t)(cc + j) * BM);
             for (int s = 1; s < p.splits; ++s) {
@@ -630,19 +632,22 @@ int launch_pair_as(const CUtensorMap& ta, const CUtensorMap& tb, const PairParam
 
 template <int BN>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const PairParams& p, int clusters, cudaStream_t stream) {
-  return p.stats ? launch_pair_as<BN, true>(ta, tb, p, clusters, stream) : launch_pair_as<BN, false>(ta, tb, p, clusters, stream);
+  if constexpr (BN == 224) return p.stats ? -4 : launch_pair_as<BN, false>(ta, tb, p, clusters, stream);
+  else return p.stats ? launch_pair_as<BN, true>(ta, tb, p, clusters, stream) : launch_pair_as<BN, false>(ta, tb, p, clusters, stream);
 }
 
 // Estimated microseconds of a plan, without what gemm_pair_plan adds to the best one. Fitted to sweeps of every tile width and up to six splits over
 // token counts 100..8000 and the projections of an 8B decoder and a 12B image transformer. A k-block costs more the fuller the chip
 // is (operand traffic, power): 0.29 us at BN = 256 on half of the pairs, 0.35 us on all of them. Narrower tiles move the same A for less
 // work but fill a last wave better: 975 x 9216 x 3072 takes 41.8 us at 256, 45.9 at 192, 52.3 at 128; 700 x 4096 x 4096 takes 27.2, 22.5, 32.1.
+// 224 is for counts of row tiles that leave a wave of 256 partly empty without filling two of 192 (1231 x 3072 x 15360: 85.3 us at 256, 82.5 at 224, 118.5 at
+// 192; 1231 x 9216 x 3072: 54.5, 51.7, 57.7; 975 x 12288 x 3072: 56.1, 54.2, 59.3); with k-splits the other widths fill the chip as well.
 // k-splits pay for parking and reading back partial sums: 100 x 3072 x 12288 takes 43.4 us at 128, 25.3 in three splits, 33.5 in four.
 double plan_cost(int bn, int splits, long tiles, int kblocks, int pairs) {
   const long items = tiles * splits, waves = (items + pairs - 1) / pairs;
   const int per = (kblocks + splits - 1) / splits;
   const double fill = (double)items / (double)(waves * pairs);
-  const double t = bn == 256 ? 0.22 + 0.14 * fill : bn == 192 ? 0.17 + 0.11 * fill : bn == 128 ? 0.15 + 0.085 * fill : 0.13 + 0.1 * fill;
+  const double t = bn == 256 ? 0.22 + 0.14 * fill : bn == 224 ? 0.195 + 0.125 * fill : bn == 192 ? 0.17 + 0.11 * fill : bn == 128 ? 0.15 + 0.085 * fill : 0.13 + 0.1 * fill;
   return waves * (per * t + 0.5) + (splits > 1 ? bn / 256.0 * (2.0 + 2.0 * splits) : 0.0);
 }
 
@@ -663,11 +668,11 @@ double gemm_pair_plan(int T, int N, int K, size_t sum_bytes, int* block_n, int* 
   const int kblocks = (K + BK - 1) / BK;
   const long tm = (T + 2 * BM - 1) / (2 * BM);
   double best = 1e30;
-  for (int bn : {256, 192, 128, 64}) {
+  for (int bn : {256, 224, 192, 128, 64}) {
     if ((bn > 64 && bn >= 2 * N) || multiple % bn) continue;
     const long tiles = tm * ((N + bn - 1) / bn);
     for (int s = 1; s <= 8; ++s) {
-      if (s > 1 && (kblocks / s < 8 || sum_bytes < split_bytes(T, N, bn, s) || !counters_suffice(tiles) || tiles > pairs)) break;
+      if (s > 1 && (bn == 224 || kblocks / s < 8 || sum_bytes < split_bytes(T, N, bn, s) || !counters_suffice(tiles) || tiles > pairs)) break;
       const double c = plan_cost(bn, s, tiles, kblocks, pairs);
       if (c < best) best = c, *block_n = bn, *splits = s;
     }
@@ -773,13 +778,14 @@ int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t st
       splits = 1;
     } else {
       int s = 1;
-      // a convolution's and a group list's rows are not T: plan with the row tiles they have
-      gemm_pair_plan(a.conv_c || a.group_tiles ? p.tiles_m * 2 * BM : a.T, a.N, a.K, sum_bytes, &block_n, &s, a.D2 ? a.first_n : 0);
+      // a convolution's and a group list's rows are not T: plan with the row tiles they have. 768: all widths whose warps' columns do not differ (the
+      // group sums of a convolution take them for equal)
+      gemm_pair_plan(a.conv_c || a.group_tiles ? p.tiles_m * 2 * BM : a.T, a.N, a.K, sum_bytes, &block_n, &s, a.D2 ? a.first_n : a.conv_c ? 768 : 0);
       splits = splits > 0 ? splits : s;
     }
   }
   splits = std::max(1, splits);
-  if (block_n != 256 && block_n != 192 && block_n != 128 && block_n != 64 && block_n != 32) return -4;
+  if (block_n != 256 && block_n != 224 && block_n != 192 && block_n != 128 && block_n != 64 && block_n != 32) return -4;
   if (gemm_act_pairs(a.act) && block_n < 64) return -4;
   r = make_tmap_bf16_2d(&tb, a.W, a.group_tiles ? a.groups * a.N : a.N, a.K, a.ldw, block_n / 2);
   if (r) return r;
@@ -799,6 +805,7 @@ int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t st
     case 32: return launch_pair<32>(ta, tb, p, clusters, stream);
     case 64: return launch_pair<64>(ta, tb, p, clusters, stream);
     case 128: return launch_pair<128>(ta, tb, p, clusters, stream);
+    case 224: return launch_pair<224>(ta, tb, p, clusters, stream);
     case 192: return launch_pair<192>(ta, tb, p, clusters, stream);
     default: return launch_pair<256>(ta, tb, p, clusters, stream);
   }

@@ -189,6 +189,13 @@ def test_pairs_of_sms(T, N, K, block_n, splits):
         close(y, (z + b.float()) * gate.float()[torch.arange(T, device="cuda") // rows] + r.float())
 
 
+@pytest.mark.parametrize("splits", [1, 2])
+@pytest.mark.parametrize("T,N,K", [(65, 128, 64), (255, 232, 584), (257, 352, 1096), (1000, 784, 2048), (300, 4480, 1024)])
+def test_pairs_of_sms_with_tiles_of_224_columns(T, N, K, splits):
+    """One half of the warps has 128 columns of a tile, the other 96; the same cases and tolerances as the other widths."""
+    test_pairs_of_sms(T, N, K, 224, splits)
+
+
 @pytest.mark.parametrize("T,N,K", [(1100, 2048, 512), (300, 12288, 3072)])
 def test_residual_in_place_above_256_rows(T, N, K):
     """The same product in place on the kernel of its choice (one SM a tile here) and on pairs of SMs: one rounding of fp32 sums each."""
