@@ -6,9 +6,10 @@
 // half) with the 128-byte swizzle into a 3-stage ring, completing on an mbarrier. Warps 0..3 each take a
 // 16-token slice of every tile: S = Q K^T and O += P V on mma.sync with ldmatrix from the swizzled ring,
 // online softmax in registers, then a cross-warp merge in shared memory. The <=16 MMA rows are the GQA
-// group's query heads times the (1..4) query tokens of the step. With num_splits > 1 the CTA writes an
-// un-normalised partial (O, max, sum); the last split CTA of a (sequence, kv head) to finish merges them (ticket
-// counter in the workspace, reset by the merger), so split-KV decode is still one launch.
+// group's query heads times the (1..4) query tokens of the step. With num_splits > 1 each CTA has an
+// un-normalised partial (O, max, sum). Splits that fit a thread-block cluster keep theirs in shared memory, and every CTA merges a share of
+// the rows from there; others (and the differential maps' in either case) go to the workspace, where the first CTA of the cluster or the last
+// one to finish (ticket counter, reset by the merger) merges them. Split-KV decode is one launch either way.
 // The decode step is bandwidth bound (KV bytes >> FLOPs), so the design goal is bytes in flight:
 // 2 CTAs/SM x 3 stages x 32 KB with no per-thread address arithmetic on the load path.
 #include "attention_common.cuh"
