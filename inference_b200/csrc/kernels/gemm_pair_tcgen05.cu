@@ -779,8 +779,8 @@ int gemm_pair_launch(const GemmArgs& a, int block_n, int splits, cudaStream_t st
     } else {
       int s = 1;
       // a convolution's and a group list's rows are not T: plan with the row tiles they have. 768: all widths whose warps' columns do not differ (the
-      // group sums of a convolution take them for equal)
-      gemm_pair_plan(a.conv_c || a.group_tiles ? p.tiles_m * 2 * BM : a.T, a.N, a.K, sum_bytes, &block_n, &s, a.D2 ? a.first_n : a.conv_c ? 768 : 0);
+      // group sums of a convolution take them for equal; the number of a list's tiles is a bound, so how full its last wave is is not known)
+      gemm_pair_plan(a.conv_c || a.group_tiles ? p.tiles_m * 2 * BM : a.T, a.N, a.K, sum_bytes, &block_n, &s, a.D2 ? a.first_n : a.conv_c || a.group_tiles ? 768 : 0);
       splits = splits > 0 ? splits : s;
     }
   }
