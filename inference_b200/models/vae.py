@@ -6,8 +6,9 @@ upsample + conv3x3 between levels) -> GroupNorm(32) -> swish -> conv_out. Latent
 z / scale_factor + shift_factor.
 
 GPU execution keeps activations NHWC bf16: every convolution is a tcgen05 GEMM (3x3 implicitly, the first one's 16 channels
-through a patch gather, 1x1 directly) with bias and the residual add fused in the epilogue; GroupNorm + SiLU is one fused pass after a
-statistics pass; the mid-block attention is GEMM -> row softmax -> GEMM."""
+through a patch gather, 1x1 directly) with bias and the residual add fused in the epilogue; GroupNorm + SiLU is one fused pass over
+sums that the convolution in front of it has added up (or a pass of their own); the last norm is part of conv_out's kernel; the mid-block attention is
+GEMM -> row softmax -> GEMM."""
 from __future__ import annotations
 
 from dataclasses import dataclass

@@ -100,9 +100,10 @@ def test_convolution_adds_up_the_sums_of_its_output(N, H, W, C, cout, G, residua
     assert (a.float() - b.float()).abs().max() <= 2.0 ** -7 * b.float().abs().max()
 
 
-@pytest.mark.parametrize("N,H,W,C,G", [(1, 1, 1, 64, 32), (1, 8, 32, 128, 32), (2, 9, 33, 128, 32), (3, 17, 31, 64, 16), (1, 7, 200, 128, 4), (5, 130, 75, 128, 32)])
+@pytest.mark.parametrize("N,H,W,C,G", [(1, 1, 1, 64, 32), (1, 8, 32, 128, 32), (2, 9, 33, 128, 32), (3, 17, 31, 64, 16), (1, 7, 200, 128, 4), (5, 130, 75, 128, 32),
+                                       (2, 300, 200, 64, 32), (3, 333, 210, 128, 32)])
 def test_last_convolution_norms_its_input(N, H, W, C, G):
-    """One kernel against the norm and the convolution apart: the operands of the products are rounded alike (a scale that is contracted otherwise may move one in some
+    """One kernel against the norm and the convolution apart (the last two shapes have more tiles than CTAs): the operands of the products are rounded alike (a scale that is contracted otherwise may move one in some
     thousand by 2^-8 of itself), so what is left is the order of fp32 sums and one rounding to bf16."""
     from inference_b200 import ops
 
