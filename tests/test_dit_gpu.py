@@ -93,8 +93,11 @@ def test_convolution_adds_up_the_sums_of_its_output(N, H, W, C, cout, G, residua
     assert torch.equal(y, ops.conv3x3_nhwc(x, w, bias, res))
     t = y.double().reshape(N, H * W, G, cout // G)
     n = H * W * cout // G
-    assert ((sums[..., 0].double() - t.sum((1, 3))).abs() <= n * 2.0 ** -20 * t.abs().mean((1, 3))).all()      # fp32 sums, in parts of some thousand
-    assert ((sums[..., 1].double() - t.pow(2).sum((1, 3))).abs() <= n * 2.0 ** -20 * t.pow(2).mean((1, 3))).all()
+    # A warp adds the parts of 32 pixels to its sum (some 30 additions deep) and that to the one in memory, in any order: at most H W / 32 additions there.
+    # Each is off by half of the last of 24 bits of a sum that is never above the whole one of magnitudes.
+    bound = (H * W / 32 + 32) * 2.0 ** -24 * n
+    assert ((sums[..., 0].double() - t.sum((1, 3))).abs() <= bound * t.abs().mean((1, 3))).all()
+    assert ((sums[..., 1].double() - t.pow(2).sum((1, 3))).abs() <= bound * t.pow(2).mean((1, 3))).all()
     gamma, beta = (torch.randn(cout, device="cuda", generator=g).bfloat16() for _ in range(2))
     a, b = ops.groupnorm_nhwc(y, gamma, beta, G, silu=True, sums=sums), ops.groupnorm_nhwc(y, gamma, beta, G, silu=True)
     assert (a.float() - b.float()).abs().max() <= 2.0 ** -7 * b.float().abs().max()
