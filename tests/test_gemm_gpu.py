@@ -196,6 +196,22 @@ def test_pairs_of_sms_with_tiles_of_224_columns(T, N, K, splits):
     test_pairs_of_sms(T, N, K, 224, splits)
 
 
+@pytest.mark.parametrize("T,N,K", [(65, 64, 2048), (256, 120, 520), (257, 96, 2048), (3863, 64, 2048), (1000, 72, 64)])
+def test_few_columns_of_fp32(T, N, K):
+    """Routers above 64 rows: k-splits on pairs of SMs, in the workspace or on scratch of the call's own. fp32 sums of K terms of size K^-0.5."""
+    from inference_b200 import ops
+    from inference_b200._native import kernels
+
+    assert kernels().swb_gemm_takes_pairs(T, N, K, 0, 0, 0, 1, -1, 0, 0) and not kernels().swb_gemm_takes_pairs(T, N, K, 0, 0, 0, 1, -2, 0, 0)
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    a = torch.randn(T, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    y = ops.gemm_bf16(a, w, out_dtype=torch.float32)
+    ops.check_status()
+    torch.testing.assert_close(y.double(), a.double() @ w.double().t(), rtol=1e-5, atol=1e-5)
+    assert torch.equal(y, ops.gemm_bf16(a, w, out_dtype=torch.float32))
+
+
 @pytest.mark.parametrize("T,N,K", [(1100, 2048, 512), (300, 12288, 3072)])
 def test_residual_in_place_above_256_rows(T, N, K):
     """The same product in place on the kernel of its choice (one SM a tile here) and on pairs of SMs: one rounding of fp32 sums each."""
