@@ -330,8 +330,8 @@ __global__ void __launch_bounds__(GV_THREADS, 1) gemv_q4k_chain_kernel(const GvP
       float y0 = y[it][0], y1 = y[it][1], ss = 0.f;
       if (lt < nt && n < p.N) {
         const bool two = n + 1 < p.N;
-        if (p.bias) y0 += __bfloat162float(p.bias[n]), y1 += two ? __bfloat162float(p.bias[n + 1]) : 0.f;
         if (p.ssq_in) y0 *= rms[it], y1 *= rms[it];
+        if (p.bias) y0 += __bfloat162float(p.bias[n]), y1 += two ? __bfloat162float(p.bias[n + 1]) : 0.f;
         if (gemm_act_pairs(p.act)) {                       // N is even
           reinterpret_cast<bf16*>(p.out)[(size_t)t * p.ldd + (n >> 1)] = __float2bfloat16((p.act == SWB_ACT_GEGLU_PAIRS ? gelu_tanh_f(y0) : silu_f(y0)) * y1);
         } else {

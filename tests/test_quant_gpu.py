@@ -128,6 +128,37 @@ def test_q4k_matvec_chain_links(T, N, K):
             assert ((u.double() - f(gate) * up).abs() - bound - 2.0 ** -8 * (f(gate) * up).abs()).max().item() <= 1e-6
 
 
+@pytest.mark.parametrize("T,N,K", [(1, 2, 256), (4, 98, 1536), (8, 2390, 4096)])
+@pytest.mark.parametrize("act", [None, "swiglu_pairs", "geglu_pairs"])
+def test_q4k_matvec_chain_adds_the_bias_behind_the_norm(T, N, K, act):
+    """D = act(rms * A W^T + bias): the projections of a decoder with biases, whose stream is far from unit size (1 / rms is 2^-6, 1 and 2^6 of a row)."""
+    from inference_b200 import ops
+    from inference_b200.ops import quant
+
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    qw = quant.quantize_on_device((torch.randn(N, K, device="cuda", generator=g) * 0.05).bfloat16(), "Q4_K")
+    w = quant.dequantize_reference(qw).double().cuda()
+    a = (torch.randn(T, K, device="cuda", generator=g) * 64.0 ** (torch.arange(T, device="cuda") % 3 - 1)[:, None]).bfloat16()
+    bias = torch.randn(N, device="cuda", generator=g).bfloat16()
+    ssq = ops.ssq_buffer(a.device)
+    ssq[:T] = (a.double().pow(2).sum(1) * 2.0 ** 24).round().long()
+    got = ops.linear_normed(a, qw, bias=bias, act=act, ssq_in=ssq, norm_dim=K, eps=1e-5).double()
+    ops.check_status()
+    rms = (a.double().pow(2).mean(1, keepdim=True) + 1e-5).rsqrt()
+    want = a.double() @ w.T * rms + bias.double()
+    # fp32 sums of K terms and a square root; the sum with the bias
+    near = (a.double().abs() @ w.abs().T * rms) * (2.0 ** -22 + K * 2.0 ** -26) + 2.0 ** -23 * want.abs()
+    if act is None:
+        assert ((got - want).abs() - near - 2.0 ** -8 * want.abs()).max().item() <= 0
+        return
+    f = torch.nn.functional.silu if act == "swiglu_pairs" else lambda t: torch.nn.functional.gelu(t, approximate="tanh")  # noqa: E731
+    gate, up, e_gate, e_up = want[:, 0::2], want[:, 1::2], near[:, 0::2], near[:, 1::2]
+    want = f(gate) * up
+    # slopes of both functions stay below 1.2; the functions' own exponentials and quotients are good to 2^-20 of the gate
+    bound = (1.2 * e_gate + 2.0 ** -20 * gate.abs()) * (up.abs() + e_up) + f(gate).abs() * e_up
+    assert ((got - want).abs() - bound - 2.0 ** -8 * want.abs()).max().item() <= 0
+
+
 def test_q4k_matvec_chain_sees_small_activations():
     """Tokens and super-blocks of any size: what one holds is not measured by another's largest."""
     from inference_b200 import ops
@@ -183,6 +214,62 @@ def test_a_q4k_decoder_chains_its_products_in_decode():
             del os.environ["SWB_NORM_CHAIN"]
     assert launches["1"] == launches["0"] - 3 * 3 + 3        # the first norm stays, the stream is converted to 32 bits and back
     assert (logits["1"] - logits["0"]).norm() < 0.03 * logits["0"].norm()
+
+
+def test_a_q4k_decoder_with_biases_matches_the_oracle():
+    """Query, key and value biases of the size of their projections, norm weights away from one, several layers: decode and a prompt of a few tokens, on the
+    chain and with the kernels in between, against 32 bits on the weights that the packed blocks stand for."""
+    import os
+
+    from inference_b200.engine.kv_pool import PagedKvPool, PagedSequence
+    from inference_b200.engine.runner import ModelRunner
+    from inference_b200.models import ModelConfig
+    from inference_b200.models.llama import LlamaGpu
+    from inference_b200.models.oracle import OracleLlama, random_llama_weights
+    from inference_b200.ops import quant
+
+    cfg = ModelConfig.from_json({"model_type": "qwen2", "hidden_size": 512, "intermediate_size": 1024, "num_hidden_layers": 4, "num_attention_heads": 4,
+                                 "num_key_value_heads": 2, "head_dim": 128, "vocab_size": 1024, "rms_norm_eps": 1e-5, "rope_theta": 10000.0})
+    g = torch.Generator().manual_seed(11)
+    w = {k: v.bfloat16().float() for k, v in random_llama_weights(cfg, seed=4, std=0.05, bias=True).items()}
+    for k in w:
+        if k.endswith("layernorm.weight"):
+            w[k] = (torch.rand(w[k].shape, generator=g) + 0.5).bfloat16().float()
+        elif k.endswith("proj.bias"):
+            w[k] = torch.randn(w[k].shape, generator=g).bfloat16().float()
+    model = LlamaGpu(cfg, device=torch.device("cuda")).load_state_dict(w).quantize_("Q4_K")
+    seen = dict(w)          # the norm weights are part of the projections before these are packed
+    for i in range(cfg.num_layers):
+        p = f"model.layers.{i}."
+        for norm, names in (("input_layernorm", ("self_attn.q_proj", "self_attn.k_proj", "self_attn.v_proj")),
+                            ("post_attention_layernorm", ("mlp.gate_proj", "mlp.up_proj")), (None, ("self_attn.o_proj", "mlp.down_proj"))):
+            by = w[f"{p}{norm}.weight"] if norm else 1.0
+            for n in names:
+                folded = (w[f"{p}{n}.weight"] * by).bfloat16().float()
+                seen[f"{p}{n}.weight"] = quant.dequantize_reference(quant.quantize_on_device(folded, "Q4_K"))
+            if norm:
+                seen[f"{p}{norm}.weight"] = torch.ones_like(w[f"{p}{norm}.weight"])
+    oracle = OracleLlama(cfg, seen, dtype=torch.float32, device="cuda")
+    prompts, steps = [[5, 6, 7], [40, 41], [900]], ([3, 4, 5], [600, 2, 77])
+    want = [[], [], []]
+    for i, p in enumerate(prompts):
+        cache = oracle.make_cache()
+        for toks in (p, [steps[0][i]], [steps[1][i]]):
+            want[i].append(oracle.decode_logits(torch.tensor([toks], device="cuda"), cache, cache.offset)[0])
+    for chain in ("1", "0"):
+        os.environ["SWB_NORM_CHAIN"] = chain
+        try:
+            pool = PagedKvPool(cfg.num_layers, 64, model.hkv, cfg.head_dim, 16, device="cuda")
+            runner = ModelRunner(model, pool, max_batch=8, max_seq_len=64)
+            seqs = [PagedSequence(pool) for _ in prompts]
+            got = [runner.prefill(seqs, prompts, want_logits=True).clone()] + [runner.decode(seqs, list(t), want_logits=True).clone() for t in steps]
+        finally:
+            del os.environ["SWB_NORM_CHAIN"]
+        for i in range(3):
+            for step in range(3):
+                # bf16 between the kernels of four layers, int8 activations in the products of a step without the chain
+                err = (got[step][i] - want[i][step]).norm() / want[i][step].norm()
+                assert err < 0.05, (chain, i, step, err.item())
 
 
 @pytest.mark.parametrize("T", [65, 130, 256])
