@@ -21,6 +21,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 
@@ -1001,15 +1002,17 @@ int make_tmap_heads(CUtensorMap* out, const void* ptr, int hd, int heads, int to
 
 namespace {
 
-// Sum of the splits of a row and head: a warp each, a lane has four columns.
+// Sum of the splits of a row and head: a warp each, a lane has four columns. blockIdx.y = sequence; rows that no CTA of the products has taken (of no
+// sequence, of one without context, behind `covered` rows of a sequence) have no parts and stay as they are in the output.
 __global__ void __launch_bounds__(256) attn_split_merge_kernel(const float* __restrict__ part_o, const float2* __restrict__ part_ml, int splits,
-                                                              long long rows, int Hq, bf16* out, long long out_stride) {
+                                                              long long rows, int Hq, const int* __restrict__ cu_q, const int* __restrict__ kv_lens, int covered,
+                                                              bf16* out, long long out_stride) {
   pdl_launch_dependents();
   pdl_wait();
   const long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);      // heads run fastest: a row of the output is written together
-  const int lane = threadIdx.x & 31;
-  if (i >= rows * Hq) return;
-  const long long row = i / Hq, head = i - row * Hq;
+  const int lane = threadIdx.x & 31, tok0 = cu_q[blockIdx.y], mine = min(cu_q[blockIdx.y + 1] - tok0, covered);
+  if (i >= (long long)mine * Hq || kv_lens[blockIdx.y] <= 0) return;
+  const long long row = tok0 + i / Hq, head = i % Hq;
   float top = -INFINITY;
   for (int s = 0; s < splits; ++s) top = fmaxf(top, part_ml[(s * Hq + head) * rows + row].x);
   float sum = 0.f;
@@ -1148,9 +1151,10 @@ int attn_dense_tcgen05_launch(const void* q, long long q_stride_tok, int q_strid
   }
   rc = launch_tiles(head_dim, FaKind::DENSE, q_len, Hq, batch, stream, m, p);
   if (rc || splits <= 1) return rc;
-  const long long warps = (long long)total_tokens * Hq;
-  return launch_kernel(attn_split_merge_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, stream, (const float*)p.part_o, (const float2*)p.part_ml,
-                       splits, (long long)total_tokens, Hq, reinterpret_cast<bf16*>(out), out_stride_tok);
+  const int step = p.tiles * BM, covered = (q_len + step - 1) / step * step;      // rows of a sequence that the launch above takes
+  const long long warps = (long long)std::min(covered, total_tokens) * Hq;
+  return launch_kernel(attn_split_merge_kernel, dim3((unsigned)((warps + 7) / 8), (unsigned)batch), dim3(256), 0, stream, (const float*)p.part_o,
+                       (const float2*)p.part_ml, splits, (long long)total_tokens, Hq, cu_q, kv_lens, covered, reinterpret_cast<bf16*>(out), out_stride_tok);
 }
 
 size_t attn_prefill_part_bytes(int total_tokens, int Hq, int splits) { return splits > 1 ? (size_t)splits * Hq * total_tokens * (128 * 4 + 8) : 0; }

@@ -193,6 +193,32 @@ def test_paged_prefill_with_split_keys(news, olds, Hq, Hkv, bs, splits):
     assert (split - want).abs().max() <= 2.0 ** -6 * want.abs().max()
 
 
+@pytest.mark.parametrize("splits", [1, 2, 5])
+def test_paged_prefill_leaves_rows_of_no_sequence_alone(splits):
+    """Rows before the first and behind the last sequence, of a sequence without context and behind the query tiles that max_q_len asks for: the keys may be
+    split or not, such rows of the result stay as they are."""
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    Hq, Hkv, bs, first, news, lens = 4, 2, 16, 3, [40, 9, 300], [900, 0, 1300]
+    T = first + sum(news) + 70
+    table = torch.randperm(3 * 82, device="cuda", generator=g).int().view(3, 82)
+    kc, vc = (torch.randn(3 * 82, Hkv, bs, 128, device="cuda", generator=g).bfloat16() for _ in range(2))
+    q = torch.randn(T, Hq, 128, device="cuda", generator=g).bfloat16()
+    cu = torch.tensor([first, first + 40, first + 49, first + 349], dtype=torch.int32, device="cuda")
+    kvl = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    junk = torch.full((splits * Hq * T * 130,), math.nan, device="cuda")      # what the allocator hands out next
+    del junk
+    out = torch.full((T, Hq * 128), 7.0, device="cuda", dtype=torch.bfloat16)
+    ops.paged_attention(q, kc, vc, table, kvl, cu_q=cu, max_q_len=200, scale=128 ** -0.5, prefill_splits=splits, out=out)
+    ops.check_status()
+    rows = torch.zeros(T, dtype=torch.bool, device="cuda")
+    rows[first:first + 40] = True
+    rows[first + 49:first + 49 + 256] = True              # 200 rows asked for are one tile of 256
+    assert (out[~rows] == 7.0).all()
+    assert out[rows].isfinite().all() and not (out[rows] == 7.0).all(1).any()
+
+
 @pytest.mark.parametrize("T", [5, 150])
 @pytest.mark.parametrize("E,top", [(1, 1), (32, 32), (33, 4), (64, 8), (100, 7), (128, 3), (200, 40), (256, 6), (257, 5)])
 def test_routing_chooses_in_order(E, top, T):
