@@ -9,7 +9,6 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 
-import gc
 import os
 
 import numpy as np
@@ -17,6 +16,7 @@ import torch
 
 from ..models.llama import LlamaGpu, StepInputs, splits_for as _splits_for
 from ..utils import tracing
+from ..utils.graphs import recording
 from .kv_pool import PagedKvPool, PagedSequence
 
 
@@ -422,15 +422,8 @@ class ModelRunner:
         fused = self.model.comm.fused
         if fused is not None:
             fused.begin_capture()
-        # A graph of an engine that nobody holds any more must not be collected now: destroying one is an error in any capture.
-        collecting = gc.isenabled()
-        gc.disable()
-        try:
-            with torch.cuda.graph(graph):
-                toks, logits = self._decode_body(B, splits, want_logits, feedback)
-        finally:
-            if collecting:
-                gc.enable()
+        with recording(graph):
+            toks, logits = self._decode_body(B, splits, want_logits, feedback)
         if fused is not None:
             fused.end_capture()
         return _DecodeGraph(graph, toks, logits, self.model.launches)

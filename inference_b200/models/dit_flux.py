@@ -21,6 +21,7 @@ from .nn_dual import adapter_residual
 
 from .. import ops
 from ..parallel.comm import Communicator, single
+from ..utils.graphs import recording
 
 
 @dataclass
@@ -472,7 +473,7 @@ class FluxDiTGpu:
             if self.comm.world > 1:
                 self.comm.barrier()
             graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph):
+            with recording(graph):
                 static["out"] = run()
             static["launches"] = self.launches
             g = st[key] = (graph, static)

@@ -19,8 +19,8 @@ from dataclasses import dataclass
 import torch
 import torch.nn.functional as F
 
+from ..utils.graphs import recording
 from .nn_dual import adapter_residual
-
 from .dit_flux import rope_table
 
 ADALN_DIM = 256
@@ -398,7 +398,7 @@ class ZImageDiTGpu:
             torch.cuda.current_stream().wait_stream(side)
             torch.cuda.synchronize()
             graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph):
+            with recording(graph):
                 static["out"] = run()
             static["launches"] = self.launches
             g = st[key] = (graph, static)
