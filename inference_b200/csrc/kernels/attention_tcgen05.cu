@@ -79,7 +79,7 @@ struct FaParams {
   const int* kv_lens;
   const int* block_table;
   int max_blocks, block_size;
-  // Paged problems may split the keys (plain instantiation): CTAs of split z take the z-th part of the key tiles that their rows see and leave
+  // Paged problems may split the keys (the SPLIT instantiation): CTAs of split z take the z-th part of the key tiles that their rows see and leave
   // un-normalised rows in part_o [split][head][rows][VD] with their maximum (log2 units) and sum in part_ml, for attn_split_merge_kernel.
   int splits;
   long long part_rows;
@@ -251,7 +251,7 @@ __device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 6
 
 constexpr int FMA_EVERY = 8;   // one of the four pairs of exponentials of every FMA_EVERY keys leaves the special-function unit
 
-template <typename C>
+template <typename C, bool SPLIT>
 __device__ __forceinline__ void softmax_halves(const FaParams& p, Barriers* bars, uint8_t* smem, uint32_t tmem, int q_base, int q_len, int kv_len,
                                                int coff, int n_tiles, int tok0, int batch, int head, int j0, int split) {
   constexpr int VD = C::ROW_BYTES / 2, KEYS = BN / 2, OUT = VD / 2;         // scores and output columns of a thread
@@ -320,7 +320,7 @@ __device__ __forceinline__ void softmax_halves(const FaParams& p, Barriers* bars
         }
       }
     }
-    const float neg_m = m_used == -INFINITY ? 0.f : -m_used * scale_log2;     // no key of a split so far is visible to this row
+    const float neg_m = SPLIT && m_used == -INFINITY ? 0.f : -m_used * scale_log2;     // no key of a split so far is visible to this row
     const unsigned long long sc2 = pack2(scale_log2, scale_log2), nm2 = pack2(neg_m, neg_m);
     unsigned long long l0 = 0ull, l1 = 0ull;                                // two sums of +0 each
 #pragma unroll
@@ -358,7 +358,7 @@ __device__ __forceinline__ void softmax_halves(const FaParams& p, Barriers* bars
   if (!ok) return;
   tc_fence_after_sync();
   const float sum = half ? other + l : l + other, inv = sum > 0.f ? 1.f / sum : 0.f;
-  if (p.splits > 1) {
+  if constexpr (SPLIT) {
     const long long at = ((long long)split * p.Hq + head) * p.part_rows + tok0 + row;
 #pragma unroll
     for (int c = 0; c < OUT / 32; ++c) {
@@ -424,10 +424,12 @@ __device__ __forceinline__ void softmax_halves(const FaParams& p, Barriers* bars
 // the second map's result is handed to the first one's threads through shared memory for the difference and its norm. DIFF 2 is for
 // caps up to MAX_FIXED_CAP: the scores are bounded, so the exponentials are taken as they are, without a running maximum.
 // HALVES 2 (the plain problems): two threads per query row, each with 64 of a tile's 128 keys. See softmax_halves.
+// SPLIT: a plain problem whose keys are split (p.splits). An instantiation of its own: as a branch in the plain one it made whole problems slower, prompts of 45
+// tokens 7.0 -> 7.4 us, 8 x 100 tokens on 700 40.0 -> 41.3, 3000 on 3000 288.4 -> 290.4.
 template <int HALVES>
 constexpr int fa_threads() { return HALVES * 256 + 64; }
 
-template <int QK, int VD, bool EXT, bool LAT, int DIFF, int HALVES>
+template <int QK, int VD, bool EXT, bool LAT, int DIFF, int HALVES, bool SPLIT>
 __global__ void __launch_bounds__(fa_threads<HALVES>(), 1)
 attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                           const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_q2,
@@ -441,13 +443,13 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   Barriers* bars = reinterpret_cast<Barriers*>(smem + SMEM_BAR);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   static_assert(HALVES == 1 || !(EXT || LAT || DIFF), "halves: plain problems only");
+  static_assert(HALVES == 2 || !SPLIT, "split keys: plain problems only");
   constexpr int TMA_WARP = 8 * HALVES, MMA_WARP = TMA_WARP + 1;
   constexpr int TILE_STEP = DIFF ? 0 : BM;                  // query rows between the two tiles of a CTA
   const int cta_rows = DIFF ? BM : p.tiles * BM;
   // causal blocks: the last queries see the most keys and start first
-  constexpr bool PLAIN = HALVES == 2;                         // p.splits is looked at
-  const int row_tiles = PLAIN && p.splits > 1 ? (int)gridDim.x / p.splits : (int)gridDim.x;
-  const int split = PLAIN && p.splits > 1 ? (int)blockIdx.x / row_tiles : 0, row_tile = (int)blockIdx.x - split * row_tiles;
+  const int row_tiles = SPLIT ? (int)gridDim.x / p.splits : (int)gridDim.x;
+  const int split = SPLIT ? (int)blockIdx.x / row_tiles : 0, row_tile = (int)blockIdx.x - split * row_tiles;
   const int q_base = (p.causal ? row_tiles - 1 - row_tile : row_tile) * cta_rows;
   constexpr bool WIDE = EXT && !LAT && DIFF == 0;             // v_heads and out_gate are looked at
   const int head = WIDE && p.v_heads > 0 ? blockIdx.y / p.v_heads : blockIdx.y;
@@ -469,10 +471,10 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
     if (p.window > 0) first = max(first, pos - p.window + 1);
     return first;
   };
-  const int all_tiles = (kv_end + BN - 1) / BN, per_split = PLAIN && p.splits > 1 ? (all_tiles + p.splits - 1) / p.splits : all_tiles;
-  const int j0 = EXT ? first_key_of(q_base + coff) / BN : split * per_split;
-  const int n_tiles = EXT ? all_tiles - j0 : min(all_tiles, j0 + per_split) - j0;
-  if (PLAIN && n_tiles <= 0) {      // fewer key tiles than splits; uniform for the whole CTA
+  const int all_tiles = (kv_end + BN - 1) / BN, per_split = SPLIT ? (all_tiles + p.splits - 1) / p.splits : all_tiles;
+  const int j0 = EXT ? first_key_of(q_base + coff) / BN : SPLIT ? split * per_split : 0;
+  const int n_tiles = SPLIT ? min(all_tiles, j0 + per_split) - j0 : all_tiles - j0;
+  if (SPLIT && n_tiles <= 0) {      // fewer key tiles than splits; uniform for the whole CTA
     pdl_wait();
     for (int r = threadIdx.x; r < cta_rows && q_base + r < q_len; r += blockDim.x)
       p.part_ml[((long long)split * p.Hq + head) * p.part_rows + tok0 + q_base + r] = make_float2(-INFINITY, 0.f);
@@ -648,7 +650,7 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
       __syncwarp();
     }
   } else if constexpr (HALVES == 2) {
-    softmax_halves<C>(p, bars, smem, tmem, q_base, q_len, kv_len, coff, n_tiles, tok0, batch, head, j0, split);
+    softmax_halves<C, SPLIT>(p, bars, smem, tmem, q_base, q_len, kv_len, coff, n_tiles, tok0, batch, head, j0, split);
   } else {
     // ------------------------------------------------------------------ softmax warpgroups (thread = query row)
     const int q = warp >> 2;
@@ -1041,11 +1043,11 @@ struct FaMaps {
   CUtensorMap q, k, v, q2, k2;     // q2 / k2: second parts of latent attention
 };
 
-template <int QK, int VD, bool EXT, bool LAT, int DIFF = 0>
+template <int QK, int VD, bool EXT, bool LAT, int DIFF = 0, bool SPLIT = false>
 int launch_fa(dim3 grid, cudaStream_t stream, const FaMaps& m, const FaParams& p) {
   static bool configured[64] = {false};
   constexpr int HALVES = EXT || LAT || DIFF ? 1 : 2;
-  auto kernel = attn_dense_tcgen05_kernel<QK, VD, EXT, LAT, DIFF, HALVES>;
+  auto kernel = attn_dense_tcgen05_kernel<QK, VD, EXT, LAT, DIFF, HALVES, SPLIT>;
   constexpr size_t SMEM = FaCfg<QK, VD>::SMEM_BYTES + (HALVES == 2 ? FaCfg<QK, VD>::EXCHANGE_BYTES : 0);
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1079,6 +1081,7 @@ int launch_tiles(int qk, FaKind kind, int q_len, int Hq, int batch, cudaStream_t
     if (qk == 64 && p.v_dim > 64) return launch_fa<64, 128, true, false>(grid, stream, m, p);
     return qk == 64 ? launch_fa<64, 64, true, false>(grid, stream, m, p) : launch_fa<128, 128, true, false>(grid, stream, m, p);
   }
+  if (p.splits > 1) return launch_fa<128, 128, false, false, 0, true>(grid, stream, m, p);      // paged: heads of 128
   return qk == 64 ? launch_fa<64, 64, false, false>(grid, stream, m, p) : launch_fa<128, 128, false, false>(grid, stream, m, p);
 }
 
