@@ -102,10 +102,10 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_kernel(const bf16* __restrict
 }
 
 // LayerNorm without affine followed by adaLN modulation: out = LN(x) * (1 + scale) + shift, where
-// scale/shift are per-batch vectors (row / rows_per_batch selects the batch). Bound by the latency of a row's loads and sums: 1231 rows of 3072 columns take 6.6 us
-// (7.1 with 256 threads to a row, the second half of them without a second vector, and scale and shift requested behind the sums). A warp per row
-// took 8.6: its written-out code is longer than it runs.
-template <int THREADS, int VPT>
+// scale/shift are per-batch vectors (row / rows_per_batch selects the batch). With few rows bound by the latency of a row's loads and sums, with many by
+// how many rows an SM has on their way. AHEAD: all that a row meets is requested before its first sum, which takes registers: 64 rows of 3840 columns 2.97 -> 2.68
+// us, but 4608 rows 23.4 -> 27.0. layernorm_form has the lines between the forms.
+template <int THREADS, int VPT, bool AHEAD>
 __global__ void __launch_bounds__(THREADS) layernorm_mod_kernel(const bf16* __restrict__ x, int ldx,
                                                                const bf16* __restrict__ scale,
                                                                const bf16* __restrict__ shift, int ld_mod,
@@ -119,24 +119,29 @@ __global__ void __launch_bounds__(THREADS) layernorm_mod_kernel(const bf16* __re
   const int nvec = H / 8;
   const int b = rows_per_batch > 0 ? row / rows_per_batch : 0;
   float vals[VPT][8];
-  uint4 raw[VPT], sc8[VPT], sh8[VPT];      // all that the row meets is requested before its first sum
+  auto row8 = [&](int v) { return *reinterpret_cast<const uint4*>(x + (size_t)row * ldx + v * 8); };
+  auto scale8 = [&](int v) { return *reinterpret_cast<const uint4*>(scale + (size_t)b * ld_mod + v * 8); };
+  auto shift8 = [&](int v) { return *reinterpret_cast<const uint4*>(shift + (size_t)b * ld_mod + v * 8); };
+  uint4 raw[VPT], sc8[VPT], sh8[VPT];
+  if constexpr (AHEAD) {
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int v = threadIdx.x + i * THREADS;
-    if (v < nvec) raw[i] = *reinterpret_cast<const uint4*>(x + (size_t)row * ldx + v * 8);
-  }
+    for (int i = 0; i < VPT; ++i) {
+      const int v = threadIdx.x + i * THREADS;
+      if (v < nvec) raw[i] = row8(v);
+    }
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int v = threadIdx.x + i * THREADS;
-    if (v < nvec && scale) sc8[i] = *reinterpret_cast<const uint4*>(scale + (size_t)b * ld_mod + v * 8);
-    if (v < nvec && shift) sh8[i] = *reinterpret_cast<const uint4*>(shift + (size_t)b * ld_mod + v * 8);
+    for (int i = 0; i < VPT; ++i) {
+      const int v = threadIdx.x + i * THREADS;
+      if (v < nvec && scale) sc8[i] = scale8(v);
+      if (v < nvec && shift) sh8[i] = shift8(v);
+    }
   }
   float s = 0.f;
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int v = threadIdx.x + i * THREADS;
     if (v < nvec) {
-      unpack8(raw[i], vals[i]);
+      unpack8(AHEAD ? raw[i] : row8(v), vals[i]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) s += vals[i][j];
     }
@@ -176,13 +181,13 @@ __global__ void __launch_bounds__(THREADS) layernorm_mod_kernel(const bf16* __re
       }
       if (scale) {
         float sc[8];
-        unpack8(sc8[i], sc);
+        unpack8(AHEAD ? sc8[i] : scale8(v), sc);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] *= (1.f + sc[j]);
       }
       if (shift) {
         float sh[8];
-        unpack8(sh8[i], sh);
+        unpack8(AHEAD ? sh8[i] : shift8(v), sh);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] += sh[j];
       }
@@ -821,6 +826,36 @@ int launch_norm(int H, F&& f) {
   return -3;
 }
 
+// Calls f with the threads of a row, the vectors of a thread and whether loads go ahead of the sums (layernorm_mod_kernel), H <= 16384. Microseconds at 1 / 64 / 600 /
+// 1231 / 4608 rows, loads ahead and (in brackets) not:
+//   512 columns    64 x 1   1.83 2.03 2.23 2.87 6.14                          128 x 1 (2.10) (2.39) (2.55) (3.58) (7.17)
+//   1536 columns   256 x 1  2.02 2.19 4.08 4.92 13.4 (2.30 2.39 4.11 5.37 13.3)   128 x 2  2.20 2.42 3.44 4.08 11.0
+//   3072 columns   256 x 2  2.37 2.57 4.81 7.33 24.5 (2.59 2.90 5.25 6.97 21.0)   128 x 3  2.67 2.91 4.59 6.69 20.3 (2.91 3.24 5.75 6.66 17.1)
+//   3840 columns   256 x 2  2.42 2.68 5.11 8.02 27.0 (2.72 2.97 5.74 7.77 23.4)
+//   6144 columns   256 x 4  2.82 3.06 6.61 10.7 37.6 (3.24 3.43 7.34 11.4 36.4)
+// Fewer threads to a row pay once every SM has three rows; at 444 rows 128 x 2 takes 2.71 where 256 x 1 takes 3.57 (296: 2.73 and 2.56), 128 x 3 takes 4.36 where
+// 256 x 2 takes 3.58 (600: 4.59 and 5.25). Loads ahead of wide rows pay until there are more rows than the SMs hold.
+template <int THREADS, int VPT, bool AHEAD, typename F>
+int layernorm_as(F&& f) {
+  return f(std::integral_constant<int, THREADS>{}, std::integral_constant<int, VPT>{}, std::bool_constant<AHEAD>{});
+}
+template <typename F>
+int layernorm_form(int H, int T, F&& f) {
+  const int nvec = H / 8;
+  constexpr int SMS = 148;
+  if (nvec <= 64) return layernorm_as<64, 1, true>(f);
+  if (nvec <= 128) return layernorm_as<128, 1, true>(f);
+  if (nvec <= 256) return T < 3 * SMS ? layernorm_as<256, 1, true>(f) : layernorm_as<128, 2, true>(f);
+  if (nvec <= 384) {
+    if (T < 4 * SMS) return T < 3 * SMS ? layernorm_as<256, 2, true>(f) : layernorm_as<256, 2, false>(f);
+    return T < 8 * SMS ? layernorm_as<128, 3, true>(f) : layernorm_as<128, 3, false>(f);
+  }
+  if (nvec <= 512) return T < 3 * SMS ? layernorm_as<256, 2, true>(f) : layernorm_as<256, 2, false>(f);
+  if (nvec <= 1024) return T < 14 * SMS ? layernorm_as<256, 4, true>(f) : layernorm_as<256, 4, false>(f);
+  if (nvec <= 2048) return T <= SMS ? layernorm_as<512, 4, true>(f) : layernorm_as<512, 4, false>(f);
+  return -3;
+}
+
 static thread_local int launch_rc = 0;
 inline int last_err() { return launch_rc; }
 
@@ -868,15 +903,11 @@ int swb_layernorm_mod(const void* x, int ldx, const void* scale, const void* shi
   const bf16 *px = reinterpret_cast<const bf16*>(x), *psc = reinterpret_cast<const bf16*>(scale), *psh = reinterpret_cast<const bf16*>(shift),
              *pg = reinterpret_cast<const bf16*>(gamma), *pb = reinterpret_cast<const bf16*>(beta);
   bf16* po = reinterpret_cast<bf16*>(out);
-  auto launch = [&](auto TH, auto VP) {
-    constexpr int THREADS = decltype(TH)::value, VPT = decltype(VP)::value;
-    launch_rc = launch_kernel(layernorm_mod_kernel<THREADS, VPT>, dim3(T), dim3(THREADS), 0, s, px, ldx, psc, psh, ld_mod, rows_per_batch, pg, pb, po, ldo, H,
-                              eps);
+  return layernorm_form(H, T, [&](auto TH, auto VP, auto AH) {
+    launch_rc = launch_kernel(layernorm_mod_kernel<decltype(TH)::value, decltype(VP)::value, decltype(AH)::value>, dim3(T), dim3(decltype(TH)::value), 0, s, px, ldx, psc,
+                              psh, ld_mod, rows_per_batch, pg, pb, po, ldo, H, eps);
     return last_err();
-  };
-  // three whole vectors of 128 threads instead of one and a half of 256
-  if (H / 8 > 256 && H / 8 <= 384) return launch(std::integral_constant<int, 128>{}, std::integral_constant<int, 3>{});
-  return launch_norm(H, launch);
+  });
 }
 
 // fp32 = 1: qkv and both caches hold floats (q_norm_w / k_norm_w stay bf16). Dv: width of the v heads and of the v cache.

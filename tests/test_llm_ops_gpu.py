@@ -64,6 +64,13 @@ def test_layernorm_of_any_width(T, H, per, ld):
     assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()      # fp32 sums of values that are 7 times their spread
 
 
+# both sides of every line between the forms by rows of an SM, and one vector of a row
+@pytest.mark.parametrize("T,H", [(600, 8), (9, 512), (9, 520), (443, 1032), (444, 2048), (443, 2056), (591, 2056), (1183, 3072), (1184, 3072), (443, 3080), (444, 4096),
+                                 (2071, 4104), (2072, 8192), (148, 8200), (149, 16384)])
+def test_layernorm_of_many_rows(T, H):
+    test_layernorm_of_any_width(T, H, 100, H + 8)
+
+
 @pytest.mark.parametrize("interleaved", [False, True])
 @pytest.mark.parametrize("D,rot", [(128, 128), (64, 64), (128, 64), (96, 32)])
 def test_rope_kv_write(interleaved, D, rot):
