@@ -79,12 +79,6 @@ struct FaParams {
   const int* kv_lens;
   const int* block_table;
   int max_blocks, block_size;
-  // Paged problems may split the keys (the SPLIT instantiation): CTAs of split z take the z-th part of the key tiles that their rows see and leave
-  // un-normalised rows in part_o [split][head][rows][VD] with their maximum (log2 units) and sum in part_ml, for attn_split_merge_kernel.
-  int splits;
-  long long part_rows;
-  float* part_o;
-  float2* part_ml;
   // Extended problems (the EXT instantiations only):
   int chunk;           // > 0: query i sees key j <= i only if floor(i / chunk) == floor(j / chunk), positions of the sequence
   const float* sink;   // optional [Hq]: exp(sink[h]) joins the softmax denominator (no key, no value, not scaled)
@@ -101,6 +95,12 @@ struct FaParams {
   const bf16* gate;    // optional [tokens, >= Hq] logits: head outputs are scaled by their sigmoid
   long long gate_stride;
   int first_atoms;     // 64-column atoms of the first part; the second takes the rest of the tile
+  // Paged problems may split the keys (the SPLIT instantiation): CTAs of split z take the z-th part of the key tiles that their rows see and leave
+  // un-normalised rows in part_o [split][head][rows][VD] with their maximum (log2 units) and sum in part_ml, for attn_split_merge_kernel.
+  int splits;
+  long long part_rows;
+  float* part_o;
+  float2* part_ml;
 };
 
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const void* tmap, uint64_t* bar, int c0, int c1, int c2,
@@ -424,8 +424,9 @@ __device__ __forceinline__ void softmax_halves(const FaParams& p, Barriers* bars
 // the second map's result is handed to the first one's threads through shared memory for the difference and its norm. DIFF 2 is for
 // caps up to MAX_FIXED_CAP: the scores are bounded, so the exponentials are taken as they are, without a running maximum.
 // HALVES 2 (the plain problems): two threads per query row, each with 64 of a tile's 128 keys. See softmax_halves.
-// SPLIT: a plain problem whose keys are split (p.splits). An instantiation of its own: as a branch in the plain one it made whole problems slower, prompts of 45
-// tokens 7.0 -> 7.4 us, 8 x 100 tokens on 700 40.0 -> 41.3, 3000 on 3000 288.4 -> 290.4.
+// SPLIT: a plain problem whose keys are split (p.splits). An instantiation of its own, and the plain one keeps its own expression for the first row (the
+// allocation of registers hangs on it): with the splits as a branch whole problems were slower, 24 heads of 4608 x 4608 224 -> 235 us, causal prompts
+// of 3000 tokens 111 -> 117, 45 tokens on none 7.05 -> 7.4, 8 x 100 on 700 40.1 -> 41.2.
 template <int HALVES>
 constexpr int fa_threads() { return HALVES * 256 + 64; }
 
@@ -448,9 +449,9 @@ attn_dense_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   constexpr int TILE_STEP = DIFF ? 0 : BM;                  // query rows between the two tiles of a CTA
   const int cta_rows = DIFF ? BM : p.tiles * BM;
   // causal blocks: the last queries see the most keys and start first
-  const int row_tiles = SPLIT ? (int)gridDim.x / p.splits : (int)gridDim.x;
-  const int split = SPLIT ? (int)blockIdx.x / row_tiles : 0, row_tile = (int)blockIdx.x - split * row_tiles;
-  const int q_base = (p.causal ? row_tiles - 1 - row_tile : row_tile) * cta_rows;
+  const int row_tiles = SPLIT ? (int)gridDim.x / p.splits : 0, split = SPLIT ? (int)blockIdx.x / row_tiles : 0;
+  const int q_base = (SPLIT ? (p.causal ? (split + 1) * row_tiles - 1 - (int)blockIdx.x : (int)blockIdx.x - split * row_tiles)
+                            : (p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x)) * cta_rows;
   constexpr bool WIDE = EXT && !LAT && DIFF == 0;             // v_heads and out_gate are looked at
   const int head = WIDE && p.v_heads > 0 ? blockIdx.y / p.v_heads : blockIdx.y;
   // packed variable-length batch: this CTA's sequence covers tokens [tok0, tok0 + q_len) of one flat token axis
