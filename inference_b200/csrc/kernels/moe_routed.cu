@@ -475,9 +475,8 @@ __device__ __forceinline__ void grouped_pass(const GroupedRowsParams& p, const b
   __syncthreads();
 }
 
-// BLOCKS: CTAs to an SM that the registers allow. A CTA is short (32 weight rows), its loads pause while it sums its parts, and other CTAs fill the pause.
-template <int MT, int BLOCKS>
-__global__ void __launch_bounds__(GR_WARPS * 32, BLOCKS) grouped_rows_kernel(const GroupedRowsParams p) {
+template <int MT>
+__device__ __forceinline__ void grouped_rows(const GroupedRowsParams& p) {
   pdl_launch_dependents();
   __shared__ float red[GR_WARPS * 32 * (16 * MT + 1)];
   if (!p.plan_ahead) pdl_wait();
@@ -495,6 +494,13 @@ __global__ void __launch_bounds__(GR_WARPS * 32, BLOCKS) grouped_rows_kernel(con
     else grouped_pass<MT, 4>(p, wrow, f0, r, n, red);
   }
 }
+
+template <int MT>
+__global__ void __launch_bounds__(GR_WARPS * 32) grouped_rows_kernel(const GroupedRowsParams p) {
+  grouped_rows<MT>(p);
+}
+// Registers for three CTAs to an SM. A CTA is short (32 weight rows), its loads pause while it sums its parts, and other CTAs fill the pause.
+__global__ void __launch_bounds__(GR_WARPS * 32, 3) grouped_rows_three_kernel(const GroupedRowsParams p) { grouped_rows<2>(p); }
 
 }  // namespace
 }  // namespace swb
@@ -577,13 +583,15 @@ int swb_gemm_grouped_rows(const void* x, int ldx, const int* src, const int* off
   GroupedRowsParams p{reinterpret_cast<const bf16*>(x), ldx, src, offsets, active, reinterpret_cast<const bf16*>(w),
                       reinterpret_cast<bf16*>(out), ldo, N, K, act, act_a, plan_ahead};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  // 32 weight rows per CTA halve the token re-reads; 16 when that is needed to give every SM two CTAs. Three to an SM once they make two waves: both products
-  // of 64 experts of 2048 x 1024 take 105.2 us with two and 99.0 with three at 8 tokens (40 experts), 169.8 and 162.6 at 64, but 26.1 and 29.5 for one token
-  // (8 experts, 512 CTAs).
+  // 32 weight rows per CTA halve the token re-reads; 16 when that is needed to give every SM two CTAs. Three to an SM once they make two waves, and for long
+  // reductions, which pause less, once they make seven. Both products of 64 experts of 2048 x 1024 take 104.5 us with two and 98.0 with three
+  // at 8 tokens (40 experts), 172.8 and 165.1 at 64; 2048 CTAs of K 2560 43.8 and 38.4, 1024 of K 3072 21.8 and 25.7, of 14336 147.8 and 153.0; 3584 CTAs of K 3584 111.1
+  // and 109.6. (The other two kernels leave their registers to the compiler: held to 80 and 128 they spill, 512 CTAs of 16 rows x 1024 7.2 -> 8.0 us, of 32 rows 9.3 -> 9.6.)
   const long long ctas = (long long)((N + 31) / 32) * n_active;
-  if (ctas >= 2 * 3 * 148) return launch_kernel(grouped_rows_kernel<2, 3>, dim3((N + 31) / 32, n_active), dim3(GR_WARPS * 32), 0, s, p);
-  if (ctas >= 2 * 148) return launch_kernel(grouped_rows_kernel<2, 2>, dim3((N + 31) / 32, n_active), dim3(GR_WARPS * 32), 0, s, p);
-  return launch_kernel(grouped_rows_kernel<1, 3>, dim3((N + 15) / 16, n_active), dim3(GR_WARPS * 32), 0, s, p);
+  const dim3 block(GR_WARPS * 32), grid32((N + 31) / 32, n_active);
+  if (ctas >= (K <= 2560 ? 2 : 7) * 3 * 148) return launch_kernel(grouped_rows_three_kernel, grid32, block, 0, s, p);
+  if (ctas >= 2 * 148) return launch_kernel(grouped_rows_kernel<2>, grid32, block, 0, s, p);
+  return launch_kernel(grouped_rows_kernel<1>, dim3((N + 15) / 16, n_active), block, 0, s, p);
 }
 
 }  // extern "C"

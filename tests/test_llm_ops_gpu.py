@@ -248,6 +248,30 @@ def test_routing_chooses_in_order(E, top, T):
     assert torch.equal(plan.src.long()[plan.dest.long()], torch.arange(T, device="cuda")[:, None].expand(T, top))
 
 
+# 16 and 32 weight rows to a CTA; two and three CTAs to an SM on both sides of the lines (CTAs, length of the reduction); segments of one row to three passes
+@pytest.mark.parametrize("E,top,N,K,T", [(4, 2, 72, 520, 3), (8, 1, 1176, 64, 9), (8, 1, 1192, 2568, 200), (16, 2, 1800, 2560, 40), (16, 2, 1800, 2568, 40), (64, 2, 1576, 2568, 90)])
+@pytest.mark.parametrize("pairs", [False, True])
+def test_rows_of_experts_at_every_split(E, top, N, K, T, pairs):
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(T, K, device="cuda", generator=g).bfloat16()
+    w = torch.empty(E, N, K, device="cuda", dtype=torch.bfloat16).normal_(0.0, K ** -0.5, generator=g)
+    z = torch.randn(T, E, device="cuda", generator=g)
+    z[:, 0] += 2                            # one expert has most rows
+    plan, _ = ops.logits_routing(z, E, top)
+    got = ops.gemm_grouped_rows(x, w, plan, gather=True, act="swiglu_pairs" if pairs else None).double()
+    ops.check_status()
+    for e, (lo, hi) in enumerate(zip(plan.offsets.tolist(), plan.offsets.tolist()[1:])):
+        if lo == hi:
+            continue
+        want = x[plan.src[lo:hi].long()].double() @ w[e].double().T
+        if pairs:
+            want = torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]
+        # one rounding of fp32 sums of K terms of size K^-0.5
+        assert ((got[lo:hi] - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5).all()
+
+
 @pytest.mark.parametrize("value", [math.nan, math.inf, -math.inf])
 def test_routing_of_what_is_no_number_names_experts(value):
     from inference_b200 import ops
