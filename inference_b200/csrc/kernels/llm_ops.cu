@@ -322,22 +322,33 @@ __global__ void __launch_bounds__(256) rope_kv_write_kernel(
 // Head dim 128 with full rotary width. A lane has 8 (interleaved: elements 8 l ..) or 16 (half-split: 8 l .. and 64 + 8 l ..) elements of a head, so
 // that both members of each rotation pair are its own and every access is a 16-byte vector: 16 or 8 lanes to a head. A thread keeps
 // its token's cosines and sines in registers and walks over heads: read for each head they are twice the bytes of the head itself.
-// Bound by memory: 1231 tokens of 48 heads take 8.1 us and 4608 27.3 (13.8 and 48.3 with 4- and 8-byte accesses and
-// a table read per head).
+// ONE: a thread has one head, which it requests ahead of the tables, and tokens with few heads share a CTA.
+// Many heads are bound by memory: 1231 tokens of 32 + 8 + 8 heads take 8.5 us and 4608 27.2 (13.1 and 46 with 4- and 8-byte accesses and a table read per
+// head, 10.7 and 32 with the slot's page divided out in 64 bits). Few are bound by latency: 4 + 1 + 1 heads take 1.6 us for a token and 4.7 for 4608 (2.4 and 15.2
+// with a CTA to each token and the head requested behind the tables).
 // Squares are summed pair by pair in the order of a warp with four elements per lane. V heads are only touched when they have to
 // be copied into a cache.
-template <bool INTERLEAVED>
+template <bool INTERLEAVED, bool ONE>
 __global__ void __launch_bounds__(256) rope_kv_write_d128_kernel(
     bf16* qkv, int ld_qkv, const int* __restrict__ positions, const long long* __restrict__ slot_mapping,
     const float* __restrict__ cos_tab, const float* __restrict__ sin_tab, const bf16* __restrict__ q_norm_w,
     const bf16* __restrict__ k_norm_w, float norm_eps, float norm_w_offset, bf16* kcache, bf16* vcache, int block_size,
-    int Hq, int Hkv, int heads_active, int heads_cta) {
+    int T, int Hq, int Hkv, int heads_active, int heads_cta, int tokens_cta) {
   pdl_launch_dependents();
-  pdl_wait(TL_ROPE_KV);
   constexpr int D = 128, LANES = INTERLEAVED ? 16 : 8, VECS = INTERLEAVED ? 1 : 2, HEADS = 256 / LANES;
-  const int l = threadIdx.x % LANES;
-  const int t = blockIdx.x;
+  const int l = threadIdx.x % LANES, group = threadIdx.x / LANES, token = ONE ? group / heads_cta : 0;
+  const int t = ONE ? (int)blockIdx.x * tokens_cta + token : (int)blockIdx.x;
   const int h_end = min(heads_active, ((int)blockIdx.y + 1) * heads_cta);
+  int h = (int)blockIdx.y * heads_cta + group - (ONE ? token * heads_cta : 0);
+  bf16* const row = qkv + (size_t)t * ld_qkv + 8 * l;
+  pdl_wait(TL_ROPE_KV);
+  uint4 raw[VECS];
+  if constexpr (ONE) {
+    if (token >= tokens_cta || t >= T || h >= h_end) return;      // all lanes of a head together
+#pragma unroll
+    for (int u = 0; u < VECS; ++u) raw[u] = *reinterpret_cast<const uint4*>(row + (size_t)h * D + u * 64);
+  }
+  const long long slot = slot_mapping ? slot_mapping[t] : -1;
   float c[INTERLEAVED ? 4 : 8], sn[INTERLEAVED ? 4 : 8];
   {
     const size_t at = (size_t)positions[t] * 64 + (INTERLEAVED ? 4 : 8) * l;
@@ -348,13 +359,16 @@ __global__ void __launch_bounds__(256) rope_kv_write_d128_kernel(
       sn[j] = b.x, sn[j + 1] = b.y, sn[j + 2] = b.z, sn[j + 3] = b.w;
     }
   }
-  const long long slot = slot_mapping ? slot_mapping[t] : -1;
-  const long long blk = slot < 0 ? 0 : slot / block_size;
-  const int off = slot < 0 ? 0 : (int)(slot % block_size);
-  for (int h = (int)blockIdx.y * heads_cta + (int)threadIdx.x / LANES; h < h_end; h += HEADS) {
-    bf16* src = qkv + (size_t)t * ld_qkv + (size_t)h * D + 8 * l;
+  const long long blk = slot < 0 ? 0 : (slot >> 32) ? slot / block_size : (long long)((unsigned)slot / (unsigned)block_size);
+  const int off = slot < 0 ? 0 : (int)(slot - blk * block_size);
+  for (; h < h_end; h += ONE ? heads_active : HEADS) {
+    bf16* src = row + (size_t)h * D;
     const bool is_q = h < Hq;
     const bool is_k = !is_q && h < Hq + Hkv;
+    if constexpr (!ONE) {
+#pragma unroll
+      for (int u = 0; u < VECS; ++u) raw[u] = *reinterpret_cast<const uint4*>(src + u * 64);
+    }
     bf16* dst = src;
     if (!is_q && (is_k ? kcache : vcache) != nullptr) {
       const int kvh = is_k ? (h - Hq) : (h - Hq - Hkv);
@@ -363,13 +377,13 @@ __global__ void __launch_bounds__(256) rope_kv_write_d128_kernel(
     if (!is_q && !is_k) {      // values are copied
       if (dst && dst != src) {
 #pragma unroll
-        for (int u = 0; u < VECS; ++u) *reinterpret_cast<uint4*>(dst + u * 64) = *reinterpret_cast<const uint4*>(src + u * 64);
+        for (int u = 0; u < VECS; ++u) *reinterpret_cast<uint4*>(dst + u * 64) = raw[u];
       }
       continue;
     }
     float v[VECS][8];
 #pragma unroll
-    for (int u = 0; u < VECS; ++u) load_row8(src + u * 64, v[u]);
+    for (int u = 0; u < VECS; ++u) unpack8(raw[u], v[u]);
     const bf16* nw = is_q ? q_norm_w : k_norm_w;
     if (nw) {
       // a part is what a lane of four elements would have: interleaved 4 i .. 4 i + 3, else 2 i, 2 i + 1, 64 + 2 i, 65 + 2 i
@@ -924,15 +938,19 @@ int swb_rope_kv_write_ex(void* qkv, int ld_qkv, const int* positions, const long
   const bf16* kn = reinterpret_cast<const bf16*>(k_norm_w);
   auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   if (!fp32 && D == 128 && Dv == 128 && rot_dim == 128 && ld_qkv % 8 == 0 && aligned(qkv) && aligned(kcache) && aligned(vcache) && aligned(cos_tab) &&
-      aligned(sin_tab) && aligned(qn) && aligned(kn)) {
+      aligned(sin_tab) && aligned(qn) && aligned(kn) && Hq + Hkv > 0) {
     const int heads_active = Hq + Hkv + (vcache ? Hkv : 0);   // V stays where it is unless it goes to a cache
     const int at_once = interleaved ? 16 : 32;                // heads of a CTA's 256 threads
-    // enough CTAs to have every SM at work: a CTA has all heads of its token from two tokens per SM on
-    const int heads_cta = T >= 296 ? heads_active : at_once;
-    auto kern = interleaved ? rope_kv_write_d128_kernel<true> : rope_kv_write_d128_kernel<false>;
-    launch_rc = launch_kernel(kern, dim3((unsigned)T, (unsigned)((heads_active + heads_cta - 1) / heads_cta)), dim3(256), 0, st, reinterpret_cast<bf16*>(qkv),
-                              ld_qkv, positions, slot_mapping, cos_tab, sin_tab, qn, kn, norm_eps, norm_w_offset,
-                              reinterpret_cast<bf16*>(kcache), reinterpret_cast<bf16*>(vcache), block_size, Hq, Hkv, heads_active, heads_cta);
+    // A thread has one head where a token's heads fill half of a CTA at most, and with few tokens (CTAs then share a token's heads). Otherwise a CTA has all
+    // heads of its token from two tokens per SM on. One head ahead of the tables takes registers that more tokens want for other heads: 148 tokens of 24 + 24
+    // heads 2.4 us without and 2.6 with it, 64 tokens 2.4 and 2.1.
+    const bool one = heads_active <= at_once / 2 || T <= 64;
+    const int heads_cta = one ? std::min(at_once, heads_active) : T >= 296 ? heads_active : at_once, tokens_cta = one ? at_once / heads_cta : 1;
+    auto kern = interleaved ? (one ? rope_kv_write_d128_kernel<true, true> : rope_kv_write_d128_kernel<true, false>)
+                            : (one ? rope_kv_write_d128_kernel<false, true> : rope_kv_write_d128_kernel<false, false>);
+    launch_rc = launch_kernel(kern, dim3((unsigned)((T + tokens_cta - 1) / tokens_cta), (unsigned)((heads_active + heads_cta - 1) / heads_cta)), dim3(256), 0, st,
+                              reinterpret_cast<bf16*>(qkv), ld_qkv, positions, slot_mapping, cos_tab, sin_tab, qn, kn, norm_eps, norm_w_offset,
+                              reinterpret_cast<bf16*>(kcache), reinterpret_cast<bf16*>(vcache), block_size, T, Hq, Hkv, heads_active, heads_cta, tokens_cta);
     return last_err();
   }
   const long long warps = (long long)T * (Hq + 2 * Hkv);

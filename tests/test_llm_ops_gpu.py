@@ -164,6 +164,13 @@ def test_rope_of_whole_heads(interleaved, T, Hq, Hkv, ld_extra):
     assert (kc.transpose(1, 2).reshape(nblk * bs, -1)[rest] == 7.0).all() and (vc.transpose(1, 2).reshape(nblk * bs, -1)[rest] == 7.0).all()
 
 
+# heads that fill half of a CTA and one more; several tokens to a CTA, the last CTA with fewer; 64 tokens of more heads than a CTA has, and 65
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("T,Hq,Hkv", [(1, 4, 1), (301, 4, 1), (67, 12, 2), (67, 13, 2), (66, 4, 2), (66, 5, 2), (64, 40, 7), (65, 40, 7)])
+def test_rope_of_few_heads_or_tokens(interleaved, T, Hq, Hkv):
+    test_rope_of_whole_heads(interleaved, T, Hq, Hkv, 0)
+
+
 # sequences with fewer key tiles than parts, rows that see no key of the last part, one row, a last tile that ends inside a page
 @pytest.mark.parametrize("splits", [2, 3, 8])
 @pytest.mark.parametrize("news,olds,Hq,Hkv,bs", [([700], [1900], 4, 2, 16), ([130, 1, 300], [1000, 2500, 0], 2, 1, 32), ([5, 257], [3, 640], 3, 3, 64)])
