@@ -124,6 +124,26 @@ def test_last_convolution_norms_its_input(N, H, W, C, G):
     assert ops.conv3x3_of_norm(x, sums, gamma, beta, 1e-6, w[:, 9:].contiguous(), bias) is None
 
 
+# one pixel; fewer pixels than a thread takes at a time; a last round in part; rounds of several CTAs and samples
+@pytest.mark.parametrize("N,H,W,C,G", [(1, 1, 1, 64, 32), (2, 3, 5, 128, 32), (1, 33, 31, 256, 32), (3, 16, 65, 512, 32), (2, 70, 61, 2048, 16)])
+@pytest.mark.parametrize("silu", [False, True])
+def test_group_norm_of_any_number_of_pixels(N, H, W, C, G, silu):
+    """Against 64 bits. The variance, 1e-3 and more with eps, is the difference of a mean of squares and a squared mean of up to 9, each good to 2^-22: 2e-6 of it is at most
+    1e-3 of the result, times weights of up to 4; and the rounding to bf16."""
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(H * W + C)
+    x = torch.randn(N, H, W, C, device="cuda", generator=g).bfloat16()
+    gamma, beta = (torch.randn(C, device="cuda", generator=g).bfloat16() for _ in range(2))
+    d = x.double().reshape(N, H * W, G, C // G)
+    want = (d - d.mean((1, 3), keepdim=True)) * (d.var((1, 3), unbiased=False, keepdim=True) + 1e-3).rsqrt()
+    want = want.reshape(x.shape) * gamma.double() + beta.double()
+    want = torch.nn.functional.silu(want) if silu else want
+    sums = torch.stack([d.sum((1, 3)), d.pow(2).sum((1, 3))], -1).float()
+    for got in (ops.groupnorm_nhwc(x, gamma, beta, G, 1e-3, silu), ops.groupnorm_nhwc(x, gamma, beta, G, 1e-3, silu, sums=sums)):
+        assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 4e-3).all()
+
+
 def test_rope_in_place_updates_k_without_cache():
     from inference_b200 import ops
 
