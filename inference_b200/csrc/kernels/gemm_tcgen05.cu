@@ -815,12 +815,14 @@ bool gemm_bf16_prefers_one_sm(int T, int N, int K, size_t split_bytes, double ep
 // make up for it (the same product with both: 56 us on one SM, 50 on pairs). Both estimates were fitted to 890 products of 257..4000
 // rows, bare, with residual, bias or SiLU: no choice loses more than 8 % to the other kernel, 0.1 % on average. Gated pairs are for the two-SM kernel alone:
 // callers ask gemm_bf16_prefers_one_sm first. 64 to 127 columns of fp32 (routers) are few tiles, which only k-splits spread over the chip: 3863 rows x 64 x 2048 take
-// 13.7 us on one SM a tile, 10.2 in four splits; 130 rows 46.8 and 9.2; 96 columns of 512 at 3863 rows 7.5 and 7.6.
+// 13.7 us on one SM a tile, 10.2 in four splits; 130 rows 46.8 and 9.2; 96 columns of 512 at 1000 rows 7.8 and 6.9. Above 3072 rows a short reduction is mostly the
+// epilogue's time, of which one SM a tile has twice as many at work: 3863 rows x 72 x 256 6.3 us and 7.3, 8000 x 112 x 512 7.8 and 8.3, x 768 9.1 and 9.3, 3863 x 96 x 768 9.3
+// and 8.9; 3863 x 64 x 128 5.3 and 5.7, x 384 equal.
 // A caller's own tile width or number of CTAs means the one-SM kernels.
 bool gemm_bf16_takes_pairs(const GemmArgs& a) {
   if (a.gate || a.group_tiles || a.force_mode == 3) return true;
   if (a.force_mode >= 0 || a.force_ctas != 0 || a.force_block_n != 0 || a.T <= 64 || a.N < 64 || !gemm_pair_accepts(a)) return false;
-  if (a.N < 128) return a.out_fp32 && a.force_mode == -1;
+  if (a.N < 128) return a.out_fp32 && a.force_mode == -1 && (a.T <= 3072 || a.K >= (a.N > 64 ? 768 : 384));
   if (gemm_act_pairs(a.act) || a.out_fp32) return true;
   const double epilogue_us = (a.bias ? 7.45 : 0.0) + (a.act != SWB_ACT_NONE ? 8.6 : 0.0);
   return !gemm_bf16_prefers_one_sm(a.T, a.N, a.K, a.split_counters ? a.split_bytes : 0, epilogue_us, 0.0);

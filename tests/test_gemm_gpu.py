@@ -212,6 +212,22 @@ def test_few_columns_of_fp32(T, N, K):
     assert torch.equal(y, ops.gemm_bf16(a, w, out_dtype=torch.float32))
 
 
+@pytest.mark.parametrize("T,N,K,pairs", [(3072, 72, 64, 1), (3073, 72, 760, 0), (3073, 72, 768, 1), (3073, 64, 376, 0), (3073, 64, 384, 1), (4001, 120, 64, 0)])
+def test_few_columns_of_many_rows(T, N, K, pairs):
+    """On both sides of the lines up to which a short reduction of many rows goes to one SM a tile."""
+    from inference_b200 import ops
+    from inference_b200._native import kernels
+
+    assert kernels().swb_gemm_takes_pairs(T, N, K, 0, 0, 0, 1, -1, 0, 0) == pairs
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    a = torch.randn(T, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    y = ops.gemm_bf16(a, w, out_dtype=torch.float32)
+    ops.check_status()
+    torch.testing.assert_close(y.double(), a.double() @ w.double().t(), rtol=1e-5, atol=1e-5)
+
+
+
 @pytest.mark.parametrize("T,N,K", [(1100, 2048, 512), (300, 12288, 3072)])
 def test_residual_in_place_above_256_rows(T, N, K):
     """The same product in place on the kernel of its choice (one SM a tile here) and on pairs of SMs: one rounding of fp32 sums each."""
