@@ -71,6 +71,18 @@ def test_layernorm_of_many_rows(T, H):
     test_layernorm_of_any_width(T, H, 100, H + 8)
 
 
+@pytest.mark.parametrize("H", [512, 1536, 2056, 3072, 3840, 6144, 16384])
+def test_layernorm_of_a_row_whatever_comes_with_it(H):
+    from inference_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(H)
+    x = torch.randn(4608, H, device="cuda", generator=g).bfloat16()
+    mods = [(torch.randn(1, H, device="cuda", generator=g) * 0.3).bfloat16() for _ in range(2)]
+    whole = ops.layernorm_mod(x, scale=mods[0], shift=mods[1], rows_per_batch=4608)
+    for T in (5, 256, 512, 1231):
+        assert torch.equal(ops.layernorm_mod(x[:T], scale=mods[0], shift=mods[1], rows_per_batch=T), whole[:T])
+
+
 @pytest.mark.parametrize("interleaved", [False, True])
 @pytest.mark.parametrize("D,rot", [(128, 128), (64, 64), (128, 64), (96, 32)])
 def test_rope_kv_write(interleaved, D, rot):
