@@ -11,10 +11,12 @@
 //                that one, and below it to 2^-35 of it. Those of an fp32 stream are rounded to 11 bits.
 //   minima       sum over blocks of m * (sum of the block's activations): one more MMA per super-block, the sums as two f16 parts.
 // The order of the reduction index is free as long as both operands agree. d and dmin are applied to the fp32 result of each super-block.
-// The cost per weight does not depend on T. 28672 x 4096 takes 19.6 / 21.0 / 22.6 us at 1 / 4 / 8 tokens, 4096 x 14336 13.6 / 17.8 / 25.9; the kernel of single
-// products (gemv_q4k.cu: dp4a on activations that are rounded to int8) 23.5 / 34.2 / 50.4 and 13.5 / 21.6 / 32.2. What is left above the weights' arrival
-// (10.2 and 5.1 us): about 5 us of a launch before the first and behind the last weight, shared memory (activations 4 KB and weights 2.3 KB per step) and
+// A step does the same for any number of tokens; what grows with them is the conversion of the activations and the passes over a long reduction that they
+// need. 28672 x 4096 takes 19.6 / 21.0 / 22.6 us at 1 / 4 / 8 tokens, 4096 x 14336 13.6 / 17.8 / 25.9; the kernel of single products (gemv_q4k.cu: dp4a on
+// activations that are rounded to int8) 23.5 / 34.2 / 50.4 and 13.5 / 21.6 / 32.2. What is left above the weights' arrival (10.2 and 5.1 us): about 5 us of
+// a launch before the first and behind the last weight, shared memory (activations 4 KB and weights 2.3 KB per step) and
 // latency with four warps to a scheduler. A decode step of 4 tokens of an 8B decoder went from 3.27 to 2.50 ms, its error against 64 bits from 0.029 to 0.004.
+// Small models gain from 4 tokens on; at 1 and 2 a step of 8 layers of 2048 takes 320 and 343 us where nine kernels a layer took 304 and 341.
 //
 // One CTA of 16 warps per SM. A CTA has every gridDim-th tile of 16 rows; the (tile, super-block) steps of its tiles lie on one line that is cut
 // into 16 equal parts, one per warp, so that few warps meet in a tile and none is idle. Packed bytes come through a ring of
@@ -427,7 +429,7 @@ GvParams gv_params(const void* A, int lda, const void* Wq, void* D, int ldd, int
 
 }  // namespace
 
-// Whether this kernel takes the problem: T in 1..8, K a multiple of 256 up to what at most four passes hold (29 184 at eight tokens),
+// Whether this kernel takes the problem: T in 1..8, K a multiple of 256 up to what at most four passes hold (28 672 at eight tokens),
 // 16-byte aligned operands.
 static bool gemv_q4k_chain_accepts(int T, int K, int lda, const void* A, const void* Wq) {
   static const bool off = [] { const char* e = getenv("SWB_Q4K_GEMV"); return e && e[0] == '0'; }();

@@ -159,6 +159,23 @@ def test_q4k_matvec_chain_adds_the_bias_behind_the_norm(T, N, K, act):
     assert ((got - want).abs() - bound - 2.0 ** -8 * want.abs()).max().item() <= 0
 
 
+@pytest.mark.parametrize("T,most", [(8, 28672), (7, 32768)])
+def test_q4k_matvec_chain_takes_reductions_up_to_four_passes(T, most):
+    """The longest reduction of whole super-blocks that it takes, and no longer one."""
+    from inference_b200 import ops
+    from inference_b200._native import kernels
+    from inference_b200.ops import quant
+
+    assert all(kernels().swb_gemv_q4k_supported(T, k) for k in range(256, most + 1, 256)) and not kernels().swb_gemv_q4k_supported(T, most + 256)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    qw = quant.quantize_on_device((torch.randn(18, most, device="cuda", generator=g) * 0.05).bfloat16(), "Q4_K")
+    a = torch.randn(T, most, device="cuda", generator=g).bfloat16()
+    w = quant.dequantize_reference(qw).double().cuda()
+    got, want = ops.linear_normed(a, qw).double(), a.double() @ w.T
+    ops.check_status()
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + (2.0 ** -22 + most * 2.0 ** -26) * (a.double().abs() @ w.abs().T)).all()
+
+
 def test_q4k_matvec_chain_sees_small_activations():
     """Tokens and super-blocks of any size: what one holds is not measured by another's largest."""
     from inference_b200 import ops
