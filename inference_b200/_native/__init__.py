@@ -179,8 +179,6 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
     sig("swb_attn_dense_set_tiles", [c_int], None)
     sig("swb_attn_varlen_causal", [c_void_p, c_ll, c_int, c_void_p, c_void_p, c_ll, c_int, c_void_p, c_ll, c_void_p, c_int,
                                    c_int, c_int, c_int, c_int, c_float, c_void_p])
-    sig("swb_attn_paged_prefill_tc", [c_void_p, c_ll, c_int, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-                                      c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p])
     sig("swb_attn_paged_prefill_split", [c_void_p, c_ll, c_int, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_size_t, c_void_p])
     sig("swb_attn_prefill_splits", [c_int, c_int, c_int, c_int, c_ll])
@@ -232,8 +230,6 @@ def _declare_kernels(lib: ctypes.CDLL) -> None:
     sig("swb_im2col3x3", [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
     sig("swb_gemm_bf16_two", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                               c_void_p])
-    sig("swb_conv3x3_nhwc", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p,
-                             c_int, c_int, c_void_p])
     sig("swb_conv3x3_nhwc_stats", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p,
                              c_int, c_int, c_void_p, c_int, c_void_p])
     sig("swb_softmax_rows", [c_void_p, c_void_p, c_int, c_int, c_ll, c_ll, c_float, c_void_p])

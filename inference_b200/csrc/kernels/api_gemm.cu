@@ -152,10 +152,6 @@ int swb_conv3x3_nhwc_stats(const void* x, int n, int h, int w, int c, const void
   a.stats_groups = groups;
   return swb::gemm_bf16_launch(a, reinterpret_cast<cudaStream_t>(stream));
 }
-int swb_conv3x3_nhwc(const void* x, int n, int h, int w, int c, const void* W, int ldw, int cout, void* out, int ldd,
-                     const void* bias, const void* residual, int ld_res, int act, void* stream) {
-  return swb_conv3x3_nhwc_stats(x, n, h, w, c, W, ldw, cout, out, ldd, bias, residual, ld_res, act, nullptr, 0, stream);
-}
 
 // GEMM whose epilogue dispatches the output head-sharded to peers (see GemmScatter): D is not written locally.
 // peers: `world` device pointers to every rank's receive buffer [global rows, N / (heads * 128), heads_per_rank, 128].

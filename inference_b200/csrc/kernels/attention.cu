@@ -601,13 +601,6 @@ int swb_attn_paged_prefill_split(const void* q, long long q_stride_tok, int q_st
                                    nullptr, 0, 0, 0, 0, 0, causal, cu_q, total_tokens, 128, kv_lens, block_table,
                                    max_blocks, block_size, num_blocks, splits, parts, part_bytes);
 }
-int swb_attn_paged_prefill_tc(const void* q, long long q_stride_tok, int q_stride_head, void* out, long long out_stride_tok,
-                              const void* kcache, const void* vcache, const int* block_table, int max_blocks,
-                              int block_size, int num_blocks, const int* cu_q, const int* kv_lens, int num_seqs,
-                              int max_q_len, int total_tokens, int Hq, int Hkv, float scale, int causal, void* stream) {
-  return swb_attn_paged_prefill_split(q, q_stride_tok, q_stride_head, out, out_stride_tok, kcache, vcache, block_table, max_blocks, block_size, num_blocks,
-                                      cu_q, kv_lens, num_seqs, max_q_len, total_tokens, Hq, Hkv, scale, causal, 1, nullptr, 0, stream);
-}
 // How many splits of the keys a step should take (contexts of up to max_kv tokens), and the bytes of their parts (16-byte aligned; the call's own).
 int swb_attn_prefill_splits(int max_q_len, int total_tokens, int Hq, int num_seqs, long long max_kv) {
   return swb::attn_prefill_splits(max_q_len, total_tokens, Hq, num_seqs, max_kv);

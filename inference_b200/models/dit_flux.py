@@ -319,7 +319,7 @@ class FluxDiTGpu:
         SMs, six waves, and 180 + 240 of them seven."""
         p = f"single_blocks.{i}.linear1"
         W, b = self._linear1.get(i, (None, None))
-        # (adapters put other tensors in place of the parts)
+        # (a program may put other tensors in place of the parts)
         whole = W is not None and all(self.w[f"{p}_{n}.{k}"].data_ptr() == t.data_ptr() + o * t.stride(0) * t.element_size()
                                       for n, o in (("qkv", 0), ("mlp", qkv.shape[1])) for k, t in (("weight", W), ("bias", b)))
         if x.shape[0] > 256 and whole and ops.gemm_bf16_two(x, W, qkv, mlp, bias=b, act=(None, "gelu_tanh")):

@@ -430,7 +430,7 @@ class LlamaGpu:
         pf = (lambda t: t if (pf_bytes >= 0 and isinstance(t, torch.Tensor)) else None)
         ssq = (self._ssq if self.quant_format is None else torch.empty((2, ops.SSQ_WORDS), dtype=torch.int64, device=self.device).unbind(0)) if chain else None
         packed = chain and self.quant_format is not None
-        normed = ops.linear_normed if packed else ops.gemm_bf16_normed
+        normed = ops.linear_normed
         prefill_splits = None
         ssq_prev = None                 # partial sums of squares of `res` (valid while branch is None)
         H = cfg.hidden_size
@@ -575,7 +575,7 @@ class LlamaGpu:
 
         Up to rows_per_expert_small (token, expert) pairs per expert the weights are streamed past the few rows of each expert; above it
         the rows are copied into their segments and multiplied in tiles of 256 by pairs of SMs. 64 experts of
-        2048 x 1024, 8 of them per token, whole layer: 213 us streamed and 222 us in tiles at 64 tokens, 243 and 227 us at 96, 446 and 260 us at 256."""
+        2048 x 1024, 8 of them per token, whole layer: 184 us streamed and 184 us in tiles at 64 tokens, 224 and 196 us at 96, 397 and 205 us at 256."""
         moe = self.cfg.moe
         act = self.cfg.mlp_activation
         T, E, k = h.shape[0], m.router.shape[0], moe.num_experts_per_tok

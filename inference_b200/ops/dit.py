@@ -120,7 +120,7 @@ def conv3x3_nhwc(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = N
     rc = kernels().swb_conv3x3_nhwc_stats(x.data_ptr(), N, H, W, C, w.data_ptr(), w.stride(0), Cout, out.data_ptr(), out.stride(0),
                                           ptr(bias), ptr(res2), res2.stride(0) if res2 is not None else 0, ACT[act], ptr(sums),
                                           sums.shape[1] if sums is not None else 0, stream_ptr())
-    check(rc, "swb_conv3x3_nhwc")
+    check(rc, "swb_conv3x3_nhwc_stats")
     return out.view(N, H, W, Cout)
 
 
