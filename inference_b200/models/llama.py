@@ -430,7 +430,7 @@ class LlamaGpu:
         pf = (lambda t: t if (pf_bytes >= 0 and isinstance(t, torch.Tensor)) else None)
         ssq = (self._ssq if self.quant_format is None else torch.empty((2, ops.SSQ_WORDS), dtype=torch.int64, device=self.device).unbind(0)) if chain else None
         packed = chain and self.quant_format is not None
-        normed = ops.linear_normed
+        normed = ops.linear_normed if packed else ops.gemm_bf16_normed
         prefill_splits = None
         ssq_prev = None                 # partial sums of squares of `res` (valid while branch is None)
         H = cfg.hidden_size
