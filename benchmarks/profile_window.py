@@ -10,6 +10,10 @@ with cudaProfilerStart/Stop so that `ncu --profile-from-start off` sees only tho
   --what attn_dense one dense non-causal attention launch (S=4608, 24 heads)
   --what conv     one implicit-GEMM 3x3 convolution, 512 x 512 x 256 -> 256 channels (134 MB in, 134 MB out)
   --what paged_prefill  one prefill-attention launch over paged K / V: 2048 new tokens on 8192 of context, 32 / 8 heads
+  --what split_prefill  the same for 700 new tokens on 5900, whose keys are split, and the sum of the parts
+  --what q4k_chain  one gate-up link of a chain of Q4_K products (T from --shape "Tx..", 28672 x 4096)
+  --what conv_sums  one implicit-GEMM convolution that adds up its output's group sums (832 x 1216 x 128 -> 128)
+  --what last_conv  group norm, SiLU and the last convolution of a decoder (832 x 1216 x 128 -> 8)
   --what vae      one FLUX-class VAE decode, 128 x 128 latents -> 1024 x 1024 (about 115 launches, 1.3 GB live)
 """
 import argparse
@@ -86,9 +90,34 @@ def main():
         w = (torch.randn(256, 9 * 256, device=dev, generator=g) / 48).bfloat16()
         b = torch.randn(256, device=dev, generator=g).bfloat16()
         window(lambda: ops.conv3x3_nhwc(x, w, b), reps=args.reps)
-    elif args.what == "paged_prefill":
-        Hq, Hkv, D, bs, q_len, ctx = 32, 8, 128, 16, 2048, 8192
-        per = (ctx + q_len) // bs
+    elif args.what == "q4k_chain":
+        from inference_b200.ops import quant
+
+        T, N, K = int(args.shape.split("x")[0]) if args.shape != "8192x4096x4096" else 4, 28672, 4096
+        a = torch.randn(T, K, device=dev, generator=g)
+        qw = quant.quantize_on_device((torch.randn(N, K, device=dev, generator=g) * 0.02).bfloat16(), "Q4_K")
+        ssq = ops.ssq_buffer(dev)
+        ssq[:T] = (a.double().pow(2).sum(1) * 2.0 ** 24).round().long()
+        flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
+
+        def fn():
+            flush.zero_()
+            ops.linear_normed(a, qw, act="swiglu_pairs", ssq_in=ssq, norm_dim=K, eps=1e-5)
+        window(fn, reps=args.reps)
+    elif args.what in ("conv_sums", "last_conv"):
+        x = torch.randn(1, 832, 1216, 128, device=dev, generator=g).bfloat16()
+        cout = 128 if args.what == "conv_sums" else 8
+        w = (torch.randn(cout, 9 * 128, device=dev, generator=g) / 34).bfloat16()
+        b, ga, be = (torch.randn(n, device=dev, generator=g).bfloat16() for n in (cout, 128, 128))
+        d = x.float().view(1, -1, 32, 4)
+        sums = torch.stack([d.sum((1, 3)), d.pow(2).sum((1, 3))], -1)
+        if args.what == "conv_sums":
+            window(lambda: ops.conv3x3_nhwc(x, w, b, sums=sums), reps=args.reps)
+        else:
+            window(lambda: ops.conv3x3_of_norm(x, sums, ga, be, 1e-6, w, b), reps=args.reps)
+    elif args.what in ("paged_prefill", "split_prefill"):
+        Hq, Hkv, D, bs, q_len, ctx = 32, 8, 128, 16, *((2048, 8192) if args.what == "paged_prefill" else (700, 5900))
+        per = (ctx + q_len + bs - 1) // bs
         kc = torch.randn(per + 4, Hkv, bs, D, device=dev, generator=g).bfloat16()
         vc = torch.randn(per + 4, Hkv, bs, D, device=dev, generator=g).bfloat16()
         table = torch.randperm(per, device=dev, generator=g).to(torch.int32).view(1, per).contiguous()
