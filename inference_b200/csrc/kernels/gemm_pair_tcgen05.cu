@@ -197,12 +197,14 @@ __device__ __forceinline__ void copy_async16(void* smem_dst, const void* src) {
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Where the columns of a tile go.
+// Where the columns of a tile go. TWO: there is a second output. (An instantiation of its own: chosen at run time for every product, the activation was looked up
+// for every element. 897 x 14336 x 1152 with bias and GELU took 107 us so, 93 before there were two outputs and 52.7 with this; 722 x 15360 x 5120 120, 108 and 90.)
+template <bool TWO>
 struct OutSel {
   void* out;
   int ldd, act, first;       // first accumulator column of this output
   __device__ __forceinline__ OutSel(const PairParams& p, int col0) {
-    const bool second = p.first_n > 0 && col0 >= p.first_n;
+    const bool second = TWO && col0 >= p.first_n;
     out = second ? p.out2 : p.out, ldd = second ? p.ldd2 : p.ldd, act = second ? p.act2 : p.act, first = second ? p.first_n : 0;
   }
 };
@@ -254,9 +256,9 @@ struct GroupSums {
 };
 
 // cols accumulator columns of this warp's 32 rows (thread = row) -> D. `load(c, v)` gives columns c .. c + 31.
-template <bool STATS, typename Load>
+template <bool STATS, bool TWO, typename Load>
 __device__ __forceinline__ void store_columns(int cols, const PairParams& p, const RowMap& rows, int col0, uint8_t* slab, int lane, GroupSums& sums, Load load) {
-  const OutSel to(p, col0);
+  const OutSel<TWO> to(p, col0);
   const bool pairs = gemm_act_pairs(p.act);
   const long long my_row = rows(lane);
   const int swz = lane & 7;
@@ -399,7 +401,7 @@ __device__ __forceinline__ void store_columns(int cols, const PairParams& p, con
   }
 }
 
-template <int BN, bool STATS>
+template <int BN, bool STATS, bool TWO>
 __global__ void __launch_bounds__(THREADS, 1) __cluster_dims__(2, 1, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const PairParams p) {
   using Cfg = PairCfg<BN>;
@@ -551,7 +553,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         sums.img = rows.box.img, sums.col0 = col0;
       }
       if (p.splits == 1) {
-        if (!idle) store_columns<STATS>(cols, p, rows, col0, slab, lane, sums, [&](int cc, float* v) { tmem_ld_32(taddr + cc, v); });
+        if (!idle) store_columns<STATS, TWO>(cols, p, rows, col0, slab, lane, sums, [&](int cc, float* v) { tmem_ld_32(taddr + cc, v); });
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive_even(smem_u32(&bar_tempty[acc]));
@@ -585,7 +587,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         if (last && !idle) {
           __threadfence();
           const float* ws = p.workspace + tile_slot * SLOT + mine;
-          store_columns<false>(cols, p, rows, col0, slab, lane, sums, [&](int cc, float* v) {
+          store_columns<false, TWO>(cols, p, rows, col0, slab, lane, sums, [&](int cc, float* v) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __ldcg(ws + (size_t)(cc + j) * BM);
             for (int s = 1; s < p.splits; ++s) {
@@ -616,9 +618,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   }
 }
 
-template <int BN, bool STATS>
+template <int BN, bool STATS, bool TWO>
 int launch_pair_as(const CUtensorMap& ta, const CUtensorMap& tb, const PairParams& p, int clusters, cudaStream_t stream) {
-  auto kern = gemm_pair_kernel<BN, STATS>;
+  auto kern = gemm_pair_kernel<BN, STATS, TWO>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -632,8 +634,14 @@ int launch_pair_as(const CUtensorMap& ta, const CUtensorMap& tb, const PairParam
 
 template <int BN>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const PairParams& p, int clusters, cudaStream_t stream) {
-  if constexpr (BN == 224) return p.stats ? -4 : launch_pair_as<BN, false>(ta, tb, p, clusters, stream);
-  else return p.stats ? launch_pair_as<BN, true>(ta, tb, p, clusters, stream) : launch_pair_as<BN, false>(ta, tb, p, clusters, stream);
+  // sums: tiles whose warps' columns do not differ; two outputs: widths that divide the first one's 64-column pieces, as the plan gives them
+  if constexpr (BN != 224) {
+    if (p.stats) return launch_pair_as<BN, true, false>(ta, tb, p, clusters, stream);
+  }
+  if constexpr (BN != 32) {
+    if (p.first_n > 0) return launch_pair_as<BN, false, true>(ta, tb, p, clusters, stream);
+  }
+  return p.stats || p.first_n > 0 ? -4 : launch_pair_as<BN, false, false>(ta, tb, p, clusters, stream);
 }
 
 // Estimated microseconds of a plan, without what gemm_pair_plan adds to the best one. Fitted to sweeps of every tile width and up to six splits over
