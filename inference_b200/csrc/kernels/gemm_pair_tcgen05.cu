@@ -177,6 +177,21 @@ __device__ __forceinline__ float pair_act(float x, const PairParams& p, int act)
     default: return x;
   }
 }
+// The same for 32 values: one choice for all of them. Looked up for every element it was half of the time of short products: 897 x 14336 x 1152 with bias and GELU 93 us
+// (107 with the output chosen at run time too) and 52.7 so, 722 x 15360 x 5120 108 and 90, two outputs of 9216 and 12288 columns of 3072 at 4608 rows 628 and 443.
+__device__ __forceinline__ void pair_act_all(float* v, const PairParams& p, int act) {
+  auto all = [&](auto f) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = f(v[j]);
+  };
+  switch (act) {
+    case SWB_ACT_SILU: all([](float x) { return silu_f(x); }); break;
+    case SWB_ACT_GELU_TANH: all([](float x) { return gelu_tanh_f(x); }); break;
+    case SWB_ACT_RELU2: all([](float x) { return relu2_f(x); }); break;
+    case SWB_ACT_XIELU: all([&](float x) { return xielu_f(x, p.act_a, p.act_b); }); break;
+    default: break;
+  }
+}
 __device__ __forceinline__ void add_bf16x8(float* v, const uint4 u) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
@@ -197,8 +212,7 @@ __device__ __forceinline__ void copy_async16(void* smem_dst, const void* src) {
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Where the columns of a tile go. TWO: there is a second output. (An instantiation of its own: chosen at run time for every product, the activation was looked up
-// for every element. 897 x 14336 x 1152 with bias and GELU took 107 us so, 93 before there were two outputs and 52.7 with this; 722 x 15360 x 5120 120, 108 and 90.)
+// Where the columns of a tile go. TWO: there is a second output, an instantiation of its own.
 template <bool TWO>
 struct OutSel {
   void* out;
@@ -343,10 +357,7 @@ __device__ __forceinline__ void store_columns(int cols, const PairParams& p, con
         *reinterpret_cast<uint4*>(my_slab + ((k ^ swz) << 4)) = pack8(o);
         *reinterpret_cast<uint4*>(my_slab + (((k + 1) ^ swz) << 4)) = pack8(o + 8);
       } else {
-        if (to.act != SWB_ACT_NONE) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = pair_act(v[j], p, to.act);
-        }
+        pair_act_all(v, p, to.act);
         const int k0 = (c - s) >> 3;
         if (gate) {
 #pragma unroll

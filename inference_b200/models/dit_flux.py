@@ -316,7 +316,7 @@ class FluxDiTGpu:
 
     def _linear1_of(self, x, i, qkv, mlp):
         """Both parts of a single block's linear1, as one product above the sizes at which each has a kernel of its own: 1231 rows are 420 tiles on 74 pairs of
-        SMs, six waves, and 180 + 240 of them seven."""
+        SMs, six waves, and 180 + 240 of them seven: 128 us and 144; 257 rows 58 and 70, 4608 rows 443 and 470."""
         p = f"single_blocks.{i}.linear1"
         W, b = self._linear1.get(i, (None, None))
         # (a program may put other tensors in place of the parts)
